@@ -503,251 +503,365 @@ __device__ void link_particle_fast(const DevParams& P, const SetView& vd, const 
         }
     }
 }
-// link_particle_fast with the candidate scan spread over a warp.  The warp walks the 27
-// cells in order; in each cell 32 candidates at a time are tested for d < h in parallel
-// and the passing ones are handled one after another in ascending index, by the same
-// sequential rule as link_particle_fast (the dup test ends the cell, own slots are kept in
-// registers, claims go through memory).  Every lane holds the same state; lane 0 writes.
-// Results are those of link_particle_fast.
-__device__ void link_particle_warp(const DevParams& P, const SetView& vd, const snowb_particle_data& d, uint32_t i,
-                                   int dynamic, DevState* S)
+// A particle's links by one warp.  The sequential rule of link_particle_fast, for up to 32
+// candidates in traversal order (lane k holds candidate k), resolved at once:
+//  - a candidate that o is already linked to ends its cell, so it and the later candidates
+//    of its cell drop out;
+//  - of the rest, those whose partner has room (count below the cap and a free slot) are
+//    linked in order, each into o's next free slot, until o's count reaches its cap or its
+//    slots run out; a partner without room changes nothing.
+// A link changes only o and its own partner, so the partners' counts and slots are all read
+// before the first link, eight slot rows in flight at a time, and the links are written side
+// by side: a chunk costs a few dependent memory round trips, where taking the candidates one
+// after another cost two for each.  A particle that meets itself or the same partner twice in
+// a chunk (stale cell ranges) takes the candidates one by one.
+struct LinkState {
+    uint32_t o, base, tol, count, rk, skip_cell;   // rk: lane k holds slot k of particle o
+};
+struct LinkMap {
+    uint32_t slot[32], partner[32];                // by rank of the link: o's slot, the partner
+};
+// false: nothing later can change anything (cap reached or no free slot)
+__device__ __forceinline__ bool link_chunk(const DevParams& P, const snowb_particle_data& d, DevState* S, uint32_t n,
+                                           LinkState& L, LinkMap& map, bool in, uint32_t o1, uint32_t cell, float dist)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t M = P.maxc;
-    const float3 p = vd.pos(i);
-    const uint32_t o = vd.gi[i];
-    const GCell g = grid_pos(P, p, vd.scene(i));
-    const uint32_t tol = link_tolerance(P, d.T[o], dynamic);
-    const uint32_t base = o * M;
-    uint32_t count = d.iter_end[o] - base;
-    // own slots: lane k holds slot k
-    uint32_t rk = lane < M ? d.connect_record[base + lane] : 0u;
-    FOR27 {
-        uint32_t s, e;
-        if (!vd.range(P, g, ox, oy, oz, s, e)) continue;
-        bool cell_done = false;
-        for (uint32_t j0 = s; j0 < e && !cell_done; j0 += 32u) {
-            const uint32_t j = j0 + lane;
-            float d2 = 0.f;
-            bool in = false;
-            if (j < e && j != i) {
-                const float3 dv = sub3(p, vd.pos(j));
-                d2 = dot3(dv, dv);
-                in = d2 < P.h2_lt;
-            }
-            uint32_t mask = __ballot_sync(0xffffffffu, in);
-            while (mask) {
-                const int k = __ffs(mask) - 1;
-                mask &= mask - 1u;
-                if (!(count < tol)) continue;
-                const uint32_t jj = j0 + (uint32_t)k;
-                const float dk2 = __shfl_sync(0xffffffffu, d2, k);
-                const uint32_t o1 = vd.gi[jj];
-                const float dist = sqrtf(dk2);
-                const bool dup = __any_sync(0xffffffffu, lane < M && rk == o1);
-                if (dup) { cell_done = true; break; }   // the reference returns from the cell helper
-                const uint32_t freem = __ballot_sync(0xffffffffu, lane < M && rk == SNOWB_UMAX);
-                if (!freem) continue;                      // no free slot: the claim loop finds nothing
-                const int free_k = __ffs(freem) - 1;
-                if (lane == 0) d.connect_record[base + free_k] = o1;   // claim
-                if (lane == (uint32_t)free_k) rk = o1;
-                __syncwarp();
-                const uint32_t b1 = o1 * M;
-                bool valid = false;
-                if (d.iter_end[o1] < b1 + M) {
-                    const uint32_t q = lane < M ? d.connect_record[b1 + lane] : 0u;
-                    const uint32_t pm = __ballot_sync(0xffffffffu, lane < M && q == SNOWB_UMAX);
-                    if (pm) {
-                        const int pk = __ffs(pm) - 1;
-                        if (lane == 0) {
-                            d.connect_record[b1 + pk] = o;
-                            d.connect_length[b1 + pk] = dist;
-                            d.iter_end[o1]++;
-                            if (o1 >= vd.n) atomicOr(&S->tail_dirty, 1u);
-                        }
-                        if (o1 == o) {                       // self link (stale cell range)
-                            ++count;
-                            if (lane == (uint32_t)pk) rk = o;
-                        }
-                        valid = true;
-                    }
-                }
-                if (valid) {
-                    ++count;
-                    if (lane == 0) {
-                        d.connect_length[base + free_k] = dist;
-                        d.iter_end[o] = base + count;
-                        atomicAdd(&S->n_links, 1u);
-                    }
-                } else {
-                    if (lane == 0) d.connect_record[base + free_k] = SNOWB_UMAX;
-                    if (lane == (uint32_t)free_k) rk = SNOWB_UMAX;
-                }
-                __syncwarp();
-            }
-        }
-    }
-}
-// link_particle_warp replaying the snow-snow candidate list written by the substep's first
-// density pass at the same sorted positions (entries in traversal order: cells z-y-x, index
-// ascending, all with d < h, tagged with their cell).  The sequential rule is the same; a
-// dup ends the entries of its cell.
-__device__ void link_particle_list(const DevParams& P, const SetView& vd, const snowb_particle_data& d, uint32_t i,
-                                   int dynamic, DevState* S, const NList& L, uint32_t n_list)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t M = P.maxc;
-    const float3 p = vd.pos(i);
-    const uint32_t o = vd.gi[i];
-    const uint32_t tol = link_tolerance(P, d.T[o], dynamic);
-    const uint32_t base = o * M;
-    const uint32_t slot = L.cap + i;
-    uint32_t count = d.iter_end[o] - base;
-    uint32_t rk = lane < M ? d.connect_record[base + lane] : 0u;
-    uint32_t skip_cell = 0xFFu;
-    for (uint32_t k0 = 0; k0 < n_list; k0 += 32u) {
-        const uint32_t k = k0 + lane;
-        uint32_t j = 0, cell = 0xFEu, og = 0;
-        float d2 = 0.f;
-        if (k < n_list) {
-            const uint32_t en = L.e[(size_t)k * L.stride + slot];
-            j = en & NL_J_MASK;
-            cell = (en >> 25) & 31u;
-            const float3 dv = sub3(p, vd.pos(j));
-            d2 = dot3(dv, dv);
-            // the partner's index, fetched side by side for the 32 candidates (it never
-            // changes in this pass), so the walk below needs no load for a duplicate
-            og = vd.gi[j];
-        }
-        // Candidates of a cell are contiguous and in order.  Once a cell is skipped (a
-        // duplicate ends it, as the reference returns from its cell helper), its remaining
-        // candidates leave the mask in one step; once the count reaches the cap, no later
-        // candidate can do anything (counts only grow), so the walk ends.
-        if (!(count < tol)) break;
-        uint32_t mask = __ballot_sync(0xffffffffu, k < n_list && cell != skip_cell);
-        while (mask) {
-            const int kk = __ffs(mask) - 1;
-            mask &= mask - 1u;
-            const uint32_t ck = __shfl_sync(0xffffffffu, cell, kk);
-            if (!(count < tol)) break;
-            const uint32_t o1 = __shfl_sync(0xffffffffu, og, kk);
-            const bool dup = __any_sync(0xffffffffu, lane < M && rk == o1);
-            if (dup) {
-                skip_cell = ck;
-                mask &= ~__ballot_sync(0xffffffffu, cell == ck);
+    const uint32_t lane = threadIdx.x & 31u, M = P.maxc, full = 0xffffffffu, below = (1u << lane) - 1u;
+    if (!(L.count < L.tol)) return false;
+    uint32_t freem = __ballot_sync(full, lane < M && L.rk == SNOWB_UMAX);
+    if (!freem) return false;
+    in = in && cell != L.skip_cell;
+    const uint32_t b1 = o1 * M;
+    const uint32_t ie = in ? d.iter_end[o1] : 0u;
+    bool dup = false;
+    for (uint32_t q = 0; q < M; ++q) dup |= __shfl_sync(full, L.rk, q) == o1;
+    const uint32_t dupm = __ballot_sync(full, in && dup);
+    const uint32_t same = __match_any_sync(full, in ? cell : 0x100u + lane);
+    const bool elig = in && !dup && !(same & dupm & below);
+    if (dupm) L.skip_cell = __shfl_sync(full, cell, 31 - __clz(dupm));
+    const uint32_t twin = __match_any_sync(full, elig ? o1 : 0x80000000u | lane);
+    if (__any_sync(full, elig && (o1 == L.o || (twin & (twin - 1u))))) {
+        uint32_t m = __ballot_sync(full, elig);
+        uint32_t dead = 0xFFu;   // a cell that a link made in this chunk ended
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1u;
+            if (!(L.count < L.tol)) return false;
+            const uint32_t p1 = __shfl_sync(full, o1, k), pc = __shfl_sync(full, cell, k);
+            const float pd = __shfl_sync(full, dist, k);
+            if (pc == dead) continue;
+            if (__any_sync(full, lane < M && L.rk == p1)) {
+                dead = pc;
+                if (!dupm || pc > L.skip_cell) L.skip_cell = pc;   // the last ended cell carries over
                 continue;
             }
-            const float dist = sqrtf(__shfl_sync(0xffffffffu, d2, kk));
-            const uint32_t freem = __ballot_sync(0xffffffffu, lane < M && rk == SNOWB_UMAX);
-            if (!freem) continue;
-            const int free_k = __ffs(freem) - 1;
-            if (lane == 0) d.connect_record[base + free_k] = o1;
-            if (lane == (uint32_t)free_k) rk = o1;
+            freem = __ballot_sync(full, lane < M && L.rk == SNOWB_UMAX);
+            if (!freem) return false;
+            const int fk = __ffs(freem) - 1;
+            if (lane == 0) d.connect_record[L.base + fk] = p1;   // claim
+            if (lane == (uint32_t)fk) L.rk = p1;
             __syncwarp();
-            const uint32_t b1 = o1 * M;
+            const uint32_t c1 = p1 * M;
             bool valid = false;
-            if (d.iter_end[o1] < b1 + M) {
-                const uint32_t q = lane < M ? d.connect_record[b1 + lane] : 0u;
-                const uint32_t pm = __ballot_sync(0xffffffffu, lane < M && q == SNOWB_UMAX);
+            if (d.iter_end[p1] < c1 + M) {
+                const uint32_t q = lane < M ? d.connect_record[c1 + lane] : 0u;
+                const uint32_t pm = __ballot_sync(full, lane < M && q == SNOWB_UMAX);
+                __syncwarp();
                 if (pm) {
                     const int pk = __ffs(pm) - 1;
                     if (lane == 0) {
-                        d.connect_record[b1 + pk] = o;
-                        d.connect_length[b1 + pk] = dist;
-                        d.iter_end[o1]++;
-                        if (o1 >= vd.n) atomicOr(&S->tail_dirty, 1u);
+                        d.connect_record[c1 + pk] = L.o;
+                        d.connect_length[c1 + pk] = pd;
+                        d.iter_end[p1]++;
+                        if (p1 >= n) atomicOr(&S->tail_dirty, 1u);
                     }
-                    if (o1 == o) {
-                        ++count;
-                        if (lane == (uint32_t)pk) rk = o;
+                    if (p1 == L.o) {                     // self link (stale cell range)
+                        ++L.count;
+                        if (lane == (uint32_t)pk) L.rk = L.o;
                     }
                     valid = true;
                 }
             }
+            __syncwarp();
             if (valid) {
-                ++count;
+                ++L.count;
                 if (lane == 0) {
-                    d.connect_length[base + free_k] = dist;
-                    d.iter_end[o] = base + count;
+                    d.connect_length[L.base + fk] = pd;
+                    d.iter_end[L.o] = L.base + L.count;
                     atomicAdd(&S->n_links, 1u);
                 }
             } else {
-                if (lane == 0) d.connect_record[base + free_k] = SNOWB_UMAX;
-                if (lane == (uint32_t)free_k) rk = SNOWB_UMAX;
+                if (lane == 0) d.connect_record[L.base + fk] = SNOWB_UMAX;
+                if (lane == (uint32_t)fk) L.rk = SNOWB_UMAX;
             }
             __syncwarp();
         }
+        return true;
     }
+    const uint32_t most = umin32(L.tol - L.count, (uint32_t)__popc(freem));
+    uint32_t need = __ballot_sync(full, elig && ie < b1 + M), okm = 0;
+    int pk = 0;   // this lane's candidate: the partner's first free slot
+    while (need && (uint32_t)__popc(okm) < most) {
+        int k[8];
+        uint32_t q[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            k[u] = need ? __ffs(need) - 1 : -1;
+            need &= need - 1u;
+            const uint32_t row = __shfl_sync(full, b1, k[u] < 0 ? 0 : k[u]);
+            q[u] = k[u] >= 0 && lane < M ? d.connect_record[row + lane] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t pm = __ballot_sync(full, q[u] == SNOWB_UMAX);
+            if (pm) okm |= 1u << k[u];
+            if (lane == (uint32_t)k[u]) pk = __ffs(pm) - 1;
+        }
+    }
+    // the r-th candidate with room takes the r-th free slot
+    const uint32_t made = umin32(most, (uint32_t)__popc(okm)), r = __popc(okm & below), fr = __popc(freem & below);
+    const bool link = (okm >> lane & 1u) && r < made, gets = (freem >> lane & 1u) && fr < made;
+    __syncwarp();
+    if (link) map.partner[r] = o1;
+    if (gets) map.slot[fr] = lane;
+    __syncwarp();
+    if (gets) L.rk = map.partner[fr];
+    if (link) {
+        const uint32_t fk = map.slot[r];
+        d.connect_record[L.base + fk] = o1;
+        d.connect_length[L.base + fk] = dist;
+        d.connect_record[b1 + pk] = L.o;
+        d.connect_length[b1 + pk] = dist;
+        d.iter_end[o1] = ie + 1u;
+        if (o1 >= n) atomicOr(&S->tail_dirty, 1u);
+    }
+    L.count += made;
+    if (made && lane == 0) {
+        d.iter_end[L.o] = L.base + L.count;
+        atomicAdd(&S->n_links, made);
+    }
+    __syncwarp();
+    return made < most;
 }
-// One colour with one warp per super-cell: the warp walks the super-cell's particles in
-// ascending sorted index and links the active ones with link_particle_warp.
+// The candidates of sorted particle i (d < h, traversal order) handed to use(in, j, cell, d2)
+// in chunks of a warp's width, by the 27-cell traversal: lane c < 27 loads cell c's range, the
+// ranges are walked end to end in cell order, 4 x 32 entries in flight, and those within the
+// support are packed in shared memory into full chunks.  use returns false to stop.
+struct LinkGather {
+    uint32_t e[64];                         // sorted index | cell << 25
+    float d2[64];
+    uint32_t first[27], begin[27];          // flattened position and sorted index of each cell's first member
+};
+template <class F>
+__device__ __forceinline__ void link_candidates(const DevParams& P, const SetView& vd, uint32_t i, LinkGather& W, F&& use)
+{
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu;
+    const float3 p = vd.pos(i);
+    const GCell g = grid_pos(P, p, vd.scene(i));
+    uint32_t s = 0, cnt = 0;
+    if (lane < 27u) {
+        uint32_t e;
+        if (vd.range(P, g, (int)(lane % 3u) - 1, (int)((lane / 3u) % 3u) - 1, (int)(lane / 9u) - 1, s, e))
+            cnt = e > s ? e - s : 0u;
+    }
+    const uint32_t incl = warp_incl_scan(cnt);
+    __syncwarp();
+    if (lane < 27u) { W.first[lane] = incl - cnt; W.begin[lane] = s; }
+    const uint32_t total = __shfl_sync(full, incl, 26);
+    __syncwarp();
+    uint32_t held = 0, cell = 0;
+    bool more = true;
+    for (uint32_t f0 = 0; f0 < total && more; f0 += 128u) {
+        uint32_t en[4];
+        float d2[4];
+        bool in[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t f = f0 + 32u * u + lane;
+            in[u] = f < total;
+            if (in[u]) {
+                // the last cell that starts at or before f (a lane's f grows)
+                while (cell < 26u && W.first[cell + 1u] <= f) ++cell;
+                const uint32_t j = W.begin[cell] + (f - W.first[cell]);
+                in[u] = j != i;
+                en[u] = j | cell << 25;
+                const float3 dv = sub3(p, vd.pos(j));
+                d2[u] = dot3(dv, dv);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool pass = more && in[u] && d2[u] < P.h2_lt;
+            const uint32_t m = __ballot_sync(full, pass);
+            if (pass) {
+                const uint32_t at = held + __popc(m & ((1u << lane) - 1u));
+                W.e[at] = en[u];
+                W.d2[at] = d2[u];
+            }
+            held += __popc(m);
+            __syncwarp();
+            if (held >= 32u) {
+                const uint32_t ce = W.e[lane], te = W.e[32u + lane];
+                const float cd = W.d2[lane], td = W.d2[32u + lane];
+                __syncwarp();
+                held -= 32u;
+                if (lane < held) { W.e[lane] = te; W.d2[lane] = td; }
+                __syncwarp();
+                more = use(true, ce & NL_J_MASK, ce >> 25, cd);
+            }
+        }
+    }
+    if (held && more) {
+        const bool in = lane < held;
+        const uint32_t ce = in ? W.e[lane] : 0u;
+        use(in, ce & NL_J_MASK, ce >> 25, in ? W.d2[lane] : 0.f);
+    }
+    __syncwarp();
+}
+// One colour: a block takes a super-cell.  Its active particles link one after another in
+// ascending sorted index, each by warp 0 (link_chunk); what a particle's links are chosen from
+// -- its candidates -- never changes in the pass, so the block's warps fetch the candidates of
+// LINK_BATCH active particles side by side into shared memory first (partner, cell, distance;
+// a particle with more than LINK_CAND candidates has them fetched by warp 0 in its turn).
+// The chain per particle is then its own slots, the partners' counts and slots, and the
+// writes.  README-scale set-up (every particle active, 64 to a super-cell): a colour takes
+// about 210 us, 934 us with one warp per super-cell taking candidates one at a time; 415 us with
+// link_chunk but the candidates fetched in the same warp's chain.
 // L: the snow-snow candidate lists of the substep's first density pass (L.cnt null: none);
 // they are valid while no phase change re-sorted the sets.
-__global__ void k_link_colour_warp(DevParams P, DevState* S, SetView vd, snowb_particle_data dem,
-                                   const uint32_t* __restrict__ fs, const uint32_t* __restrict__ fe,
-                                   const uint8_t* __restrict__ active, uint32_t colour, int dynamic, NList L,
-                                   SCList sc)
+constexpr uint32_t LINK_TPB = 256, LINK_BATCH = 32, LINK_CAND = 64;
+__global__ void __launch_bounds__(LINK_TPB) k_link_colour_warp(DevParams P, DevState* S, SetView vd,
+                                                               snowb_particle_data dem, const uint32_t* __restrict__ fs,
+                                                               const uint32_t* __restrict__ fe,
+                                                               const uint8_t* __restrict__ active, uint32_t colour,
+                                                               int dynamic, NList L, SCList sc)
 {
+    __shared__ uint32_t c_e[LINK_BATCH][LINK_CAND];     // partner | cell << 25
+    __shared__ float c_d[LINK_BATCH][LINK_CAND];        // distance
+    __shared__ uint32_t a_i[LINK_BATCH], a_o[LINK_BATCH], a_tol[LINK_BATCH], a_n[LINK_BATCH];
+    __shared__ LinkGather gather[LINK_TPB / 32];
+    __shared__ LinkMap map;
+    __shared__ uint32_t st[8], bs[8], s_total, s_next, s_held;
     vd.n = S->n_dem;
     const bool lists = L.cnt != nullptr && S->changed == 0;
-    const uint32_t qx = P.gsx >> 2, qy = P.gsy >> 2, qz = P.gsz >> 2;
+    const uint32_t qx = P.gsx >> 2, qy = P.gsy >> 2, qz = P.gsz >> 2, M = P.maxc, full = 0xffffffffu;
     // the listed super-cells of this colour, or all of them
     const uint32_t total = sc.flag ? sc.count[colour] : qx * qy * qz;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nwarps) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
         const uint32_t t = sc.flag ? sc.list[colour * sc.per + w] : w;
         const uint32_t sx = 2u * (t % qx) + (colour & 1u);
         const uint32_t sy = 2u * ((t / qx) % qy) + ((colour >> 1) & 1u);
         const uint32_t sz = 2u * (t / (qx * qy)) + ((colour >> 2) & 1u);
         // The 8 cells (dz, dy, dx) in hash order -- ascending sorted index -- with lane c
-        // loading cell c's range; the super-cell's particles are then taken 32 at a time in
-        // that order (cell by cell, ascending index), as the cell-by-cell loops would.
-        uint32_t cb = 0, cn = 0;
-        if (lane < 8u) {
-            const uint32_t dz = lane >> 2, dy = (lane >> 1) & 1u, dx = lane & 1u;
-            const uint32_t h = ((2u * sz + dz) * P.gsy + (2u * sy + dy)) * P.gsx + (2u * sx + dx);
-            cb = fs[h];
-            cn = fe[h] - cb;
-        }
-        uint32_t incl = cn;
-#pragma unroll
-        for (uint32_t o = 1; o < 8u; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        uint32_t st[8], bs[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            st[q] = __shfl_sync(0xffffffffu, incl - cn, q);   // first flattened position of cell q
-            bs[q] = __shfl_sync(0xffffffffu, cb, q);
-        }
-        const uint32_t total_p = __shfl_sync(0xffffffffu, incl, 7);
-        for (uint32_t f0 = 0; f0 < total_p; f0 += 32u) {
-            const uint32_t f = f0 + lane;
-            uint32_t i = 0;
-            bool act = false;
-            if (f < total_p) {
-                // the last cell starting at or before f holds it (empty cells start where the
-                // next one does)
-                uint32_t s0 = st[0], b0 = bs[0];
-#pragma unroll
-                for (int r = 1; r < 8; ++r)
-                    if (st[r] <= f) { s0 = st[r]; b0 = bs[r]; }
-                i = b0 + (f - s0);
-                act = active[i] != 0;
+        // loading cell c's range; the super-cell's particles are then taken in that order
+        // (cell by cell, ascending index), as the cell-by-cell loops would.
+        if (warp == 0) {
+            uint32_t cb = 0, cn = 0;
+            if (lane < 8u) {
+                const uint32_t dz = lane >> 2, dy = (lane >> 1) & 1u, dx = lane & 1u;
+                const uint32_t h = ((2u * sz + dz) * P.gsy + (2u * sy + dy)) * P.gsx + (2u * sx + dx);
+                cb = fs[h];
+                cn = fe[h] - cb;
             }
-            uint32_t am = __ballot_sync(0xffffffffu, act);
-            while (am) {
-                const int k = __ffs(am) - 1;
-                am &= am - 1u;
-                const uint32_t ii = __shfl_sync(0xffffffffu, i, k);
-                const uint32_t lc = lists ? L.cnt[L.cap + ii] : NL_OVF;
-                if (lc & NL_OVF) link_particle_warp(P, vd, dem, ii, dynamic, S);
-                else link_particle_list(P, vd, dem, ii, dynamic, S, L, lc & 1023u);
-            }
+            const uint32_t incl = warp_incl_scan(cn);
+            if (lane < 8u) { st[lane] = incl - cn; bs[lane] = cb; }   // first flattened position of each cell
+            if (lane == 7u) s_total = incl;
+            if (lane == 0u) s_next = 0u;
         }
-        if (sc.flag && lane == 0) sc.flag[colour * sc.per + t] = 0u;   // ready for the next pass
+        __syncthreads();
+        const uint32_t total_p = s_total;
+        for (;;) {
+            // warp 0: the next LINK_BATCH active particles
+            if (warp == 0) {
+                uint32_t held = 0, f0 = s_next;
+                while (held < LINK_BATCH && f0 < total_p) {
+                    const uint32_t f = f0 + lane;
+                    uint32_t i = 0;
+                    bool act = false;
+                    if (f < total_p) {
+                        // the last cell starting at or before f holds it (empty cells start
+                        // where the next one does)
+                        uint32_t c = 0;
+#pragma unroll
+                        for (uint32_t r = 1; r < 8u; ++r)
+                            if (st[r] <= f) c = r;
+                        i = bs[c] + (f - st[c]);
+                        act = active[i] != 0;
+                    }
+                    const uint32_t am = __ballot_sync(full, act);
+                    const uint32_t at = held + __popc(am & ((1u << lane) - 1u));
+                    if (act && at < LINK_BATCH) a_i[at] = i;
+                    const uint32_t over = __ballot_sync(full, act && at >= LINK_BATCH);
+                    held = umin32(held + __popc(am), LINK_BATCH);
+                    f0 += over ? (uint32_t)__ffs(over) - 1u : 32u;   // the first left out opens the next batch
+                }
+                if (lane == 0u) { s_next = f0; s_held = held; }
+            }
+            __syncthreads();
+            const uint32_t held = s_held;
+            if (held == 0u) break;
+            for (uint32_t a = warp; a < held; a += nwarps) {
+                const uint32_t i = a_i[a];
+                const uint32_t o = vd.gi[i];
+                if (lane == 0u) { a_o[a] = o; a_tol[a] = link_tolerance(P, dem.T[o], dynamic); }
+                const uint32_t lc = lists ? L.cnt[L.cap + i] : NL_OVF;
+                uint32_t got = 0;
+                if (!(lc & NL_OVF)) {
+                    const float3 p = vd.pos(i);
+                    got = lc & 1023u;
+                    for (uint32_t k = lane; k < got && got <= LINK_CAND; k += 32u) {
+                        const uint32_t en = L.e[(size_t)k * L.stride + L.cap + i];
+                        c_e[a][k] = vd.gi[en & NL_J_MASK] | (en & (31u << 25));
+                        c_d[a][k] = len3(sub3(p, vd.pos(en & NL_J_MASK)));
+                    }
+                } else {
+                    link_candidates(P, vd, i, gather[warp], [&](bool in, uint32_t j, uint32_t cell, float d2) {
+                        const uint32_t k = got + lane;
+                        if (in && k < LINK_CAND) {
+                            c_e[a][k] = vd.gi[j] | cell << 25;
+                            c_d[a][k] = sqrtf(d2);
+                        }
+                        got += __popc(__ballot_sync(full, in));
+                        return got <= LINK_CAND;
+                    });
+                }
+                if (lane == 0u) a_n[a] = got;
+            }
+            __syncthreads();
+            if (warp == 0)
+                for (uint32_t a = 0; a < held; ++a) {
+                    const uint32_t o = a_o[a], got = a_n[a];
+                    LinkState l{o, o * M, a_tol[a], dem.iter_end[o] - o * M,
+                                lane < M ? dem.connect_record[o * M + lane] : 0u, 0xFFu};
+                    if (got <= LINK_CAND) {
+                        bool more = true;
+                        for (uint32_t k0 = 0; k0 < got && more; k0 += 32u) {
+                            const uint32_t k = k0 + lane;
+                            const bool in = k < got;
+                            const uint32_t en = in ? c_e[a][k] : 0u;
+                            more = link_chunk(P, dem, S, vd.n, l, map, in, en & NL_J_MASK, en >> 25, in ? c_d[a][k] : 0.f);
+                        }
+                    } else if (lists && !(L.cnt[L.cap + a_i[a]] & NL_OVF)) {
+                        const uint32_t i = a_i[a];
+                        const float3 p = vd.pos(i);
+                        bool more = true;
+                        for (uint32_t k0 = 0; k0 < got && more; k0 += 32u) {
+                            const uint32_t k = k0 + lane;
+                            const bool in = k < got;
+                            const uint32_t en = in ? L.e[(size_t)k * L.stride + L.cap + i] : 0u, j = en & NL_J_MASK;
+                            more = link_chunk(P, dem, S, vd.n, l, map, in, in ? vd.gi[j] : 0u, (en >> 25) & 31u,
+                                              in ? len3(sub3(p, vd.pos(j))) : 0.f);
+                        }
+                    } else {
+                        link_candidates(P, vd, a_i[a], gather[0], [&](bool in, uint32_t j, uint32_t cell, float d2) {
+                            return link_chunk(P, dem, S, vd.n, l, map, in, in ? vd.gi[j] : 0u, cell, sqrtf(d2));
+                        });
+                    }
+                }
+            __syncthreads();
+        }
+        if (sc.flag && threadIdx.x == 0) sc.flag[colour * sc.per + t] = 0u;   // ready for the next pass
+        __syncthreads();
     }
 }
 // general maximum_connection: the plain restatement with every access in memory

@@ -319,6 +319,8 @@ static SCList sc_lists(const DevParams& P)
     if (P.maxc > SNOWB_MAXC_FAST) return SCList{nullptr, nullptr, nullptr, 0u};
     return SCList{g_ctx.sc_flag, g_ctx.sc_list, g_ctx.S->sc_count, P.ncells / 64u};
 }
+// blocks of a link colour pass: one per super-cell, at most the three that fit an SM at a time
+static uint32_t link_blocks(uint32_t nsc) { return umin32(nsc, 3u * (uint32_t)g_sms); }
 static int ensure_gen(uint32_t n, uint32_t ncells)
 {
     Ctx& c = g_ctx;
@@ -809,7 +811,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
             const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);   // super-cells per colour
             for (uint32_t col = 0; col < 8; ++col) {
                 if (P.maxc <= SNOWB_MAXC_FAST)
-                    TLAUNCH(k_link_colour_warp, 256, (uint64_t)nsc * 32, 128, P, S, v, *a.dem, off, off + 1, c.active,
+                    TLAUNCH(k_link_colour_warp, LINK_TPB, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, S, v, *a.dem, off, off + 1, c.active,
                             col, a.dynamic, NL2, scl);
                 else
                     TLAUNCH(k_link_colour, 128, nsc, 64, P, S, v, *a.dem, off, off + 1, c.active, col, a.dynamic);
@@ -1518,7 +1520,7 @@ static int connect_links(const DevParams& P, snowb_particle_data* dem, uint32_t 
     const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);
     for (uint32_t col = 0; col < 8; ++col) {
         if (P.maxc <= SNOWB_MAXC_FAST)
-            LAUNCH(k_link_colour_warp, (uint64_t)nsc * 32, 128, P, c.S, vd, *dem, c.fs, c.fe, c.active, col, dynamic,
+            LAUNCH(k_link_colour_warp, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, c.S, vd, *dem, c.fs, c.fe, c.active, col, dynamic,
                    NList{nullptr, nullptr, 0u, 0u}, scl);
         else
             LAUNCH(k_link_colour, nsc, 64, P, c.S, vd, *dem, c.fs, c.fe, c.active, col, dynamic);
