@@ -516,8 +516,25 @@ __device__ void link_particle_fast(const DevParams& P, const SetView& vd, const 
 // after another cost two for each.  A particle that meets itself or the same partner twice in
 // a chunk (stale cell ranges) takes the candidates one by one.
 struct LinkState {
-    uint32_t o, base, tol, count, rk, skip_cell;   // rk: lane k holds slot k of particle o
+    uint32_t o, base, tol, count, skip_cell;
+    uint32_t rk;   // lane k < M holds slot k of particle o, the others LINK_NO_SLOT
 };
+constexpr uint32_t LINK_NO_SLOT = SNOWB_UMAX - 1u;   // no particle index and not an empty slot
+// which lanes' candidates (o1, of a cell) o is already linked to or meets after such a one in
+// its cell; carries the last ended cell over
+__device__ __forceinline__ bool link_ended(uint32_t rk, uint32_t& skip_cell, bool in, uint32_t o1, uint32_t cell,
+                                           uint32_t& dupm)
+{
+    const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
+    in = in && cell != skip_cell;
+    bool dup = false;
+#pragma unroll
+    for (int q = 0; q < SNOWB_MAXC_FAST; ++q) dup |= __shfl_sync(full, rk, q) == o1;
+    dupm = __ballot_sync(full, in && dup);
+    const uint32_t same = __match_any_sync(full, in ? cell : 0x100u + lane);
+    if (dupm) skip_cell = __shfl_sync(full, cell, 31 - __clz(dupm));
+    return !in || dup || (same & dupm & ((1u << lane) - 1u)) != 0u;
+}
 struct LinkMap {
     uint32_t slot[32], partner[32];                // by rank of the link: o's slot, the partner
 };
@@ -527,17 +544,12 @@ __device__ __forceinline__ bool link_chunk(const DevParams& P, const snowb_parti
 {
     const uint32_t lane = threadIdx.x & 31u, M = P.maxc, full = 0xffffffffu, below = (1u << lane) - 1u;
     if (!(L.count < L.tol)) return false;
-    uint32_t freem = __ballot_sync(full, lane < M && L.rk == SNOWB_UMAX);
+    uint32_t freem = __ballot_sync(full, L.rk == SNOWB_UMAX);
     if (!freem) return false;
-    in = in && cell != L.skip_cell;
     const uint32_t b1 = o1 * M;
     const uint32_t ie = in ? d.iter_end[o1] : 0u;
-    bool dup = false;
-    for (uint32_t q = 0; q < M; ++q) dup |= __shfl_sync(full, L.rk, q) == o1;
-    const uint32_t dupm = __ballot_sync(full, in && dup);
-    const uint32_t same = __match_any_sync(full, in ? cell : 0x100u + lane);
-    const bool elig = in && !dup && !(same & dupm & below);
-    if (dupm) L.skip_cell = __shfl_sync(full, cell, 31 - __clz(dupm));
+    uint32_t dupm;
+    const bool elig = !link_ended(L.rk, L.skip_cell, in, o1, cell, dupm);   // every lane takes part
     const uint32_t twin = __match_any_sync(full, elig ? o1 : 0x80000000u | lane);
     if (__any_sync(full, elig && (o1 == L.o || (twin & (twin - 1u))))) {
         uint32_t m = __ballot_sync(full, elig);
@@ -549,12 +561,12 @@ __device__ __forceinline__ bool link_chunk(const DevParams& P, const snowb_parti
             const uint32_t p1 = __shfl_sync(full, o1, k), pc = __shfl_sync(full, cell, k);
             const float pd = __shfl_sync(full, dist, k);
             if (pc == dead) continue;
-            if (__any_sync(full, lane < M && L.rk == p1)) {
+            if (__any_sync(full, L.rk == p1)) {
                 dead = pc;
                 if (!dupm || pc > L.skip_cell) L.skip_cell = pc;   // the last ended cell carries over
                 continue;
             }
-            freem = __ballot_sync(full, lane < M && L.rk == SNOWB_UMAX);
+            freem = __ballot_sync(full, L.rk == SNOWB_UMAX);
             if (!freem) return false;
             const int fk = __ffs(freem) - 1;
             if (lane == 0) d.connect_record[L.base + fk] = p1;   // claim
@@ -720,12 +732,15 @@ __device__ __forceinline__ void link_candidates(const DevParams& P, const SetVie
 // One colour: a block takes a super-cell.  Its active particles link one after another in
 // ascending sorted index, each by warp 0 (link_chunk); what a particle's links are chosen from
 // -- its candidates -- never changes in the pass, so the block's warps fetch the candidates of
-// LINK_BATCH active particles side by side into shared memory first (partner, cell, distance;
-// a particle with more than LINK_CAND candidates has them fetched by warp 0 in its turn).
-// The chain per particle is then its own slots, the partners' counts and slots, and the
-// writes.  README-scale set-up (every particle active, 64 to a super-cell): a colour takes
-// about 210 us, 934 us with one warp per super-cell taking candidates one at a time; 415 us with
-// link_chunk but the candidates fetched in the same warp's chain.
+// LINK_BATCH active particles side by side into shared memory first.  They also leave out what
+// can no longer link when the batch begins: links are only added and counts only grow in the
+// pass, so a candidate that is linked already (with the rest of its cell) or whose count has
+// reached the cap stays without effect.  A particle left without candidates costs nothing in
+// the chain; the others' own slots, the partners' counts and slots and the writes remain.  (A
+// particle with more than LINK_CAND of them has all candidates fetched in its turn.)
+// README-scale set-up (every particle active, 64 to a super-cell): a colour takes about 180 us,
+// 934 us with one warp per super-cell taking candidates one at a time; 415 us with link_chunk
+// but the candidates fetched in the same warp's chain.
 // L: the snow-snow candidate lists of the substep's first density pass (L.cnt null: none);
 // they are valid while no phase change re-sorted the sets.
 constexpr uint32_t LINK_TPB = 256, LINK_BATCH = 32, LINK_CAND = 64;
@@ -802,37 +817,46 @@ __global__ void __launch_bounds__(LINK_TPB) k_link_colour_warp(DevParams P, DevS
             if (held == 0u) break;
             for (uint32_t a = warp; a < held; a += nwarps) {
                 const uint32_t i = a_i[a];
-                const uint32_t o = vd.gi[i];
-                if (lane == 0u) { a_o[a] = o; a_tol[a] = link_tolerance(P, dem.T[o], dynamic); }
+                const uint32_t o = vd.gi[i], tol = link_tolerance(P, dem.T[o], dynamic);
+                const uint32_t rk = lane < M ? dem.connect_record[o * M + lane] : LINK_NO_SLOT;
                 const uint32_t lc = lists ? L.cnt[L.cap + i] : NL_OVF;
-                uint32_t got = 0;
-                if (!(lc & NL_OVF)) {
+                uint32_t got = 0, skip_cell = 0xFFu;
+                auto keep = [&](bool in, uint32_t o1, uint32_t cell, float dist) {
+                    const bool room = in && dem.iter_end[o1] < (o1 + 1u) * M;
+                    uint32_t dupm;
+                    in = !link_ended(rk, skip_cell, in, o1, cell, dupm) && room;
+                    const uint32_t m = __ballot_sync(full, in), k = got + __popc(m & ((1u << lane) - 1u));
+                    if (in && k < LINK_CAND) { c_e[a][k] = o1 | cell << 25; c_d[a][k] = dist; }
+                    got += __popc(m);
+                    return got <= LINK_CAND;
+                };
+                const uint32_t end = dem.iter_end[o];
+                if ((end >= o * M && end - o * M >= tol) || !__any_sync(full, rk == SNOWB_UMAX)) {
+                    // at its cap (a count below zero, which dynamic caps can leave, may rise
+                    // past zero in this pass) or out of slots
+                } else if (!(lc & NL_OVF)) {
                     const float3 p = vd.pos(i);
-                    got = lc & 1023u;
-                    for (uint32_t k = lane; k < got && got <= LINK_CAND; k += 32u) {
-                        const uint32_t en = L.e[(size_t)k * L.stride + L.cap + i];
-                        c_e[a][k] = vd.gi[en & NL_J_MASK] | (en & (31u << 25));
-                        c_d[a][k] = len3(sub3(p, vd.pos(en & NL_J_MASK)));
+                    const uint32_t nl = lc & 1023u;
+                    bool more = true;
+                    for (uint32_t k0 = 0; k0 < nl && more; k0 += 32u) {
+                        const bool in = k0 + lane < nl;
+                        const uint32_t en = in ? L.e[(size_t)(k0 + lane) * L.stride + L.cap + i] : 0u, j = en & NL_J_MASK;
+                        more = keep(in, in ? vd.gi[j] : 0u, (en >> 25) & 31u, in ? len3(sub3(p, vd.pos(j))) : 0.f);
                     }
                 } else {
                     link_candidates(P, vd, i, gather[warp], [&](bool in, uint32_t j, uint32_t cell, float d2) {
-                        const uint32_t k = got + lane;
-                        if (in && k < LINK_CAND) {
-                            c_e[a][k] = vd.gi[j] | cell << 25;
-                            c_d[a][k] = sqrtf(d2);
-                        }
-                        got += __popc(__ballot_sync(full, in));
-                        return got <= LINK_CAND;
+                        return keep(in, in ? vd.gi[j] : 0u, cell, sqrtf(d2));
                     });
                 }
-                if (lane == 0u) a_n[a] = got;
+                if (lane == 0u) { a_o[a] = o; a_tol[a] = tol; a_n[a] = got; }
             }
             __syncthreads();
             if (warp == 0)
                 for (uint32_t a = 0; a < held; ++a) {
                     const uint32_t o = a_o[a], got = a_n[a];
-                    LinkState l{o, o * M, a_tol[a], dem.iter_end[o] - o * M,
-                                lane < M ? dem.connect_record[o * M + lane] : 0u, 0xFFu};
+                    if (got == 0u) continue;
+                    LinkState l{o, o * M, a_tol[a], dem.iter_end[o] - o * M, 0xFFu,
+                                lane < M ? dem.connect_record[o * M + lane] : LINK_NO_SLOT};
                     if (got <= LINK_CAND) {
                         bool more = true;
                         for (uint32_t k0 = 0; k0 < got && more; k0 += 32u) {
@@ -844,10 +868,11 @@ __global__ void __launch_bounds__(LINK_TPB) k_link_colour_warp(DevParams P, DevS
                     } else if (lists && !(L.cnt[L.cap + a_i[a]] & NL_OVF)) {
                         const uint32_t i = a_i[a];
                         const float3 p = vd.pos(i);
+                        const uint32_t nl = L.cnt[L.cap + i] & 1023u;
                         bool more = true;
-                        for (uint32_t k0 = 0; k0 < got && more; k0 += 32u) {
+                        for (uint32_t k0 = 0; k0 < nl && more; k0 += 32u) {
                             const uint32_t k = k0 + lane;
-                            const bool in = k < got;
+                            const bool in = k < nl;
                             const uint32_t en = in ? L.e[(size_t)k * L.stride + L.cap + i] : 0u, j = en & NL_J_MASK;
                             more = link_chunk(P, dem, S, vd.n, l, map, in, in ? vd.gi[j] : 0u, (en >> 25) & 31u,
                                               in ? len3(sub3(p, vd.pos(j))) : 0.f);
