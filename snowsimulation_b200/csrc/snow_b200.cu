@@ -136,6 +136,7 @@ struct SetBufs {
     float4* p4 = nullptr;
     float *invm = nullptr, *contrib = nullptr, *lambda = nullptr, *mass = nullptr;
     uint32_t* sid = nullptr;   // scene id per sorted particle (batched runs)
+    BndBase base{nullptr, nullptr};   // boundary only
 };
 
 struct Ctx {
@@ -184,7 +185,7 @@ static uint64_t g_ctx_gen = 0;   // bumped whenever the scratch buffers are (re)
 static void free_set(SetBufs& s)
 {
     void* ptrs[] = {s.key, s.slot, s.tmp, s.cnt, s.off, s.bsum, s.val, s.p4, s.invm, s.contrib, s.lambda, s.mass,
-                    s.sid};
+                    s.sid, s.base.rho, s.base.gs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     s = SetBufs();
@@ -251,6 +252,7 @@ static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
     for (auto& s : c.s) TRY(alloc_sort(s, c.cap, ncells, true));
     TRY(dalloc(&c.b.p4, c.bcap)); TRY(dalloc(&c.b.invm, c.bcap)); TRY(dalloc(&c.b.mass, c.bcap));
     TRY(dalloc(&c.b.lambda, c.bcap)); TRY(dalloc(&c.b.sid, c.bcap));
+    TRY(dalloc(&c.b.base.rho, c.bcap)); TRY(dalloc(&c.b.base.gs, c.bcap));
     TRY(dalloc(&c.fl_s, c.cap)); TRY(dalloc(&c.fl_d, c.cap)); TRY(dalloc(&c.rk_s, c.cap)); TRY(dalloc(&c.rk_d, c.cap));
     TRY(dalloc(&c.sbsum, 4 * (c.cap / SCAN_CHUNK + 2)));
     TRY(dalloc(&c.active, c.cap));
@@ -391,9 +393,10 @@ static inline unsigned blocks_for(uint64_t work, int tpb)
     if (b > (uint64_t)g_max_blocks) b = g_max_blocks;
     return (unsigned)b;
 }
-#define KL(kernel, grid, tpb, ...)                                                         \
+#define KL(kernel, grid, tpb, ...) KL_AS(#kernel, kernel, grid, tpb, __VA_ARGS__)
+#define KL_AS(name, kernel, grid, tpb, ...)                                                \
     do {                                                                                   \
-        prof_begin(#kernel);                                                               \
+        prof_begin(name);                                                                  \
         kernel<<<(grid), (tpb), 0, g_stream>>>(__VA_ARGS__);                               \
         prof_end();                                                                        \
         cudaError_t _e = cudaGetLastError();                                               \
@@ -450,6 +453,14 @@ static void tune_pick(const char* name, uint64_t work, int tpb0, int max_tpb, in
         unsigned _grid;                                                                      \
         tune_pick(#kernel, (work), (tpb0), (max_tpb), _tpb, _grid);                          \
         KL(kernel, _grid, _tpb, __VA_ARGS__);                                                \
+    } while (0)
+// a pass with several forms is profiled and tuned under the pass's name, whichever form runs
+#define TLAUNCH_AS(name, kernel, max_tpb, work, tpb0, ...)                                   \
+    do {                                                                                     \
+        int _tpb;                                                                            \
+        unsigned _grid;                                                                      \
+        tune_pick(name, (work), (tpb0), (max_tpb), _tpb, _grid);                             \
+        KL_AS(name, kernel, _grid, _tpb, __VA_ARGS__);                                       \
     } while (0)
 // tunable only when `tunable` holds (else the built-in shape)
 #define TLAUNCH_IF(tunable, kernel, max_tpb, work, tpb0, ...)                                \
@@ -516,6 +527,8 @@ struct StepArgs {
     const uint32_t *sid_sph, *sid_dem, *sid_bnd;   // batched runs: scene id per slot (else null)
     uint32_t* sid_buf;
     int xsph_thread[2];   // XSPH of the water / snow set in the one-thread form (sizes at the call)
+    uint32_t particles;   // water + snow at the call (phase changes keep the sum)
+    int small;            // the neighbour passes in their one-warp forms (particles at the call)
 };
 
 
@@ -743,7 +756,14 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // iterations' density+lambda passes before anything reads them, so a whole substep with
     // iterations leaves the boundary out here.
     const int bnd_first = !(beside && a.iterations > 0);
-    TLAUNCH(k_density<false>, 256, bnd_first ? work3 : 2 * full, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL2, bnd_first);
+    // warps of the one-warp density form: a particle each, 32 boundary particles each
+    const uint64_t dwork = 32ull * (a.particles + (a.nb + 31u) / 32u);
+    if (a.small)
+        TLAUNCH_AS("k_density<false>", k_density_warp<false>, 256, bnd_first ? dwork : 32ull * a.particles, 128, P, S, vs,
+                   vd, vb, X, ss, sd, sb, NL2, bnd_first, c.b.base);
+    else
+        TLAUNCH(k_density<false>, 256, bnd_first ? work3 : 2 * full, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL2,
+                bnd_first, c.b.base);
     STOP(2);
     // in a whole substep the phase flags pass commits the new temperatures itself
     const int commit_in_flags = beside && a.temperature && a.change_phase;
@@ -811,8 +831,8 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
             const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);   // super-cells per colour
             for (uint32_t col = 0; col < 8; ++col) {
                 if (P.maxc <= SNOWB_MAXC_FAST)
-                    TLAUNCH(k_link_colour_warp, LINK_TPB, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, S, v, *a.dem, off, off + 1, c.active,
-                            col, a.dynamic, NL2, scl);
+                    TLAUNCH(k_link_colour_warp, LINK_TPB, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, S, v, *a.dem,
+                            off, off + 1, c.active, col, a.dynamic, NL2, scl);
                 else
                     TLAUNCH(k_link_colour, 128, nsc, 64, P, S, v, *a.dem, off, off + 1, c.active, col, a.dynamic);
             }
@@ -868,7 +888,11 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         const bool links_beside = beside && a.interlink;
         if (links_beside) TRY(on_side(c.side, c.fork, link_terms));
         // density + lambda in one pass (stage boundaries base+1 and base+2 coincide)
-        TLAUNCH(k_density<true>, 256, work3, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1);
+        if (a.small)
+            TLAUNCH_AS("k_density<true>", k_density_warp<true>, 256, dwork, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1,
+                       c.b.base);
+        else
+            TLAUNCH(k_density<true>, 256, work3, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1, c.b.base);
         STOP(base + 2);
         // with the interlink pass beside, the passes that finish a correction apply it (no
         // k_apply launch): the water PBF passes for the water, k_link_apply for the snow
@@ -1403,7 +1427,8 @@ static int run_steps(snowb_particle_data* sph, uint32_t* sph_size, snowb_particl
                fl[0], fl[1], fl[2], fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10], dTe, opt.stop_after,
                batch ? batch->scene_sph : nullptr, batch ? batch->scene_dem : nullptr,
                batch ? batch->scene_boundary : nullptr, batch ? batch->scene_buffer : nullptr,
-               {xs_s > XSPH_WARP_MAX ? 1 : 0, xs_d > XSPH_WARP_MAX ? 1 : 0}};
+               {xs_s > XSPH_WARP_MAX ? 1 : 0, xs_d > XSPH_WARP_MAX ? 1 : 0}, *sph_size + *dem_size,
+               *sph_size + *dem_size <= DENSITY_WARP_MAX ? 1 : 0};
     LAUNCH1(k_set_state, c.S, *sph_size, *dem_size, nb);
     if (batch)
         LAUNCH(k_check_scenes, full > nb ? full : nb, 256, P, c.S, a.sid_sph, a.sid_dem, a.sid_bnd);
@@ -1520,8 +1545,8 @@ static int connect_links(const DevParams& P, snowb_particle_data* dem, uint32_t 
     const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);
     for (uint32_t col = 0; col < 8; ++col) {
         if (P.maxc <= SNOWB_MAXC_FAST)
-            LAUNCH(k_link_colour_warp, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, c.S, vd, *dem, c.fs, c.fe, c.active, col, dynamic,
-                   NList{nullptr, nullptr, 0u, 0u}, scl);
+            LAUNCH(k_link_colour_warp, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, c.S, vd, *dem, c.fs, c.fe,
+                   c.active, col, dynamic, NList{nullptr, nullptr, 0u, 0u}, scl);
         else
             LAUNCH(k_link_colour, nsc, 64, P, c.S, vd, *dem, c.fs, c.fe, c.active, col, dynamic);
     }

@@ -374,16 +374,76 @@ __device__ __forceinline__ void acc_WG(const DevParams& P, float& rho, float& gs
         if (LAMBDA) gs += cg;
     }
 }
+// Sums over the boundary set of every boundary particle (own term included): the opening
+// terms of its density and lambda sums, the same in every pass of a call since the boundary
+// does not move.  The call's first pass over the boundary forms them, the later ones read them
+// (by sorted index; DevState::base_ready).
+struct BndBase {
+    float *rho, *gs;
+};
+// which of the water (bit 0) and snow (bit 1) sets have an entry, stale ones included, in the
+// 27 cells around g; the loads are independent
+__device__ __forceinline__ uint32_t occupied27(const DevParams& P, GCell g, const SetView& vs, const SetView& vd)
+{
+    uint32_t w = 0, s = 0;
+#pragma unroll
+    for (int oz = -1; oz <= 1; ++oz)
+#pragma unroll
+        for (int oy = -1; oy <= 1; ++oy)
+#pragma unroll
+            for (int ox = -1; ox <= 1; ++ox) {
+                const uint32_t h = grid_hash(P, g, ox, oy, oz);
+                w |= ~__ldg(vs.cs + h);     // SNOWB_EMPTY is all ones
+                s |= ~__ldg(vd.cs + h);
+            }
+    return (w ? 1u : 0u) | (s ? 2u : 0u);
+}
+// The 27 cell ranges are loaded first (independent loads), then the occupied cells walked: one
+// layer of boundary particles fills about 9 of them.
+__device__ __forceinline__ void boundary_base(const DevParams& P, const SetView& vb, const Sets& X, const Sorted& sb,
+                                              uint32_t i, uint32_t o, float3 p, GCell g, bool ready, const BndBase& base,
+                                              float& rho, float& gs)
+{
+    if (ready) {
+        rho = base.rho[i];
+        gs = base.gs[i];
+        return;
+    }
+    uint32_t s[27], e[27], m = 0;
+#pragma unroll
+    for (int c = 0; c < 27; ++c) {
+        const uint32_t h = grid_hash(P, g, c % 3 - 1, (c / 3) % 3 - 1, c / 9 - 1);
+        s[c] = __ldg(vb.cs + h);
+        e[c] = __ldg(vb.ce + h);
+        if (s[c] != SNOWB_EMPTY) m |= 1u << c;
+    }
+    rho = (P.rho0 * X.bnd.volume[o]) * P.W0;
+    gs = 0.f;
+    while (m) {
+        const int c = __ffs(m) - 1;
+        m &= m - 1u;
+        float cs = 0.f, cg = 0.f;
+        for (uint32_t j = s[c]; j < e[c]; ++j)
+            if (j != i)
+                wg_term<true>(P, cs, cg, vb.pw(j), p, j, true, 2, 0.f, vb.attr(sb.mass, X.bnd.mass, j), nullptr, 0, 0);
+        rho += cs;
+        gs += cg;
+    }
+    base.rho[i] = rho;
+    base.gs[i] = gs;
+}
+
 template <bool LAMBDA>
 // with_bnd = 0: water and snow only (the boundary particles' density, C and lambda are then
 // left as they were; a later density+lambda pass of the substep rewrites them).  The water
 // and snow sums take the boundary's terms either way, through its compact sorted copies.
 __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restrict__ S, SetView vs, SetView vd,
                                                  SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, NList L,
-                                                 int with_bnd)
+                                                 int with_bnd, BndBase base)
 {
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b, nbt = with_bnd ? nb : 0u;
     vs.n = ns; vd.n = nd; vb.n = nb;
+    const bool ready = S->base_ready != 0u;
     const float3 z = f3(0.f, 0.f, 0.f);
     if (LAMBDA && blockIdx.x == 0 && threadIdx.x == 0) S->far_move = 0u;   // the lists are new
     GRID_LOOP(t, ns + nd + nbt) {
@@ -420,27 +480,31 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
                 L.cnt[wr.slot] = n_own > NLIST_K ? NL_OVF : n_own;
             }
         } else {
-            // boundary: density sums the sets in the order (b, snow, water), lambda (b, water, snow)
+            // boundary: density sums the sets in the order (b, snow, water), lambda (b, water,
+            // snow); the sums over the boundary itself open both, and most boundary particles
+            // have no other neighbour
             i = t - ns - nd; o = vb.gi[i];
             float3 p = xyz(vb.p4[i]); GCell g = grid_pos(P, p, vb.scene(i));
-            const Nbhd nb = make_nbhd(P, g, p, P.h2_cull);
-            rho = (P.rho0 * X.bnd.volume[o]) * P.W0;
-            acc_WG<LAMBDA>(P, rho, gs, vb, p, nb, i, true, 2, 0.f, sb.mass, X.bnd.mass);
-            if (LAMBDA) {
+            boundary_base(P, vb, X, sb, i, o, p, g, ready, base, rho, gs);
+            const uint32_t near = occupied27(P, g, vs, vd);
+            if (LAMBDA && near) {
                 // one traversal per set for both sums: water first (its lambda terms come
                 // before the snow's), its density partials kept aside and added after the
                 // snow's, cell by cell in order -- the two orders of the separate passes
+                const Nbhd nb = make_nbhd(P, g, p, P.h2_cull);
                 float wpart[27];
                 uint32_t wmask = 0;
-                acc_WG<true>(P, rho, gs, vs, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr, nullptr, 0, wpart,
-                             &wmask);
-                acc_WG<true>(P, rho, gs, vd, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr);
+                if (near & 1u)
+                    acc_WG<true>(P, rho, gs, vs, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr, nullptr, 0, wpart,
+                                 &wmask);
+                if (near & 2u) acc_WG<true>(P, rho, gs, vd, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr);
                 while (wmask) {
                     const int c = __ffs(wmask) - 1;
                     wmask &= wmask - 1u;
                     rho += wpart[c];
                 }
-            } else {
+            } else if (near) {
+                const Nbhd nb = make_nbhd(P, g, p, P.h2_cull);
                 float unused = 0.f;
                 acc_WG<false>(P, rho, unused, vd, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr);
                 acc_WG<false>(P, rho, unused, vs, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr);
@@ -455,6 +519,181 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
             float lam = (-c) / (gs + P.eps);
             D->lambda[o] = lam;
             lam_s[i] = lam;
+        }
+    }
+}
+
+constexpr uint32_t DENSITY_WARP_MAX = 40000;
+// The same pass with one warp per particle, for sets too small to fill the GPU with threads
+// (DENSITY_WARP_MAX): one thread walking 81 cells is a chain of some 160 dependent loads, 80 to
+// 120 us whatever the set's size.  Lane c < 27 takes cell c of each set: it marks the
+// candidates within the support, the counts' prefix over the lanes places its list entries in
+// traversal order, it forms the cell's partial sums in index order, and the partials are added
+// in cell order with shuffles -- the operations of the one-thread form in the same order.  A
+// warp takes 32 boundary particles: each lane tests whether its particle has water or snow
+// around it, and the few that do are taken by the whole warp one after another.
+// Density + lambda, both forms, us a launch: 67 -> 18 at 208 particles, 105 -> 33 at 5,096, 119
+// -> 55 at 16,380.  Whole frames, one thread against one warp each: 2.66 against 2.03 ms at
+// 15.8k particles, 3.24 against 3.03 at 35.7k, 3.32 against 3.80 at 58k; the line lies between.
+struct CellHits {
+    uint32_t s, e, n, mask;     // range, candidates within the support, which of the first 32
+};
+__device__ __forceinline__ CellHits cell_hits(const DevParams& P, const SetView& v, float3 p, uint32_t h, bool live,
+                                              uint32_t skip)
+{
+    CellHits c{0u, 0u, 0u, 0u};
+    if (!live) return c;
+    c.s = __ldg(v.cs + h);
+    c.e = __ldg(v.ce + h);
+    if (c.s == SNOWB_EMPTY) c.e = c.s = 0u;
+    for (uint32_t j0 = c.s; j0 < c.e; j0 += 4u) {
+        float d2[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u) {
+            const float3 dv = sub3(p, v.pos(umin32(j0 + u, c.e - 1u)));
+            d2[u] = dot3(dv, dv);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u)
+            if (j0 + u < c.e && d2[u] < P.h2_lt && j0 + u != skip) {
+                ++c.n;
+                if (j0 + u - c.s < 32u) c.mask |= 1u << (j0 + u - c.s);
+            }
+    }
+    return c;
+}
+// the cell's partial sums and, with e set, its list entries from position k on
+template <bool LAMBDA>
+__device__ __forceinline__ void cell_sums(const DevParams& P, const SetView& v, float3 p, const CellHits& c,
+                                          uint32_t skip, bool vol, int mode, float m_self, NLWriter* wr, int cell,
+                                          int set, float& cs, float& cg)
+{
+    cs = cg = 0.f;
+    uint32_t m = c.mask;
+    while (m) {
+        const uint32_t j = c.s + (uint32_t)__ffs(m) - 1u;
+        m &= m - 1u;
+        wg_term<LAMBDA>(P, cs, cg, v.pw(j), p, j, vol, mode, m_self, 0.f, wr, cell, set);
+    }
+    for (uint32_t j = c.s + 32u; j < c.e; ++j)
+        if (j != skip) wg_term<LAMBDA>(P, cs, cg, v.pw(j), p, j, vol, mode, m_self, 0.f, wr, cell, set);
+}
+// adds the cells' partials in cell order (partials are never negative and the totals never -0,
+// so a cell whose partials are both +0 is left out)
+__device__ __forceinline__ void warp_ordered_add(float& a, float& b, float pa, float pb)
+{
+    uint32_t m = __ballot_sync(0xffffffffu, (__float_as_uint(pa) | __float_as_uint(pb)) != 0u);
+    while (m) {
+        const int k = __ffs(m) - 1;
+        m &= m - 1u;
+        a += __shfl_sync(0xffffffffu, pa, k);
+        b += __shfl_sync(0xffffffffu, pb, k);
+    }
+}
+template <bool LAMBDA>
+__global__ void __launch_bounds__(256) k_density_warp(DevParams P, DevState* __restrict__ S, SetView vs, SetView vd,
+                                                      SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, NList L,
+                                                      int with_bnd, BndBase base)
+{
+    const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b, nbg = with_bnd ? (nb + 31u) / 32u : 0u;
+    vs.n = ns; vd.n = nd; vb.n = nb;
+    const bool ready = S->base_ready != 0u;
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu;
+    const bool cl = lane < 27u;
+    const int ox = (int)(lane % 3u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane / 9u) - 1;
+    if (LAMBDA && blockIdx.x == 0 && threadIdx.x == 0) S->far_move = 0u;   // the lists are new
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ns + nd + nbg; t += nwarps) {
+        if (t < ns + nd) {
+            const bool w = t < ns;
+            const uint32_t i = w ? t : t - ns;
+            const SetView& own = w ? vs : vd;
+            const SetView& oth = w ? vd : vs;
+            const snowb_particle_data& D = w ? X.sph : X.dem;
+            const uint32_t o = own.gi[i];
+            const float3 p = xyz(own.p4[i]);
+            const uint32_t h = grid_hash(P, grid_pos(P, p, own.scene(i)), ox, oy, oz);
+            const float mass = D.mass[o];
+            const CellHits c0 = cell_hits(P, own, p, h, cl, i), c1 = cell_hits(P, oth, p, h, cl, SNOWB_UMAX),
+                           c2 = cell_hits(P, vb, p, h, cl, SNOWB_UMAX);
+            // list positions: the lambda pass lists all three sets, the first density pass the
+            // snow-snow candidates
+            const bool l0 = LAMBDA || !w;
+            const uint32_t slot = (w ? 0u : L.cap) + i;
+            const uint32_t i0 = l0 ? warp_incl_scan(c0.n) : 0u, n0 = __shfl_sync(full, i0, 31);
+            const uint32_t i1 = LAMBDA ? warp_incl_scan(c1.n) : 0u, n1 = __shfl_sync(full, i1, 31);
+            const uint32_t i2 = LAMBDA ? warp_incl_scan(c2.n) : 0u, n2 = __shfl_sync(full, i2, 31);
+            float rho = mass * P.W0, gs = 0.f, pa, pb;
+            NLWriter wr{L.e, L.stride, slot, i0 - c0.n};
+            cell_sums<LAMBDA>(P, own, p, c0, i, false, 0, 0.f, l0 ? &wr : nullptr, (int)lane, 0, pa, pb);
+            warp_ordered_add(rho, gs, pa, pb);
+            wr.n = n0 + i1 - c1.n;
+            cell_sums<LAMBDA>(P, oth, p, c1, SNOWB_UMAX, false, 0, 0.f, LAMBDA ? &wr : nullptr, (int)lane, 1, pa, pb);
+            warp_ordered_add(rho, gs, pa, pb);
+            wr.n = n0 + n1 + i2 - c2.n;
+            cell_sums<LAMBDA>(P, vb, p, c2, SNOWB_UMAX, true, 1, mass, LAMBDA ? &wr : nullptr, (int)lane, 2, pa, pb);
+            warp_ordered_add(rho, gs, pa, pb);
+            if (lane == 0) {
+                const uint32_t n = n0 + n1 + n2;
+                if (l0) {
+                    L.cnt[slot] = n > NLIST_K ? NL_OVF : (n0 | (n1 << 10) | (n2 << 20));
+                    if (LAMBDA && n > NLIST_K) atomicAdd(&S->n_nl_ovf, 1u);
+                }
+                float c = (rho / P.rho0) - 1.f;
+                c = c > 0.f ? c : 0.f;
+                D.density[o] = rho;
+                D.C[o] = c;
+                if (LAMBDA) {
+                    const float lam = (-c) / (gs + P.eps);
+                    D.lambda[o] = lam;
+                    (w ? ss.lambda : sd.lambda)[i] = lam;
+                }
+            }
+        } else {
+            // a warp's boundary particles lie nbg apart: those with neighbours come in patches
+            const uint32_t i = (t - ns - nd) + lane * nbg;
+            const bool live = i < nb;
+            float3 p = f3(0.f, 0.f, 0.f);
+            GCell g{};
+            float rho = 0.f, gs = 0.f;
+            uint32_t near = 0;
+            if (live) {
+                p = xyz(vb.p4[i]);
+                g = grid_pos(P, p, vb.scene(i));
+                boundary_base(P, vb, X, sb, i, vb.gi[i], p, g, ready, base, rho, gs);
+                near = occupied27(P, g, vs, vd);
+            }
+            uint32_t m = __ballot_sync(full, near != 0u);
+            while (m) {
+                const int k = __ffs(m) - 1;
+                m &= m - 1u;
+                const float3 q = f3(__shfl_sync(full, p.x, k), __shfl_sync(full, p.y, k), __shfl_sync(full, p.z, k));
+                const GCell gk{__shfl_sync(full, g.x, k), __shfl_sync(full, g.y, k), __shfl_sync(full, g.z, k),
+                               __shfl_sync(full, g.bx, k), __shfl_sync(full, g.bz, k)};
+                const uint32_t h = grid_hash(P, gk, ox, oy, oz);
+                float wa, wb, sa, sb2, r = __shfl_sync(full, rho, k), s = __shfl_sync(full, gs, k), none = 0.f;
+                cell_sums<LAMBDA>(P, vs, q, cell_hits(P, vs, q, h, cl, SNOWB_UMAX), SNOWB_UMAX, false, 0, 0.f, nullptr,
+                                  0, 0, wa, wb);
+                cell_sums<LAMBDA>(P, vd, q, cell_hits(P, vd, q, h, cl, SNOWB_UMAX), SNOWB_UMAX, false, 0, 0.f, nullptr,
+                                  0, 0, sa, sb2);
+                warp_ordered_add(r, none, sa, 0.f);     // density: snow, then water
+                warp_ordered_add(r, none, wa, 0.f);
+                warp_ordered_add(s, none, wb, 0.f);     // lambda: water, then snow
+                warp_ordered_add(s, none, sb2, 0.f);
+                if (lane == (uint32_t)k) { rho = r; gs = s; }
+            }
+            if (live) {
+                const uint32_t o = vb.gi[i];
+                float c = (rho / P.rho0) - 1.f;
+                c = c > 0.f ? c : 0.f;
+                X.bnd.density[o] = rho;
+                X.bnd.C[o] = c;
+                if (LAMBDA) {
+                    const float lam = (-c) / (gs + P.eps);
+                    X.bnd.lambda[o] = lam;
+                    sb.lambda[i] = lam;
+                }
+            }
         }
     }
 }
@@ -499,6 +738,8 @@ __global__ void __launch_bounds__(256) k_pbf(DevParams P, DevState* __restrict__
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b;
     vs.n = ns; vd.n = nd; vb.n = nb;
     const bool ref = P.quirks == SNOWB_QUIRKS_REFERENCE;
+    // the density + lambda pass before this one has formed the boundary sums
+    if (blockIdx.x == 0 && threadIdx.x == 0) S->base_ready = 1u;
     // up to PBF_WARP_MAX_WATER water particles the water terms come from k_pbf_water_warp;
     // the snow particles keep the thread mapping t = ns + i of the reference's launch (its
     // float atomics, Q3, follow it)
@@ -1362,6 +1603,7 @@ __global__ void k_set_state(DevState* S, uint32_t ns, uint32_t nd, uint32_t nb)
         for (int k = 0; k < 2; ++k) { S->moved[k] = 1u; S->sorts_full[k] = 0u; S->sorts_kept[k] = 0u; }
         for (int c = 0; c < 8; ++c) S->sc_count[c] = 0u;
         S->clean_hi[0] = SNOWB_UMAX; S->clean_hi[1] = SNOWB_UMAX;
+        S->base_ready = 0u;   // ... and the boundary
     }
 }
 // batched runs: every live slot's scene id must name a scene of the batch
