@@ -9,10 +9,16 @@
 // a differentiated substep and every contrib is 1 (the fields the adjoint assumes).
 //
 // All adjoint and field arrays are in original index order (like the caller's state); the
-// gathers run over the sorted views of the positions being differentiated, exactly like
-// the forward neighbour loops.  Every kernel is a gather: a particle accumulates every
+// gathers run over the sorted views of the positions being differentiated, over the
+// neighbours of the forward loops.  Every kernel is a gather: a particle accumulates every
 // term in which it takes part, from its own constraint and from its neighbours', so no
 // atomics are needed except for the scalar parameter gradients.
+//
+// The neighbour passes run one warp per particle (warp_neighbors): with the few thousand
+// particles that are differentiated, one thread each left most of the GPU idle while it
+// walked up to 81 cells one candidate after another (9,216 particles, us a launch: fields
+// 90 -> 43, lambda adjoint 99 -> 19, positions 130 -> 43, friction 81 -> 25, XSPH 79 -> 20,
+// heat 94 -> 31).
 //
 // Notation: r = x_i - x_j, d = |r|.  For a radial vector function F(r) = f(d) r its
 // Jacobian is J = f I + (f'(d)/d) r r^T (symmetric, even in r).
@@ -82,54 +88,198 @@ __device__ __forceinline__ float3 grad_gsq(const DevParams& P, float3 r, float d
     return sc3(2.f, jv_spiky(P, r, d, G));
 }
 
+// ------------------------------------------------------- a particle's neighbours by a warp
+// Ordered sums over the entries j != skip of set v within d2 < cut of p.  Lane c < 27 scans cell c
+// (h: its hash), four entries in flight; the counts' prefix over the lanes lists those accepted
+// in shared memory in traversal order (cells z-y-x, index ascending), and 32 of them at a time
+// are evaluated side by side: terms(j, out) writes M addends for each of NA sums, sum-major.
+// Lane a < NA then adds the addends of sum a to its `acc`, neighbour by neighbour in order -- the
+// additions that one thread walking the cells makes, so the sums round alike, while the costly
+// terms run with full warps although a cell accepts few of its entries.  An absent addend is 0.
+// (Views of a full sort: every range is current.)
+constexpr uint32_t ADJ_TPB = 128, ADJ_LIST = 96, ADJ_TERMS = 24;
+struct AdjBuf {
+    uint32_t j[ADJ_LIST];
+    float t[32 * (ADJ_TERMS + 1)];    // a lane's addends; an odd row keeps the lanes off each other's banks
+};
+template <int NA, int M, class F>
+__device__ __forceinline__ void warp_neighbors(const SetView& v, float3 p, uint32_t h, uint32_t skip, float cut,
+                                               AdjBuf& W, float& acc, F&& terms)
+{
+    static_assert(NA * M <= (int)ADJ_TERMS, "addends of a neighbour");
+    constexpr int ROW = (NA * M) | 1;
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu;
+    uint32_t s = 0, e = 0;
+    if (lane < 27u) {
+        s = __ldg(v.cs + h);
+        e = __ldg(v.ce + h);
+        if (s == SNOWB_EMPTY) s = e = 0u;
+    }
+    auto hit = [&](uint32_t j) {
+        const float3 r = sub3(p, xyz(__ldg(v.p4 + j)));
+        return dot3(r, r) < cut && j != skip;
+    };
+    uint32_t n = 0, mask = 0;   // accepted, and which of the first 32 entries
+    for (uint32_t k = 0; k < e - s; k += 4u)
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u)
+            if (hit(umin32(s + k + u, e - 1u)) && s + k + u < e) {
+                ++n;
+                if (k + u < 32u) mask |= 1u << (k + u);
+            }
+    const uint32_t first = warp_incl_scan(n) - n, total = __shfl_sync(full, first + n, 31);
+    for (uint32_t w0 = 0; w0 < total; w0 += ADJ_LIST) {
+        __syncwarp();
+        uint32_t at = first, m = mask;
+        while (m) {
+            const uint32_t j = s + (uint32_t)__ffs(m) - 1u;
+            m &= m - 1u;
+            if (at - w0 < ADJ_LIST) W.j[at - w0] = j;
+            ++at;
+        }
+        for (uint32_t j = s + 32u; j < e; ++j)
+            if (hit(j)) {
+                if (at - w0 < ADJ_LIST) W.j[at - w0] = j;
+                ++at;
+            }
+        __syncwarp();
+        const uint32_t held = umin32(total - w0, ADJ_LIST);
+        for (uint32_t b = 0; b < held; b += 32u) {
+            if (b + lane < held) terms(W.j[b + lane], W.t + lane * ROW);
+            __syncwarp();
+            if (lane < (uint32_t)NA)
+                for (uint32_t k = 0; k < umin32(held - b, 32u); ++k)
+#pragma unroll
+                    for (int q = 0; q < M; ++q) acc += W.t[k * ROW + lane * M + q];
+            __syncwarp();
+        }
+    }
+}
+// sum a of the ordered sums, for every lane
+__device__ __forceinline__ float sum_of(float acc, int a) { return __shfl_sync(0xffffffffu, acc, a); }
+__device__ __forceinline__ float3 sum3_of(float acc, int a) { return f3(sum_of(acc, a), sum_of(acc, a + 1), sum_of(acc, a + 2)); }
+// addend q of the three sums from a on (M addends each)
+template <int M>
+__device__ __forceinline__ void put3(float* out, int a, int q, float3 x)
+{
+    out[a * M + q] = x.x;
+    out[(a + 1) * M + q] = x.y;
+    out[(a + 2) * M + q] = x.z;
+}
+// lane c < 27: hash of cell c around g
+__device__ __forceinline__ uint32_t lane_cell(const DevParams& P, GCell g)
+{
+    const uint32_t c = threadIdx.x & 31u;
+    return c < 27u ? grid_hash(P, g, (int)(c % 3u) - 1, (int)((c / 3u) % 3u) - 1, (int)(c / 9u) - 1) : 0u;
+}
+// warps of the launch, and this one's number
+#define WARP_LOOP(t, n) \
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < (n); t += (gridDim.x * blockDim.x) >> 5)
+// A warp takes 32 boundary particles (nbg apart: those with neighbours come in patches): lane by
+// lane they are looked over (near(i): is anything around?), and those with something around are
+// taken by the whole warp, one after another (take(i), every lane).
+template <class N, class T>
+__device__ __forceinline__ void boundary_patch(uint32_t t, uint32_t nb, N&& near, T&& take)
+{
+    const uint32_t nbg = (nb + 31u) / 32u, i = t + (threadIdx.x & 31u) * nbg;
+    uint32_t m = __ballot_sync(0xffffffffu, i < nb && near(i));
+    while (m) {
+        const uint32_t k = (uint32_t)__ffs(m) - 1u;
+        m &= m - 1u;
+        take(t + k * nbg);
+    }
+}
+
 // ---------------------------------------------------------------- fields at positions
 // density, C, gradient-square sum and lambda of every particle of the three sets (the
 // quantities of k_density<true>, fixed quirks), stored in original order.
-__global__ void __launch_bounds__(128) ka_fields(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
-                                                 SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
-                                                 AdjField fb)
+__device__ __forceinline__ void field_store(const DevParams& P, const AdjField& F, uint32_t o, float rho, float S)
 {
+    const float C = (rho / P.rho0) - 1.f > 0.f ? (rho / P.rho0) - 1.f : 0.f;
+    F.rho[o] = rho;
+    F.C[o] = C;
+    F.S[o] = S;
+    F.lam[o] = -C / (S + P.eps);
+}
+// a particle's density (sum 0) and gradient-square (sum 1) terms from the entries of set v (vol:
+// the boundary, whose lambda denominator scales with the volume over m_of(j))
+template <class F>
+__device__ __forceinline__ void field_terms(const DevParams& P, const SetView& v, float3 p, uint32_t h, uint32_t skip,
+                                            bool vol, AdjBuf& W, float& acc, F&& m_of)
+{
+    warp_neighbors<2, 1>(v, p, h, skip, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+        const float4 q = __ldg(v.p4 + j);
+        const float3 r = sub3(p, xyz(q));
+        const float d = sqrtf(dot3(r, r));
+        out[0] = (vol ? P.rho0 * q.w : q.w) * W_poly6(P, d);
+        const float sc = vol ? P.inv_rho0 * ((P.rho0 * q.w) / m_of(j)) : P.inv_rho0;
+        const float3 G = G_spiky(P, r, d);
+        out[1] = (sc * sc) * dot3(G, G);
+    });
+}
+// the sums of a boundary particle without water or snow around it: the boundary does not move,
+// so they are the same in every pass of a backward call (by sorted index)
+__global__ void __launch_bounds__(ADJ_TPB) ka_boundary_base(DevParams P, uint32_t nb, SetView vb, Sets X, float* rho0,
+                                                            float* S0)
+{
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    vb.n = nb;
+    WARP_LOOP(i, nb) {
+        const float3 p = xyz(vb.p4[i]);
+        float acc = lane == 0u ? (P.rho0 * X.bnd.volume[vb.gi[i]]) * P.W0 : 0.f;
+        field_terms(P, vb, p, lane_cell(P, grid_pos(P, p)), i, true, W, acc,
+                    [&](uint32_t j) { return X.bnd.mass[vb.gi[j]]; });
+        if (lane == 0u) rho0[i] = acc;
+        if (lane == 1u) S0[i] = acc;
+    }
+}
+__global__ void __launch_bounds__(ADJ_TPB) ka_fields(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
+                                                     SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
+                                                     AdjField fb, const float* __restrict__ rho0,
+                                                     const float* __restrict__ S0)
+{
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns; vb.n = nb;
-    GRID_LOOP(t, nw + ns + nb) {
-        const int set = t < nw ? 0 : (t < nw + ns ? 1 : 2);
-        const uint32_t i = set == 0 ? t : (set == 1 ? t - nw : t - nw - ns);
-        const SetView& own = set == 0 ? vw : (set == 1 ? vs : vb);
-        const uint32_t o = own.gi[i];
-        const float3 p = xyz(own.p4[i]);
-        const GCell g = grid_pos(P, p);
-        const float wi = set == 2 ? P.rho0 * X.bnd.volume[o] : (set == 0 ? X.sph.mass[o] : X.dem.mass[o]);
-        const float mi = set == 0 ? X.sph.mass[o] : (set == 1 ? X.dem.mass[o] : X.bnd.mass[o]);
-        float rho = wi * P.W0, S = 0.f;
-        for (int k = 0; k < 3; ++k) {
-            const SetView& v = k == 0 ? vw : (k == 1 ? vs : vb);
-            const bool self = k == set;
-            FOR27 {
-                uint32_t s, e;
-                if (!v.range(P, g, ox, oy, oz, s, e)) continue;
-                for (uint32_t j = s; j < e; ++j) {
-                    if (self && j == i) continue;
-                    const float4 q = v.p4[j];
-                    const float3 r = sub3(p, xyz(q));
-                    const float d2 = dot3(r, r);
-                    if (!(d2 < P.h2_lt)) continue;
-                    const float d = sqrtf(d2);
-                    const float wj = k == 2 ? P.rho0 * q.w : q.w;
-                    rho += wj * W_poly6(P, d);
-                    // lambda denominator scale (modes of the three lambda kernels)
-                    float sc = P.inv_rho0;
-                    if (set != 2 && k == 2) sc = P.inv_rho0 * ((P.rho0 * q.w) / mi);
-                    if (set == 2 && k == 2) sc = P.inv_rho0 * ((P.rho0 * q.w) / X.bnd.mass[v.gi[j]]);
-                    const float3 G = G_spiky(P, r, d);
-                    S += (sc * sc) * dot3(G, G);
-                }
-            }
+    const uint32_t lane = threadIdx.x & 31u;
+    WARP_LOOP(t, nw + ns + (nb + 31u) / 32u) {
+        if (t < nw + ns) {
+            const bool w = t < nw;
+            const uint32_t i = w ? t : t - nw;
+            const SetView& own = w ? vw : vs;
+            const uint32_t o = own.gi[i];
+            const float3 p = xyz(own.p4[i]);
+            const uint32_t h = lane_cell(P, grid_pos(P, p));
+            const float mi = (w ? X.sph.mass : X.dem.mass)[o];
+            auto m_of = [&](uint32_t) { return mi; };
+            float acc = lane == 0u ? mi * P.W0 : 0.f;
+            field_terms(P, vw, p, h, w ? i : SNOWB_UMAX, false, W, acc, m_of);
+            field_terms(P, vs, p, h, w ? SNOWB_UMAX : i, false, W, acc, m_of);
+            field_terms(P, vb, p, h, SNOWB_UMAX, true, W, acc, m_of);
+            const float S = sum_of(acc, 1);
+            if (lane == 0u) field_store(P, w ? fw : fs, o, acc, S);
+        } else {
+            boundary_patch(
+                t - nw - ns, nb,
+                [&](uint32_t i) {
+                    const bool near = occupied27(P, grid_pos(P, xyz(vb.p4[i])), vw, vs) != 0u;
+                    if (!near) field_store(P, fb, vb.gi[i], rho0[i], S0[i]);
+                    return near;
+                },
+                [&](uint32_t i) {
+                    const float3 p = xyz(vb.p4[i]);
+                    const uint32_t o = vb.gi[i], h = lane_cell(P, grid_pos(P, p));
+                    auto m_of = [&](uint32_t j) { return X.bnd.mass[vb.gi[j]]; };
+                    float acc = lane == 0u ? (P.rho0 * X.bnd.volume[o]) * P.W0 : 0.f;
+                    field_terms(P, vw, p, h, SNOWB_UMAX, false, W, acc, m_of);
+                    field_terms(P, vs, p, h, SNOWB_UMAX, false, W, acc, m_of);
+                    field_terms(P, vb, p, h, i, true, W, acc, m_of);
+                    const float S = sum_of(acc, 1);
+                    if (lane == 0u) field_store(P, fb, o, acc, S);
+                });
         }
-        const AdjField& F = set == 0 ? fw : (set == 1 ? fs : fb);
-        const float C = (rho / P.rho0) - 1.f > 0.f ? (rho / P.rho0) - 1.f : 0.f;
-        F.rho[o] = rho;
-        F.C[o] = C;
-        F.S[o] = S;
-        F.lam[o] = -C / (S + P.eps);
     }
 }
 
@@ -137,72 +287,75 @@ __global__ void __launch_bounds__(128) ka_fields(DevParams P, uint32_t nw, uint3
 // lambda-bar of every particle from u (sor times the adjoint of the corrected water
 // positions), then C-, S- and rho-bar (rho-bar is added to, so other terms at the same
 // positions can be accumulated first).
-__global__ void __launch_bounds__(128) ka_pbf_lambar(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
-                                                     SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
-                                                     AdjField fb, AdjSet aw)
+__device__ __forceinline__ void lambar_store(const DevParams& P, const AdjField& F, uint32_t o, float lb)
 {
+    const float den = F.S[o] + P.eps;
+    const float Cb = -lb / den;
+    F.lamb[o] = lb;
+    F.Sb[o] = lb * F.C[o] / (den * den);
+    if ((F.rho[o] / P.rho0) - 1.f > 0.f) F.rhob[o] += Cb * P.inv_rho0;
+}
+// snow (snow: the coupling's support) and boundary particles take part in the water's PBF sums
+__device__ __forceinline__ float lambar_of_water(const DevParams& P, const SetView& vw, float3 p, bool snow,
+                                                 const float* contrib, const snowb_float3* u, AdjBuf& W)
+{
+    float acc = 0.f;
+    warp_neighbors<1, 1>(vw, p, lane_cell(P, grid_pos(P, p)), SNOWB_UMAX, snow ? P.r2_le : P.h2_lt, W, acc,
+                         [&](uint32_t j, float* out) {
+        const float3 r = sub3(p, xyz(__ldg(vw.p4 + j)));   // r = x_i - x_k, the water term uses -r
+        const float d = sqrtf(dot3(r, r));
+        const uint32_t ok = vw.gi[j];
+        out[0] = -(contrib[ok] * dot3(ldv3(u, ok), snow ? G_poly6(P, r, d) : G_spiky(P, r, d)));
+    });
+    return acc;   // in lane 0
+}
+__global__ void __launch_bounds__(ADJ_TPB) ka_pbf_lambar(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
+                                                         SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
+                                                         AdjField fb, AdjSet aw)
+{
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns; vb.n = nb;
-    GRID_LOOP(t, nw + ns + nb) {
-        const int set = t < nw ? 0 : (t < nw + ns ? 1 : 2);
-        const uint32_t i = set == 0 ? t : (set == 1 ? t - nw : t - nw - ns);
-        const SetView& own = set == 0 ? vw : (set == 1 ? vs : vb);
-        const uint32_t o = own.gi[i];
-        const float3 p = xyz(own.p4[i]);
-        const GCell g = grid_pos(P, p);
-        float lb = 0.f;
-        if (set == 0) {
+    const uint32_t lane = threadIdx.x & 31u;
+    WARP_LOOP(t, nw + ns + (nb + 31u) / 32u) {
+        if (t < nw) {
+            const uint32_t o = vw.gi[t];
+            const float3 p = xyz(vw.p4[t]);
+            const uint32_t h = lane_cell(P, grid_pos(P, p));
             const float ci = X.sph.contrib[o];
             const float3 ui = ldv3(aw.u, o);
             float acc = 0.f;
-            for (int k = 0; k < 3; ++k) {
-                const SetView& v = k == 0 ? vw : (k == 1 ? vs : vb);
-                FOR27 {
-                    uint32_t s, e;
-                    if (!v.range(P, g, ox, oy, oz, s, e)) continue;
-                    for (uint32_t j = s; j < e; ++j) {
-                        if (k == 0 && j == i) continue;
-                        const float3 r = sub3(p, xyz(v.p4[j]));
-                        const float d2 = dot3(r, r);
-                        const float d = sqrtf(d2);
-                        if (k == 0 && d2 < P.h2_lt) {
-                            const uint32_t oj = v.gi[j];
-                            const float cj = X.sph.contrib[oj];
-                            const float3 uj = ldv3(aw.u, oj);
-                            acc += (ci * cj) * dot3(sub3(ui, uj), G_spiky(P, r, d));
-                        } else if (k == 1 && d2 < P.r2_le) {
-                            acc += ci * dot3(ui, G_poly6(P, r, d));
-                        } else if (k == 2 && d2 < P.h2_lt) {
-                            acc += ci * dot3(ui, G_spiky(P, r, d));
-                        }
-                    }
-                }
-            }
-            lb = acc * P.inv_rho0;
+            warp_neighbors<1, 1>(vw, p, h, t, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+                const float3 r = sub3(p, xyz(__ldg(vw.p4 + j)));
+                const uint32_t oj = vw.gi[j];
+                out[0] = (ci * X.sph.contrib[oj]) * dot3(sub3(ui, ldv3(aw.u, oj)), G_spiky(P, r, sqrtf(dot3(r, r))));
+            });
+            warp_neighbors<1, 1>(vs, p, h, SNOWB_UMAX, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+                const float3 r = sub3(p, xyz(__ldg(vs.p4 + j)));
+                out[0] = ci * dot3(ui, G_poly6(P, r, sqrtf(dot3(r, r))));
+            });
+            warp_neighbors<1, 1>(vb, p, h, SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+                const float3 r = sub3(p, xyz(__ldg(vb.p4 + j)));
+                out[0] = ci * dot3(ui, G_spiky(P, r, sqrtf(dot3(r, r))));
+            });
+            if (lane == 0u) lambar_store(P, fw, o, acc * P.inv_rho0);
+        } else if (t < nw + ns) {
+            const uint32_t i = t - nw;
+            const float acc = lambar_of_water(P, vw, xyz(vs.p4[i]), true, X.sph.contrib, aw.u, W);
+            if (lane == 0u) lambar_store(P, fs, vs.gi[i], acc * P.inv_rho0);
         } else {
-            // snow and boundary particles take part in the water particles' PBF sums
-            float acc = 0.f;
-            FOR27 {
-                uint32_t s, e;
-                if (!vw.range(P, g, ox, oy, oz, s, e)) continue;
-                for (uint32_t j = s; j < e; ++j) {
-                    const float3 r = sub3(p, xyz(vw.p4[j]));   // r = x_i - x_k, the water term uses -r
-                    const float d2 = dot3(r, r);
-                    const uint32_t ok = vw.gi[j];
-                    const float ck = X.sph.contrib[ok];
-                    const float3 uk = ldv3(aw.u, ok);
-                    const float d = sqrtf(d2);
-                    if (set == 1 && d2 < P.r2_le) acc -= ck * dot3(uk, G_poly6(P, r, d));
-                    if (set == 2 && d2 < P.h2_lt) acc -= ck * dot3(uk, G_spiky(P, r, d));
-                }
-            }
-            lb = acc * P.inv_rho0;
+            boundary_patch(
+                t - nw - ns, nb,
+                [&](uint32_t i) {
+                    const bool near = (occupied27(P, grid_pos(P, xyz(vb.p4[i])), vw, vw) & 1u) != 0u;
+                    if (!near) lambar_store(P, fb, vb.gi[i], 0.f);
+                    return near;
+                },
+                [&](uint32_t i) {
+                    const float acc = lambar_of_water(P, vw, xyz(vb.p4[i]), false, X.sph.contrib, aw.u, W);
+                    if (lane == 0u) lambar_store(P, fb, vb.gi[i], acc * P.inv_rho0);
+                });
         }
-        const AdjField& F = set == 0 ? fw : (set == 1 ? fs : fb);
-        const float den = F.S[o] + P.eps;
-        const float Cb = -lb / den;
-        F.lamb[o] = lb;
-        F.Sb[o] = lb * F.C[o] / (den * den);
-        if ((F.rho[o] / P.rho0) - 1.f > 0.f) F.rhob[o] += Cb * P.inv_rho0;
     }
 }
 
@@ -212,19 +365,21 @@ __global__ void __launch_bounds__(128) ka_pbf_lambar(DevParams P, uint32_t nw, u
 // terms of rho-bar (which also carries the XSPH and heat contributions at these
 // positions when they were accumulated before).  pbf != 0 adds the constraint terms;
 // pbf == 0 runs the density part alone (heat, substep start).
-__global__ void __launch_bounds__(128) ka_pos_rev(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
+__global__ void __launch_bounds__(ADJ_TPB) ka_pos_rev(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
                                                   SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
-                                                  AdjField fb, AdjSet aw, AdjSet as, AdjParams G, int pbf, int contact)
+                                                  AdjField fb, AdjSet aw, AdjSet as, float* __restrict__ kst, int pbf, int contact)
 {
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns; vb.n = nb;
-    float kst_acc = 0.f;
-    GRID_LOOP(t, nw + ns) {
+    const uint32_t lane = threadIdx.x & 31u;
+    WARP_LOOP(t, nw + ns) {
         const int set = t < nw ? 0 : 1;
         const uint32_t i = set == 0 ? t : t - nw;
         const SetView& own = set == 0 ? vw : vs;
         const uint32_t o = own.gi[i];
         const float3 p = xyz(own.p4[i]);
-        const GCell g = grid_pos(P, p);
+        const uint32_t h = lane_cell(P, grid_pos(P, p));
         const AdjField& Fi = set == 0 ? fw : fs;
         const AdjSet& Ai = set == 0 ? aw : as;
         const snowb_particle_data& Di = set == 0 ? X.sph : X.dem;
@@ -232,97 +387,111 @@ __global__ void __launch_bounds__(128) ka_pos_rev(DevParams P, uint32_t nw, uint
         const float rhob_i = Fi.rhob[o], Sb_i = Fi.Sb[o];
         const float lam_i = pbf ? Fi.lam[o] : 0.f;
         const float3 ui = pbf ? ldv3(Ai.u, o) : f3(0.f, 0.f, 0.f);
-        float3 xb = f3(0.f, 0.f, 0.f);
-        float3 kst_dir = f3(0.f, 0.f, 0.f);
+        // sums 0..2: position adjoint (up to four addends a neighbour); 3..5: k_stretch direction
+        float acc = 0.f;
         for (int k = 0; k < 3; ++k) {
             const SetView& v = k == 0 ? vw : (k == 1 ? vs : vb);
             const AdjField& Fj = k == 0 ? fw : (k == 1 ? fs : fb);
             const bool self = k == set;
-            FOR27 {
-                uint32_t s, e;
-                if (!v.range(P, g, ox, oy, oz, s, e)) continue;
-                for (uint32_t j = s; j < e; ++j) {
-                    if (self && j == i) continue;
-                    const float4 q = v.p4[j];
-                    const float3 r = sub3(p, xyz(q));
-                    const float d2 = dot3(r, r);
-                    if (!(d2 < P.h2_lt)) continue;
-                    const float d = sqrtf(d2);
-                    const uint32_t oj = v.gi[j];
-                    const float wj = k == 2 ? P.rho0 * q.w : q.w;
-                    // density: d rho_i/dx_i = w_j Gp(r); d rho_j/dx_i = w_i Gp(r)
-                    xb = add3(xb, sc3(wj * rhob_i + mi * Fj.rhob[oj], G_poly6(P, r, d)));
-                    if (!pbf) continue;
-                    // S through lambda: s_ij^2 Sbar_i + s_ji^2 Sbar_j
-                    {
-                        float sij = P.inv_rho0, sji = P.inv_rho0;
-                        if (k == 2) sij = P.inv_rho0 * ((P.rho0 * q.w) / mi);
-                        const float a = (sij * sij) * Sb_i + (sji * sji) * Fj.Sb[oj];
-                        xb = add3(xb, sc3(a, grad_gsq(P, r, d)));
-                    }
-                    if (set == 0) {
-                        // water: PBF own / coupling / boundary terms
-                        if (k == 0) {
-                            const float cj = X.sph.contrib[oj];
-                            const float3 uj = ldv3(aw.u, oj);
-                            const float a = (ci * cj) * P.inv_rho0 * (lam_i + Fj.lam[oj]);
-                            xb = add3(xb, sc3(a, jv_spiky(P, r, d, sub3(ui, uj))));
-                        } else if (k == 1) {
-                            if (d2 < P.r2_le) {
-                                const float a = ci * P.inv_rho0 * (lam_i + Fj.lam[oj]);
-                                xb = add3(xb, sc3(a, jv_gpoly6(P, r, d, ui)));
-                            }
-                            if (contact && d2 < P.r2_lt) {
-                                // snow particle j pushed by this water particle: -k_st c_j kappa_ji Jc u_j
-                                const float wj_inv = X.dem.massInv[oj];
-                                const float kap = (-wj_inv) * (1.f / (wj_inv + wi_inv));
-                                const float a = -(P.k_stretch * X.dem.contrib[oj]) * kap;
-                                xb = add3(xb, sc3(a, jv_contact(P, r, d, ldv3(as.u, oj), P.two_r)));
-                            }
-                        } else {
+            warp_neighbors<6, 4>(v, p, h, self ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+#pragma unroll
+                for (int q = 0; q < 24; ++q) out[q] = 0.f;
+                const float4 q = __ldg(v.p4 + j);
+                const float3 r = sub3(p, xyz(q));
+                const float d2 = dot3(r, r);
+                const float d = sqrtf(d2);
+                const uint32_t oj = v.gi[j];
+                const float wj = k == 2 ? P.rho0 * q.w : q.w;
+                // density: d rho_i/dx_i = w_j Gp(r); d rho_j/dx_i = w_i Gp(r)
+                put3<4>(out, 0, 0, sc3(wj * rhob_i + mi * Fj.rhob[oj], G_poly6(P, r, d)));
+                if (!pbf) return;
+                // S through lambda: s_ij^2 Sbar_i + s_ji^2 Sbar_j
+                {
+                    float sij = P.inv_rho0, sji = P.inv_rho0;
+                    if (k == 2) sij = P.inv_rho0 * ((P.rho0 * q.w) / mi);
+                    const float a = (sij * sij) * Sb_i + (sji * sji) * Fj.Sb[oj];
+                    put3<4>(out, 0, 1, sc3(a, grad_gsq(P, r, d)));
+                }
+                if (set == 0) {
+                    // water: PBF own / coupling / boundary terms
+                    if (k == 0) {
+                        const float cj = X.sph.contrib[oj];
+                        const float3 uj = ldv3(aw.u, oj);
+                        const float a = (ci * cj) * P.inv_rho0 * (lam_i + Fj.lam[oj]);
+                        put3<4>(out, 0, 2, sc3(a, jv_spiky(P, r, d, sub3(ui, uj))));
+                    } else if (k == 1) {
+                        if (d2 < P.r2_le) {
                             const float a = ci * P.inv_rho0 * (lam_i + Fj.lam[oj]);
-                            xb = add3(xb, sc3(a, jv_spiky(P, r, d, ui)));
+                            put3<4>(out, 0, 2, sc3(a, jv_gpoly6(P, r, d, ui)));
+                        }
+                        if (contact && d2 < P.r2_lt) {
+                            // snow particle j pushed by this water particle: -k_st c_j kappa_ji Jc u_j
+                            const float wj_inv = X.dem.massInv[oj];
+                            const float kap = (-wj_inv) * (1.f / (wj_inv + wi_inv));
+                            const float a = -(P.k_stretch * X.dem.contrib[oj]) * kap;
+                            put3<4>(out, 0, 3, sc3(a, jv_contact(P, r, d, ldv3(as.u, oj), P.two_r)));
                         }
                     } else {
-                        // snow: coupling term of water neighbours, contact terms
-                        if (k == 0) {
-                            if (d2 < P.r2_le) {
-                                const float ck = X.sph.contrib[oj];
-                                const float a = -(ck * P.inv_rho0) * (Fj.lam[oj] + lam_i);
-                                xb = add3(xb, sc3(a, jv_gpoly6(P, r, d, ldv3(aw.u, oj))));
-                            }
-                            if (contact && d2 < P.r2_lt) {
-                                const float wj_inv = X.sph.massInv[oj];
-                                const float kap = (-wi_inv) * (1.f / (wi_inv + wj_inv));
-                                const float a = (P.k_stretch * ci) * kap;
-                                xb = add3(xb, sc3(a, jv_contact(P, r, d, ui, P.two_r)));
-                                kst_dir = add3(kst_dir, sc3(ci * kap, phi_contact(P, r, d)));
-                            }
-                        } else if (k == 1) {
-                            if (d2 < P.r2_lt) {
-                                const float wj_inv = X.dem.massInv[oj];
-                                const float kij = ci * ((-wi_inv) * (1.f / (wi_inv + wj_inv)));
-                                const float kji = X.dem.contrib[oj] * ((-wj_inv) * (1.f / (wj_inv + wi_inv)));
-                                const float3 y = sub3(sc3(kij, ui), sc3(kji, ldv3(as.u, oj)));
-                                xb = add3(xb, jv_contact(P, r, d, y, P.two_r));
-                            }
-                        } else {
-                            if (d2 < P.r2_lt) {
-                                const float wj_inv = X.bnd.massInv[oj];
-                                const float kij = ci * ((-wi_inv) * (1.f / (wi_inv + wj_inv)));
-                                xb = add3(xb, jv_contact(P, r, d, sc3(kij, ui), P.two_r));
-                            }
+                        const float a = ci * P.inv_rho0 * (lam_i + Fj.lam[oj]);
+                        put3<4>(out, 0, 2, sc3(a, jv_spiky(P, r, d, ui)));
+                    }
+                } else {
+                    // snow: coupling term of water neighbours, contact terms
+                    if (k == 0) {
+                        if (d2 < P.r2_le) {
+                            const float ck = X.sph.contrib[oj];
+                            const float a = -(ck * P.inv_rho0) * (Fj.lam[oj] + lam_i);
+                            put3<4>(out, 0, 2, sc3(a, jv_gpoly6(P, r, d, ldv3(aw.u, oj))));
+                        }
+                        if (contact && d2 < P.r2_lt) {
+                            const float wj_inv = X.sph.massInv[oj];
+                            const float kap = (-wi_inv) * (1.f / (wi_inv + wj_inv));
+                            const float a = (P.k_stretch * ci) * kap;
+                            put3<4>(out, 0, 3, sc3(a, jv_contact(P, r, d, ui, P.two_r)));
+                            put3<4>(out, 3, 0, sc3(ci * kap, phi_contact(P, r, d)));
+                        }
+                    } else if (k == 1) {
+                        if (d2 < P.r2_lt) {
+                            const float wj_inv = X.dem.massInv[oj];
+                            const float kij = ci * ((-wi_inv) * (1.f / (wi_inv + wj_inv)));
+                            const float kji = X.dem.contrib[oj] * ((-wj_inv) * (1.f / (wj_inv + wi_inv)));
+                            const float3 y = sub3(sc3(kij, ui), sc3(kji, ldv3(as.u, oj)));
+                            put3<4>(out, 0, 2, jv_contact(P, r, d, y, P.two_r));
+                        }
+                    } else {
+                        if (d2 < P.r2_lt) {
+                            const float wj_inv = X.bnd.massInv[oj];
+                            const float kij = ci * ((-wi_inv) * (1.f / (wi_inv + wj_inv)));
+                            put3<4>(out, 0, 2, jv_contact(P, r, d, sc3(kij, ui), P.two_r));
                         }
                     }
                 }
-            }
+            });
         }
-        st3(Ai.xb, o, add3(ldv3(Ai.xb, o), xb));
-        if (set == 1) kst_acc += dot3(ui, kst_dir);
+        const float3 xb = sum3_of(acc, 0), kst_dir = sum3_of(acc, 3);
+        if (lane == 0u) {
+            st3(Ai.xb, o, add3(ldv3(Ai.xb, o), xb));
+            if (pbf) kst[t] = set == 1 ? dot3(ui, kst_dir) : 0.f;
+        }
     }
-    // k_stretch gradient: warp sum, one atomic per warp
-    for (int s = 16; s > 0; s >>= 1) kst_acc += __shfl_down_sync(0xffffffffu, kst_acc, s);
-    if ((threadIdx.x & 31) == 0 && kst_acc != 0.f) atomicAdd(G.g + 1, (double)kst_acc);
+}
+// Scalar parameter gradients from per-particle values a (and b, when not null): warp sums in
+// float, one double atomic per warp.
+__global__ void ka_param_sum(uint32_t n, const float* __restrict__ a, const float* __restrict__ b, double* ga, double* gb)
+{
+    float x = 0.f, y = 0.f;
+    GRID_LOOP(t, n) {
+        x += a[t];
+        if (b) y += b[t];
+    }
+    for (int s = 16; s > 0; s >>= 1) {
+        x += __shfl_down_sync(0xffffffffu, x, s);
+        y += __shfl_down_sync(0xffffffffu, y, s);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (x != 0.f) atomicAdd(ga, (double)x);
+        if (b && y != 0.f) atomicAdd(gb, (double)y);
+    }
 }
 
 // --------------------------------------------------------------- interlink adjoint
@@ -448,67 +617,58 @@ __device__ __forceinline__ void friction_vjp(const DevParams& P, float3 dx, floa
 }
 // snow particles at the friction pass's positions (sorted view vs) and the start
 // positions after integration x0p; u = sor * adjoint of the positions after friction.
-__global__ void __launch_bounds__(128) ka_friction_rev(DevParams P, uint32_t ns, uint32_t nb, SetView vs, SetView vb,
-                                                       Sets X, AdjSet as)
+__global__ void __launch_bounds__(ADJ_TPB) ka_friction_rev(DevParams P, uint32_t ns, uint32_t nb, SetView vs, SetView vb,
+                                                           Sets X, AdjSet as)
 {
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
     vs.n = ns; vb.n = nb;
-    GRID_LOOP(i, ns) {
+    WARP_LOOP(i, ns) {
         const uint32_t o = vs.gi[i];
         const float3 p = xyz(vs.p4[i]);
-        const GCell g = grid_pos(P, p);
+        const uint32_t h = lane_cell(P, grid_pos(P, p));
         const float3 op0 = ldv3(as.x0p, o);
         const float w0 = X.dem.massInv[o];
         const float3 ui = ldv3(as.u, o);
-        float3 pb = f3(0.f, 0.f, 0.f), x0b = f3(0.f, 0.f, 0.f);
-        FOR27 {
-            uint32_t s, e;
-            if (!vs.range(P, g, ox, oy, oz, s, e)) continue;
-            for (uint32_t j = s; j < e; ++j) {
-                if (j == i) continue;
-                const float3 pp1 = xyz(vs.p4[j]);
-                const float3 r = sub3(p, pp1);
-                const float d2 = dot3(r, r);
-                if (!(d2 < P.r2_le)) continue;
-                const float d = sqrtf(d2);
-                const uint32_t oj = vs.gi[j];
-                const float3 op1 = ldv3(as.x0p, oj);
-                const float w1 = X.dem.massInv[oj];
-                const float3 dx = add3(sub3(p, op0), sub3(pp1, op1));
-                float3 dxb, rb;
-                friction_vjp(P, dx, w0, w1, d, r, ui, dxb, rb);        // term of i
-                pb = add3(pb, add3(dxb, rb));
-                x0b = sub3(x0b, dxb);
-                friction_vjp(P, dx, w1, w0, d, sc3(-1.f, r), ldv3(as.u, oj), dxb, rb);   // term of j
-                pb = add3(pb, sub3(dxb, rb));
-                x0b = sub3(x0b, dxb);
-            }
+        float acc = 0.f;   // sums 0..2: positions, 3..5: start positions; two addends a neighbour
+        warp_neighbors<6, 2>(vs, p, h, i, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+            const float3 pp1 = xyz(__ldg(vs.p4 + j));
+            const float3 r = sub3(p, pp1);
+            const float d = sqrtf(dot3(r, r));
+            const uint32_t oj = vs.gi[j];
+            const float3 op1 = ldv3(as.x0p, oj);
+            const float w1 = X.dem.massInv[oj];
+            const float3 dx = add3(sub3(p, op0), sub3(pp1, op1));
+            float3 dxb, rb;
+            friction_vjp(P, dx, w0, w1, d, r, ui, dxb, rb);        // term of i
+            put3<2>(out, 0, 0, add3(dxb, rb));
+            put3<2>(out, 3, 0, sc3(-1.f, dxb));
+            friction_vjp(P, dx, w1, w0, d, sc3(-1.f, r), ldv3(as.u, oj), dxb, rb);   // term of j
+            put3<2>(out, 0, 1, sub3(dxb, rb));
+            put3<2>(out, 3, 1, sc3(-1.f, dxb));
+        });
+        warp_neighbors<6, 1>(vb, p, h, SNOWB_UMAX, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+            const float3 r = sub3(p, xyz(__ldg(vb.p4 + j)));
+            float3 dxb, rb;
+            friction_vjp(P, sub3(p, op0), w0, X.bnd.massInv[vb.gi[j]], sqrtf(dot3(r, r)), r, ui, dxb, rb);
+            put3<1>(out, 0, 0, add3(dxb, rb));
+            put3<1>(out, 3, 0, sc3(-1.f, dxb));
+        });
+        const float3 pb = sum3_of(acc, 0), x0b = sum3_of(acc, 3);
+        if ((threadIdx.x & 31u) == 0u) {
+            st3(as.xb, o, add3(ldv3(as.xb, o), pb));
+            st3(as.x0b, o, add3(ldv3(as.x0b, o), x0b));
         }
-        FOR27 {
-            uint32_t s, e;
-            if (!vb.range(P, g, ox, oy, oz, s, e)) continue;
-            for (uint32_t j = s; j < e; ++j) {
-                const float3 r = sub3(p, xyz(vb.p4[j]));
-                const float d2 = dot3(r, r);
-                if (!(d2 < P.r2_le)) continue;
-                const float d = sqrtf(d2);
-                float3 dxb, rb;
-                friction_vjp(P, sub3(p, op0), w0, X.bnd.massInv[vb.gi[j]], d, r, ui, dxb, rb);
-                pb = add3(pb, add3(dxb, rb));
-                x0b = sub3(x0b, dxb);
-            }
-        }
-        st3(as.xb, o, add3(ldv3(as.xb, o), pb));
-        st3(as.x0b, o, add3(ldv3(as.x0b, o), x0b));
     }
 }
 
 // -------------------------------------------------------------------- XSPH adjoint
 // XSPH of set A (own) over A and B with velocities vA, vB, viscosity c; gb = adjoint of
-// A's new velocities.  One launch handles both roles: threads [0, nA) are particles of A
-// (own sum: velocity, position and density adjoints), threads [nA, nA + nB) particles of
+// A's new velocities.  One launch handles both roles: warps [0, nA) take particles of A
+// (own sum: velocity, position and density adjoints), warps [nA, nA + nB) particles of
 // B (as neighbours of A).  Outputs are added to vbA/vbB (velocity adjoints), xbA/xbB and
 // rhobA/rhobB.  A's own velocity adjoint keeps its identity term.
-__global__ void __launch_bounds__(128) ka_xsph_rev(DevParams P, uint32_t nA, uint32_t nB, SetView vA, SetView vB,
+__global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA, uint32_t nB, SetView vA, SetView vB,
                                                    const snowb_float3* __restrict__ velA,
                                                    const snowb_float3* __restrict__ velB,
                                                    const float* __restrict__ massA, const float* __restrict__ massB,
@@ -517,75 +677,67 @@ __global__ void __launch_bounds__(128) ka_xsph_rev(DevParams P, uint32_t nA, uin
                                                    snowb_float3* vbA, snowb_float3* vbB, snowb_float3* xbA,
                                                    snowb_float3* xbB, float* rhobA, float* rhobB)
 {
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
     vA.n = nA; vB.n = nB;
-    GRID_LOOP(t, nA + nB) {
+    const uint32_t lane = threadIdx.x & 31u;
+    WARP_LOOP(t, nA + nB) {
         const bool inA = t < nA;
         const uint32_t i = inA ? t : t - nA;
         const SetView& own = inA ? vA : vB;
         const uint32_t o = own.gi[i];
         const float3 p = xyz(own.p4[i]);
-        const GCell g = grid_pos(P, p);
+        const uint32_t h = lane_cell(P, grid_pos(P, p));
         const float3 vi = ldv3(inA ? velA : velB, o);
         const float mi = (inA ? massA : massB)[o], rhoi = (inA ? rhoA : rhoB)[o];
         const float ai = mi / rhoi;
-        float3 vb = f3(0.f, 0.f, 0.f), xb = f3(0.f, 0.f, 0.f);
-        float rb = 0.f;
+        // sums 0..2: positions (two addends a neighbour), 3..5: velocities, 6: density, 7: weights
+        float acc = 0.f;
+        // i as a neighbour of A-particle j: c a_i (v_i - v_j) W, adjoint g_j
+        auto as_neighbor = [&](float* out, int q, uint32_t oj, float3 vj, float3 r, float d, float Wd) {
+            const float3 gj = ldv3(gb, oj);
+            put3<2>(out, 3, 0, sc3(c * ai * Wd, gj));
+            put3<2>(out, 0, q, sc3(c * ai * dot3(sub3(vi, vj), gj), G_poly6(P, r, d)));
+            out[12] = -c * (mi / (rhoi * rhoi)) * Wd * dot3(sub3(vi, vj), gj);
+        };
+        float3 vb;
         if (inA) {
             const float3 gi = ldv3(gb, o);
-            float wsum = 0.f;
+#pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const SetView& v = k == 0 ? vA : vB;
-                FOR27 {
-                    uint32_t s, e;
-                    if (!v.range(P, g, ox, oy, oz, s, e)) continue;
-                    for (uint32_t j = s; j < e; ++j) {
-                        if (k == 0 && j == i) continue;
-                        const float3 r = sub3(p, xyz(v.p4[j]));
-                        const float d2 = dot3(r, r);
-                        if (!(d2 < P.h2_lt)) continue;
-                        const float d = sqrtf(d2);
-                        const uint32_t oj = v.gi[j];
-                        const float3 vj = ldv3(k == 0 ? velA : velB, oj);
-                        const float aj = (k == 0 ? massA : massB)[oj] / (k == 0 ? rhoA : rhoB)[oj];
-                        const float W = W_poly6(P, d);
-                        wsum += aj * W;
-                        // own term: c a_j (v_j - v_i) W(r)
-                        xb = add3(xb, sc3(c * aj * dot3(sub3(vj, vi), gi), G_poly6(P, r, d)));
-                        if (k == 0) {
-                            // i as neighbour j' of A-particle j: c a_i (v_i - v_j) W, adjoint g_j
-                            const float3 gj = ldv3(gb, oj);
-                            vb = add3(vb, sc3(c * ai * W, gj));
-                            xb = add3(xb, sc3(c * ai * dot3(sub3(vi, vj), gj), G_poly6(P, r, d)));
-                            rb += -c * (mi / (rhoi * rhoi)) * W * dot3(sub3(vi, vj), gj);
-                        }
-                    }
-                }
+                warp_neighbors<8, 2>(v, p, h, k == 0 ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+                    for (int q = 0; q < 16; ++q) out[q] = 0.f;
+                    const float3 r = sub3(p, xyz(__ldg(v.p4 + j)));
+                    const float d = sqrtf(dot3(r, r));
+                    const uint32_t oj = v.gi[j];
+                    const float3 vj = ldv3(k == 0 ? velA : velB, oj);
+                    const float aj = (k == 0 ? massA : massB)[oj] / (k == 0 ? rhoA : rhoB)[oj];
+                    const float Wd = W_poly6(P, d);
+                    out[14] = aj * Wd;
+                    // own term: c a_j (v_j - v_i) W(r)
+                    put3<2>(out, 0, 0, sc3(c * aj * dot3(sub3(vj, vi), gi), G_poly6(P, r, d)));
+                    if (k == 0) as_neighbor(out, 1, oj, vj, r, d, Wd);
+                });
             }
-            vb = add3(vb, sc3(1.f - c * wsum, gi));
-            st3(vbA, o, add3(ldv3(vbA, o), vb));
-            st3(xbA, o, add3(ldv3(xbA, o), xb));
-            rhobA[o] += rb;
+            vb = add3(sum3_of(acc, 3), sc3(1.f - c * sum_of(acc, 7), gi));
         } else {
-            FOR27 {
-                uint32_t s, e;
-                if (!vA.range(P, g, ox, oy, oz, s, e)) continue;
-                for (uint32_t j = s; j < e; ++j) {
-                    const float3 r = sub3(p, xyz(vA.p4[j]));
-                    const float d2 = dot3(r, r);
-                    if (!(d2 < P.h2_lt)) continue;
-                    const float d = sqrtf(d2);
-                    const uint32_t oj = vA.gi[j];
-                    const float3 vj = ldv3(velA, oj);
-                    const float3 gj = ldv3(gb, oj);
-                    const float W = W_poly6(P, d);
-                    vb = add3(vb, sc3(c * ai * W, gj));
-                    xb = add3(xb, sc3(c * ai * dot3(sub3(vi, vj), gj), G_poly6(P, r, d)));
-                    rb += -c * (mi / (rhoi * rhoi)) * W * dot3(sub3(vi, vj), gj);
-                }
-            }
-            st3(vbB, o, add3(ldv3(vbB, o), vb));
-            st3(xbB, o, add3(ldv3(xbB, o), xb));
-            rhobB[o] += rb;
+            warp_neighbors<8, 2>(vA, p, h, SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+                for (int q = 0; q < 16; ++q) out[q] = 0.f;
+                const float3 r = sub3(p, xyz(__ldg(vA.p4 + j)));
+                const float d = sqrtf(dot3(r, r));
+                const uint32_t oj = vA.gi[j];
+                as_neighbor(out, 0, oj, ldv3(velA, oj), r, d, W_poly6(P, d));
+            });
+            vb = sum3_of(acc, 3);
+        }
+        const float3 xb = sum3_of(acc, 0);
+        const float rb = sum_of(acc, 6);
+        if (lane == 0u) {
+            snowb_float3 *const vo = inA ? vbA : vbB, *const xo = inA ? xbA : xbB;
+            st3(vo, o, add3(ldv3(vo, o), vb));
+            st3(xo, o, add3(ldv3(xo, o), xb));
+            (inA ? rhobA : rhobB)[o] += rb;
         }
     }
 }
@@ -595,21 +747,24 @@ __global__ void __launch_bounds__(128) ka_xsph_rev(DevParams P, uint32_t nA, uin
 // both sets (fixed quirks).  Tb = adjoint of T1 in, T0b = adjoint of T out; rho-bar and
 // position adjoints added; conductivity gradients accumulated.
 __device__ __forceinline__ float kh(float ki, float kj) { return ((4.f * ki) * kj) / (ki + kj); }
-__global__ void __launch_bounds__(128) ka_heat_rev(DevParams P, uint32_t nw, uint32_t ns, SetView vw, SetView vs,
+__global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw, uint32_t ns, SetView vw, SetView vs,
                                                    Sets X, const float* __restrict__ Tw, const float* __restrict__ Ts,
                                                    const float* __restrict__ Tbw, const float* __restrict__ Tbs,
                                                    float* T0bw, float* T0bs, AdjField fw, AdjField fs, AdjSet aw,
-                                                   AdjSet as, AdjParams G, float dt)
+                                                   AdjSet as, float* __restrict__ gkw_t, float* __restrict__ gks_t,
+                                                       float dt)
 {
+    __shared__ AdjBuf bufs[ADJ_TPB / 32];
+    AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns;
-    float gkw = 0.f, gks = 0.f;
-    GRID_LOOP(t, nw + ns) {
+    const uint32_t lane = threadIdx.x & 31u;
+    WARP_LOOP(t, nw + ns) {
         const int set = t < nw ? 0 : 1;
         const uint32_t i = set == 0 ? t : t - nw;
         const SetView& own = set == 0 ? vw : vs;
         const uint32_t o = own.gi[i];
         const float3 p = xyz(own.p4[i]);
-        const GCell g = grid_pos(P, p);
+        const uint32_t h = lane_cell(P, grid_pos(P, p));
         const float Ti = (set == 0 ? Tw : Ts)[o];
         const float Tbi = (set == 0 ? Tbw : Tbs)[o];
         const float ki = set == 0 ? P.k_water : P.k_snow;
@@ -617,8 +772,8 @@ __global__ void __launch_bounds__(128) ka_heat_rev(DevParams P, uint32_t nw, uin
         const float mi = (set == 0 ? X.sph.mass : X.dem.mass)[o];
         const float rhoi = (set == 0 ? fw.rho : fs.rho)[o];
         const float bi = dt / (Ci * rhoi);
-        float T0b = 0.f, lsum = 0.f, dT = 0.f, rb = 0.f;
-        float3 xb = f3(0.f, 0.f, 0.f);
+        // sums 0: T, 1: weights, 2: dT, 3: density, 4, 5: conductivities, 6..8: positions
+        float acc = 0.f;
         for (int k = 0; k < 2; ++k) {
             const SetView& v = k == 0 ? vw : vs;
             const float kj = k == 0 ? P.k_water : P.k_snow;
@@ -632,53 +787,44 @@ __global__ void __launch_bounds__(128) ka_heat_rev(DevParams P, uint32_t nw, uin
                 dkw = 4.f * P.k_snow * P.k_snow / s2;
                 dks = 4.f * P.k_water * P.k_water / s2;
             }
-            FOR27 {
-                uint32_t s, e;
-                if (!v.range(P, g, ox, oy, oz, s, e)) continue;
-                for (uint32_t j = s; j < e; ++j) {
-                    if (k == set && j == i) continue;
-                    const float3 r = sub3(p, xyz(v.p4[j]));
-                    const float d2 = dot3(r, r);
-                    if (!(d2 < P.h2_lt)) continue;
-                    const float d = sqrtf(d2);
-                    const uint32_t oj = v.gi[j];
-                    const float Tj = (k == 0 ? Tw : Ts)[oj];
-                    const float Tbj = (k == 0 ? Tbw : Tbs)[oj];
-                    const float mj = (k == 0 ? X.sph.mass : X.dem.mass)[oj];
-                    const float rhoj = (k == 0 ? fw.rho : fs.rho)[oj];
-                    const float bj = dt / (Cj * rhoj);
-                    const float L = L_visc(P, d);
-                    const float aij = (mj / rhoj) * kk, aji = (mi / rhoi) * kk;
-                    // temperatures
-                    lsum += aij * L;
-                    T0b += Tbj * bj * aji * L;
-                    dT += aij * (Tj - Ti) * L;
-                    // this particle's density in the neighbour's term
-                    rb += Tbj * bj * (-(mi / (rhoi * rhoi)) * kk) * (Ti - Tj) * L;
-                    // positions through L(d): dL/dx_i = -visc_lap r/d
-                    const float a = Tbi * bi * aij * (Tj - Ti) + Tbj * bj * aji * (Ti - Tj);
-                    if (d > 0.f) xb = add3(xb, sc3(a * (-P.visc_lap) / d, r));
-                    // conductivities (own term only: every pair is counted once per end)
-                    const float q = Tbi * bi * (mj / rhoj) * (Tj - Ti) * L;
-                    gkw += q * dkw;
-                    gks += q * dks;
-                }
-            }
+            warp_neighbors<9, 1>(v, p, h, k == set ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+                const float3 r = sub3(p, xyz(__ldg(v.p4 + j)));
+                const float d = sqrtf(dot3(r, r));
+                const uint32_t oj = v.gi[j];
+                const float Tj = (k == 0 ? Tw : Ts)[oj];
+                const float Tbj = (k == 0 ? Tbw : Tbs)[oj];
+                const float mj = (k == 0 ? X.sph.mass : X.dem.mass)[oj];
+                const float rhoj = (k == 0 ? fw.rho : fs.rho)[oj];
+                const float bj = dt / (Cj * rhoj);
+                const float L = L_visc(P, d);
+                const float aij = (mj / rhoj) * kk, aji = (mi / rhoi) * kk;
+                // temperatures
+                out[1] = aij * L;
+                out[0] = Tbj * bj * aji * L;
+                out[2] = aij * (Tj - Ti) * L;
+                // this particle's density in the neighbour's term
+                out[3] = Tbj * bj * (-(mi / (rhoi * rhoi)) * kk) * (Ti - Tj) * L;
+                // positions through L(d): dL/dx_i = -visc_lap r/d
+                const float a = Tbi * bi * aij * (Tj - Ti) + Tbj * bj * aji * (Ti - Tj);
+                put3<1>(out, 6, 0, d > 0.f ? sc3(a * (-P.visc_lap) / d, r) : f3(0.f, 0.f, 0.f));
+                // conductivities (own term only: every pair is counted once per end)
+                const float q = Tbi * bi * (mj / rhoj) * (Tj - Ti) * L;
+                out[4] = q * dkw;
+                out[5] = q * dks;
+            });
         }
-        T0b += Tbi * (1.f - bi * lsum);
-        rb += -Tbi * (bi / rhoi) * dT;
-        (set == 0 ? T0bw : T0bs)[o] = T0b;
-        (set == 0 ? fw.rhob : fs.rhob)[o] += rb;
-        const AdjSet& A = set == 0 ? aw : as;
-        st3(A.xb, o, add3(ldv3(A.xb, o), xb));
-    }
-    for (int s = 16; s > 0; s >>= 1) {
-        gkw += __shfl_down_sync(0xffffffffu, gkw, s);
-        gks += __shfl_down_sync(0xffffffffu, gks, s);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (gkw != 0.f) atomicAdd(G.g + 2, (double)gkw);
-        if (gks != 0.f) atomicAdd(G.g + 3, (double)gks);
+        const float T0b = sum_of(acc, 0) + Tbi * (1.f - bi * sum_of(acc, 1));
+        const float rb = sum_of(acc, 3) + -Tbi * (bi / rhoi) * sum_of(acc, 2);
+        const float gkw = sum_of(acc, 4), gks = sum_of(acc, 5);
+        const float3 xb = sum3_of(acc, 6);
+        if (lane == 0u) {
+            (set == 0 ? T0bw : T0bs)[o] = T0b;
+            (set == 0 ? fw.rhob : fs.rhob)[o] += rb;
+            const AdjSet& A = set == 0 ? aw : as;
+            st3(A.xb, o, add3(ldv3(A.xb, o), xb));
+            gkw_t[t] = gkw;
+            gks_t[t] = gks;
+        }
     }
 }
 

@@ -1026,10 +1026,11 @@ struct AdjBufs {
     snowb_cell_data cd[2] = {};
     SetBufs sb[2];
     float4* bp4 = nullptr;
-    float *binvm = nullptr, *bmass = nullptr;
+    float *binvm = nullptr, *bmass = nullptr, *brho0 = nullptr, *bS0 = nullptr;   // rho0, S0: sums over the boundary itself
     float* f[3][7] = {};            // rho, C, S, lam, lamb, rhob, Sb
     float *XB[2] = {}, *U[2] = {}, *X0B[2] = {}, *VB[2] = {}, *XBX[2] = {}, *XH[2] = {}, *T0B[2] = {};
     float* GVW = nullptr;
+    float* part[2] = {};            // per-particle parts of the parameter gradients (water, then snow)
     uint32_t* nbuf = nullptr;
     double* gp = nullptr;
     std::vector<void*> bufs;
@@ -1062,7 +1063,9 @@ static int adj_ensure(uint32_t cap, uint32_t bcap, uint32_t ncells)
     for (int s = 0; s < 3; ++s)
         for (int k = 0; k < 7; ++k) TRY(A(&B.f[s][k], s == 2 ? bcap : cap));
     TRY(A(&B.bp4, bcap)); TRY(A(&B.binvm, bcap)); TRY(A(&B.bmass, bcap));
+    TRY(A(&B.brho0, bcap)); TRY(A(&B.bS0, bcap));
     TRY(A(&B.GVW, (size_t)cap * 3));
+    for (float*& q : B.part) TRY(A(&q, 2 * (size_t)cap));
     TRY(A(&B.nbuf, 4)); TRY(A(&B.gp, 4));
     return SNOWB_OK;
 }
@@ -1110,8 +1113,10 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         for (int s = 0; s < 3; ++s) TRY(zero(F[s].rhob, fb[s]));
         return SNOWB_OK;
     };
+    // a warp per water and snow particle, one per 32 boundary particles
+    const uint64_t bwork = 32ull * ((uint64_t)nw + ns + (nb + 31u) / 32u);
     auto fields = [&]() -> int {
-        LAUNCH(ka_fields, nw + ns + nb, 128, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2]);
+        LAUNCH(ka_fields, bwork, ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], B.brho0, B.bS0);
         return SNOWB_OK;
     };
     // 1. fields at the last iteration's input positions (densities read by the XSPH)
@@ -1125,12 +1130,12 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
     for (int s = 0; s < 2; ++s) { TRY(zero(B.VB[s], b3[s])); TRY(zero(B.XBX[s], b3[s])); }
     TRY(dcopy(B.GVW, gv[0], b3[0]));
     if (tp.dem_visc)
-        LAUNCH(ka_xsph_rev, ns + nw, 128, P, ns, nw, vs, vw, F3(T.vf[1]), F3(T.vw1), tp.dem.mass, tp.sph.mass,
+        LAUNCH(ka_xsph_rev, 32ull * (ns + nw), ADJ_TPB, P, ns, nw, vs, vw, F3(T.vf[1]), F3(T.vw1), tp.dem.mass, tp.sph.mass,
                F[1].rho, F[0].rho, P.dem_visc, F3(gv[1]), F3(B.VB[1]), F3(B.GVW), F3(B.XBX[1]), F3(B.XBX[0]),
                F[1].rhob, F[0].rhob);
     else
         TRY(dcopy(B.VB[1], gv[1], b3[1]));
-    LAUNCH(ka_xsph_rev, nw + ns, 128, P, nw, ns, vw, vs, F3(T.vf[0]), F3(T.vf[1]), tp.sph.mass, tp.dem.mass, F[0].rho,
+    LAUNCH(ka_xsph_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, vw, vs, F3(T.vf[0]), F3(T.vf[1]), tp.sph.mass, tp.dem.mass, F[0].rho,
            F[1].rho, P.sph_visc, F3(B.GVW), F3(B.VB[0]), F3(B.VB[1]), F3(B.XBX[0]), F3(B.XBX[1]), F[0].rhob,
            F[1].rhob);
     // 3. finalize: x = x_new, v = (x_new - x0p)/dt
@@ -1146,16 +1151,17 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         if (tp.friction) {
             if (it != last) TRY(sort2(T.xmid[0][it], T.xmid[1][it]));
             LAUNCH(ka_scale3, ns, 256, ns, F3(B.U[1]), P.sor, F3(B.XB[1]));
-            LAUNCH(ka_friction_rev, ns, 128, P, ns, nb, vs, vb, X, AS);
+            LAUNCH(ka_friction_rev, 32ull * ns, ADJ_TPB, P, ns, nb, vs, vb, X, AS);
         }
         if (it == last && tp.friction)
             for (int s = 0; s < 2; ++s) LAUNCH(ka_axpy3, n[s], 256, n[s], F3(B.XB[s]), F3(B.XB[s]), 1.f, F3(B.XBX[s]));
         TRY(sort2(T.xit[0][it], T.xit[1][it]));
         TRY(fields());
         for (int s = 0; s < 2; ++s) LAUNCH(ka_scale3, n[s], 256, n[s], F3(B.U[s]), P.sor, F3(B.XB[s]));
-        LAUNCH(ka_pbf_lambar, nw + ns + nb, 128, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW);
-        LAUNCH(ka_pos_rev, nw + ns, 128, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW, AS, G, 1,
-               tp.correct_dem);
+        LAUNCH(ka_pbf_lambar, bwork, ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW);
+        LAUNCH(ka_pos_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW, AS, B.part[0],
+               1, tp.correct_dem);
+        LAUNCH(ka_param_sum, nw + ns, 128, nw + ns, B.part[0], nullptr, G.g + 1, nullptr);
         if (tp.interlink)
             LAUNCH(ka_interlink_rev, ns, 128, P, ns, F3(T.xit[1][it]), T.rec[it], T.len[it], tp.dem.massInv, AS, G,
                    gL);
@@ -1172,9 +1178,11 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         TRY(fields());
         AdjSet HW{F3(B.XH[0]), F3(B.U[0]), F3(B.X0B[0]), F3(T.x0p[0])};
         AdjSet HS{F3(B.XH[1]), F3(B.U[1]), F3(B.X0B[1]), F3(T.x0p[1])};
-        LAUNCH(ka_heat_rev, nw + ns, 128, P, nw, ns, vw, vs, X, T.T0[0], T.T0[1], gT[0], gT[1], B.T0B[0], B.T0B[1],
-               F[0], F[1], HW, HS, G, tp.dt);
-        LAUNCH(ka_pos_rev, nw + ns, 128, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], HW, HS, G, 0, 0);
+        LAUNCH(ka_heat_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, vw, vs, X, T.T0[0], T.T0[1], gT[0], gT[1], B.T0B[0], B.T0B[1],
+               F[0], F[1], HW, HS, B.part[0], B.part[1], tp.dt);
+        LAUNCH(ka_param_sum, nw + ns, 128, nw + ns, B.part[0], B.part[1], G.g + 2, G.g + 3);
+        LAUNCH(ka_pos_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], HW, HS, B.part[0], 0,
+               0);
         TRY(zero_rhob());
         for (int s = 0; s < 2; ++s) TRY(dcopy(gT[s], B.T0B[s], fb[s]));
     }
@@ -1207,6 +1215,11 @@ static int adjoint_backward(const snowb_adjoint_io* io)
     CUDA_TRY(cudaMemsetAsync(B.gp, 0, 4 * sizeof(double), g_stream));
     LAUNCH(k_boundary_prep, tp.nb, 256, tp.bcd, tp.bnd.volume, tp.bnd.massInv, tp.bnd.mass, tp.nb, B.bp4, B.binvm,
            B.bmass, nullptr, nullptr);
+    {
+        Sets X{tp.sph, tp.dem, tp.bnd};
+        LAUNCH(ka_boundary_base, 32ull * tp.nb, ADJ_TPB, tp.P, tp.nb, make_view(tp.bcd, B.bp4, tp.bnd.volume), X, B.brho0,
+               B.bS0);
+    }
     float* gx[2] = {io->gx_sph, io->gx_dem};
     float* gv[2] = {io->gv_sph, io->gv_dem};
     float* gT[2] = {io->gT_sph, io->gT_dem};
