@@ -72,6 +72,7 @@ struct DevState {
     uint32_t sc_count[8];           // super-cells listed for each link colour (SCList)
     uint32_t clean_hi[2];           // per set: every slot from here on is clean (k_commit_sizes)
     uint32_t base_ready;            // the call's boundary sums (BndBase) are formed
+    uint32_t table_any[2];          // per set: the caller may have written the cell table (no sort since the call began)
 };
 #define SNOWB_DEVERR_SCATTER 1u
 #define SNOWB_DEVERR_SCENE 2u      // a batched scene id >= the scene count

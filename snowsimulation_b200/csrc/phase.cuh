@@ -136,58 +136,73 @@ __device__ __forceinline__ bool compaction_moves(const snowb_particle_data& d, u
 {
     return d.predicate[i] == 1 && d.scan_index[i] != i;
 }
-// copy_to_target (:4451-4460) into the caller's phase-change buffer.  removed: the
-// number of particles the set loses (none: no particle moves)
-__global__ void k_copy_to_buffer(DevParams P, const DevState* __restrict__ S, snowb_particle_data d,
-                                 snowb_particle_data buf, uint32_t full, const uint32_t* __restrict__ sid,
-                                 uint32_t* __restrict__ sid_buf, const uint32_t* __restrict__ removed)
+// The two sets' compactions, side by side in the same launches: the water set through the
+// caller's phase-change buffer, the snow set through the library's.
+struct CompactSide {
+    snowb_particle_data d, buf;
+    uint32_t *sid, *sid_buf;      // scene ids (batched runs) or null
+    const uint32_t* removed;      // the number of particles the set loses (none: no particle moves)
+    int rebase;
+};
+struct CompactPair {
+    CompactSide a[2];
+};
+// copy_to_target (:4451-4460) into the phase-change buffer
+__global__ void k_copy_to_buffer(DevParams P, const DevState* __restrict__ S, const __grid_constant__ CompactPair Q,
+                                 uint32_t full)
 {
-    if (S->changed == 0 || *removed == 0) return;
+    if (S->changed == 0) return;
     const uint32_t M = P.maxc;
-    GRID_LOOP(k, full * (M + 1)) {
-        if (k < full) {
-            if (!compaction_moves(d, k)) continue;
-            copy_fields(d, buf, k, k);
-            if (sid) sid_buf[k] = sid[k];
-        } else {
-            const uint32_t s = k - full;
-            if (!compaction_moves(d, s / M)) continue;
-            buf.connect_record[s] = d.connect_record[s];
-            buf.connect_length[s] = d.connect_length[s];
+#pragma unroll 1
+    for (int set = 0; set < 2; ++set) {
+        const CompactSide& A = Q.a[set];
+        GRID_LOOP(k, *A.removed ? full * (M + 1) : 0u) {
+            if (k < full) {
+                if (!compaction_moves(A.d, k)) continue;
+                copy_fields(A.d, A.buf, k, k);
+                if (A.sid) A.sid_buf[k] = A.sid[k];
+            } else {
+                const uint32_t s = k - full;
+                if (!compaction_moves(A.d, s / M)) continue;
+                A.buf.connect_record[s] = A.d.connect_record[s];
+                A.buf.connect_length[s] = A.d.connect_length[s];
+            }
         }
     }
 }
 // scatter (:4462-4480).  rebase (fixed quirks, snow set): a moved particle keeps its link
 // count, iter_end = t*M + count; the reference copies iter_end verbatim (Q13).  A particle
 // that stays keeps its iter_end either way.
-__global__ void k_scatter_set(DevParams P, DevState* S, snowb_particle_data d, snowb_particle_data buf, uint32_t full,
-                              uint32_t* __restrict__ sid, const uint32_t* __restrict__ sid_buf, int rebase,
-                              const uint32_t* __restrict__ removed)
+__global__ void k_scatter_set(DevParams P, DevState* S, const __grid_constant__ CompactPair Q, uint32_t full)
 {
     if (S->changed == 0) return;
     const uint32_t M = P.maxc;
-    // with nothing removed every kept particle stays: only new_index is written
-    GRID_LOOP(k, *removed ? full * (M + 1) : full) {
-        if (k < full) {
-            const uint32_t i = k;
-            if (d.predicate[i] == 1) {
-                const uint32_t t = d.scan_index[i];
-                if (t >= full) { atomicOr(&S->err, SNOWB_DEVERR_SCATTER); continue; }
-                if (t != i) {
-                    copy_fields(buf, d, i, t);
-                    if (rebase) d.iter_end[t] = M * t + (buf.iter_end[i] - M * i);
-                    if (sid) sid[t] = sid_buf[i];
-                }
-                d.new_index[i] = t;
-            } else d.new_index[i] = SNOWB_UMAX;
-        } else {
-            const uint32_t s = k - full, i = s / M;
-            if (d.predicate[i] != 1) continue;
-            const uint32_t t = d.scan_index[i];
-            if (t >= full || t == i) continue;
-            const uint32_t q = t * M + (s - i * M);
-            d.connect_record[q] = buf.connect_record[s];
-            d.connect_length[q] = buf.connect_length[s];
+#pragma unroll 1
+    for (int set = 0; set < 2; ++set) {
+        const CompactSide& A = Q.a[set];
+        // with nothing removed every kept particle stays: only new_index is written
+        GRID_LOOP(k, *A.removed ? full * (M + 1) : full) {
+            if (k < full) {
+                const uint32_t i = k;
+                if (A.d.predicate[i] == 1) {
+                    const uint32_t t = A.d.scan_index[i];
+                    if (t >= full) { atomicOr(&S->err, SNOWB_DEVERR_SCATTER); continue; }
+                    if (t != i) {
+                        copy_fields(A.buf, A.d, i, t);
+                        if (A.rebase) A.d.iter_end[t] = M * t + (A.buf.iter_end[i] - M * i);
+                        if (A.sid) A.sid[t] = A.sid_buf[i];
+                    }
+                    A.d.new_index[i] = t;
+                } else A.d.new_index[i] = SNOWB_UMAX;
+            } else {
+                const uint32_t s = k - full, i = s / M;
+                if (A.d.predicate[i] != 1) continue;
+                const uint32_t t = A.d.scan_index[i];
+                if (t >= full || t == i) continue;
+                const uint32_t q = t * M + (s - i * M);
+                A.d.connect_record[q] = A.buf.connect_record[s];
+                A.d.connect_length[q] = A.buf.connect_length[s];
+            }
         }
     }
 }
@@ -318,6 +333,13 @@ __device__ __forceinline__ void list_supercell(const DevParams& P, const SCList&
         sc.list[colour * sc.per + atomicAdd(sc.count + colour, 1u)] = t;
 }
 
+// the particles of hash cell h in the current sort: their number and first sorted index (a stale
+// range does not begin with an entry of its own cell)
+__device__ __forceinline__ uint32_t current_range(const SetView& v, uint32_t h, uint32_t& b)
+{
+    b = v.cs[h];
+    return b != SNOWB_EMPTY && b < v.n && v.gh[b] == h ? v.ce[h] - b : 0u;
+}
 // L: the snow-snow candidate lists of the substep's first density pass (L.cnt null: none),
 // replayed instead of the traversal while no phase change re-sorted the sets.
 constexpr uint32_t LF_G = 4;
@@ -744,9 +766,8 @@ __device__ __forceinline__ void link_candidates(const DevParams& P, const SetVie
 // L: the snow-snow candidate lists of the substep's first density pass (L.cnt null: none);
 // they are valid while no phase change re-sorted the sets.
 constexpr uint32_t LINK_TPB = 256, LINK_BATCH = 32, LINK_CAND = 64;
-__global__ void __launch_bounds__(LINK_TPB) k_link_colour_warp(DevParams P, DevState* S, SetView vd,
-                                                               snowb_particle_data dem, const uint32_t* __restrict__ fs,
-                                                               const uint32_t* __restrict__ fe,
+__global__ void __launch_bounds__(LINK_TPB, 3) k_link_colour_warp(DevParams P, DevState* S, SetView vd,
+                                                               snowb_particle_data dem,
                                                                const uint8_t* __restrict__ active, uint32_t colour,
                                                                int dynamic, NList L, SCList sc)
 {
@@ -775,8 +796,7 @@ __global__ void __launch_bounds__(LINK_TPB) k_link_colour_warp(DevParams P, DevS
             if (lane < 8u) {
                 const uint32_t dz = lane >> 2, dy = (lane >> 1) & 1u, dx = lane & 1u;
                 const uint32_t h = ((2u * sz + dz) * P.gsy + (2u * sy + dy)) * P.gsx + (2u * sx + dx);
-                cb = fs[h];
-                cn = fe[h] - cb;
+                cn = current_range(vd, h, cb);
             }
             const uint32_t incl = warp_incl_scan(cn);
             if (lane < 8u) { st[lane] = incl - cn; bs[lane] = cb; }   // first flattened position of each cell
@@ -936,16 +956,15 @@ __device__ void link_particle(const DevParams& P, const SetView& vd, const snowb
     }
 }
 // Link formation's copy of the snow set's sorted view (the arrays its passes read: the
-// sorted copies, grid index and hash, the cell table and the sort's cell offsets), taken
-// after the sort point before it, so that the first iteration's sort point may rewrite the
+// sorted copies, grid index and hash, and the cell table), taken after the sort point before it, so that the first iteration's sort point may rewrite the
 // set's view while link formation runs.  `full` entries of the particle arrays (the
 // caller's arrays hold that many), `ncells` of the cell table.
-__global__ void k_copy_link_view(SetView v, uint32_t full, uint32_t ncells, const uint32_t* __restrict__ off,
-                                 float4* __restrict__ p4, snowb_float3* __restrict__ sp, uint32_t* __restrict__ gi,
+__global__ void k_copy_link_view(SetView v, uint32_t full, uint32_t ncells, float4* __restrict__ p4,
+                                 snowb_float3* __restrict__ sp, uint32_t* __restrict__ gi,
                                  uint32_t* __restrict__ gh, uint32_t* __restrict__ sid, uint32_t* __restrict__ cs,
-                                 uint32_t* __restrict__ ce, uint32_t* __restrict__ off_o)
+                                 uint32_t* __restrict__ ce)
 {
-    const uint32_t m = full > ncells + 1 ? full : ncells + 1;
+    const uint32_t m = full > ncells ? full : ncells;
     GRID_LOOP(k, m) {
         if (k < full) {
             p4[k] = v.p4[k];
@@ -955,13 +974,10 @@ __global__ void k_copy_link_view(SetView v, uint32_t full, uint32_t ncells, cons
             if (v.sid) sid[k] = v.sid[k];
         }
         if (k < ncells) { cs[k] = v.cs[k]; ce[k] = v.ce[k]; }
-        if (k <= ncells) off_o[k] = off[k];
     }
 }
-// one colour: one thread per super-cell of that colour; fs/fe give each hash cell's
-// current (non-stale) sorted range
+// one colour: one thread per super-cell of that colour
 __global__ void k_link_colour(DevParams P, DevState* S, SetView vd, snowb_particle_data dem,
-                              const uint32_t* __restrict__ fs, const uint32_t* __restrict__ fe,
                               const uint8_t* __restrict__ active, uint32_t colour, int dynamic)
 {
     vd.n = S->n_dem;
@@ -975,8 +991,9 @@ __global__ void k_link_colour(DevParams P, DevState* S, SetView vd, snowb_partic
             for (uint32_t dy = 0; dy < 2; ++dy)
                 for (uint32_t dx = 0; dx < 2; ++dx) {
                     const uint32_t h = ((2u * sz + dz) * P.gsy + (2u * sy + dy)) * P.gsx + (2u * sx + dx);
-                    const uint32_t b = fs[h], e = fe[h];
-                    for (uint32_t i = b; i < e; ++i)
+                    uint32_t b = 0;
+                    const uint32_t n = current_range(vd, h, b);
+                    for (uint32_t i = b; i < b + n; ++i)
                         if (active[i]) {
                             if (P.maxc <= SNOWB_MAXC_FAST) link_particle_fast(P, vd, dem, i, dynamic, S);
                             else link_particle(P, vd, dem, i, dynamic, S);

@@ -132,6 +132,7 @@ static int dalloc(T** p, size_t count)
 
 struct SetBufs {
     uint32_t *key = nullptr, *slot = nullptr, *tmp = nullptr, *cnt = nullptr, *off = nullptr, *bsum = nullptr;
+    uint32_t *sup = nullptr, *dirty = nullptr;
     uint32_t* val = nullptr;
     float4* p4 = nullptr;
     float *invm = nullptr, *contrib = nullptr, *lambda = nullptr, *mass = nullptr;
@@ -149,7 +150,6 @@ struct Ctx {
     uint32_t *fl_s = nullptr, *fl_d = nullptr, *rk_s = nullptr, *rk_d = nullptr, *sbsum = nullptr;
     uint8_t* active = nullptr;
     uint32_t *sc_flag = nullptr, *sc_list = nullptr;   // link super-cell lists (SCList)
-    uint32_t *fs = nullptr, *fe = nullptr;
     snowb_float3* tmp_vel = nullptr;
     uint32_t *nl_e = nullptr, *nl_cnt = nullptr;
     uint32_t *nl2_e = nullptr, *nl2_cnt = nullptr;   // the first density pass's snow lists (link formation)
@@ -157,8 +157,7 @@ struct Ctx {
     // precedes it, so that the first iteration's sort may run beside it
     float4* lf_p4 = nullptr;
     snowb_float3* lf_sp = nullptr;
-    uint32_t *lf_gi = nullptr, *lf_gh = nullptr, *lf_sid = nullptr, *lf_cs = nullptr, *lf_ce = nullptr,
-             *lf_off = nullptr;
+    uint32_t *lf_gi = nullptr, *lf_gh = nullptr, *lf_sid = nullptr, *lf_cs = nullptr, *lf_ce = nullptr;
     float4* link_terms = nullptr;         // one interlink term per slot (k_link_terms)
     float4* contact = nullptr;            // two snow contact sums per particle (k_dem_corr<true>)
     // the snow set's phase-change buffer (the caller's serves the water set), so that the two
@@ -185,7 +184,7 @@ static uint64_t g_ctx_gen = 0;   // bumped whenever the scratch buffers are (re)
 static void free_set(SetBufs& s)
 {
     void* ptrs[] = {s.key, s.slot, s.tmp, s.cnt, s.off, s.bsum, s.val, s.p4, s.invm, s.contrib, s.lambda, s.mass,
-                    s.sid, s.base.rho, s.base.gs};
+                    s.sid, s.sup, s.dirty, s.base.rho, s.base.gs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     s = SetBufs();
@@ -195,14 +194,14 @@ static void free_ctx(Ctx& c)
     for (auto& s : c.s) free_set(s);
     free_set(c.b);
     free_set(c.gen);
-    void* ptrs[] = {c.fl_s, c.fl_d, c.rk_s, c.rk_d, c.sbsum, c.active, c.sc_flag, c.sc_list, c.fs, c.fe, c.tmp_vel,
+    void* ptrs[] = {c.fl_s, c.fl_d, c.rk_s, c.rk_d, c.sbsum, c.active, c.sc_flag, c.sc_list, c.tmp_vel,
                     c.epart, c.eout, c.link_terms, c.contact, c.psid,
                     c.pbuf.positions, c.pbuf.predict_positions, c.pbuf.new_positions, c.pbuf.velocity, c.pbuf.force,
                     c.pbuf.correction, c.pbuf.mass, c.pbuf.massInv, c.pbuf.contrib, c.pbuf.density, c.pbuf.C,
                     c.pbuf.lambda, c.pbuf.T, c.pbuf.new_T, c.pbuf.trackId, c.pbuf.iter_end, c.pbuf.connect_record,
                     c.pbuf.connect_length,
                     c.S, c.err_dev, c.nl_e, c.nl_cnt, c.nl2_e, c.nl2_cnt, c.lf_p4, c.lf_sp, c.lf_gi, c.lf_gh,
-                    c.lf_sid, c.lf_cs, c.lf_ce, c.lf_off};
+                    c.lf_sid, c.lf_cs, c.lf_ce};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c.S_host) cudaFreeHost(c.S_host);
@@ -228,6 +227,9 @@ static int alloc_sort(SetBufs& s, uint32_t cap, uint32_t ncells, bool attrs)
     TRY(dalloc(&s.bsum, ncells / SCAN_CHUNK + 2));
     CUDA_TRY(cudaMemset(s.cnt, 0, sizeof(uint32_t) * ncells));
     CUDA_TRY(cudaMemset(s.bsum, 0, sizeof(uint32_t) * (ncells / SCAN_CHUNK + 2)));
+    TRY(dalloc(&s.sup, ncells / SCAN_CHUNK / SUP_CHUNKS + 2)); TRY(dalloc(&s.dirty, ncells / SCAN_CHUNK + 2));
+    CUDA_TRY(cudaMemset(s.sup, 0, sizeof(uint32_t) * (ncells / SCAN_CHUNK / SUP_CHUNKS + 2)));
+    CUDA_TRY(cudaMemset(s.dirty, 0xff, sizeof(uint32_t) * (ncells / SCAN_CHUNK + 2)));
     if (attrs) {
         TRY(dalloc(&s.p4, cap)); TRY(dalloc(&s.invm, cap)); TRY(dalloc(&s.contrib, cap)); TRY(dalloc(&s.lambda, cap));
         TRY(dalloc(&s.sid, cap));
@@ -258,7 +260,6 @@ static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
     TRY(dalloc(&c.active, c.cap));
     TRY(dalloc(&c.sc_flag, ncells / 8 + 1)); TRY(dalloc(&c.sc_list, ncells / 8 + 1));
     CUDA_TRY(cudaMemset(c.sc_flag, 0, sizeof(uint32_t) * (ncells / 8 + 1)));
-    TRY(dalloc(&c.fs, ncells)); TRY(dalloc(&c.fe, ncells));
     TRY(dalloc(&c.tmp_vel, c.cap));
     TRY(dalloc(&c.nl_e, (size_t)NLIST_K * 2 * c.cap));
     TRY(dalloc(&c.nl_cnt, 2 * (size_t)c.cap));
@@ -266,7 +267,7 @@ static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
     TRY(dalloc(&c.nl2_cnt, 2 * (size_t)c.cap));
     TRY(dalloc(&c.lf_p4, c.cap)); TRY(dalloc(&c.lf_sp, c.cap)); TRY(dalloc(&c.lf_gi, c.cap));
     TRY(dalloc(&c.lf_gh, c.cap)); TRY(dalloc(&c.lf_sid, c.cap)); TRY(dalloc(&c.lf_cs, (size_t)c.ncells));
-    TRY(dalloc(&c.lf_ce, (size_t)c.ncells)); TRY(dalloc(&c.lf_off, (size_t)c.ncells + 1));
+    TRY(dalloc(&c.lf_ce, (size_t)c.ncells));
     c.maxc = maxc;
     TRY(dalloc(&c.link_terms, (size_t)c.cap * maxc));
     TRY(dalloc(&c.contact, (size_t)c.cap * 2));
@@ -472,34 +473,31 @@ static void tune_pick(const char* name, uint64_t work, int tpb0, int max_tpb, in
 
 static inline unsigned scan_blocks(uint32_t n) { return (n + SCAN_CHUNK - 1) / SCAN_CHUNK + (n == 0); }
 
-// exclusive scan of in[0, n) (n from the device when n_ptr is set; `cap` bounds it)
-static int scan(const uint32_t* in, const uint32_t* n_ptr, uint32_t n_fixed, uint32_t cap, uint32_t* bsum,
-                uint32_t* out, uint32_t* total, const uint32_t* cond)
+// exclusive scans of two arrays (sizes from the device when n_ptr is set; `cap` bounds them)
+static int scan_pair(const ScanPair& Q, uint32_t cap)
 {
-    const uint32_t nb = scan_blocks(n_ptr ? cap : n_fixed);
-    KL(k_scan_sums, nb, SCAN_TPB, in, n_ptr, n_fixed, bsum, cond);
-    KL(k_scan_apply, nb, SCAN_TPB, in, n_ptr, n_fixed, bsum, out, total, cond);
+    const uint32_t nb = scan_blocks(cap);
+    KL(k_scan_sums, 2 * nb, SCAN_TPB, Q, nb);
+    KL(k_scan_apply, 2 * nb, SCAN_TPB, Q, nb);
     return SNOWB_OK;
 }
 
-// hash + stable sort + reorder of one set (sort_and_reorder :398-420), writing the
-// caller's cell data and the compact sorted copies.  cond: skip unless *cond != 0.
-// gate.S set: a sort point of the substep, which decides for itself whether the set keeps
-// its last sort (cond then points at that decision, DevState::resort)
-static int sort_set(const DevParams& P, SetBufs& B, const snowb_particle_data& D, const snowb_cell_data& cd,
-                    const uint32_t* n_ptr, uint32_t cap, const uint32_t* cond, bool clear_all,
-                    const uint32_t* sid_o = nullptr, SortGate gate = SortGate{nullptr, 0, 0})
+// one set of a sort (sort_and_reorder :398-420): hash + stable sort + reorder, writing the
+// caller's cell data and the compact sorted copies
+static SortSide sort_side(SetBufs& B, const snowb_particle_data& D, const snowb_cell_data& cd, const uint32_t* n,
+                          const uint32_t* sid_o = nullptr)
 {
-    const uint32_t nc = P.ncells;
-    const unsigned nb = (nc + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    // chunk counts come from the hash pass (bsum is all zero between sorts)
-    LAUNCH(k_hash_count, cap, 256, P, D.predict_positions, n_ptr, 0u, B.key, B.slot, B.cnt, cond, sid_o, B.bsum,
-           gate);
-    KL(k_cell_scan, nb, SCAN_TPB, B.cnt, B.bsum, nc, B.off, cd.cell_start, n_ptr, 0u, clear_all ? 1 : 0, cond,
-       gate.S ? &gate.S->moved[gate.set] : nullptr);
-    LAUNCH(k_scatter, cap, 256, B.key, B.slot, B.off, B.tmp, n_ptr, 0u, cond, B.bsum, nb);
-    LAUNCH(k_rank_reorder, cap, 256, B.key, B.off, B.tmp, D.predict_positions, D.mass, D.massInv, D.contrib, cd, B.p4,
-           B.invm, B.contrib, n_ptr, 0u, cond, sid_o, sid_o ? B.sid : nullptr);
+    return SortSide{D.predict_positions, D.mass, D.massInv, D.contrib, n, B.key, B.slot, B.tmp, B.cnt, B.off, B.bsum,
+                    B.sup, B.dirty, sid_o, sid_o ? B.sid : nullptr, cd, B.p4, B.invm, B.contrib};
+}
+// work: particles of the sorted sets together
+static int sort_sets(const DevParams& P, const SortPair& Q, uint64_t work)
+{
+    const unsigned chunks = (P.ncells + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    LAUNCH(k_sort_hash, work, 256, P, Q);
+    KL(k_sort_scan, 2 * chunks, SCAN_TPB, Q, chunks);
+    LAUNCH(k_sort_scatter, work, 256, Q, chunks);
+    LAUNCH(k_sort_rank, work, 256, Q);
     return SNOWB_OK;
 }
 
@@ -681,13 +679,6 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     bool dirty_s = true, dirty_d = true;
     auto track = [&](int set) { return SortTrack{c.s[set].key, set ? a.sid_dem : a.sid_sph, &S->moved[set]}; };
     const SortTrack track_s = track(0), track_d = track(1);
-    // a sort point of one set: the full sort when the set moved, else only the refresh of the
-    // gathered outputs
-    auto sort_if = [&](int set, bool begin) -> int {
-        TRY(sort_set(P, c.s[set], set ? *a.dem : *a.sph, set ? a.dcd : a.scd, set ? n_d : n_s, cap, &S->resort[set],
-                     !ref, set ? a.sid_dem : a.sid_sph, SortGate{S, set, begin ? 1 : 0}));
-        return SNOWB_OK;
-    };
     // launches on a side stream forked from the main one; join_side makes the main stream
     // wait for them
     auto on_side = [&](cudaStream_t st, cudaEvent_t ev, auto&& launch) -> int {
@@ -709,40 +700,24 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // contact passes, so they run beside them on the side streams when the substep runs
     // whole (a stage stop keeps every launch on the main stream).
     const bool beside = a.stop_after == 0;
-    // The two sets' sorts share no buffer: the water sort runs on a side stream beside the
-    // snow sort (a fork and a join of the captured graph), so the small set's chain of
-    // latency-bound launches overlaps the large one's.  after_phase: the sort point after
+    // A sort point sorts both sets in the same launches.  after_phase: the sort point after
     // the phase change, where only a compaction (which marks both sets moved) alters the
-    // result.
-    // begin: the substep's first sort point, whose snow hash pass also opens the substep
+    // result.  begin: the substep's first sort point, whose hash pass also opens the substep
     // (both sets are dirty there)
-    // defer_water: the friction sort point, whose passes read no water data: its water sort
-    // stays on the side stream beside the friction and apply passes, joined by the next
-    // sort point or by join_water
-    bool water_pending = false;
-    auto join_water = [&]() -> int {
-        if (water_pending) TRY(join_side(c.side, c.join));
-        water_pending = false;
-        return SNOWB_OK;
-    };
     // link formation beside the integration and the first iteration (see below): the snow
     // sort waits for link formation's copy of the snow view, the first interlink terms for
     // the links
     bool view_pending = false, links_pending = false;
-    auto sort_pair = [&](bool after_phase, bool begin = false, bool defer_water = false) -> int {
-        TRY(join_water());
+    auto sort_pair = [&](bool after_phase, bool begin = false) -> int {
         const bool need_s = dirty_s || after_phase, need_d = dirty_d || after_phase;
         if (!need_s && !need_d) return SNOWB_OK;
-        if (need_s) TRY(on_side(c.side, c.fork, [&]() { return sort_if(0, false); }));
         if (need_d && view_pending) {
             CUDA_TRY(cudaStreamWaitEvent(g_stream, c.ev_view, 0));
             view_pending = false;
         }
-        if (need_d) TRY(sort_if(1, begin));
-        if (need_s) {
-            if (defer_water) water_pending = true;
-            else TRY(join_side(c.side, c.join));
-        }
+        const SortPair Q{{sort_side(c.s[0], *a.sph, a.scd, n_s, a.sid_sph), sort_side(c.s[1], *a.dem, a.dcd, n_d, a.sid_dem)},
+                         {need_s ? 1 : 0, need_d ? 1 : 0}, S, begin ? 1 : 0, P.ncells, ref ? 0 : 1};
+        TRY(sort_sets(P, Q, full));
         dirty_s = dirty_d = false;
         return SNOWB_OK;
     };
@@ -775,46 +750,20 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     if (a.change_phase) {
         LAUNCH(k_phase_flags, 2 * full, 256, P, S, *a.sph, *a.dem, a.freezing, a.melting, c.fl_s, c.fl_d,
                commit_in_flags, a.dTe, step_sph ? 1 : 0, step_dem ? 1 : 0);
-        const uint32_t sb_stride = cap / SCAN_CHUNK + 2;
-        // the two sets' scans share nothing: in a whole substep the snow set's runs beside
-        auto scan_pair = [&](auto&& scan_s, auto&& scan_d) -> int {
-            if (beside) {
-                TRY(on_side(c.side, c.fork, scan_d));
-                TRY(scan_s());
-                TRY(join_side(c.side, c.join));
-            } else {
-                TRY(scan_s());
-                TRY(scan_d());
-            }
-            return SNOWB_OK;
-        };
-        TRY(scan_pair([&]() { return scan(c.fl_s, n_s, 0, cap, c.sbsum, c.rk_s, &S->n_freeze, nullptr); },
-                      [&]() { return scan(c.fl_d, n_d, 0, cap, c.sbsum + sb_stride, c.rk_d, &S->n_melt, nullptr); }));
+        uint32_t *const bs0 = c.sbsum, *const bs1 = c.sbsum + cap / SCAN_CHUNK + 2;
+        TRY(scan_pair(ScanPair{{{c.fl_s, n_s, 0u, bs0, c.rk_s, &S->n_freeze}, {c.fl_d, n_d, 0u, bs1, c.rk_d, &S->n_melt}}},
+                      full));
         LAUNCH(k_phase_move, 2 * full, 256, P, S, *a.sph, *a.dem, c.fl_s, c.rk_s, c.fl_d, c.rk_d, scn);
         // compact_and_clean (:4495-4589): predicate scans run every substep (they define
         // scan_index), the data movement only after a phase change.
-        TRY(scan_pair(
-            [&]() { return scan(a.sph->predicate, nullptr, full, full, c.sbsum, a.sph->scan_index, &S->new_sph, nullptr); },
-            [&]() {
-                return scan(a.dem->predicate, nullptr, full, full, c.sbsum + sb_stride, a.dem->scan_index, &S->new_dem,
-                            nullptr);
-            }));
-        const uint64_t cw = (uint64_t)full * (P.maxc + 1);   // a thread per particle and per link slot
-        // the water set loses the freezing particles, the snow set the melting ones; in a whole
-        // substep the water set compacts through the caller's buffer beside the snow set
-        // compacting through the library's
-        auto compact_water = [&]() -> int {
-            LAUNCH(k_copy_to_buffer, cw, 256, P, S, *a.sph, *a.buf, full, scn.sph, scn.buf, &S->n_freeze);
-            LAUNCH(k_scatter_set, cw, 256, P, S, *a.sph, *a.buf, full, scn.sph, scn.buf, 0, &S->n_freeze);
-            return SNOWB_OK;
-        };
-        const snowb_particle_data& dbuf = beside ? c.pbuf : *a.buf;
-        uint32_t* dsid = beside ? c.psid : scn.buf;
-        if (beside) TRY(on_side(c.side, c.fork, compact_water));
-        else TRY(compact_water());
-        LAUNCH(k_copy_to_buffer, cw, 256, P, S, *a.dem, dbuf, full, scn.dem, dsid, &S->n_melt);
-        LAUNCH(k_scatter_set, cw, 256, P, S, *a.dem, dbuf, full, scn.dem, dsid, ref ? 0 : 1, &S->n_melt);
-        if (beside) TRY(join_side(c.side, c.join));
+        TRY(scan_pair(ScanPair{{{a.sph->predicate, nullptr, full, bs0, a.sph->scan_index, &S->new_sph},
+                                {a.dem->predicate, nullptr, full, bs1, a.dem->scan_index, &S->new_dem}}}, full));
+        // the water set loses the freezing particles, the snow set the melting ones; a thread
+        // per particle and per link slot of each set
+        const CompactPair cp{{{*a.sph, *a.buf, scn.sph, scn.buf, &S->n_freeze, 0},
+                              {*a.dem, c.pbuf, scn.dem, c.psid, &S->n_melt, ref ? 0 : 1}}};
+        LAUNCH(k_copy_to_buffer, (uint64_t)full * (P.maxc + 1), 256, P, S, cp, full);
+        LAUNCH(k_scatter_set, (uint64_t)full * (P.maxc + 1), 256, P, S, cp, full);
         LAUNCH(k_compact_finish, 2 * full + (uint64_t)P.maxc * full, 256, P, S, *a.sph, *a.dem, full, 1);
         LAUNCH1(k_commit_sizes, S);
     }
@@ -825,16 +774,16 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     STOP(5);
     if (a.interlink) {
         // link formation over a view of the snow set: the set's own, or its copy
-        auto form = [&](const SetView& v, const uint32_t* off) -> int {
+        auto form = [&](const SetView& v) -> int {
             const SCList scl = sc_lists(P);
             TLAUNCH(k_link_filter, 256, full, 128, P, S, v, *a.dem, a.dynamic, c.active, NL2, scl);
             const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);   // super-cells per colour
             for (uint32_t col = 0; col < 8; ++col) {
                 if (P.maxc <= SNOWB_MAXC_FAST)
                     TLAUNCH(k_link_colour_warp, LINK_TPB, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, S, v, *a.dem,
-                            off, off + 1, c.active, col, a.dynamic, NL2, scl);
+                            c.active, col, a.dynamic, NL2, scl);
                 else
-                    TLAUNCH(k_link_colour, 128, nsc, 64, P, S, v, *a.dem, off, off + 1, c.active, col, a.dynamic);
+                    TLAUNCH(k_link_colour, 128, nsc, 64, P, S, v, *a.dem, c.active, col, a.dynamic);
             }
             if (a.dynamic) LAUNCH1(k_adjust_links, P, S, *a.dem, full);
             return SNOWB_OK;
@@ -850,16 +799,16 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
             vl.p4 = c.lf_p4; vl.sp = c.lf_sp; vl.gi = c.lf_gi; vl.gh = c.lf_gh; vl.cs = c.lf_cs; vl.ce = c.lf_ce;
             vl.sid = vd.sid ? c.lf_sid : nullptr;
             TRY(on_side(c.side4, c.fork4, [&]() -> int {
-                LAUNCH(k_copy_link_view, (full > P.ncells + 1 ? full : P.ncells + 1), 256, vd, full, P.ncells,
-                       c.s[1].off, c.lf_p4, c.lf_sp, c.lf_gi, c.lf_gh, c.lf_sid, c.lf_cs, c.lf_ce, c.lf_off);
+                LAUNCH(k_copy_link_view, (full > P.ncells ? full : P.ncells), 256, vd, full, P.ncells, c.lf_p4, c.lf_sp,
+                       c.lf_gi, c.lf_gh, c.lf_sid, c.lf_cs, c.lf_ce);
                 CUDA_TRY(cudaEventRecord(c.ev_view, g_stream));
-                TRY(form(vl, c.lf_off));
+                TRY(form(vl));
                 CUDA_TRY(cudaEventRecord(c.ev_links, g_stream));
                 return SNOWB_OK;
             }));
             view_pending = links_pending = true;
         } else {
-            TRY(form(vd, c.s[1].off));
+            TRY(form(vd));
         }
     }
     STOP(6);
@@ -942,7 +891,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         TAPE_HOOK(3, it);
         STOP(base + 6);
         if (a.friction && step_dem) {
-            TRY(sort_pair(false, false, beside));
+            TRY(sort_pair(false));
             // a whole substep applies the friction correction in the friction pass itself
             if (beside) {
                 TLAUNCH(k_friction<true>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, track_d);
@@ -954,7 +903,6 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         }
         STOP(base + 7);
     }
-    TRY(join_water());
     if (step_sph || step_dem)
         LAUNCH(k_finalize, 2 * full, 256, P, S, X, a.dt, step_sph ? 1 : 0, step_dem ? 1 : 0);
     TAPE_HOOK(4, 0);
@@ -1089,7 +1037,7 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
     Tape& tp = g_tape;
     AdjBufs& B = g_adj;
     const DevParams& P = tp.P;
-    const uint32_t n[2] = {tp.n[0], tp.n[1]}, nw = n[0], ns = n[1], nb = tp.nb, cap = B.cap;
+    const uint32_t n[2] = {tp.n[0], tp.n[1]}, nw = n[0], ns = n[1], nb = tp.nb;
     const size_t b3[2] = {(size_t)nw * 12, (size_t)ns * 12};
     const int last = tp.iterations - 1;
     Sets X{tp.sph, tp.dem, tp.bnd};
@@ -1105,8 +1053,8 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         snowb_particle_data dw = tp.sph, ds = tp.dem;
         dw.predict_positions = const_cast<snowb_float3*>(F3(pw));
         ds.predict_positions = const_cast<snowb_float3*>(F3(ps));
-        TRY(sort_set(P, B.sb[0], dw, B.cd[0], B.nbuf + 0, cap, nullptr, true));
-        TRY(sort_set(P, B.sb[1], ds, B.cd[1], B.nbuf + 1, cap, nullptr, true));
+        TRY(sort_sets(P, SortPair{{sort_side(B.sb[0], dw, B.cd[0], B.nbuf + 0), sort_side(B.sb[1], ds, B.cd[1], B.nbuf + 1)},
+                                  {1, 1}, nullptr, 0, P.ncells, 1}, (uint64_t)nw + ns));
         return SNOWB_OK;
     };
     auto zero_rhob = [&]() -> int {
@@ -1503,9 +1451,8 @@ static int sort_pairs(uint32_t nc, snowb_cell_data cd, uint32_t n)
     LAUNCH(k_key_count, n, 256, cd.grid_hash, cd.grid_index, n, nc, B.key, B.val, B.slot, B.cnt, g_ctx.err_dev);
     const unsigned nb = (nc + SCAN_CHUNK - 1) / SCAN_CHUNK;
     KL(k_block_sums, nb, SCAN_TPB, B.cnt, nc, B.bsum, nullptr);
-    // cell_start is not touched by a plain sort: clear nothing (clear_all = 0, n = 0)
-    KL(k_cell_scan, nb, SCAN_TPB, B.cnt, B.bsum, nc, B.off, nullptr, nullptr, 0u, 0, nullptr);
-    LAUNCH(k_scatter, n, 256, B.key, B.slot, B.off, B.tmp, nullptr, n, nullptr);
+    KL(k_cell_scan, nb, SCAN_TPB, B.cnt, B.bsum, nc, B.off);
+    LAUNCH(k_scatter, n, 256, B.key, B.slot, B.off, B.tmp, n);
     LAUNCH(k_rank_pairs, n, 256, B.key, B.val, B.off, B.tmp, cd.grid_hash, cd.grid_index, n);
     uint32_t err = 0;
     CUDA_TRY(cudaMemcpyAsync(&err, g_ctx.err_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, g_stream));
@@ -1546,9 +1493,6 @@ static int connect_links(const DevParams& P, snowb_particle_data* dem, uint32_t 
     TRY(ensure_ctx(g_ctx.cap > n ? g_ctx.cap : n, g_ctx.bcap ? g_ctx.bcap : 1, P.ncells));
     Ctx& c = g_ctx;
     LAUNCH1(k_set_state, c.S, 0u, n, 0u);
-    CUDA_TRY(cudaMemsetAsync(c.fs, 0, sizeof(uint32_t) * P.ncells, g_stream));
-    CUDA_TRY(cudaMemsetAsync(c.fe, 0, sizeof(uint32_t) * P.ncells, g_stream));
-    LAUNCH(k_fresh_ranges, n, 256, dcd.grid_hash, n, c.fs, c.fe);
     // the view's compact copy (and sorted scene ids) are filled from sorted_pos
     LAUNCH(k_boundary_prep, n, 256, dcd, dem->mass, dem->massInv, dem->mass, n, c.s[1].p4, c.s[1].invm, c.s[1].lambda,
            sid, sid ? c.s[1].sid : nullptr);
@@ -1558,10 +1502,10 @@ static int connect_links(const DevParams& P, snowb_particle_data* dem, uint32_t 
     const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);
     for (uint32_t col = 0; col < 8; ++col) {
         if (P.maxc <= SNOWB_MAXC_FAST)
-            LAUNCH(k_link_colour_warp, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, c.S, vd, *dem, c.fs, c.fe,
+            LAUNCH(k_link_colour_warp, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, c.S, vd, *dem,
                    c.active, col, dynamic, NList{nullptr, nullptr, 0u, 0u}, scl);
         else
-            LAUNCH(k_link_colour, nsc, 64, P, c.S, vd, *dem, c.fs, c.fe, c.active, col, dynamic);
+            LAUNCH(k_link_colour, nsc, 64, P, c.S, vd, *dem, c.active, col, dynamic);
     }
     CUDA_TRY(cudaStreamSynchronize(g_stream));
     return SNOWB_OK;
@@ -1705,8 +1649,8 @@ int snowb_sort_particles_static(snowb_cell_data cd, uint32_t n)
     const unsigned nb = (nc + SCAN_CHUNK - 1) / SCAN_CHUNK;
     KL_PLAIN(k_key_count, blocks_for(n, 256), 256, cd.grid_hash, cd.grid_index, n, nc, key, val, slot, cnt, err);
     KL_PLAIN(k_block_sums, nb, SCAN_TPB, cnt, nc, bsum, nullptr);
-    KL_PLAIN(k_cell_scan, nb, SCAN_TPB, cnt, bsum, nc, off, nullptr, nullptr, 0u, 0, nullptr);
-    KL_PLAIN(k_scatter, blocks_for(n, 256), 256, key, slot, off, tmp, nullptr, n, nullptr);
+    KL_PLAIN(k_cell_scan, nb, SCAN_TPB, cnt, bsum, nc, off);
+    KL_PLAIN(k_scatter, blocks_for(n, 256), 256, key, slot, off, tmp, n);
     KL_PLAIN(k_rank_pairs, blocks_for(n, 256), 256, key, val, off, tmp, cd.grid_hash, cd.grid_index, n);
     uint32_t herr = 0;
     CUDA_TRY(cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, g_stream));

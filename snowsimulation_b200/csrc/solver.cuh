@@ -1600,7 +1600,7 @@ __global__ void k_set_state(DevState* S, uint32_t ns, uint32_t nd, uint32_t nb)
         // of a call cleans the tail as the reference's does every substep
         S->tail_dirty = 1u;
         // ... and the particles: the first sort point of a call sorts both sets in full
-        for (int k = 0; k < 2; ++k) { S->moved[k] = 1u; S->sorts_full[k] = 0u; S->sorts_kept[k] = 0u; }
+        for (int k = 0; k < 2; ++k) { S->moved[k] = 1u; S->table_any[k] = 1u; S->sorts_full[k] = 0u; S->sorts_kept[k] = 0u; }
         for (int c = 0; c < 8; ++c) S->sc_count[c] = 0u;
         S->clean_hi[0] = SNOWB_UMAX; S->clean_hi[1] = SNOWB_UMAX;
         S->base_ready = 0u;   // ... and the boundary

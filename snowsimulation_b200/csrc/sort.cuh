@@ -6,7 +6,7 @@
 // permutation:
 //   1. hash + count: each particle's cell key, and an (unordered) slot in its cell
 //      from an atomic counter;
-//   2. exclusive scan of the per-cell counts (num_cells + 1 offsets); the same pass
+//   2. exclusive scan of the per-cell counts of the occupied scan chunks; the same pass
 //      re-zeroes the counters and clears cell_start over the range the reference clears;
 //   3. scatter each particle into its cell's range (unordered inside the cell);
 //   4. rank inside the cell by original index (cells hold a handful of particles),
@@ -67,18 +67,44 @@ __device__ __forceinline__ uint32_t prefix_of_blocks(const uint32_t* bsum, uint3
     return warp_sum(s);
 }
 
-// ------------------------------------------------------------------ 1. hash + count
-// Fused path: hash of pos[o] for o < n (calcHashD :194-212).  Also adds every particle to
-// the count of its scan chunk (bsum, SCAN_CHUNK cells each, one atomic per chunk and warp),
-// which the cell scan needs; the scatter pass re-zeroes bsum for the next sort.
-// Sort points of a substep decide for themselves (gate.S set): the hash pass turns the
-// set's moved flag into the decision (DevState::resort, read by the later passes; the scan
-// pass clears the flag), and returns at once when the set keeps its last sort.  The first
-// sort point of a substep also opens it (begin).  gate.S null: `cond` alone decides.
-struct SortGate {
-    DevState* S;
-    int set, begin;
+// One or two sets sorted by the same four launches (the water and the snow set of a sort
+// point): the particle passes run over both sets' particles end to end, the scan over both
+// cell tables.  Two chains of launches on two streams, forked and joined at each sort point,
+// were 56 launches and 32 event calls a substep; these are 28 launches (issuing a substep: 330 ->
+// 230 us of host time; one substep of 208 particles 512 -> 480 us).
+struct SortSide {
+    const snowb_float3* pos;
+    const float *w, *invm, *contrib;      // mass, massInv, contrib by original index
+    const uint32_t* n;                    // set size (device)
+    uint32_t *key, *slot, *tmp, *cnt, *off;
+    uint32_t *bsum, *sup;                 // particles per scan chunk, and per SUP_CHUNKS chunks; zero between sorts
+    uint32_t* dirty;                      // per scan chunk: its part of cell_start may hold entries
+    const uint32_t* sid_o;                // scene ids by original index (batched runs) or null
+    uint32_t* sid_s;
+    snowb_cell_data cd;
+    float4* p4;
+    float *invm_s, *contrib_s;
 };
+struct SortPair {
+    SortSide a[2];
+    int on[2];                            // set k is sorted
+    // A sort point of the substep decides for itself (S set): the hash pass turns a set's moved
+    // flag into the decision (DevState::resort, read by the later passes; the scan pass clears the
+    // flag); a set that keeps its last sort only has its gathered outputs refreshed.  The first
+    // sort point of a substep also opens it (begin).  S null: both sets sort in full.
+    DevState* S;
+    int begin;
+    uint32_t ncells;
+    int clear_all;
+    __device__ __forceinline__ bool sorts(int k) const { return on[k] && (!S || S->resort[k] != 0u); }
+    __device__ __forceinline__ uint32_t size(int k) const { return on[k] ? *a[k].n : 0u; }
+};
+constexpr uint32_t SUP_CHUNKS = 64;       // scan chunks per entry of `sup`, used past SUP_MIN chunks
+constexpr uint32_t SUP_MIN = 1024;
+
+// ------------------------------------------------------------------ 1. hash + count
+// Hash of pos[o] (calcHashD :194-212) and its cell's and scan chunk's counts (one chunk atomic
+// per chunk and warp), which the cell scan needs; the scatter pass re-zeroes the chunk counts.
 // substep start: launch sizes, phase-change and link counters
 __device__ __forceinline__ void begin_substep(DevState* S)
 {
@@ -86,38 +112,43 @@ __device__ __forceinline__ void begin_substep(DevState* S)
     S->n_freeze = 0; S->n_melt = 0; S->changed = 0; S->n_active = 0; S->n_links = 0; S->n_nl_ovf = 0;
     for (int c = 0; c < 8; ++c) S->sc_count[c] = 0u;
 }
-__global__ void k_hash_count(DevParams P, const snowb_float3* __restrict__ pos, const uint32_t* n_ptr,
-                             uint32_t n_fixed, uint32_t* __restrict__ key_o, uint32_t* __restrict__ slot_o,
-                             uint32_t* __restrict__ cnt, const uint32_t* cond, const uint32_t* __restrict__ sid_o,
-                             uint32_t* __restrict__ bsum, SortGate gate)
+__global__ void k_sort_hash(DevParams P, const __grid_constant__ SortPair Q)
 {
-    if (gate.S) {
-        const uint32_t m = gate.S->moved[gate.set];
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            if (gate.begin) begin_substep(gate.S);
-            gate.S->resort[gate.set] = m;
-            if (m) ++gate.S->sorts_full[gate.set];
-            else ++gate.S->sorts_kept[gate.set];
-        }
-        if (m == 0) return;
-    } else if (cond && *cond == 0) return;
-    const uint32_t n = n_ptr ? *n_ptr : n_fixed;
+    uint32_t m[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) m[k] = !Q.on[k] ? 0u : (Q.S ? Q.S->moved[k] : 1u);
+    if (Q.S && blockIdx.x == 0 && threadIdx.x == 0) {
+        if (Q.begin) begin_substep(Q.S);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (Q.on[k]) {
+                Q.S->resort[k] = m[k];
+                if (m[k]) ++Q.S->sorts_full[k];
+                else ++Q.S->sorts_kept[k];
+            }
+    }
+    const uint32_t n0 = m[0] ? Q.size(0) : 0u, n = n0 + (m[1] ? Q.size(1) : 0u);
     const uint32_t lane = threadIdx.x & 31u;
     // whole warps iterate together so the chunk counts can be aggregated with warp votes
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        const uint32_t o = base + lane;
-        const bool live = o < n;
+        const uint32_t t = base + lane;
+        const int k = t < n0 ? 0 : 1;
+        const SortSide& A = Q.a[k];
+        const uint32_t o = k ? t - n0 : t;
+        const bool live = t < n;
         uint32_t chunk = 0xFFFFFFFFu;
         if (live) {
-            float3 p = ldv3(pos, o);
-            uint32_t h = grid_hash(P, grid_pos(P, p, sid_o ? sid_o[o] : 0u), 0, 0, 0);
-            key_o[o] = h;
-            slot_o[o] = atomicAdd(cnt + h, 1u);
+            const uint32_t h = grid_hash(P, grid_pos(P, ldv3(A.pos, o), A.sid_o ? A.sid_o[o] : 0u), 0, 0, 0);
+            A.key[o] = h;
+            A.slot[o] = atomicAdd(A.cnt + h, 1u);
             chunk = h / (uint32_t)SCAN_CHUNK;
         }
-        const uint32_t peers = __match_any_sync(0xffffffffu, chunk);
-        if (live && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(bsum + chunk, (uint32_t)__popc(peers));
+        const uint32_t peers = __match_any_sync(0xffffffffu, chunk | (uint32_t)k << 30);
+        if (live && lane == (uint32_t)(__ffs(peers) - 1)) {
+            atomicAdd(A.bsum + chunk, (uint32_t)__popc(peers));
+            if (Q.ncells > SUP_MIN * SCAN_CHUNK) atomicAdd(A.sup + chunk / SUP_CHUNKS, (uint32_t)__popc(peers));
+        }
     }
 }
 // sort_particles path: keys and values already in (grid_hash, grid_index).
@@ -155,25 +186,14 @@ __global__ void k_block_sums(const uint32_t* __restrict__ cnt, uint32_t ncells, 
     }
 }
 
-// off[c] = exclusive prefix of cnt; off[ncells] = total; cnt re-zeroed; cell_start cleared
-// for c < clear (clear = min(n, ncells) reproduces the reference's partial memset, Q1).
-// moved: the set's moved flag, cleared here once the hash pass has read it (null: none)
-__global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restrict__ bsum, uint32_t ncells,
-                            uint32_t* __restrict__ off, uint32_t* __restrict__ cell_start,
-                            const uint32_t* n_ptr, uint32_t n_fixed, int clear_all, const uint32_t* cond,
-                            uint32_t* moved = nullptr)
+// off[c] = exclusive prefix of cnt (c <= ncells), cnt re-zeroed, for the scan chunk `chunk` whose
+// particles come after `prefix` others; cells from `clear` on keep their cell_start (null: none
+// is cleared)
+__device__ __forceinline__ void scan_chunk(uint32_t* __restrict__ cnt, uint32_t ncells, uint32_t* __restrict__ off,
+                                           uint32_t* __restrict__ cell_start, uint32_t clear, uint32_t chunk,
+                                           uint32_t prefix, uint32_t* sm)
 {
-    if (moved && blockIdx.x == 0 && threadIdx.x == 0) *moved = 0u;
-    if (cond && *cond == 0) return;
-    __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
-    __shared__ uint32_t s_prefix;
-    if (threadIdx.x < 32) {
-        uint32_t p = prefix_of_blocks(bsum, blockIdx.x);
-        if (threadIdx.x == 0) s_prefix = p;
-    }
-    const uint32_t n = n_ptr ? *n_ptr : n_fixed;
-    const uint32_t clear = clear_all ? ncells : umin32(n, ncells);
-    const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
+    const uint32_t base = chunk * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS], t = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
@@ -181,31 +201,98 @@ __global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restri
         t += v[k];
     }
     uint32_t total;
-    __syncthreads();
-    uint32_t ex = block_excl_scan(t, sm, total) + s_prefix;
+    uint32_t ex = block_excl_scan(t, sm, total) + prefix;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
-        uint32_t c = base + k;
+        const uint32_t c = base + k;
         if (c < ncells) {
             off[c] = ex;
             cnt[c] = 0u;
-            if (c < clear) cell_start[c] = SNOWB_EMPTY;
-            if (c == ncells - 1) off[ncells] = ex + v[k];
+            if (cell_start && c < clear) cell_start[c] = SNOWB_EMPTY;
+            // the chunk's end: the next chunk, if it is walked, writes the same value
+            if (c == ncells - 1 || (k == SCAN_ITEMS - 1 && threadIdx.x == SCAN_TPB - 1)) off[c + 1] = ex + v[k];
         }
         ex += v[k];
     }
 }
+// sort_particles path: every chunk, no cell table
+__global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restrict__ bsum, uint32_t ncells,
+                            uint32_t* __restrict__ off)
+{
+    __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
+    __shared__ uint32_t s_prefix;
+    if (threadIdx.x < 32) {
+        const uint32_t p = prefix_of_blocks(bsum, blockIdx.x);
+        if (threadIdx.x == 0) s_prefix = p;
+    }
+    __syncthreads();
+    scan_chunk(cnt, ncells, off, nullptr, 0u, blockIdx.x, s_prefix, sm);
+}
+// A block takes a scan chunk of a set.  A chunk without particles only has its part of
+// cell_start cleared, if entries may be left there (dirty); its offsets are not written, and no
+// pass reads them: most chunks of a batch's wide grid, or above a scene, are empty (32 scenes,
+// 8,192 chunks, where every block also summed all earlier chunks: 79 us a set, 26 us both).
+// cell_start is cleared for c < clear (min(n, ncells) reproduces the reference's partial memset, Q1).
+__global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ SortPair Q, uint32_t chunks)
+{
+    __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
+    __shared__ uint32_t s_prefix;
+    const int k = blockIdx.x < chunks ? 0 : 1;
+    const uint32_t chunk = blockIdx.x - (k ? chunks : 0u);
+    const SortSide& A = Q.a[k];
+    if (Q.S && Q.on[k] && chunk == 0 && threadIdx.x == 0) Q.S->moved[k] = 0u;   // the hash pass has read it
+    if (!Q.sorts(k)) return;
+    const uint32_t here = A.bsum[chunk], begin = chunk * SCAN_CHUNK, end = umin32(begin + SCAN_CHUNK, Q.ncells);
+    const uint32_t clear = Q.clear_all ? Q.ncells : umin32(Q.size(k), Q.ncells);
+    const bool dirty = !Q.S || Q.S->table_any[k] != 0u || A.dirty[chunk] != 0u;
+    if (here == 0u) {
+        if (dirty)
+            for (uint32_t c = begin + threadIdx.x; c < umin32(end, clear); c += SCAN_TPB) A.cd.cell_start[c] = SNOWB_EMPTY;
+        __syncthreads();
+        if (threadIdx.x == 0) A.dirty[chunk] = dirty && end > clear ? 1u : 0u;
+        return;
+    }
+    if (threadIdx.x < 32) {
+        uint32_t p = 0;
+        if (Q.ncells > SUP_MIN * SCAN_CHUNK) {
+            const uint32_t s0 = chunk / SUP_CHUNKS;
+            p = prefix_of_blocks(A.sup, s0) + prefix_of_blocks(A.bsum + s0 * SUP_CHUNKS, chunk - s0 * SUP_CHUNKS);
+        } else {
+            p = prefix_of_blocks(A.bsum, chunk);
+        }
+        if (threadIdx.x == 0) {
+            s_prefix = p;
+            A.dirty[chunk] = 1u;
+        }
+    }
+    __syncthreads();
+    scan_chunk(A.cnt, Q.ncells, A.off, A.cd.cell_start, clear, chunk, s_prefix, sm);
+}
 
 // ------------------------------------------------------------------ 3. scatter
 __global__ void k_scatter(const uint32_t* __restrict__ key_o, const uint32_t* __restrict__ slot_o,
-                          const uint32_t* __restrict__ off, uint32_t* __restrict__ tmp,
-                          const uint32_t* n_ptr, uint32_t n_fixed, const uint32_t* cond,
-                          uint32_t* __restrict__ bsum_zero = nullptr, uint32_t nbsum = 0)
+                          const uint32_t* __restrict__ off, uint32_t* __restrict__ tmp, uint32_t n)
 {
-    if (cond && *cond == 0) return;
-    const uint32_t n = n_ptr ? *n_ptr : n_fixed;
     GRID_LOOP(o, n) tmp[off[key_o[o]] + slot_o[o]] = o;
-    if (bsum_zero) GRID_LOOP(k, nbsum) bsum_zero[k] = 0u;
+}
+__global__ void k_sort_scatter(const __grid_constant__ SortPair Q, uint32_t chunks)
+{
+    const bool s0 = Q.sorts(0), s1 = Q.sorts(1);
+    if (Q.S && blockIdx.x == 0 && threadIdx.x == 0) {   // the scan pass has cleared what was left in the tables
+        if (s0) Q.S->table_any[0] = 0u;
+        if (s1) Q.S->table_any[1] = 0u;
+    }
+    const uint32_t n0 = s0 ? Q.size(0) : 0u, n = n0 + (s1 ? Q.size(1) : 0u);
+    GRID_LOOP(t, n) {
+        const int k = t < n0 ? 0 : 1;
+        const SortSide& A = Q.a[k];
+        const uint32_t o = k ? t - n0 : t;
+        A.tmp[A.off[A.key[o]] + A.slot[o]] = o;
+    }
+    GRID_LOOP(c, chunks) {
+        if (s0) { Q.a[0].bsum[c] = 0u; Q.a[0].sup[c / SUP_CHUNKS] = 0u; }
+        if (s1) { Q.a[1].bsum[c] = 0u; Q.a[1].sup[c / SUP_CHUNKS] = 0u; }
+    }
 }
 
 // rank of element o among the (unordered) members of its cell, by ascending o
@@ -218,44 +305,35 @@ __device__ __forceinline__ uint32_t stable_rank(const uint32_t* __restrict__ tmp
 
 // ------------------------------------------------------------------ 4. rank + outputs
 // Fused path (sort_and_reorder :398-420 with hash = cell of pos).  Also gathers the
-// compact sorted attributes: p4 = (pos, w[o]), invm_s, contrib_s.  With *cond == 0 the
-// sort point keeps the last sort (no particle left its cell, same set size): grid_hash,
-// grid_index and the cell table are already what this sort would write, so only the
-// gathered outputs are refreshed, sorted slot by sorted slot.
-__global__ void k_rank_reorder(const uint32_t* __restrict__ key_o, const uint32_t* __restrict__ off,
-                               const uint32_t* __restrict__ tmp, const snowb_float3* __restrict__ pos,
-                               const float* __restrict__ w, const float* __restrict__ invm,
-                               const float* __restrict__ contrib, snowb_cell_data cd, float4* __restrict__ p4,
-                               float* __restrict__ invm_s, float* __restrict__ contrib_s,
-                               const uint32_t* n_ptr, uint32_t n_fixed, const uint32_t* cond,
-                               const uint32_t* __restrict__ sid_o, uint32_t* __restrict__ sid_s)
+// compact sorted attributes: p4 = (pos, w[o]), invm_s, contrib_s.  A set that keeps its last
+// sort (no particle left its cell, same set size): grid_hash, grid_index and the cell table are
+// already what this sort would write, so only the gathered outputs are refreshed, sorted slot
+// by sorted slot.
+__global__ void k_sort_rank(const __grid_constant__ SortPair Q)
 {
-    const uint32_t n = n_ptr ? *n_ptr : n_fixed;
-    if (cond && *cond == 0) {
-        GRID_LOOP(p, n) {
-            const uint32_t o = cd.grid_index[p];
-            const float3 q = ldv3(pos, o);
-            st3(cd.sorted_pos, p, q);
-            if (p4) p4[p] = make_float4(q.x, q.y, q.z, w ? w[o] : 0.f);
-            if (invm_s) invm_s[p] = invm[o];
-            if (contrib_s) contrib_s[p] = contrib[o];
-            if (sid_s) sid_s[p] = sid_o[o];
+    const bool s0 = Q.sorts(0), s1 = Q.sorts(1);
+    const uint32_t n0 = Q.size(0), n = n0 + Q.size(1);
+    GRID_LOOP(t, n) {
+        const int k = t < n0 ? 0 : 1;
+        const SortSide& A = Q.a[k];
+        uint32_t o, p;
+        if (k ? s1 : s0) {
+            o = k ? t - n0 : t;
+            const uint32_t h = A.key[o], b = A.off[h], e = A.off[h + 1], r = stable_rank(A.tmp, b, e, o);
+            p = b + r;
+            A.cd.grid_index[p] = o;
+            A.cd.grid_hash[p] = h;
+            if (r == 0) { A.cd.cell_start[h] = b; A.cd.cell_end[h] = e; }
+        } else {
+            p = k ? t - n0 : t;
+            o = A.cd.grid_index[p];
         }
-        return;
-    }
-    GRID_LOOP(o, n) {
-        const uint32_t h = key_o[o], b = off[h], e = off[h + 1];
-        const uint32_t r = stable_rank(tmp, b, e, o);
-        const uint32_t p = b + r;
-        cd.grid_index[p] = o;
-        cd.grid_hash[p] = h;
-        if (r == 0) { cd.cell_start[h] = b; cd.cell_end[h] = e; }
-        float3 q = ldv3(pos, o);
-        st3(cd.sorted_pos, p, q);
-        if (p4) p4[p] = make_float4(q.x, q.y, q.z, w ? w[o] : 0.f);
-        if (invm_s) invm_s[p] = invm[o];
-        if (contrib_s) contrib_s[p] = contrib[o];
-        if (sid_s) sid_s[p] = sid_o[o];
+        const float3 q = ldv3(A.pos, o);
+        st3(A.cd.sorted_pos, p, q);
+        A.p4[p] = make_float4(q.x, q.y, q.z, A.w[o]);
+        A.invm_s[p] = A.invm[o];
+        A.contrib_s[p] = A.contrib[o];
+        if (A.sid_s) A.sid_s[p] = A.sid_o[o];
     }
 }
 // A set whose particles all kept their cells since its last sort sorts to the same
@@ -308,73 +386,69 @@ __global__ void k_reorder(snowb_cell_data cd, const snowb_float3* __restrict__ p
         st3(cd.sorted_pos, i, ldv3(pos, cd.grid_index[i]));
     }
 }
-// Occupied ranges of a sorted hash array (fresh, without stale entries); the tables are
-// zeroed beforehand so empty cells read [0, 0).
-__global__ void k_fresh_ranges(const uint32_t* __restrict__ hash, uint32_t n, uint32_t* __restrict__ fs,
-                               uint32_t* __restrict__ fe)
-{
-    GRID_LOOP(i, n) {
-        const uint32_t h = hash[i];
-        if (i == 0 || hash[i - 1] != h) fs[h] = i;
-        if (i == n - 1 || hash[i + 1] != h) fe[h] = i + 1;
-    }
-}
-
 // ------------------------------------------------------------------ generic scan
-// Exclusive scan of in[0, n) into out (n from device or fixed), total into *total.
-__global__ void k_scan_sums(const uint32_t* __restrict__ in, const uint32_t* n_ptr, uint32_t n_fixed,
-                            uint32_t* __restrict__ bsum, const uint32_t* cond)
+// Exclusive scans of two arrays in[0, n) into out, totals into *total, by the same two launches
+// (blocks [0, blocks) take the first array, the rest the second).
+struct ScanSide {
+    const uint32_t* in;
+    const uint32_t* n_ptr;     // null: n
+    uint32_t n;
+    uint32_t *bsum, *out, *total;
+};
+struct ScanPair {
+    ScanSide a[2];
+};
+__global__ void k_scan_sums(const __grid_constant__ ScanPair Q, uint32_t blocks)
 {
-    if (cond && *cond == 0) return;
-    const uint32_t n = n_ptr ? *n_ptr : n_fixed;
+    const int k = blockIdx.x < blocks ? 0 : 1;
+    const ScanSide& A = Q.a[k];
+    const uint32_t b = blockIdx.x - (k ? blocks : 0u), n = A.n_ptr ? *A.n_ptr : A.n;
     __shared__ uint32_t sm[SCAN_TPB / 32];
-    const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
-    if (blockIdx.x * SCAN_CHUNK >= n && blockIdx.x != 0) { if (threadIdx.x == 0) bsum[blockIdx.x] = 0; return; }
+    const uint32_t base = b * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
+    if (b * SCAN_CHUNK >= n && b != 0) { if (threadIdx.x == 0) A.bsum[b] = 0; return; }
     uint32_t s = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k)
-        if (base + k < n) s += in[base + k];
+    for (int k2 = 0; k2 < SCAN_ITEMS; ++k2)
+        if (base + k2 < n) s += A.in[base + k2];
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x < 32) {
         uint32_t v = threadIdx.x < SCAN_TPB / 32 ? sm[threadIdx.x] : 0u;
         v = warp_sum(v);
-        if (threadIdx.x == 0) bsum[blockIdx.x] = v;
+        if (threadIdx.x == 0) A.bsum[b] = v;
     }
 }
-__global__ void k_scan_apply(const uint32_t* __restrict__ in, const uint32_t* n_ptr, uint32_t n_fixed,
-                             const uint32_t* __restrict__ bsum, uint32_t* __restrict__ out, uint32_t* total,
-                             const uint32_t* cond)
+__global__ void k_scan_apply(const __grid_constant__ ScanPair Q, uint32_t blocks)
 {
-    if (cond && *cond == 0) return;
-    const uint32_t n = n_ptr ? *n_ptr : n_fixed;
-    const uint32_t nblocks = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    if (n == 0) { if (blockIdx.x == 0 && threadIdx.x == 0 && total) *total = 0; return; }
-    if (blockIdx.x >= nblocks) return;
+    const int k = blockIdx.x < blocks ? 0 : 1;
+    const ScanSide& A = Q.a[k];
+    const uint32_t b = blockIdx.x - (k ? blocks : 0u), n = A.n_ptr ? *A.n_ptr : A.n;
+    if (n == 0) { if (b == 0 && threadIdx.x == 0) *A.total = 0; return; }
+    if (b >= (n + SCAN_CHUNK - 1) / SCAN_CHUNK) return;
     __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
     __shared__ uint32_t s_prefix;
     if (threadIdx.x < 32) {
-        uint32_t p = prefix_of_blocks(bsum, blockIdx.x);
+        uint32_t p = prefix_of_blocks(A.bsum, b);
         if (threadIdx.x == 0) s_prefix = p;
     }
-    const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
+    const uint32_t base = b * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS], t = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0u;
-        t += v[k];
+    for (int k2 = 0; k2 < SCAN_ITEMS; ++k2) {
+        v[k2] = base + k2 < n ? A.in[base + k2] : 0u;
+        t += v[k2];
     }
     uint32_t tot;
     __syncthreads();
     uint32_t ex = block_excl_scan(t, sm, tot) + s_prefix;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < n) {
-            if (out) out[base + k] = ex;
-            if (base + k == n - 1 && total) *total = ex + v[k];
+    for (int k2 = 0; k2 < SCAN_ITEMS; ++k2) {
+        if (base + k2 < n) {
+            A.out[base + k2] = ex;
+            if (base + k2 == n - 1) *A.total = ex + v[k2];
         }
-        ex += v[k];
+        ex += v[k2];
     }
 }
 
