@@ -166,15 +166,6 @@ __device__ __forceinline__ void put3(float* out, int a, int q, float3 x)
     out[(a + 1) * M + q] = x.y;
     out[(a + 2) * M + q] = x.z;
 }
-// lane c < 27: hash of cell c around g
-__device__ __forceinline__ uint32_t lane_cell(const DevParams& P, GCell g)
-{
-    const uint32_t c = threadIdx.x & 31u;
-    return c < 27u ? grid_hash(P, g, (int)(c % 3u) - 1, (int)((c / 3u) % 3u) - 1, (int)(c / 9u) - 1) : 0u;
-}
-// warps of the launch, and this one's number
-#define WARP_LOOP(t, n) \
-    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < (n); t += (gridDim.x * blockDim.x) >> 5)
 // A warp takes 32 boundary particles (nbg apart: those with neighbours come in patches): lane by
 // lane they are looked over (near(i): is anything around?), and those with something around are
 // taken by the whole warp, one after another (take(i), every lane).

@@ -526,7 +526,9 @@ struct StepArgs {
     uint32_t* sid_buf;
     int xsph_thread[2];   // XSPH of the water / snow set in the one-thread form (sizes at the call)
     uint32_t particles;   // water + snow at the call (phase changes keep the sum)
-    int small;            // the neighbour passes in their one-warp forms (particles at the call)
+    // passes in their one-warp forms (set sizes at the call): density and link filter, heat,
+    // snow contacts, friction (1: unless the neighbour lists hold, 2: always)
+    int small, small_heat, small_contact, small_friction;
 };
 
 
@@ -743,7 +745,8 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // in a whole substep the phase flags pass commits the new temperatures itself
     const int commit_in_flags = beside && a.temperature && a.change_phase;
     if (a.temperature) {
-        TLAUNCH(k_heat, 256, 2 * full, 128, P, S, vs, vd, X, a.dt);
+        if (a.small_heat) TLAUNCH_AS("k_heat", k_heat_warp, SMALL_TPB, 32ull * a.particles, SMALL_TPB, P, S, vs, vd, X, a.dt);
+        else TLAUNCH(k_heat, 256, 2 * full, 128, P, S, vs, vd, X, a.dt);
         if (!commit_in_flags) LAUNCH(k_heat_commit, 2 * full, 256, S, X, a.dTe, step_sph ? 1 : 0, step_dem ? 1 : 0);
     }
     STOP(3);
@@ -776,7 +779,11 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         // link formation over a view of the snow set: the set's own, or its copy
         auto form = [&](const SetView& v) -> int {
             const SCList scl = sc_lists(P);
-            TLAUNCH(k_link_filter, 256, full, 128, P, S, v, *a.dem, a.dynamic, c.active, NL2, scl);
+            if (a.small && P.maxc <= SNOWB_MAXC_FAST)
+                TLAUNCH_AS("k_link_filter", k_link_filter_warp, 128, 32ull * full, 128, P, S, v, *a.dem, a.dynamic,
+                           c.active, NL2, scl);
+            else
+                TLAUNCH(k_link_filter, 256, full, 128, P, S, v, *a.dem, a.dynamic, c.active, NL2, scl);
             const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);   // super-cells per colour
             for (uint32_t col = 0; col < 8; ++col) {
                 if (P.maxc <= SNOWB_MAXC_FAST)
@@ -856,14 +863,24 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         // the snow contact sums, kept apart for k_link_apply, beside the snow PBF pass
         if (links_beside)
             TRY(on_side(c.side3, c.fork3, [&]() -> int {
-                TLAUNCH(k_dem_corr<true>, 256, full, 128, P, S, vs, vd, vb, X, ss, sd, sb, F, NL, c.contact);
+                if (a.small_contact)
+                    TLAUNCH_AS("k_dem_corr<true>", k_dem_corr_warp<true>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd,
+                               vb, X, ss, sd, sb, F, c.contact);
+                else
+                    TLAUNCH(k_dem_corr<true>, 256, full, 128, P, S, vs, vd, vb, X, ss, sd, sb, F, NL, c.contact);
                 return SNOWB_OK;
             }));
         // the reference's snow PBF pass adds into repeated targets with float atomics (Q3):
         // its order follows the launch shape, so that pass keeps the built-in shape
         TLAUNCH_IF(!ref, k_pbf, 256, 2 * full, 128, P, S, vs, vd, vb, X, ss, sd, sb, a.dt, F, NL, apply_w, track_s);
         STOP(base + 3);
-        if (!links_beside) TLAUNCH(k_dem_corr<false>, 256, full, 128, P, S, vs, vd, vb, X, ss, sd, sb, F, NL, nullptr);
+        if (!links_beside) {
+            if (a.small_contact)
+                TLAUNCH_AS("k_dem_corr<false>", k_dem_corr_warp<false>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd,
+                           vb, X, ss, sd, sb, F, nullptr);
+            else
+                TLAUNCH(k_dem_corr<false>, 256, full, 128, P, S, vs, vd, vb, X, ss, sd, sb, F, NL, nullptr);
+        }
         if (a.interlink) {
             if (links_beside) {
                 TRY(join_side(c.side3, c.join3));
@@ -893,10 +910,19 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         if (a.friction && step_dem) {
             TRY(sort_pair(false));
             // a whole substep applies the friction correction in the friction pass itself
+            const int unless = a.small_friction == 1 ? 1 : 0;
             if (beside) {
-                TLAUNCH(k_friction<true>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, track_d);
+                if (a.small_friction)
+                    TLAUNCH_AS("k_friction<true>", k_friction_warp<true>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vd,
+                               vb, X, sd, sb, fr_lists ? 1 : 0, unless, track_d);
+                if (a.small_friction != 2)
+                    TLAUNCH(k_friction<true>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, unless, track_d);
             } else {
-                TLAUNCH(k_friction<false>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, track_d);
+                if (a.small_friction)
+                    TLAUNCH_AS("k_friction<false>", k_friction_warp<false>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vd,
+                               vb, X, sd, sb, fr_lists ? 1 : 0, unless, track_d);
+                if (a.small_friction != 2)
+                    TLAUNCH(k_friction<false>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, unless, track_d);
                 TLAUNCH(k_apply, 1024, full, 256, P, S, vs, vd, X, 0, 1, track_s, track_d);
             }
             dirty_d = true;
@@ -1389,7 +1415,10 @@ static int run_steps(snowb_particle_data* sph, uint32_t* sph_size, snowb_particl
                batch ? batch->scene_sph : nullptr, batch ? batch->scene_dem : nullptr,
                batch ? batch->scene_boundary : nullptr, batch ? batch->scene_buffer : nullptr,
                {xs_s > XSPH_WARP_MAX ? 1 : 0, xs_d > XSPH_WARP_MAX ? 1 : 0}, *sph_size + *dem_size,
-               *sph_size + *dem_size <= DENSITY_WARP_MAX ? 1 : 0};
+               *sph_size + *dem_size <= DENSITY_WARP_MAX ? 1 : 0,
+               *sph_size + *dem_size <= (opt.quirks == SNOWB_QUIRKS_REFERENCE ? HEAT_WARP_MAX_REF : HEAT_WARP_MAX) ? 1 : 0,
+               *dem_size <= CONTACT_WARP_MAX ? 1 : 0,
+               *dem_size <= FRICTION_WARP_MAX ? 2 : (*dem_size <= FRICTION_BOTH_MAX ? 1 : 0)};
     LAUNCH1(k_set_state, c.S, *sph_size, *dem_size, nb);
     if (batch)
         LAUNCH(k_check_scenes, full > nb ? full : nb, 256, P, c.S, a.sid_sph, a.sid_dem, a.sid_bnd);

@@ -698,6 +698,107 @@ __global__ void __launch_bounds__(256) k_density_warp(DevParams P, DevState* __r
     }
 }
 
+// ------------------------------------------------- ordered per-cell sums by a warp (small sets)
+// The sums of a one-thread neighbour loop -- per cell a partial sum in index order, the partials
+// added in cell order -- over the entries j != skip of set v within d2 < cut of p, for sets too
+// small to fill the GPU with threads.  Lane c < 27 scans cell c (h: its hash; live: the lane takes
+// part), four entries in flight; the counts' prefix over the lanes lists those accepted in
+// traversal order, 32 of them at a time are evaluated side by side (terms(j, out) writes one
+// addend for each of NA sums), and lane a < NA adds the addends of sum a in order, a partial
+// closed where the cell changes.  acc carries on from the sets before.
+constexpr uint32_t CELL_LIST = 96;
+struct CellBuf {
+    uint32_t e[CELL_LIST];           // j | cell << 25
+    float t[32 * 3];
+};
+template <int NA, class F>
+__device__ __forceinline__ void warp_cell_sums(const SetView& v, float3 p, uint32_t h, bool live, uint32_t skip, float cut,
+                                               CellBuf& W, float& acc, F&& terms)
+{
+    static_assert(NA == 1 || NA == 3, "addends of a neighbour");
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu;
+    uint32_t s = 0, e = 0;
+    if (live) {
+        s = __ldg(v.cs + h);
+        e = __ldg(v.ce + h);
+        if (s == SNOWB_EMPTY || e < s) s = e = 0u;
+    }
+    auto hit = [&](uint32_t j) {
+        const float3 r = sub3(p, v.pos(j));
+        return dot3(r, r) < cut && j != skip;
+    };
+    uint32_t n = 0, mask = 0;   // accepted, and which of the first 32 entries
+    for (uint32_t k = 0; k < e - s; k += 4u)
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u)
+            if (hit(umin32(s + k + u, e - 1u)) && s + k + u < e) {
+                ++n;
+                if (k + u < 32u) mask |= 1u << (k + u);
+            }
+    if (!__any_sync(full, n != 0u)) return;
+    const uint32_t first = warp_incl_scan(n) - n, total = __shfl_sync(full, first + n, 31);
+    float cs = 0.f;
+    uint32_t cur = 0xFFu;
+    for (uint32_t w0 = 0; w0 < total; w0 += CELL_LIST) {
+        __syncwarp();
+        uint32_t at = first, m = mask;
+        while (m) {
+            const uint32_t j = s + (uint32_t)__ffs(m) - 1u;
+            m &= m - 1u;
+            if (at - w0 < CELL_LIST) W.e[at - w0] = j | lane << 25;
+            ++at;
+        }
+        for (uint32_t j = s + 32u; j < e; ++j)
+            if (hit(j)) {
+                if (at - w0 < CELL_LIST) W.e[at - w0] = j | lane << 25;
+                ++at;
+            }
+        __syncwarp();
+        const uint32_t held = umin32(total - w0, CELL_LIST);
+        for (uint32_t b = 0; b < held; b += 32u) {
+            if (b + lane < held) terms(W.e[b + lane] & NL_J_MASK, W.t + lane * NA);
+            __syncwarp();
+            if (lane < (uint32_t)NA)
+                for (uint32_t k = 0; k < umin32(held - b, 32u); ++k) {
+                    const uint32_t cell = W.e[b + k] >> 25;
+                    if (cell != cur) {
+                        if (cur != 0xFFu) acc += cs;
+                        cs = 0.f;
+                        cur = cell;
+                    }
+                    cs += W.t[k * NA + lane];
+                }
+            __syncwarp();
+        }
+    }
+    acc += cs;
+}
+__device__ __forceinline__ float3 warp_vec3(float acc)
+{
+    return f3(__shfl_sync(0xffffffffu, acc, 0), __shfl_sync(0xffffffffu, acc, 1), __shfl_sync(0xffffffffu, acc, 2));
+}
+// lane c < 27: hash of cell c around g
+__device__ __forceinline__ uint32_t lane_cell(const DevParams& P, GCell g)
+{
+    const uint32_t c = threadIdx.x & 31u;
+    return c < 27u ? grid_hash(P, g, (int)(c % 3u) - 1, (int)((c / 3u) % 3u) - 1, (int)(c / 9u) - 1) : 0u;
+}
+#define WARP_LOOP(t, n) \
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < (n); t += (gridDim.x * blockDim.x) >> 5)
+constexpr uint32_t SMALL_TPB = 128;
+// Where the lines lie, by whole frames (ms, one thread against one warp per particle):
+// contacts (by snow particles): 1.651 / 1.538 at 4.8k, 1.848 / 1.753 at 8.6k, 2.046 / 2.073 at
+// 14.1k and 2.362 / 2.509 at 23.1k at rest; in the melt, where lists are long, 4.431 / 3.912 at
+// 8.6k and 4.432 / 3.952 at 14.1k.  Heat: fixed quirks (27 cells of both sets) 3.238 / 3.061 at
+// 24.8k and 3.798 / 3.646 at 35.7k; reference quirks (the own cell) even at 5k, 2.362 / 2.447 at
+// 24.8k.  Friction: 1.651 / 1.606 at 4.8k; beyond FRICTION_WARP_MAX the one-thread form's list
+// replay is the faster one (2.046 / 2.133 at 14.1k), the traversal it falls back to when the lists
+// do not hold is the slower one up to about twice that (eight substeps of 13.8k: 6.20 / 5.57),
+// so up to FRICTION_BOTH_MAX both are launched and one returns at once.
+constexpr uint32_t CONTACT_WARP_MAX = 16000;
+constexpr uint32_t HEAT_WARP_MAX = 40000, HEAT_WARP_MAX_REF = 6000;
+constexpr uint32_t FRICTION_WARP_MAX = 9000, FRICTION_BOTH_MAX = 24000;
+
 // ======================================================== applying a correction
 // apply_correction (:1342-1380) for one particle: new and predicted position q + sor * corr,
 // the correction cleared, the set marked when the particle left its cell.  Passes that
@@ -878,6 +979,55 @@ __global__ void __launch_bounds__(256) k_dem_corr(DevParams P, const DevState* _
     }
     (void)ns; (void)nb;
 }
+// the same with one warp per particle, by traversal (small sets; 28 -> 18 us at 5,096 particles)
+template <bool SUMS>
+__global__ void __launch_bounds__(SMALL_TPB) k_dem_corr_warp(DevParams P, const DevState* __restrict__ S, SetView vs,
+                                                             SetView vd, SetView vb, Sets X, Sorted ss, Sorted sd,
+                                                             Sorted sb, StageFlags F, float4* __restrict__ sums)
+{
+    __shared__ CellBuf bufs[SMALL_TPB / 32];
+    CellBuf& W = bufs[threadIdx.x >> 5];
+    const uint32_t nd = S->n_dem, lane = threadIdx.x & 31u;
+    vs.n = S->n_sph; vd.n = nd; vb.n = S->n_b;
+    const float3 z = f3(0.f, 0.f, 0.f);
+    WARP_LOOP(i, nd) {
+        const uint32_t o = vd.gi[i];
+        const float3 p = xyz(vd.p4[i]);
+        const uint32_t h = lane_cell(P, grid_pos(P, p, vd.scene(i)));
+        const float w0 = X.dem.massInv[o], ci = X.dem.contrib[o];
+        auto contact = [&](const SetView& v, uint32_t skip, const float* invm_s, const float* invm_o, float& acc) {
+            warp_cell_sums<3>(v, p, h, lane < 27u, skip, P.r2_lt, W, acc, [&](uint32_t j, float* out) {
+                const float3 dv = sub3(p, v.pos(j));
+                const float d = sqrtf(dot3(dv, dv));
+                const float ws = w0 + v.attr(invm_s, invm_o, j), C = d - P.two_r;
+                const float3 t = sc3(((-w0) * (1.f / ws)) * C, div3(dv, d + P.pbd_eps));
+                out[0] = t.x; out[1] = t.y; out[2] = t.z;
+            });
+        };
+        float3 dw = z;
+        if (F.correct_dem) {
+            float acc = 0.f;
+            contact(vs, SNOWB_UMAX, ss.invm, X.sph.massInv, acc);
+            dw = sc3(P.k_stretch * ci, warp_vec3(acc));
+            if (nan3(dw)) dw = z;
+        }
+        float acc = 0.f;
+        contact(vd, i, sd.invm, X.dem.massInv, acc);
+        contact(vb, SNOWB_UMAX, sb.invm, X.bnd.massInv, acc);
+        float3 d = sc3(ci, warp_vec3(acc));
+        if (nan3(d)) d = z;
+        if (lane == 0u) {
+            if (SUMS) {
+                sums[2 * (size_t)o] = make_float4(dw.x, dw.y, dw.z, 0.f);
+                sums[2 * (size_t)o + 1] = make_float4(d.x, d.y, d.z, 0.f);
+            } else {
+                float3 c = ldv3(X.dem.correction, o);
+                if (F.correct_dem) c = add3(c, dw);
+                st3(X.dem.correction, o, add3(c, d));
+            }
+        }
+    }
+}
 // solve_snow_interlink_constraint_d (:4742-4765) with compute_interlink_correction
 // (:4661-4739), in two passes.  Each particle's slots are summed in slot order, which one
 // thread per particle walking its slots does with about 11 dependent link terms in a row
@@ -1041,16 +1191,23 @@ constexpr uint32_t FR_K = 16;
 // position it reads is this pass's p: new and predicted positions, a zero correction, the
 // moved mark of the set), without k_apply's far-move flag, which the next density+lambda
 // pass clears before any friction pass reads it.
+// only_lists: k_friction_warp takes the pass unless the lists hold.
+__device__ __forceinline__ bool friction_lists(const DevState* S, int lists)
+{
+    return lists && S->resort[1] == 0u && S->far_move == 0u;
+}
 template <bool APPLY>
 __global__ void __launch_bounds__(256) k_friction(DevParams P, const DevState* __restrict__ S, SetView vd, SetView vb,
-                                                  Sets X, Sorted sd, Sorted sb, NList L, int lists, SortTrack td)
+                                                  Sets X, Sorted sd, Sorted sb, NList L, int lists, int only_lists,
+                                                  SortTrack td)
 {
     __shared__ uint32_t rec_sh[FR_K * 256];
     uint32_t* const rec = rec_sh + threadIdx.x;     // entry k at rec[k * blockDim.x]
     const uint32_t bd = blockDim.x;
     vd.n = S->n_dem; vb.n = S->n_b;
     const uint32_t ld = launch_limit(P, S->n0_dem, S->n_dem);
-    const bool list_ok = lists && S->resort[1] == 0u && S->far_move == 0u;
+    const bool list_ok = friction_lists(S, lists);
+    if (only_lists && !list_ok) return;
     GRID_LOOP(i, ld) {
         const uint32_t o = vd.gi[i];
         float3 p = xyz(vd.p4[i]);
@@ -1215,6 +1372,45 @@ __global__ void __launch_bounds__(256) k_friction(DevParams P, const DevState* _
     }
 }
 
+// the same with one warp per particle, by traversal (at 16,380 particles, where the one-thread
+// form mostly walked the cells, 55 -> 29 us)
+template <bool APPLY>
+__global__ void __launch_bounds__(SMALL_TPB) k_friction_warp(DevParams P, const DevState* __restrict__ S, SetView vd,
+                                                             SetView vb, Sets X, Sorted sd, Sorted sb, int lists,
+                                                             int unless_lists, SortTrack td)
+{
+    if (unless_lists && friction_lists(S, lists)) return;   // k_friction replays them
+    __shared__ CellBuf bufs[SMALL_TPB / 32];
+    CellBuf& W = bufs[threadIdx.x >> 5];
+    vd.n = S->n_dem; vb.n = S->n_b;
+    const uint32_t ld = launch_limit(P, S->n0_dem, S->n_dem), lane = threadIdx.x & 31u;
+    WARP_LOOP(i, ld) {
+        const uint32_t o = vd.gi[i];
+        const float3 p = xyz(vd.p4[i]);
+        const uint32_t h = lane_cell(P, grid_pos(P, p, vd.scene(i)));
+        const float3 op0 = ldv3(X.dem.positions, o), dx0 = sub3(p, op0);
+        const float w0 = X.dem.massInv[o];
+        float acc = 0.f;
+        warp_cell_sums<3>(vd, p, h, lane < 27u, i, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+            const float3 pp1 = vd.pos(j), v = sub3(p, pp1);
+            const float3 dx = add3(dx0, sub3(pp1, ldv3(X.dem.positions, vd.gi[j])));
+            const float3 t = friction_term(P, dx, w0, vd.attr(sd.invm, X.dem.massInv, j), sqrtf(dot3(v, v)), v);
+            out[0] = t.x; out[1] = t.y; out[2] = t.z;
+        });
+        warp_cell_sums<3>(vb, p, h, lane < 27u, SNOWB_UMAX, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+            const float3 v = sub3(p, vb.pos(j));
+            const float3 t = friction_term(P, dx0, w0, vb.attr(sb.invm, X.bnd.massInv, j), sqrtf(dot3(v, v)), v);
+            out[0] = t.x; out[1] = t.y; out[2] = t.z;
+        });
+        float3 c = warp_vec3(acc);
+        if (nan3(c)) c = f3(0.f, 0.f, 0.f);
+        if (lane == 0u) {
+            if (APPLY) apply_one(P, X.dem, td, o, p, c, vd.scene(i));
+            else st3(X.dem.correction, o, c);
+        }
+    }
+}
+
 // =================================================================== integrate
 // integrate_pbd_cd_d (:467-540) / integrate_pbd_d (:447-465).  The reference kernel has no
 // bounds check, so it runs over its whole launch (clamped to the allocation here).
@@ -1347,6 +1543,55 @@ __global__ void __launch_bounds__(256) k_heat(DevParams P, const DevState* __res
         dT = heat_sum(P, dT, oth, B, g, SNOWB_UMAX, p, Ti, w ? kws : ksw);
         dT = dT / ((w ? P.C_water : P.C_snow) * A.density[o]);
         A.new_T[o] = Ti + dT * dt;
+    }
+}
+// the same with one warp per particle (small sets; fixed quirks at 16,380 particles, 27 cells of
+// both sets: 141 -> 35 us)
+__global__ void __launch_bounds__(SMALL_TPB) k_heat_warp(DevParams P, const DevState* __restrict__ S, SetView vs,
+                                                         SetView vd, Sets X, float dt)
+{
+    __shared__ CellBuf bufs[SMALL_TPB / 32];
+    CellBuf& W = bufs[threadIdx.x >> 5];
+    const uint32_t ns = S->n_sph, nd = S->n_dem, lane = threadIdx.x & 31u;
+    vs.n = ns; vd.n = nd;
+    const bool ref = P.quirks == SNOWB_QUIRKS_REFERENCE;
+    const float kww = ((4.f * P.k_water) * P.k_water) / (P.k_water + P.k_water);
+    const float kss = ((4.f * P.k_snow) * P.k_snow) / (P.k_snow + P.k_snow);
+    const float kws = ((4.f * P.k_water) * P.k_snow) / (P.k_water + P.k_snow);
+    const float ksw = ((4.f * P.k_snow) * P.k_water) / (P.k_snow + P.k_water);
+    WARP_LOOP(t, ns + nd) {
+        const bool w = t < ns;
+        const uint32_t i = w ? t : t - ns;
+        const SetView& own = w ? vs : vd;
+        const snowb_particle_data& A = w ? X.sph : X.dem;
+        const uint32_t o = own.gi[i];
+        const float3 p = xyz(own.p4[i]);
+        const uint32_t h = lane_cell(P, grid_pos(P, p, own.scene(i)));
+        const float Ti = A.T[o];
+        float dT = 0.f;   // the sum so far, in lane 0
+        auto add = [&](const SetView& v, const snowb_particle_data& O, uint32_t skip, float kk) {
+            auto term = [&](uint32_t j, float* out) {
+                const float3 dv = sub3(p, v.pos(j));
+                const uint32_t oj = v.gi[j];
+                out[0] = (((O.mass[oj] / O.density[oj]) * kk) * (O.T[oj] - Ti)) * L_visc(P, sqrtf(dot3(dv, dv)));
+            };
+            if (ref) {   // Q7: the particle's own cell, 27 times
+                float s = 0.f;
+                warp_cell_sums<1>(v, p, h, lane == 13u, skip, P.h2_lt, W, s, term);
+                for (int k = 0; k < 27; ++k) dT += s;
+            } else {
+                warp_cell_sums<1>(v, p, h, lane < 27u, skip, P.h2_lt, W, dT, term);
+            }
+        };
+        if (w) {
+            add(vs, X.sph, i, kww);
+            add(vd, X.dem, SNOWB_UMAX, kws);
+        } else {
+            add(vd, X.dem, i, kss);
+            add(vs, X.sph, SNOWB_UMAX, ksw);
+        }
+        dT = dT / ((w ? P.C_water : P.C_snow) * A.density[o]);
+        if (lane == 0u) A.new_T[o] = Ti + dT * dt;
     }
 }
 // thrust::copy new_T -> T (:3968-3969) then environmental_heat_transfer (:4847-4859)
