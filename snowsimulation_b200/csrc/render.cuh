@@ -101,12 +101,41 @@ __device__ __forceinline__ bool sprite_fragment(const SpriteVtx& v, int px, int 
              fminf(fmaxf(diff * v.col.z, 0.f), 1.f));
     return true;
 }
-__global__ void kr_depth(RenderCam c, RenderColour rc, const snowb_float3* __restrict__ pos,
-                         const float* __restrict__ T, uint32_t n, uint32_t draw,
-                         unsigned long long* __restrict__ zbuf)
+// Splats: SPLAT lanes take a particle and walk its covered pixels row by row, so one access of
+// a warp falls into fewer sectors of the image than 32 sprites' addresses would, and a lane has
+// a few pixels in turn instead of a whole sprite.  Draws of 148k and 6k sprites of 6 x 6 pixels
+// on 1280 x 720, mean: 24.3 us with one thread per particle, 16.9 with 4 lanes (2: 19.7; 8: 19.6).
+// READ: the depth that stands at a pixel is read first and a fragment that cannot win is dropped
+// before its arithmetic and its atomic (depths only fall during a launch, so an old value drops
+// nothing that belongs in the image).  It takes the wait for a read per pixel and saves atomics
+// on one address: the fluid view's default camera, whose far snow block puts about 200 sprites
+// on a pixel, 36.7 -> 27.1 us; the point view at about 25 a pixel, 16.9 -> 21.0 us, so it stays
+// out there.
+constexpr uint32_t SPLAT = 4;
+template <class F>
+__device__ __forceinline__ void splat_pixels(int x0, int x1, int y0, int y1, F&& f)
 {
-    GRID_LOOP(i, n) {
-        const SpriteVtx v = sprite_vertex(c, rc, ldv3(pos, i), T ? T[i] : 0.f);
+    const int w = x1 - x0;
+    if (w <= 0) return;
+    int px = x0 + (int)(threadIdx.x & (SPLAT - 1u)), py = y0;
+    while (true) {
+        while (px >= x1) { px -= w; ++py; }
+        if (py >= y1) return;
+        f(px, py);
+        px += (int)SPLAT;
+    }
+}
+#define SPLAT_LOOP(i, n, block, blocks)                                                    \
+    for (uint32_t i = ((block) * blockDim.x + threadIdx.x) / SPLAT; i < (n);               \
+         i += (blocks) * blockDim.x / SPLAT)
+
+template <bool READ>
+__device__ __forceinline__ void splat_points(const RenderCam& c, const RenderColour& rc,
+                                             const snowb_float3* __restrict__ pos, uint32_t n, uint32_t draw,
+                                             unsigned long long* zbuf, uint32_t block, uint32_t blocks)
+{
+    SPLAT_LOOP(i, n, block, blocks) {
+        const SpriteVtx v = sprite_vertex(c, rc, ldv3(pos, i), 0.f);   // the colour is not used here
         if (!v.live) continue;
         int x0, x1, y0, y1;
         sprite_span(v.xw, v.side, c.W, x0, x1);
@@ -114,36 +143,55 @@ __global__ void kr_depth(RenderCam c, RenderColour rc, const snowb_float3* __res
         uint32_t db;
         memcpy(&db, &v.depth, 4);
         const unsigned long long key = ((unsigned long long)db << 32) | ((unsigned long long)draw << 27) | i;
-        for (int py = y0; py < y1; ++py)
-            for (int px = x0; px < x1; ++px) {
-                float3 rgb;
-                if (sprite_fragment(v, px, py, rgb)) atomicMin(zbuf + (size_t)py * c.W + px, key);
-            }
+        splat_pixels(x0, x1, y0, y1, [&](int px, int py) {
+            unsigned long long* const z = zbuf + (size_t)py * c.W + px;
+            float3 rgb;
+            if ((!READ || key < *z) && sprite_fragment(v, px, py, rgb)) atomicMin(z, key);
+        });
     }
+}
+__global__ void __launch_bounds__(128) kr_depth(RenderCam c, RenderColour rc, const snowb_float3* __restrict__ pos,
+                                                uint32_t n, uint32_t draw, unsigned long long* zbuf)
+{
+    splat_points<false>(c, rc, pos, n, draw, zbuf, blockIdx.x, gridDim.x);
+}
+// one pixel of the image, in one 16-byte store where the image is aligned for it (v4)
+__device__ __forceinline__ void put_pixel(float* __restrict__ rgba, uint32_t k, float4 o, int v4)
+{
+    if (v4) {
+        reinterpret_cast<float4*>(rgba)[k] = o;
+    } else {
+        rgba[4 * (size_t)k] = o.x; rgba[4 * (size_t)k + 1] = o.y; rgba[4 * (size_t)k + 2] = o.z;
+        rgba[4 * (size_t)k + 3] = o.w;
+    }
+}
+// pixel k's winning sprite, shaded; false when draw did not win it
+__device__ __forceinline__ bool shade_pixel(const RenderCam& c, const RenderColour& rc,
+                                            const snowb_float3* __restrict__ pos, const float* __restrict__ T,
+                                            uint32_t draw, unsigned long long key, uint32_t k, float4& o)
+{
+    if (key == ~0ull || ((key >> 27) & 31ull) != draw) return false;
+    const uint32_t i = (uint32_t)(key & ((1u << 27) - 1u));
+    const SpriteVtx v = sprite_vertex(c, rc, ldv3(pos, i), T ? T[i] : 0.f);
+    float3 rgb = f3(0.f, 0.f, 0.f);
+    sprite_fragment(v, (int)(k % c.W), (int)(k / c.W), rgb);
+    o = make_float4(rgb.x, rgb.y, rgb.z, 1.f);
+    return true;
 }
 __global__ void kr_shade(RenderCam c, RenderColour rc, const snowb_float3* __restrict__ pos,
                          const float* __restrict__ T, uint32_t draw, const unsigned long long* __restrict__ zbuf,
-                         float* __restrict__ rgba)
+                         float* __restrict__ rgba, int v4)
 {
     GRID_LOOP(k, c.W * c.H) {
-        const unsigned long long key = zbuf[k];
-        if (key == ~0ull || ((key >> 27) & 31ull) != draw) continue;
-        const uint32_t i = (uint32_t)(key & ((1u << 27) - 1u));
-        const SpriteVtx v = sprite_vertex(c, rc, ldv3(pos, i), T ? T[i] : 0.f);
-        float3 rgb = f3(0.f, 0.f, 0.f);
-        sprite_fragment(v, (int)(k % c.W), (int)(k / c.W), rgb);
-        rgba[4 * (size_t)k] = rgb.x;
-        rgba[4 * (size_t)k + 1] = rgb.y;
-        rgba[4 * (size_t)k + 2] = rgb.z;
-        rgba[4 * (size_t)k + 3] = 1.f;
+        float4 o;
+        if (shade_pixel(c, rc, pos, T, draw, zbuf[k], k, o)) put_pixel(rgba, k, o, v4);
     }
 }
-__global__ void kr_clear(uint32_t npix, unsigned long long* zbuf, float* rgba, float4 clear)
+__global__ void kr_clear(uint32_t npix, unsigned long long* zbuf, float* rgba, float4 clear, int v4)
 {
     GRID_LOOP(k, npix) {
         zbuf[k] = ~0ull;
-        rgba[4 * (size_t)k] = clear.x; rgba[4 * (size_t)k + 1] = clear.y; rgba[4 * (size_t)k + 2] = clear.z;
-        rgba[4 * (size_t)k + 3] = clear.w;
+        put_pixel(rgba, k, clear, v4);
     }
 }
 

@@ -1954,6 +1954,7 @@ int snowb_autotune_reset(void)
 }
 
 // ------------------------------------------------------------------ point-sprite rendering
+static int aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 ? 1 : 0; }
 static int render_cam(const snowb_camera* cam, RenderCam& c)
 {
     if (!cam) return fail(SNOWB_ERR_INVALID, "null camera");
@@ -1974,7 +1975,7 @@ int snowb_render_clear(const snowb_camera* cam, float* rgba, unsigned long long*
     RenderCam c;
     TRY(render_cam(cam, c));
     if (!rgba || !zbuf) return fail(SNOWB_ERR_INVALID, "null image");
-    LAUNCH(kr_clear, (uint64_t)c.W * c.H, 256, c.W * c.H, zbuf, rgba, make_float4(0.f, 0.f, 0.f, 0.f));
+    LAUNCH(kr_clear, (uint64_t)c.W * c.H, 256, c.W * c.H, zbuf, rgba, make_float4(0.f, 0.f, 0.f, 0.f), aligned16(rgba));
     return SNOWB_OK;
 }
 
@@ -1984,8 +1985,28 @@ int snowb_render_clear_colour(const snowb_camera* cam, const float* clear_rgba, 
     TRY(render_cam(cam, c));
     if (!rgba || !zbuf || !clear_rgba) return fail(SNOWB_ERR_INVALID, "null pointer");
     LAUNCH(kr_clear, (uint64_t)c.W * c.H, 256, c.W * c.H, zbuf, rgba,
-           make_float4(clear_rgba[0], clear_rgba[1], clear_rgba[2], clear_rgba[3]));
+           make_float4(clear_rgba[0], clear_rgba[1], clear_rgba[2], clear_rgba[3]), aligned16(rgba));
     return SNOWB_OK;
+}
+
+// one block per SPLAT * n threads, not fewer that loop: sprites differ in size and finished
+// blocks make room for the next
+static unsigned splat_blocks(uint32_t n, int tpb)
+{
+    const uint64_t b = ((uint64_t)SPLAT * n + tpb - 1) / tpb;
+    return b < 1 ? 1u : (b > 0xffffffull ? 0xffffffu : (unsigned)b);
+}
+
+static RenderColour render_colour(const snowb_point_colour* colour)
+{
+    RenderColour rc;
+    std::memcpy(rc.rgb, colour->rgb, sizeof(rc.rgb));
+    rc.temp = colour->use_temperature ? 1 : 0;
+    std::memcpy(rc.cool, colour->coolest_rgb, sizeof(rc.cool));
+    std::memcpy(rc.hot, colour->hottest_rgb, sizeof(rc.hot));
+    rc.t_cool = colour->coolest_T;
+    rc.t_hot = colour->hottest_T;
+    return rc;
 }
 
 int snowb_render_points(const snowb_particle_data* set, uint32_t n, const snowb_camera* cam,
@@ -1997,16 +2018,10 @@ int snowb_render_points(const snowb_particle_data* set, uint32_t n, const snowb_
     if (draw > 31) return fail(SNOWB_ERR_INVALID, "at most 32 draws between clears");
     if (n >= (1u << 27)) return fail(SNOWB_ERR_INVALID, "more than 2^27 particles in one draw");
     if (n == 0) return SNOWB_OK;
-    RenderColour rc;
-    std::memcpy(rc.rgb, colour->rgb, sizeof(rc.rgb));
-    rc.temp = colour->use_temperature ? 1 : 0;
-    std::memcpy(rc.cool, colour->coolest_rgb, sizeof(rc.cool));
-    std::memcpy(rc.hot, colour->hottest_rgb, sizeof(rc.hot));
-    rc.t_cool = colour->coolest_T;
-    rc.t_hot = colour->hottest_T;
+    const RenderColour rc = render_colour(colour);
     const float* T = rc.temp ? set->T : nullptr;
-    LAUNCH(kr_depth, n, 128, c, rc, set->positions, T, n, draw, zbuf);
-    LAUNCH(kr_shade, (uint64_t)c.W * c.H, 256, c, rc, set->positions, T, draw, zbuf, rgba);
+    KL(kr_depth, splat_blocks(n, 128), 128, c, rc, set->positions, n, draw, zbuf);
+    LAUNCH(kr_shade, (uint64_t)c.W * c.H, 256, c, rc, set->positions, T, draw, zbuf, rgba, aligned16(rgba));
     return SNOWB_OK;
 }
 
@@ -2104,7 +2119,7 @@ int snowb_ssfr_sphere_depth(const snowb_particle_data* set, uint32_t n, const sn
     TRY(ssfr_cam(cam, ssfr, c));
     if (!set || !ssfr || !depth) return fail(SNOWB_ERR_INVALID, "null pointer");
     if (n == 0) return SNOWB_OK;
-    LAUNCH(ks_sphere_depth, n, 128, c, set->positions, n, reinterpret_cast<uint32_t*>(depth));
+    KL(ks_sphere_depth, splat_blocks(n, 128), 128, c, set->positions, n, reinterpret_cast<uint32_t*>(depth));
     return SNOWB_OK;
 }
 
@@ -2114,7 +2129,7 @@ int snowb_ssfr_thickness(const snowb_particle_data* set, uint32_t n, const snowb
     TRY(ssfr_cam(cam, nullptr, c));
     if (!set || !thick) return fail(SNOWB_ERR_INVALID, "null pointer");
     if (n == 0) return SNOWB_OK;
-    LAUNCH(ks_thickness, n, 128, c, set->positions, n, thick);
+    KL(ks_thickness, splat_blocks(n, 128), 128, c, set->positions, n, thick);
     return SNOWB_OK;
 }
 
@@ -2139,7 +2154,8 @@ int snowb_ssfr_compose(const snowb_camera* cam, const snowb_ssfr* ssfr, const fl
     TRY(ssfr_cam(cam, ssfr, c));
     TRY(ssfr_shade(ssfr, s));
     if (!depth || !thick || !scene_rgba || !scene_depth || !rgba) return fail(SNOWB_ERR_INVALID, "null pointer");
-    LAUNCH(ks_compose, (uint64_t)c.W * c.H, 256, c, s, depth, thick, scene_rgba, scene_depth, rgba);
+    LAUNCH(ks_compose, (uint64_t)c.W * c.H, 256, c, s, depth, thick, scene_rgba, scene_depth, rgba,
+           aligned16(scene_rgba), aligned16(rgba));
     return SNOWB_OK;
 }
 
@@ -2169,17 +2185,22 @@ int snowb_render_fluid(const snowb_particle_data* sph, uint32_t n_sph, const sno
     float* fdepth = scene_depth + np;
     float* tmp = fdepth + np;
     float* smooth = tmp + np;
-    // scene: the snow as point sprites over the clear colour, and its sphere depth
-    TRY(snowb_render_clear_colour(cam, ssfr->clear_color, scene, zbuf));
-    TRY(snowb_render_points(dem, n_dem, cam, snow_colour, 0, scene, zbuf));
-    TRY(snowb_ssfr_clear(cam, scene_depth, thick));
-    TRY(snowb_ssfr_clear(cam, fdepth, nullptr));
-    TRY(snowb_ssfr_sphere_depth(dem, n_dem, cam, ssfr, scene_depth));
-    // water: sphere depth, smoothed, thickness, composite
-    TRY(snowb_ssfr_sphere_depth(sph, n_sph, cam, ssfr, fdepth));
-    TRY(snowb_ssfr_smooth(cam, ssfr, fdepth, tmp, smooth));
-    TRY(snowb_ssfr_thickness(sph, n_sph, cam, thick));
-    TRY(snowb_ssfr_compose(cam, ssfr, smooth, thick, scene, scene_depth, rgba));
+    SsfrCam c;
+    SsfrShade s;
+    TRY(ssfr_cam(cam, ssfr, c));
+    TRY(ssfr_shade(ssfr, s));
+    if (n_dem >= (1u << 27)) return fail(SNOWB_ERR_INVALID, "more than 2^27 particles in one draw");
+    const RenderColour col = render_colour(snow_colour);
+    uint32_t* const sdepth = reinterpret_cast<uint32_t*>(scene_depth);
+    LAUNCH(ks_view_clear, np, 256, (uint32_t)np, zbuf, thick, sdepth, reinterpret_cast<uint32_t*>(fdepth));
+    const uint32_t b_snow = splat_blocks(n_dem, 128), b_water = splat_blocks(n_sph, 128);
+    KL(ks_view_splat, b_snow + b_water, 128, rc, col, c, dem->positions, n_dem, sph->positions, n_sph, zbuf,
+       reinterpret_cast<uint32_t*>(fdepth), thick, b_snow);
+    const uint32_t b_px = blocks_for(np, 256), b_depth = splat_blocks(n_dem, 256);
+    KL(ks_view_filter, b_px + b_depth, 256, rc, col, c, s, dem->positions, col.temp ? dem->T : nullptr, n_dem, zbuf,
+       scene, fdepth, tmp, sdepth, b_px);
+    LAUNCH(ks_bilateral, np, 256, c, s, tmp, smooth, 1);
+    LAUNCH(ks_compose, np, 256, c, s, smooth, thick, scene, scene_depth, rgba, 1, aligned16(rgba));
     return SNOWB_OK;
 }
 
