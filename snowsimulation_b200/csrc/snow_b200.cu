@@ -151,6 +151,7 @@ struct Ctx {
     uint8_t* active = nullptr;
     uint32_t *sc_flag = nullptr, *sc_list = nullptr;   // link super-cell lists (SCList)
     snowb_float3* tmp_vel = nullptr;
+    float4 *attr_s = nullptr, *attr_d = nullptr;   // neighbour attributes by sorted index (heat, XSPH)
     uint32_t *nl_e = nullptr, *nl_cnt = nullptr;
     uint32_t *nl2_e = nullptr, *nl2_cnt = nullptr;   // the first density pass's snow lists (link formation)
     // link formation's copy of the snow set's sorted view, taken after the sort point that
@@ -194,7 +195,7 @@ static void free_ctx(Ctx& c)
     for (auto& s : c.s) free_set(s);
     free_set(c.b);
     free_set(c.gen);
-    void* ptrs[] = {c.fl_s, c.fl_d, c.rk_s, c.rk_d, c.sbsum, c.active, c.sc_flag, c.sc_list, c.tmp_vel,
+    void* ptrs[] = {c.fl_s, c.fl_d, c.rk_s, c.rk_d, c.sbsum, c.active, c.sc_flag, c.sc_list, c.tmp_vel, c.attr_s, c.attr_d,
                     c.epart, c.eout, c.link_terms, c.contact, c.psid,
                     c.pbuf.positions, c.pbuf.predict_positions, c.pbuf.new_positions, c.pbuf.velocity, c.pbuf.force,
                     c.pbuf.correction, c.pbuf.mass, c.pbuf.massInv, c.pbuf.contrib, c.pbuf.density, c.pbuf.C,
@@ -260,7 +261,7 @@ static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
     TRY(dalloc(&c.active, c.cap));
     TRY(dalloc(&c.sc_flag, ncells / 8 + 1)); TRY(dalloc(&c.sc_list, ncells / 8 + 1));
     CUDA_TRY(cudaMemset(c.sc_flag, 0, sizeof(uint32_t) * (ncells / 8 + 1)));
-    TRY(dalloc(&c.tmp_vel, c.cap));
+    TRY(dalloc(&c.tmp_vel, c.cap)); TRY(dalloc(&c.attr_s, c.cap)); TRY(dalloc(&c.attr_d, c.cap));
     TRY(dalloc(&c.nl_e, (size_t)NLIST_K * 2 * c.cap));
     TRY(dalloc(&c.nl_cnt, 2 * (size_t)c.cap));
     TRY(dalloc(&c.nl2_e, (size_t)NLIST_K * 2 * c.cap));
@@ -746,7 +747,12 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     const int commit_in_flags = beside && a.temperature && a.change_phase;
     if (a.temperature) {
         if (a.small_heat) TLAUNCH_AS("k_heat", k_heat_warp, SMALL_TPB, 32ull * a.particles, SMALL_TPB, P, S, vs, vd, X, a.dt);
-        else TLAUNCH(k_heat, 256, 2 * full, 128, P, S, vs, vd, X, a.dt);
+        else if (P.quirks == SNOWB_QUIRKS_REFERENCE) {
+            TLAUNCH_AS("k_heat", k_heat<true>, 256, 2 * full, 128, P, S, vs, vd, X, a.dt, nullptr, nullptr);
+        } else {
+            LAUNCH(k_pair_attrs, 2 * full, 256, S, vs, vd, X, 1, c.attr_s, c.attr_d);
+            TLAUNCH_AS("k_heat", k_heat<false>, 256, 2 * full, 128, P, S, vs, vd, X, a.dt, c.attr_s, c.attr_d);
+        }
         if (!commit_in_flags) LAUNCH(k_heat_commit, 2 * full, 256, S, X, a.dTe, step_sph ? 1 : 0, step_dem ? 1 : 0);
     }
     STOP(3);
@@ -935,21 +941,27 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     STOP(90);
     // apply_XSPH_viscosity (:3663-3711), Jacobi
     // both forms give the same results; the choice only follows the set sizes at the call
-    if (step_sph) {
-        if (a.xsph_thread[0])
-            TLAUNCH(k_xsph_thread, 256, full, 128, P, S, vs, vd, *a.sph, *a.dem, 1, P.sph_visc, c.tmp_vel);
+    bool attrs = false;   // the neighbour attributes of the one-thread form are formed
+    auto xsph = [&](bool water) -> int {
+        const bool thread = a.xsph_thread[water ? 0 : 1] != 0;
+        const SetView &own = water ? vs : vd, &oth = water ? vd : vs;
+        const snowb_particle_data &A = water ? *a.sph : *a.dem, &B = water ? *a.dem : *a.sph;
+        float4 *const aown = water ? c.attr_s : c.attr_d, *const aoth = water ? c.attr_d : c.attr_s;
+        const float visc = water ? P.sph_visc : P.dem_visc;
+        if (thread && !attrs) {
+            LAUNCH(k_pair_attrs, 2 * full, 256, S, vs, vd, X, 0, c.attr_s, c.attr_d);
+            attrs = true;
+        }
+        if (thread)
+            TLAUNCH(k_xsph_thread, 256, full, 128, P, S, own, oth, A, B, aown, aoth, water ? 1 : 0, visc, c.tmp_vel);
         else
-            TLAUNCH(k_xsph_warp, 256, (uint64_t)full * 32, 128, P, S, vs, vd, *a.sph, *a.dem, 1, P.sph_visc, c.tmp_vel);
-        LAUNCH(k_xsph_commit, full, 256, P, S, vs, 1, c.tmp_vel, a.sph->velocity);
-    }
+            TLAUNCH(k_xsph_warp, 256, (uint64_t)full * 32, 128, P, S, own, oth, A, B, water ? 1 : 0, visc, c.tmp_vel);
+        LAUNCH(k_xsph_commit, full, 256, P, S, own, water ? 1 : 0, c.tmp_vel, A.velocity, attrs ? aown : nullptr);
+        return SNOWB_OK;
+    };
+    if (step_sph) TRY(xsph(true));
     TAPE_HOOK(5, 0);
-    if (a.dem_visc && step_dem) {
-        if (a.xsph_thread[1])
-            TLAUNCH(k_xsph_thread, 256, full, 128, P, S, vd, vs, *a.dem, *a.sph, 0, P.dem_visc, c.tmp_vel);
-        else
-            TLAUNCH(k_xsph_warp, 256, (uint64_t)full * 32, 128, P, S, vd, vs, *a.dem, *a.sph, 0, P.dem_visc, c.tmp_vel);
-        LAUNCH(k_xsph_commit, full, 256, P, S, vd, 0, c.tmp_vel, a.dem->velocity);
-    }
+    if (a.dem_visc && step_dem) TRY(xsph(false));
     TAPE_HOOK(6, 0);
 #undef STOP
     return SNOWB_OK;

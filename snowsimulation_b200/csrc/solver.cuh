@@ -1486,6 +1486,54 @@ __global__ void k_finalize(DevParams P, const DevState* __restrict__ S, Sets X, 
     }
 }
 
+// One-thread walk of the 27 cells around p: hit(j, d2) for every member with d2 < lim but skip,
+// in cell order, index ascending, close() after each cell that has members in reach.  Current
+// ranges are screened two members at a time with packed arithmetic against the slightly larger
+// cull, then the exact test (see d2_pair).
+template <class H, class C>
+__device__ __forceinline__ void walk27(const SetView& v, const Nbhd& nb, float3 p, uint32_t skip, float lim, float cull,
+                                       H&& hit, C&& close)
+{
+    const P2 pp = bcast2(p);
+    FOR27 {
+        uint32_t s, e;
+        if (!v.range_nb(nb, ox, oy, oz, s, e)) continue;
+        auto test = [&](uint32_t j, float3 q) {
+            const float3 d = sub3(p, q);
+            const float d2 = dot3(d, d);
+            if (d2 < lim && j != skip) hit(j, d2);
+        };
+        if (e <= v.n) {
+            for (uint32_t j = s; j < e; j += 2u) {
+                const bool two = j + 1u < e;
+                const float4 q0 = __ldg(v.p4 + j), q1 = __ldg(v.p4 + (two ? j + 1u : j));
+                const float2 dd = d2_pair(pp, q0, q1);
+                if (dd.x < cull) test(j, xyz(q0));
+                if (dd.y < cull && two) test(j + 1u, xyz(q1));
+            }
+        } else {
+            for (uint32_t j = s; j < e; ++j) test(j, v.pos(j));
+        }
+        close();
+    }
+}
+// Neighbour attributes of heat and XSPH by sorted index, for the one-thread forms: (velocity, or
+// (T, 0, 0), mass / density).  A hit then costs one 16-byte load beside its position instead of
+// a gather of its index, three to five gathers behind it and a division, all of them once per
+// pair (32 scenes of 11,155 particles: heat 336 -> 261 us, XSPH 188 -> 144 us, this pass 4 us).
+__global__ void k_pair_attrs(const DevState* __restrict__ S, SetView vs, SetView vd, Sets X, int heat,
+                             float4* __restrict__ as, float4* __restrict__ ad)
+{
+    const uint32_t ns = S->n_sph, nd = S->n_dem;
+    GRID_LOOP(t, ns + nd) {
+        const bool w = t < ns;
+        const uint32_t i = w ? t : t - ns, o = w ? vs.gi[i] : vd.gi[i];
+        const snowb_particle_data& D = w ? X.sph : X.dem;
+        const float r = D.mass[o] / D.density[o];
+        const float3 a = heat ? f3(D.T[o], 0.f, 0.f) : ldv3(D.velocity, o);
+        (w ? as : ad)[i] = make_float4(a.x, a.y, a.z, r);
+    }
+}
 // ======================================================================== heat
 // heat_transfer_cell (:3764-3810) over one cell
 __device__ __forceinline__ float heat_cell(const DevParams& P, const SetView& v, const snowb_particle_data& O,
@@ -1506,21 +1554,38 @@ __device__ __forceinline__ float heat_cell(const DevParams& P, const SetView& v,
         }
     return res;
 }
+// dT plus the cells' sums over one set; attr: see k_pair_attrs (fixed quirks)
+template <bool REF>
 __device__ __forceinline__ float heat_sum(const DevParams& P, float dT, const SetView& v, const snowb_particle_data& O,
-                                          GCell g, uint32_t skip, float3 p, float Ti, float kk)
+                                          const float4* __restrict__ attr, GCell g, uint32_t skip, float3 p, float Ti,
+                                          float kk)
 {
-    if (P.quirks == SNOWB_QUIRKS_REFERENCE) {
+    if (REF) {
         // Q7: the reference passes the particle's own cell to all 27 calls
         const float s = heat_cell(P, v, O, g, 0, 0, 0, skip, p, Ti, kk);
         for (int k = 0; k < 27; ++k) dT += s;
         return dT;
     }
-    FOR27 dT += heat_cell(P, v, O, g, ox, oy, oz, skip, p, Ti, kk);
+    const Nbhd nb = make_nbhd(P, g, p, P.h2_cull);
+    float cs = 0.f;
+    walk27(v, nb, p, skip, P.h2_lt, P.h2_cull, [&](uint32_t j, float d2) {
+        float T, r;
+        if (j < v.n) {
+            const float4 a = __ldg(attr + j);
+            T = a.x; r = a.w;
+        } else {
+            const uint32_t oj = v.gi[j];
+            T = O.T[oj]; r = O.mass[oj] / O.density[oj];
+        }
+        cs += ((r * kk) * (T - Ti)) * L_visc(P, sqrtf(d2));
+    }, [&]() { dT += cs; cs = 0.f; });
     return dT;
 }
 // transfer_heat_sph / transfer_heat_dem (:3812-3937): new_T from T
+template <bool REF>   // the reference's quirk mode
 __global__ void __launch_bounds__(256) k_heat(DevParams P, const DevState* __restrict__ S, SetView vs, SetView vd,
-                                              Sets X, float dt)
+                                              Sets X, float dt, const float4* __restrict__ as,
+                                              const float4* __restrict__ ad)
 {
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     vs.n = ns; vd.n = nd;
@@ -1539,8 +1604,8 @@ __global__ void __launch_bounds__(256) k_heat(DevParams P, const DevState* __res
         float3 p = xyz(own.p4[i]); GCell g = grid_pos(P, p, own.scene(i));
         const float Ti = A.T[o];
         float dT = 0.f;
-        dT = heat_sum(P, dT, own, A, g, i, p, Ti, w ? kww : kss);
-        dT = heat_sum(P, dT, oth, B, g, SNOWB_UMAX, p, Ti, w ? kws : ksw);
+        dT = heat_sum<REF>(P, dT, own, A, w ? as : ad, g, i, p, Ti, w ? kww : kss);
+        dT = heat_sum<REF>(P, dT, oth, B, w ? ad : as, g, SNOWB_UMAX, p, Ti, w ? kws : ksw);
         dT = dT / ((w ? P.C_water : P.C_snow) * A.density[o]);
         A.new_T[o] = Ti + dT * dt;
     }
@@ -1754,40 +1819,67 @@ __global__ void __launch_bounds__(256) k_xsph_warp(DevParams P, const DevState* 
 // write the Jacobi results back (only the processed particles)
 // The same sums with one thread per particle, for sets large enough to fill the GPU with
 // threads (the warp form's 27-way split then costs more than it hides): the cell partials
-// are added in the same cell order as warp_ordered_sum adds them.
+// are added in the same cell order as warp_ordered_sum adds them, cells out of reach left out
+// (they would add 0).
+__device__ __forceinline__ float3 xsph_sum(const DevParams& P, float3 c, const SetView& v, const snowb_particle_data& O,
+                                           const float4* __restrict__ attr, const Nbhd& nb, float3 p, uint32_t skip,
+                                           float3 vi)
+{
+    float3 cs = f3(0.f, 0.f, 0.f);
+    walk27(v, nb, p, skip, P.h2_lt, P.h2_cull, [&](uint32_t j, float d2) {
+        float3 vj;
+        float a;
+        if (j < v.n) {
+            const float4 q = __ldg(attr + j);
+            vj = xyz(q); a = q.w;
+        } else {
+            const uint32_t oj = v.gi[j];
+            vj = ldv3(O.velocity, oj); a = O.mass[oj] / O.density[oj];
+        }
+        const float3 vij = sub3(vj, vi);
+        const float wgt = W_poly6(P, sqrtf(d2));
+        cs = add3(cs, f3((a * vij.x) * wgt, (a * vij.y) * wgt, (a * vij.z) * wgt));
+    }, [&]() { c = add3(c, cs); cs = f3(0.f, 0.f, 0.f); });
+    return c;
+}
 __global__ void __launch_bounds__(256) k_xsph_thread(DevParams P, const DevState* __restrict__ S, SetView vown,
                                                      SetView voth, snowb_particle_data A, snowb_particle_data B,
-                                                     int own_is_sph, float visc, snowb_float3* __restrict__ out_vel)
+                                                     const float4* __restrict__ attr_own,
+                                                     const float4* __restrict__ attr_oth, int own_is_sph, float visc,
+                                                     snowb_float3* __restrict__ out_vel)
 {
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     vown.n = own_is_sph ? ns : nd;
     voth.n = own_is_sph ? nd : ns;
     const uint32_t limit = own_is_sph ? ns
                          : (P.quirks == SNOWB_QUIRKS_REFERENCE ? umin32(coverage(ns), nd) : nd);
-    const float3 z = f3(0.f, 0.f, 0.f);
     GRID_LOOP(i, limit) {
         const uint32_t o = vown.gi[i];
         const float3 p = xyz(vown.p4[i]);
-        const GCell g = grid_pos(P, p, vown.scene(i));
+        const Nbhd nb = make_nbhd(P, grid_pos(P, p, vown.scene(i)), p, P.h2_cull);
         const float3 vi = ldv3(A.velocity, o);
-        float3 c = z;
-        FOR27 c = add3(c, xsph_cell(P, vown, A, A.velocity, p, g, ox, oy, oz, i, vi));
-        FOR27 c = add3(c, xsph_cell(P, voth, B, B.velocity, p, g, ox, oy, oz, SNOWB_UMAX, vi));
+        float3 c = f3(0.f, 0.f, 0.f);
+        c = xsph_sum(P, c, vown, A, attr_own, nb, p, i, vi);
+        c = xsph_sum(P, c, voth, B, attr_oth, nb, p, SNOWB_UMAX, vi);
         c = sc3(visc, c);
         st3(out_vel, o, add3(vi, c));
     }
 }
 // Sets processed by XSPH above this many particles take the one-thread form.
 constexpr uint32_t XSPH_WARP_MAX = 65536;
+// attr: the set's neighbour attributes that a later XSPH pass reads (or null)
 __global__ void k_xsph_commit(DevParams P, const DevState* __restrict__ S, SetView vown, int own_is_sph,
-                              const snowb_float3* __restrict__ in_vel, snowb_float3* __restrict__ vel)
+                              const snowb_float3* __restrict__ in_vel, snowb_float3* __restrict__ vel,
+                              float4* __restrict__ attr)
 {
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     const uint32_t limit = own_is_sph ? ns
                          : (P.quirks == SNOWB_QUIRKS_REFERENCE ? umin32(coverage(ns), nd) : nd);
     GRID_LOOP(i, limit) {
         const uint32_t o = vown.gi[i];
-        st3(vel, o, ldv3(in_vel, o));
+        const float3 v = ldv3(in_vel, o);
+        st3(vel, o, v);
+        if (attr) attr[i] = make_float4(v.x, v.y, v.z, attr[i].w);
     }
 }
 
