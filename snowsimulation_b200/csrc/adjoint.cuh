@@ -213,6 +213,7 @@ __device__ __forceinline__ void field_terms(const DevParams& P, const SetView& v
 __global__ void __launch_bounds__(ADJ_TPB) ka_boundary_base(DevParams P, uint32_t nb, SetView vb, Sets X, float* rho0,
                                                             float* S0)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_fields(DevParams P, uint32_t nw, u
                                                      AdjField fb, const float* __restrict__ rho0,
                                                      const float* __restrict__ S0)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns; vb.n = nb;
@@ -304,6 +306,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_pbf_lambar(DevParams P, uint32_t n
                                                          SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
                                                          AdjField fb, AdjSet aw)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns; vb.n = nb;
@@ -360,6 +363,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_pos_rev(DevParams P, uint32_t nw, 
                                                   SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
                                                   AdjField fb, AdjSet aw, AdjSet as, float* __restrict__ kst, int pbf, int contact)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns; vb.n = nb;
@@ -470,6 +474,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_pos_rev(DevParams P, uint32_t nw, 
 // float, one double atomic per warp.
 __global__ void ka_param_sum(uint32_t n, const float* __restrict__ a, const float* __restrict__ b, double* ga, double* gb)
 {
+    wait_prior();
     float x = 0.f, y = 0.f;
     GRID_LOOP(t, n) {
         x += a[t];
@@ -506,6 +511,7 @@ __global__ void ka_interlink_rev(DevParams P, uint32_t ns, const snowb_float3* _
                                  const uint32_t* __restrict__ rec, const float* __restrict__ len,
                                  const float* __restrict__ invm, AdjSet as, AdjParams G, float* Lbar)
 {
+    wait_prior();
     const uint32_t M = P.maxc;
     float kref_acc = 0.f;
     GRID_LOOP(i, ns) {
@@ -553,6 +559,7 @@ __global__ void ka_linkform_rev(DevParams P, uint32_t ns, const snowb_float3* __
                                 const uint32_t* __restrict__ rec_pre, const uint32_t* __restrict__ rec0,
                                 float* Lbar, snowb_float3* xb)
 {
+    wait_prior();
     const uint32_t M = P.maxc;
     GRID_LOOP(i, ns) {
         const float3 xi = ldv3(x0, i);
@@ -611,6 +618,7 @@ __device__ __forceinline__ void friction_vjp(const DevParams& P, float3 dx, floa
 __global__ void __launch_bounds__(ADJ_TPB) ka_friction_rev(DevParams P, uint32_t ns, uint32_t nb, SetView vs, SetView vb,
                                                            Sets X, AdjSet as)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     vs.n = ns; vb.n = nb;
@@ -668,6 +676,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA,
                                                    snowb_float3* vbA, snowb_float3* vbB, snowb_float3* xbA,
                                                    snowb_float3* xbB, float* rhobA, float* rhobB)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     vA.n = nA; vB.n = nB;
@@ -745,6 +754,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw,
                                                    AdjSet as, float* __restrict__ gkw_t, float* __restrict__ gks_t,
                                                        float dt)
 {
+    wait_prior();
     __shared__ AdjBuf bufs[ADJ_TPB / 32];
     AdjBuf& W = bufs[threadIdx.x >> 5];
     vw.n = nw; vs.n = ns;
@@ -825,6 +835,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw,
 __global__ void ka_finalize_rev(uint32_t n, float dt, const snowb_float3* __restrict__ vb, snowb_float3* xb,
                                 snowb_float3* x0b)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         const float3 v = div3(ldv3(vb, i), dt);
         st3(xb, i, add3(ldv3(xb, i), v));
@@ -838,6 +849,7 @@ __global__ void ka_integrate_rev(DevParams P, uint32_t n, float dt, int cd_on, c
                                  const snowb_float3* __restrict__ v0, const snowb_float3* __restrict__ xpb,
                                  const snowb_float3* __restrict__ x0b, snowb_float3* xout, snowb_float3* vout)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         const float3 xp_b = ldv3(xpb, i);
         float3 posb = add3(ldv3(x0b, i), xp_b);
@@ -882,6 +894,7 @@ __global__ void ka_integrate_rev(DevParams P, uint32_t n, float dt, int cd_on, c
 __global__ void ka_check_contrib(uint32_t nw, uint32_t ns, const float* __restrict__ cw, const float* __restrict__ cs,
                                  uint32_t* viol)
 {
+    wait_prior();
     GRID_LOOP(t, nw + ns) {
         const float c = t < nw ? cw[t] : cs[t - nw];
         if (c != 1.f) atomicOr(viol, 2u);
@@ -889,17 +902,20 @@ __global__ void ka_check_contrib(uint32_t nw, uint32_t ns, const float* __restri
 }
 __global__ void ka_check_phase(const DevState* __restrict__ S, uint32_t* viol)
 {
+    wait_prior();
     if (blockIdx.x == 0 && threadIdx.x == 0 && S->changed) atomicOr(viol, 1u);
 }
 // out = s * a
 __global__ void ka_scale3(uint32_t n, snowb_float3* out, float s, const snowb_float3* __restrict__ a)
 {
+    wait_prior();
     GRID_LOOP(i, n) st3(out, i, sc3(s, ldv3(a, i)));
 }
 // out = a + s * b  (float3 arrays, first n entries)
 __global__ void ka_axpy3(uint32_t n, snowb_float3* out, const snowb_float3* __restrict__ a, float s,
                          const snowb_float3* __restrict__ b)
 {
+    wait_prior();
     GRID_LOOP(i, n) st3(out, i, add3(ldv3(a, i), sc3(s, ldv3(b, i))));
 }
 

@@ -78,6 +78,11 @@ struct DevState {
 #define SNOWB_DEVERR_SCENE 2u      // a batched scene id >= the scene count
 
 // ---------------------------------------------------------------- float3 helpers
+// The first statement of every kernel.  Kernels are launched with programmatic stream
+// serialization (launch_prior in snow_b200.cu): their launch overlaps the end of the kernel before
+// them, whose writes are there only behind this wait.  A kernel without it could also finish
+// before the one ahead of its predecessor.
+__device__ __forceinline__ void wait_prior() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 __device__ __forceinline__ float3 add3(float3 a, float3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ float3 sub3(float3 a, float3 b) { return f3(a.x - b.x, a.y - b.y, a.z - b.z); }

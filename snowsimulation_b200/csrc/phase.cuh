@@ -72,6 +72,7 @@ __global__ void k_phase_flags(DevParams P, const DevState* __restrict__ S, snowb
                               snowb_particle_data dem, int freeze, int melt, uint32_t* __restrict__ fl_s,
                               uint32_t* __restrict__ fl_d, int commit, float dTe, int env_sph, int env_dem)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     GRID_LOOP(t, ns + nd) {
         const bool w = t < ns;
@@ -100,6 +101,7 @@ __global__ void k_phase_move(DevParams P, DevState* __restrict__ S, snowb_partic
                              const uint32_t* __restrict__ rk_s, const uint32_t* __restrict__ fl_d,
                              const uint32_t* __restrict__ rk_d, SceneIds sc)
 {
+    wait_prior();
     const bool changed = (S->n_freeze + S->n_melt) != 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) S->changed = changed ? 1u : 0u;
     if (!changed) return;
@@ -151,6 +153,7 @@ struct CompactPair {
 __global__ void k_copy_to_buffer(DevParams P, const DevState* __restrict__ S, const __grid_constant__ CompactPair Q,
                                  uint32_t full)
 {
+    wait_prior();
     if (S->changed == 0) return;
     const uint32_t M = P.maxc;
 #pragma unroll 1
@@ -175,6 +178,7 @@ __global__ void k_copy_to_buffer(DevParams P, const DevState* __restrict__ S, co
 // that stays keeps its iter_end either way.
 __global__ void k_scatter_set(DevParams P, DevState* S, const __grid_constant__ CompactPair Q, uint32_t full)
 {
+    wait_prior();
     if (S->changed == 0) return;
     const uint32_t M = P.maxc;
 #pragma unroll 1
@@ -222,6 +226,7 @@ __device__ __forceinline__ void update_record(const DevParams& P, const DevState
 __global__ void k_compact_finish(DevParams P, DevState* S, snowb_particle_data sph, snowb_particle_data dem,
                                  uint32_t full, int records)
 {
+    wait_prior();
     const bool full_clean = S->changed || S->tail_dirty;
     const uint32_t sn = S->new_sph, dn = S->new_dem, M = P.maxc;
     const uint32_t hs = S->tail_dirty ? full : umin32(full, umax32(S->clean_hi[0], S->n_sph + S->n_melt));
@@ -254,6 +259,7 @@ __global__ void k_compact_finish(DevParams P, DevState* S, snowb_particle_data s
 // the clean mark of the tails, and the tail flag cleared.
 __global__ void k_commit_sizes(DevState* S)
 {
+    wait_prior();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // after a clean every slot past the new sizes is clean
         if (S->changed || S->tail_dirty) { S->clean_hi[0] = S->new_sph; S->clean_hi[1] = S->new_dem; }
@@ -347,6 +353,7 @@ __global__ void __launch_bounds__(256) k_link_filter(DevParams P, DevState* S, S
                                                      snowb_particle_data dem, int dynamic,
                                                      uint8_t* __restrict__ active, NList L, SCList sc)
 {
+    wait_prior();
     const uint32_t nd = S->n_dem, M = P.maxc;
     vd.n = nd;
     const bool lists = L.cnt != nullptr && S->changed == 0;
@@ -757,6 +764,7 @@ constexpr uint32_t LINK_TPB = 256;
 __global__ void __launch_bounds__(128) k_link_filter_warp(DevParams P, DevState* S, SetView vd, snowb_particle_data dem,
                                                           int dynamic, uint8_t* __restrict__ active, NList L, SCList sc)
 {
+    wait_prior();
     __shared__ LinkGather gather[4];
     const uint32_t nd = S->n_dem, M = P.maxc, lane = threadIdx.x & 31u, full = 0xffffffffu;
     vd.n = nd;
@@ -824,6 +832,7 @@ __global__ void __launch_bounds__(LINK_TPB, 3) k_link_colour_warp(DevParams P, D
                                                                const uint8_t* __restrict__ active, uint32_t colour,
                                                                int dynamic, NList L, SCList sc)
 {
+    wait_prior();
     __shared__ uint32_t c_e[LINK_BATCH][LINK_CAND];     // partner | cell << 25
     __shared__ float c_d[LINK_BATCH][LINK_CAND];        // distance
     __shared__ uint32_t a_i[LINK_BATCH], a_o[LINK_BATCH], a_tol[LINK_BATCH], a_n[LINK_BATCH];
@@ -1017,6 +1026,7 @@ __global__ void k_copy_link_view(SetView v, uint32_t full, uint32_t ncells, floa
                                  uint32_t* __restrict__ gh, uint32_t* __restrict__ sid, uint32_t* __restrict__ cs,
                                  uint32_t* __restrict__ ce)
 {
+    wait_prior();
     const uint32_t m = full > ncells ? full : ncells;
     GRID_LOOP(k, m) {
         if (k < full) {
@@ -1033,6 +1043,7 @@ __global__ void k_copy_link_view(SetView v, uint32_t full, uint32_t ncells, floa
 __global__ void k_link_colour(DevParams P, DevState* S, SetView vd, snowb_particle_data dem,
                               const uint8_t* __restrict__ active, uint32_t colour, int dynamic)
 {
+    wait_prior();
     vd.n = S->n_dem;
     const uint32_t qx = P.gsx >> 2, qy = P.gsy >> 2, qz = P.gsz >> 2;
     const uint32_t total = qx * qy * qz;
@@ -1059,6 +1070,7 @@ __global__ void k_link_colour(DevParams P, DevState* S, SetView vd, snowb_partic
 // cap (an out-of-bounds read); that partner loop is skipped here.
 __global__ void k_adjust_links(DevParams P, DevState* S, snowb_particle_data d, uint32_t full)
 {
+    wait_prior();
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     const uint32_t n = S->n_dem, M = P.maxc;
     for (uint32_t i = 0; i < n; ++i) {

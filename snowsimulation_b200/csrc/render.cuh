@@ -153,6 +153,7 @@ __device__ __forceinline__ void splat_points(const RenderCam& c, const RenderCol
 __global__ void __launch_bounds__(128) kr_depth(RenderCam c, RenderColour rc, const snowb_float3* __restrict__ pos,
                                                 uint32_t n, uint32_t draw, unsigned long long* zbuf)
 {
+    wait_prior();
     splat_points<false>(c, rc, pos, n, draw, zbuf, blockIdx.x, gridDim.x);
 }
 // one pixel of the image, in one 16-byte store where the image is aligned for it (v4)
@@ -182,6 +183,7 @@ __global__ void kr_shade(RenderCam c, RenderColour rc, const snowb_float3* __res
                          const float* __restrict__ T, uint32_t draw, const unsigned long long* __restrict__ zbuf,
                          float* __restrict__ rgba, int v4)
 {
+    wait_prior();
     GRID_LOOP(k, c.W * c.H) {
         float4 o;
         if (shade_pixel(c, rc, pos, T, draw, zbuf[k], k, o)) put_pixel(rgba, k, o, v4);
@@ -189,6 +191,7 @@ __global__ void kr_shade(RenderCam c, RenderColour rc, const snowb_float3* __res
 }
 __global__ void kr_clear(uint32_t npix, unsigned long long* zbuf, float* rgba, float4 clear, int v4)
 {
+    wait_prior();
     GRID_LOOP(k, npix) {
         zbuf[k] = ~0ull;
         put_pixel(rgba, k, clear, v4);

@@ -441,6 +441,7 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
                                                  SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, NList L,
                                                  int with_bnd, BndBase base)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b, nbt = with_bnd ? nb : 0u;
     vs.n = ns; vd.n = nd; vb.n = nb;
     const bool ready = S->base_ready != 0u;
@@ -595,6 +596,7 @@ __global__ void __launch_bounds__(256) k_density_warp(DevParams P, DevState* __r
                                                       SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, NList L,
                                                       int with_bnd, BndBase base)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b, nbg = with_bnd ? (nb + 31u) / 32u : 0u;
     vs.n = ns; vd.n = nd; vb.n = nb;
     const bool ready = S->base_ready != 0u;
@@ -836,6 +838,7 @@ __global__ void __launch_bounds__(256) k_pbf(DevParams P, DevState* __restrict__
                                              SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, float dt,
                                              StageFlags F, NList L, int apply, SortTrack ts)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b;
     vs.n = ns; vd.n = nd; vb.n = nb;
     const bool ref = P.quirks == SNOWB_QUIRKS_REFERENCE;
@@ -946,6 +949,7 @@ __global__ void __launch_bounds__(256) k_dem_corr(DevParams P, const DevState* _
                                                   SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, StageFlags F,
                                                   NList L, float4* __restrict__ sums)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b;
     vs.n = ns; vd.n = nd; vb.n = nb;
     const float3 z = f3(0.f, 0.f, 0.f);
@@ -985,6 +989,7 @@ __global__ void __launch_bounds__(SMALL_TPB) k_dem_corr_warp(DevParams P, const 
                                                              SetView vd, SetView vb, Sets X, Sorted ss, Sorted sd,
                                                              Sorted sb, StageFlags F, float4* __restrict__ sums)
 {
+    wait_prior();
     __shared__ CellBuf bufs[SMALL_TPB / 32];
     CellBuf& W = bufs[threadIdx.x >> 5];
     const uint32_t nd = S->n_dem, lane = threadIdx.x & 31u;
@@ -1060,6 +1065,7 @@ __device__ __forceinline__ float3 link_term(const DevParams& P, const snowb_part
 __global__ void __launch_bounds__(256) k_link_terms(DevParams P, const DevState* __restrict__ S,
                                                     snowb_particle_data dem, float4* __restrict__ terms)
 {
+    wait_prior();
     const uint32_t nd = S->n_dem, M = P.maxc;
     // Plain (cached) loads: a record that a partner deletes during the pass is one whose term
     // is zero at both ends, so whether this thread still sees it, or sees its length already
@@ -1077,6 +1083,7 @@ __global__ void __launch_bounds__(256) k_link_terms(DevParams P, const DevState*
 __global__ void __launch_bounds__(256) k_link_sum(DevParams P, const DevState* __restrict__ S,
                                                   snowb_particle_data dem, const float4* __restrict__ terms)
 {
+    wait_prior();
     const uint32_t nd = S->n_dem, M = P.maxc;
     const float3 z = f3(0.f, 0.f, 0.f);
     GRID_LOOP(o, nd) {
@@ -1106,6 +1113,7 @@ __global__ void __launch_bounds__(256) k_link_apply(DevParams P, DevState* __res
                                                     const float4* __restrict__ sums, int correct_dem, int apply,
                                                     SortTrack td)
 {
+    wait_prior();
     const uint32_t nd = S->n_dem, M = P.maxc;
     const uint32_t ld = apply ? launch_limit(P, S->n0_dem, nd) : 0u;
     const float3 z = f3(0.f, 0.f, 0.f);
@@ -1142,6 +1150,7 @@ __global__ void __launch_bounds__(256) k_link_apply(DevParams P, DevState* __res
 __global__ void k_apply(DevParams P, DevState* __restrict__ S, SetView vs, SetView vd, Sets X, int do_sph,
                         int do_dem, SortTrack ts, SortTrack td)
 {
+    wait_prior();
     const uint32_t ls = do_sph ? launch_limit(P, S->n0_sph, S->n_sph) : 0u;
     const uint32_t ld = do_dem ? launch_limit(P, S->n0_dem, S->n_dem) : 0u;
     GRID_LOOP(t, ls + ld) {
@@ -1201,6 +1210,7 @@ __global__ void __launch_bounds__(256) k_friction(DevParams P, const DevState* _
                                                   Sets X, Sorted sd, Sorted sb, NList L, int lists, int only_lists,
                                                   SortTrack td)
 {
+    wait_prior();
     __shared__ uint32_t rec_sh[FR_K * 256];
     uint32_t* const rec = rec_sh + threadIdx.x;     // entry k at rec[k * blockDim.x]
     const uint32_t bd = blockDim.x;
@@ -1379,6 +1389,7 @@ __global__ void __launch_bounds__(SMALL_TPB) k_friction_warp(DevParams P, const 
                                                              SetView vb, Sets X, Sorted sd, Sorted sb, int lists,
                                                              int unless_lists, SortTrack td)
 {
+    wait_prior();
     if (unless_lists && friction_lists(S, lists)) return;   // k_friction replays them
     __shared__ CellBuf bufs[SMALL_TPB / 32];
     CellBuf& W = bufs[threadIdx.x >> 5];
@@ -1453,6 +1464,7 @@ __device__ __forceinline__ void integrate_one(const DevParams& P, const snowb_pa
 __global__ void k_integrate(DevParams P, const DevState* __restrict__ S, Sets X, uint32_t full, float dt, int cd_on,
                             int do_sph, int do_dem, SortTrack ts, SortTrack td)
 {
+    wait_prior();
     const bool ref = P.quirks == SNOWB_QUIRKS_REFERENCE;
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     const uint32_t ls = do_sph ? (ref ? umin32(coverage(ns), full) : ns) : 0u;
@@ -1472,6 +1484,7 @@ __global__ void k_integrate(DevParams P, const DevState* __restrict__ S, Sets X,
 // finalize_correction (:1383-1408)
 __global__ void k_finalize(DevParams P, const DevState* __restrict__ S, Sets X, float dt, int do_sph, int do_dem)
 {
+    wait_prior();
     const uint32_t ls = do_sph ? launch_limit(P, S->n0_sph, S->n_sph) : 0u;
     const uint32_t ld = do_dem ? launch_limit(P, S->n0_dem, S->n_dem) : 0u;
     GRID_LOOP(t, ls + ld) {
@@ -1524,6 +1537,7 @@ __device__ __forceinline__ void walk27(const SetView& v, const Nbhd& nb, float3 
 __global__ void k_pair_attrs(const DevState* __restrict__ S, SetView vs, SetView vd, Sets X, int heat,
                              float4* __restrict__ as, float4* __restrict__ ad)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     GRID_LOOP(t, ns + nd) {
         const bool w = t < ns;
@@ -1587,6 +1601,7 @@ __global__ void __launch_bounds__(256) k_heat(DevParams P, const DevState* __res
                                               Sets X, float dt, const float4* __restrict__ as,
                                               const float4* __restrict__ ad)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     vs.n = ns; vd.n = nd;
     const float kww = ((4.f * P.k_water) * P.k_water) / (P.k_water + P.k_water);
@@ -1615,6 +1630,7 @@ __global__ void __launch_bounds__(256) k_heat(DevParams P, const DevState* __res
 __global__ void __launch_bounds__(SMALL_TPB) k_heat_warp(DevParams P, const DevState* __restrict__ S, SetView vs,
                                                          SetView vd, Sets X, float dt)
 {
+    wait_prior();
     __shared__ CellBuf bufs[SMALL_TPB / 32];
     CellBuf& W = bufs[threadIdx.x >> 5];
     const uint32_t ns = S->n_sph, nd = S->n_dem, lane = threadIdx.x & 31u;
@@ -1662,6 +1678,7 @@ __global__ void __launch_bounds__(SMALL_TPB) k_heat_warp(DevParams P, const DevS
 // thrust::copy new_T -> T (:3968-3969) then environmental_heat_transfer (:4847-4859)
 __global__ void k_heat_commit(const DevState* __restrict__ S, Sets X, float dTe, int env_sph, int env_dem)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     GRID_LOOP(t, ns + nd) {
         const bool w = t < ns;
@@ -1721,6 +1738,7 @@ __global__ void __launch_bounds__(256) k_pbf_water_warp(DevParams P, DevState* _
                                                         SetView vd, SetView vb, Sets X, Sorted ss, Sorted sd,
                                                         Sorted sb, float dt, StageFlags F, int apply, SortTrack ts)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph;
     if (ns > PBF_WARP_MAX_WATER) return;   // k_pbf runs the water terms one thread each
     vs.n = ns; vd.n = S->n_dem; vb.n = S->n_b;
@@ -1793,6 +1811,7 @@ __global__ void __launch_bounds__(256) k_xsph_warp(DevParams P, const DevState* 
                                                    SetView voth, snowb_particle_data A, snowb_particle_data B,
                                                    int own_is_sph, float visc, snowb_float3* __restrict__ out_vel)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     vown.n = own_is_sph ? ns : nd;
     voth.n = own_is_sph ? nd : ns;
@@ -1848,6 +1867,7 @@ __global__ void __launch_bounds__(256) k_xsph_thread(DevParams P, const DevState
                                                      const float4* __restrict__ attr_oth, int own_is_sph, float visc,
                                                      snowb_float3* __restrict__ out_vel)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     vown.n = own_is_sph ? ns : nd;
     voth.n = own_is_sph ? nd : ns;
@@ -1872,6 +1892,7 @@ __global__ void k_xsph_commit(DevParams P, const DevState* __restrict__ S, SetVi
                               const snowb_float3* __restrict__ in_vel, snowb_float3* __restrict__ vel,
                               float4* __restrict__ attr)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem;
     const uint32_t limit = own_is_sph ? ns
                          : (P.quirks == SNOWB_QUIRKS_REFERENCE ? umin32(coverage(ns), nd) : nd);
@@ -1889,6 +1910,7 @@ __global__ void k_xsph_commit(DevParams P, const DevState* __restrict__ S, SetVi
 __global__ void k_boundary_volume(DevParams P, snowb_cell_data cd, const float* __restrict__ mass,
                                   float* __restrict__ volume, uint32_t n, const uint32_t* __restrict__ sid_o)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         const uint32_t o = cd.grid_index[i];
         float3 p = ldv3(cd.sorted_pos, i);
@@ -1918,6 +1940,7 @@ __global__ void k_boundary_prep(snowb_cell_data cd, const float* __restrict__ vo
                                 float* __restrict__ invm_s, float* __restrict__ mass_s,
                                 const uint32_t* __restrict__ sid_o, uint32_t* __restrict__ sid_s)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         const uint32_t o = cd.grid_index[i];
         float3 q = ldv3(cd.sorted_pos, i);
@@ -1929,6 +1952,7 @@ __global__ void k_boundary_prep(snowb_cell_data cd, const float* __restrict__ vo
 }
 __global__ void k_set_state(DevState* S, uint32_t ns, uint32_t nd, uint32_t nb)
 {
+    wait_prior();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         S->n_sph = ns; S->n_dem = nd; S->n_b = nb;
         S->n0_sph = ns; S->n0_dem = nd;
@@ -1947,6 +1971,7 @@ __global__ void k_set_state(DevState* S, uint32_t ns, uint32_t nd, uint32_t nb)
 __global__ void k_check_scenes(DevParams P, DevState* S, const uint32_t* __restrict__ sph,
                                const uint32_t* __restrict__ dem, const uint32_t* __restrict__ bnd)
 {
+    wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b;
     const uint32_t n = ns > nd ? (ns > nb ? ns : nb) : (nd > nb ? nd : nb);
     GRID_LOOP(i, n) {
@@ -1960,6 +1985,7 @@ __global__ void k_check_scenes(DevParams P, DevState* S, const uint32_t* __restr
 __global__ void k_energy_partial(const snowb_particle_data sph, uint32_t ns, const snowb_particle_data dem,
                                  uint32_t nd, double Cw, double Cs, double* __restrict__ part)
 {
+    wait_prior();
     __shared__ double sm[4][256];
     double a[4] = {0, 0, 0, 0};
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ns + nd; t += gridDim.x * blockDim.x) {
@@ -1983,6 +2009,7 @@ __global__ void k_energy_partial(const snowb_particle_data sph, uint32_t ns, con
 }
 __global__ void k_energy_final(const double* __restrict__ part, int nblocks, double* __restrict__ out)
 {
+    wait_prior();
     if (threadIdx.x < 4) {
         double s = 0;
         for (int b = 0; b < nblocks; ++b) s += part[4 * b + threadIdx.x];

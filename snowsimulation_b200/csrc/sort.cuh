@@ -114,6 +114,7 @@ __device__ __forceinline__ void begin_substep(DevState* S)
 }
 __global__ void k_sort_hash(DevParams P, const __grid_constant__ SortPair Q)
 {
+    wait_prior();
     uint32_t m[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) m[k] = !Q.on[k] ? 0u : (Q.S ? Q.S->moved[k] : 1u);
@@ -156,6 +157,7 @@ __global__ void k_key_count(const uint32_t* __restrict__ keys, const uint32_t* _
                             uint32_t ncells, uint32_t* __restrict__ key_o, uint32_t* __restrict__ val_o,
                             uint32_t* __restrict__ slot_o, uint32_t* __restrict__ cnt, uint32_t* err)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         uint32_t h = keys[i];
         if (h >= ncells) { atomicOr(err, 2u); h = ncells - 1; }
@@ -169,6 +171,7 @@ __global__ void k_key_count(const uint32_t* __restrict__ keys, const uint32_t* _
 __global__ void k_block_sums(const uint32_t* __restrict__ cnt, uint32_t ncells, uint32_t* __restrict__ bsum,
                              const uint32_t* cond)
 {
+    wait_prior();
     if (cond && *cond == 0) return;
     __shared__ uint32_t sm[SCAN_TPB / 32];
     const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
@@ -219,6 +222,7 @@ __device__ __forceinline__ void scan_chunk(uint32_t* __restrict__ cnt, uint32_t 
 __global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restrict__ bsum, uint32_t ncells,
                             uint32_t* __restrict__ off)
 {
+    wait_prior();
     __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
     __shared__ uint32_t s_prefix;
     if (threadIdx.x < 32) {
@@ -235,6 +239,7 @@ __global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restri
 // cell_start is cleared for c < clear (min(n, ncells) reproduces the reference's partial memset, Q1).
 __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ SortPair Q, uint32_t chunks)
 {
+    wait_prior();
     __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
     __shared__ uint32_t s_prefix;
     const int k = blockIdx.x < chunks ? 0 : 1;
@@ -273,10 +278,12 @@ __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ 
 __global__ void k_scatter(const uint32_t* __restrict__ key_o, const uint32_t* __restrict__ slot_o,
                           const uint32_t* __restrict__ off, uint32_t* __restrict__ tmp, uint32_t n)
 {
+    wait_prior();
     GRID_LOOP(o, n) tmp[off[key_o[o]] + slot_o[o]] = o;
 }
 __global__ void k_sort_scatter(const __grid_constant__ SortPair Q, uint32_t chunks)
 {
+    wait_prior();
     const bool s0 = Q.sorts(0), s1 = Q.sorts(1);
     if (Q.S && blockIdx.x == 0 && threadIdx.x == 0) {   // the scan pass has cleared what was left in the tables
         if (s0) Q.S->table_any[0] = 0u;
@@ -311,6 +318,7 @@ __device__ __forceinline__ uint32_t stable_rank(const uint32_t* __restrict__ tmp
 // by sorted slot.
 __global__ void k_sort_rank(const __grid_constant__ SortPair Q)
 {
+    wait_prior();
     const bool s0 = Q.sorts(0), s1 = Q.sorts(1);
     const uint32_t n0 = Q.size(0), n = n0 + Q.size(1);
     GRID_LOOP(t, n) {
@@ -355,6 +363,7 @@ __global__ void k_rank_pairs(const uint32_t* __restrict__ key_o, const uint32_t*
                              const uint32_t* __restrict__ off, const uint32_t* __restrict__ tmp,
                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         const uint32_t h = key_o[i], b = off[h], e = off[h + 1];
         const uint32_t p = b + stable_rank(tmp, b, e, i);
@@ -367,6 +376,7 @@ __global__ void k_rank_pairs(const uint32_t* __restrict__ key_o, const uint32_t*
 __global__ void k_calc_hash(DevParams P, snowb_cell_data cd, const snowb_float3* __restrict__ pos, uint32_t n,
                             const uint32_t* __restrict__ sid_o)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         float3 p = ldv3(pos, i);
         cd.grid_hash[i] = grid_hash(P, grid_pos(P, p, sid_o ? sid_o[i] : 0u), 0, 0, 0);
@@ -376,6 +386,7 @@ __global__ void k_calc_hash(DevParams P, snowb_cell_data cd, const snowb_float3*
 // reorderDataAndFindCellStartD (:242-301) alone; cell_start cleared beforehand
 __global__ void k_reorder(snowb_cell_data cd, const snowb_float3* __restrict__ pos, uint32_t n)
 {
+    wait_prior();
     GRID_LOOP(i, n) {
         const uint32_t h = cd.grid_hash[i];
         if (i == 0 || h != cd.grid_hash[i - 1]) {
@@ -400,6 +411,7 @@ struct ScanPair {
 };
 __global__ void k_scan_sums(const __grid_constant__ ScanPair Q, uint32_t blocks)
 {
+    wait_prior();
     const int k = blockIdx.x < blocks ? 0 : 1;
     const ScanSide& A = Q.a[k];
     const uint32_t b = blockIdx.x - (k ? blocks : 0u), n = A.n_ptr ? *A.n_ptr : A.n;
@@ -421,6 +433,7 @@ __global__ void k_scan_sums(const __grid_constant__ ScanPair Q, uint32_t blocks)
 }
 __global__ void k_scan_apply(const __grid_constant__ ScanPair Q, uint32_t blocks)
 {
+    wait_prior();
     const int k = blockIdx.x < blocks ? 0 : 1;
     const ScanSide& A = Q.a[k];
     const uint32_t b = blockIdx.x - (k ? blocks : 0u), n = A.n_ptr ? *A.n_ptr : A.n;

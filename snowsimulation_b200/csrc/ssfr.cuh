@@ -130,11 +130,13 @@ __device__ __forceinline__ void splat_spheres(const SsfrCam& c, const snowb_floa
 __global__ void __launch_bounds__(128) ks_sphere_depth(SsfrCam c, const snowb_float3* __restrict__ pos, uint32_t n,
                                                        uint32_t* depth)
 {
+    wait_prior();
     splat_spheres<true, false, false>(c, pos, n, depth, nullptr, nullptr, blockIdx.x, gridDim.x);
 }
 __global__ void __launch_bounds__(128) ks_thickness(SsfrCam c, const snowb_float3* __restrict__ pos, uint32_t n,
                                                     unsigned long long* thick)
 {
+    wait_prior();
     splat_spheres<false, true, false>(c, pos, n, nullptr, thick, nullptr, blockIdx.x, gridDim.x);
 }
 __device__ __forceinline__ float thickness_value(unsigned long long q, float clear_r)
@@ -193,6 +195,7 @@ __device__ __forceinline__ void bilateral(const SsfrCam& c, const SsfrShade& s, 
 __global__ void __launch_bounds__(256) ks_bilateral(SsfrCam c, SsfrShade s, const float* __restrict__ in,
                                                     float* __restrict__ out, int horizontal)
 {
+    wait_prior();
     __shared__ BilateralTaps B;
     bilateral(c, s, in, out, horizontal, B, blockIdx.x, gridDim.x);
 }
@@ -208,6 +211,7 @@ __global__ void ks_compose(SsfrCam c, SsfrShade s, const float* __restrict__ D, 
                            const float* __restrict__ scene, const float* __restrict__ SD, float* __restrict__ out,
                            int scene4, int out4)
 {
+    wait_prior();
     auto scene_at = [&](size_t t) {
         if (scene4) return __ldg(reinterpret_cast<const float4*>(scene) + t);
         return make_float4(scene[4 * t], scene[4 * t + 1], scene[4 * t + 2], scene[4 * t + 3]);
@@ -274,6 +278,7 @@ __global__ void ks_compose(SsfrCam c, SsfrShade s, const float* __restrict__ D, 
 __global__ void ks_fill(uint32_t npix, uint32_t* __restrict__ depth_bits, uint32_t value,
                         unsigned long long* __restrict__ thick)
 {
+    wait_prior();
     GRID_LOOP(k, npix) {
         if (depth_bits) depth_bits[k] = value;
         if (thick) thick[k] = 0ull;
@@ -295,6 +300,7 @@ __global__ void ks_view_clear(uint32_t npix, unsigned long long* __restrict__ zb
                               unsigned long long* __restrict__ thick, uint32_t* __restrict__ scene_depth,
                               uint32_t* __restrict__ fluid_depth)
 {
+    wait_prior();
     GRID_LOOP(k, npix) {
         zbuf[k] = ~0ull;
         thick[k] = 0ull;
@@ -307,6 +313,7 @@ __global__ void __launch_bounds__(128) ks_view_splat(RenderCam rc, RenderColour 
                                                      unsigned long long* zbuf, uint32_t* fluid_depth,
                                                      unsigned long long* thick, uint32_t split)
 {
+    wait_prior();
     if (blockIdx.x < split) splat_points<true>(rc, col, snow, n_snow, 0u, zbuf, blockIdx.x, split);
     else
         splat_spheres<true, true, false>(c, water, n_water, fluid_depth, thick, nullptr, blockIdx.x - split,
@@ -319,6 +326,7 @@ __global__ void __launch_bounds__(256) ks_view_filter(RenderCam rc, RenderColour
                                                       float* __restrict__ scene, const float* __restrict__ fluid_depth,
                                                       float* __restrict__ tmp, uint32_t* scene_depth, uint32_t split)
 {
+    wait_prior();
     __shared__ BilateralTaps B;
     if (blockIdx.x >= split) {
         splat_spheres<true, false, true>(c, snow, n_snow, scene_depth, nullptr, fluid_depth, blockIdx.x - split,
