@@ -35,6 +35,7 @@ struct DevParams {
     float h2_lt, r2_lt, r2_le;
     // box-culling thresholds: the cut-offs with a relative safety margin
     float h2_cull, r2_cull;
+    float s2, s2_cull, skin_move2;   // snow lists with a skin (NL_SKIN)
     // walls at x = wx0, wx1 and z = wz0, wz1, floor at y = floor_y (the reference: +-1, 0)
     float wx0, wx1, wz0, wz1, floor_y;
     int quirks;
@@ -73,6 +74,9 @@ struct DevState {
     uint32_t clean_hi[2];           // per set: every slot from here on is clean (k_commit_sizes)
     uint32_t base_ready;            // the call's boundary sums (BndBase) are formed
     uint32_t table_any[2];          // per set: the caller may have written the cell table (no sort since the call began)
+    // Snow lists with a skin (NL_SKIN): skin_ok while the snow keeps the sort that this substep's
+    // lists were made in; epoch counts the substeps (marks in SkinCells).
+    uint32_t skin_ok, epoch;
 };
 #define SNOWB_DEVERR_SCATTER 1u
 #define SNOWB_DEVERR_SCENE 2u      // a batched scene id >= the scene count

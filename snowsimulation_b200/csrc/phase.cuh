@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(256) k_link_filter(DevParams P, DevState* S, S
                 for (uint32_t u = 0; u < LF_G; ++u) {
                     if (k0 + u >= nl || act) break;
                     const uint32_t cell = (en[u] >> 25) & 31u;
-                    if (cell == skip_cell) continue;
+                    if (cell == skip_cell || (en[u] & NL_FAR)) continue;
                     if (o1[u] == o) { act = 1; break; }
                     bool found = false;
                     if (fast) {
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(128) k_link_filter_warp(DevParams P, DevState*
                 for (uint32_t k0 = 0; k0 < nl && more; k0 += 32u) {
                     const bool in = k0 + lane < nl;
                     const uint32_t en = in ? L.e[(size_t)(k0 + lane) * L.stride + L.cap + i] : 0u;
-                    more = look(in, in ? vd.gi[en & NL_J_MASK] : 0u, (en >> 25) & 31u);
+                    more = look(in && !(en & NL_FAR), in ? vd.gi[en & NL_J_MASK] : 0u, (en >> 25) & 31u);
                 }
             } else {
                 link_candidates(P, vd, i, gather[threadIdx.x >> 5], [&](bool in, uint32_t j, uint32_t cell, float) {
@@ -923,7 +923,8 @@ __global__ void __launch_bounds__(LINK_TPB, 3) k_link_colour_warp(DevParams P, D
                     for (uint32_t k0 = 0; k0 < nl && more; k0 += 32u) {
                         const bool in = k0 + lane < nl;
                         const uint32_t en = in ? L.e[(size_t)(k0 + lane) * L.stride + L.cap + i] : 0u, j = en & NL_J_MASK;
-                        more = keep(in, in ? vd.gi[j] : 0u, (en >> 25) & 31u, in ? len3(sub3(p, vd.pos(j))) : 0.f);
+                        more = keep(in && !(en & NL_FAR), in ? vd.gi[j] : 0u, (en >> 25) & 31u,
+                                    in ? len3(sub3(p, vd.pos(j))) : 0.f);
                     }
                 } else {
                     link_candidates(P, vd, i, gather[warp], [&](bool in, uint32_t j, uint32_t cell, float d2) {
@@ -956,8 +957,8 @@ __global__ void __launch_bounds__(LINK_TPB, 3) k_link_colour_warp(DevParams P, D
                             const uint32_t k = k0 + lane;
                             const bool in = k < nl;
                             const uint32_t en = in ? L.e[(size_t)k * L.stride + L.cap + i] : 0u, j = en & NL_J_MASK;
-                            more = link_chunk(P, dem, S, vd.n, l, map, in, in ? vd.gi[j] : 0u, (en >> 25) & 31u,
-                                              in ? len3(sub3(p, vd.pos(j))) : 0.f);
+                            more = link_chunk(P, dem, S, vd.n, l, map, in && !(en & NL_FAR), in ? vd.gi[j] : 0u,
+                                              (en >> 25) & 31u, in ? len3(sub3(p, vd.pos(j))) : 0.f);
                         }
                     } else {
                         link_candidates(P, vd, a_i[a], gather[0], [&](bool in, uint32_t j, uint32_t cell, float d2) {

@@ -106,6 +106,11 @@ static DevParams derive(const snowb_sim_params& s)
     P.r2_le = smallest_with_sqrt_gt(P.two_r);
     P.h2_cull = P.h2_lt * (1.f + 1e-5f);
     P.r2_cull = P.r2_le * (1.f + 1e-5f);
+    // pairs within h + skin when listed hold those within h after moves below 0.499 skin (the rest
+    // covers the rounding of the distances)
+    P.s2 = (P.h + NL_SKIN * P.h) * (P.h + NL_SKIN * P.h);
+    P.s2_cull = P.s2 * (1.f + 1e-5f);
+    P.skin_move2 = (0.499f * NL_SKIN * P.h) * (0.499f * NL_SKIN * P.h);
     P.quirks = SNOWB_QUIRKS_REFERENCE;
     {   // the s_corr term is -0 inside the support when scorr_coeff is +0 and its quotient
         // W / scorr_divisor (at most W(0) / scorr_divisor) stays finite to the fourth power
@@ -151,6 +156,8 @@ struct Ctx {
     uint8_t* active = nullptr;
     uint32_t *sc_flag = nullptr, *sc_list = nullptr;   // link super-cell lists (SCList)
     snowb_float3* tmp_vel = nullptr;
+    float4* skin_p4 = nullptr;           // the snow's positions when its lists with a skin were made
+    uint32_t* skin_far = nullptr;        // per cell: the last substep in which it was marked (NL_SKIN)
     float4 *attr_s = nullptr, *attr_d = nullptr;   // neighbour attributes by sorted index (heat, XSPH)
     uint32_t *nl_e = nullptr, *nl_cnt = nullptr;
     uint32_t *nl2_e = nullptr, *nl2_cnt = nullptr;   // the first density pass's snow lists (link formation)
@@ -195,7 +202,7 @@ static void free_ctx(Ctx& c)
     for (auto& s : c.s) free_set(s);
     free_set(c.b);
     free_set(c.gen);
-    void* ptrs[] = {c.fl_s, c.fl_d, c.rk_s, c.rk_d, c.sbsum, c.active, c.sc_flag, c.sc_list, c.tmp_vel, c.attr_s, c.attr_d,
+    void* ptrs[] = {c.fl_s, c.fl_d, c.rk_s, c.rk_d, c.sbsum, c.active, c.sc_flag, c.sc_list, c.tmp_vel, c.skin_p4, c.skin_far, c.attr_s, c.attr_d,
                     c.epart, c.eout, c.link_terms, c.contact, c.psid,
                     c.pbuf.positions, c.pbuf.predict_positions, c.pbuf.new_positions, c.pbuf.velocity, c.pbuf.force,
                     c.pbuf.correction, c.pbuf.mass, c.pbuf.massInv, c.pbuf.contrib, c.pbuf.density, c.pbuf.C,
@@ -261,7 +268,9 @@ static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
     TRY(dalloc(&c.active, c.cap));
     TRY(dalloc(&c.sc_flag, ncells / 8 + 1)); TRY(dalloc(&c.sc_list, ncells / 8 + 1));
     CUDA_TRY(cudaMemset(c.sc_flag, 0, sizeof(uint32_t) * (ncells / 8 + 1)));
-    TRY(dalloc(&c.tmp_vel, c.cap)); TRY(dalloc(&c.attr_s, c.cap)); TRY(dalloc(&c.attr_d, c.cap));
+    TRY(dalloc(&c.tmp_vel, c.cap)); TRY(dalloc(&c.skin_p4, c.cap));
+    TRY(dalloc(&c.skin_far, ncells));
+    CUDA_TRY(cudaMemset(c.skin_far, 0, sizeof(uint32_t) * ncells)); TRY(dalloc(&c.attr_s, c.cap)); TRY(dalloc(&c.attr_d, c.cap));
     TRY(dalloc(&c.nl_e, (size_t)NLIST_K * 2 * c.cap));
     TRY(dalloc(&c.nl_cnt, 2 * (size_t)c.cap));
     TRY(dalloc(&c.nl2_e, (size_t)NLIST_K * 2 * c.cap));
@@ -520,7 +529,7 @@ static int sort_sets(const DevParams& P, const SortPair& Q, uint64_t work)
     LAUNCH(k_sort_hash, work, 256, P, Q);
     KL(k_sort_scan, 2 * chunks, SCAN_TPB, Q, chunks);
     LAUNCH(k_sort_scatter, work, 256, Q, chunks);
-    LAUNCH(k_sort_rank, work, 256, Q);
+    LAUNCH(k_sort_rank, work, 256, P, Q);
     return SNOWB_OK;
 }
 
@@ -686,10 +695,10 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     Sorted sd{c.s[1].invm, c.s[1].contrib, c.s[1].lambda, nullptr};
     Sorted sb{c.b.invm, nullptr, c.b.lambda, c.b.mass};
     StageFlags F{a.correct_dem, a.sph_sph, a.interlink, step_sph ? 1 : 0, step_dem ? 1 : 0};
-    NList NL{c.nl_e, c.nl_cnt, 2 * cap, cap};
-    // the substep's first density pass lists the snow-snow candidates for link formation in
-    // a list of their own, which the iterations' density passes leave alone
-    NList NL2{c.nl2_e, c.nl2_cnt, 2 * cap, cap};
+    // the substep's first density pass lists the snow-snow candidates, for link formation and with
+    // a skin for the iterations' density passes (NL_SKIN), in a list of their own
+    NList NL2{c.nl2_e, c.nl2_cnt, 2 * cap, cap, nullptr, nullptr, nullptr};
+    NList NL{c.nl_e, c.nl_cnt, 2 * cap, cap, c.nl2_e, c.nl2_cnt, c.skin_far};
     // the friction pass may replay the density+lambda lists when a contact (d <= 2r) after a
     // move of at most FR_LIST_MOVE per particle was within h before it
     const bool fr_lists = P.two_r + 2.f * FR_LIST_MOVE < 0.9f * P.h;
@@ -741,7 +750,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
             view_pending = false;
         }
         const SortPair Q{{sort_side(c.s[0], *a.sph, a.scd, n_s, a.sid_sph), sort_side(c.s[1], *a.dem, a.dcd, n_d, a.sid_dem)},
-                         {need_s ? 1 : 0, need_d ? 1 : 0}, S, begin ? 1 : 0, P.ncells, ref ? 0 : 1};
+                         {need_s ? 1 : 0, need_d ? 1 : 0}, S, begin ? 1 : 0, P.ncells, ref ? 0 : 1, c.skin_p4, c.skin_far};
         TRY(sort_sets(P, Q, full));
         dirty_s = dirty_d = false;
         return SNOWB_OK;
@@ -763,7 +772,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
                    vd, vb, X, ss, sd, sb, NL2, bnd_first, c.b.base);
     else
         TLAUNCH(k_density<false>, 256, bnd_first ? work3 : 2 * full, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL2,
-                bnd_first, c.b.base);
+                bnd_first, c.b.base, c.skin_p4);
     STOP(2);
     // in a whole substep the phase flags pass commits the new temperatures itself
     const int commit_in_flags = beside && a.temperature && a.change_phase;
@@ -876,7 +885,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
             TLAUNCH_AS("k_density<true>", k_density_warp<true>, 256, dwork, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1,
                        c.b.base);
         else
-            TLAUNCH(k_density<true>, 256, work3, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1, c.b.base);
+            TLAUNCH(k_density<true>, 256, work3, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1, c.b.base, nullptr);
         STOP(base + 2);
         // with the interlink pass beside, the passes that finish a correction apply it (no
         // k_apply launch): the water PBF passes for the water, k_link_apply for the snow
@@ -1114,7 +1123,7 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         dw.predict_positions = const_cast<snowb_float3*>(F3(pw));
         ds.predict_positions = const_cast<snowb_float3*>(F3(ps));
         TRY(sort_sets(P, SortPair{{sort_side(B.sb[0], dw, B.cd[0], B.nbuf + 0), sort_side(B.sb[1], ds, B.cd[1], B.nbuf + 1)},
-                                  {1, 1}, nullptr, 0, P.ncells, 1}, (uint64_t)nw + ns));
+                                  {1, 1}, nullptr, 0, P.ncells, 1, nullptr, nullptr}, (uint64_t)nw + ns));
         return SNOWB_OK;
     };
     auto zero_rhob = [&]() -> int {
@@ -1561,12 +1570,12 @@ static int connect_links(const DevParams& P, snowb_particle_data* dem, uint32_t 
            sid, sid ? c.s[1].sid : nullptr);
     SetView vd = make_view(dcd, c.s[1].p4, dem->mass, sid ? c.s[1].sid : nullptr);
     const SCList scl = sc_lists(P);
-    LAUNCH(k_link_filter, n, 128, P, c.S, vd, *dem, dynamic, c.active, NList{nullptr, nullptr, 0u, 0u}, scl);
+    LAUNCH(k_link_filter, n, 128, P, c.S, vd, *dem, dynamic, c.active, NList{}, scl);
     const uint32_t nsc = (P.gsx / 4) * (P.gsy / 4) * (P.gsz / 4);
     for (uint32_t col = 0; col < 8; ++col) {
         if (P.maxc <= SNOWB_MAXC_FAST)
             LAUNCH(k_link_colour_warp, (uint64_t)link_blocks(nsc) * LINK_TPB, LINK_TPB, P, c.S, vd, *dem,
-                   c.active, col, dynamic, NList{nullptr, nullptr, 0u, 0u}, scl);
+                   c.active, col, dynamic, NList{}, scl);
         else
             LAUNCH(k_link_colour, nsc, 64, P, c.S, vd, *dem, c.active, col, dynamic);
     }

@@ -36,11 +36,32 @@ struct Sorted {
 constexpr uint32_t NLIST_K = SNOWB_NLIST_K;
 constexpr uint32_t NL_J_MASK = (1u << 25) - 1u;
 constexpr uint32_t NL_OVF = 1u << 31;
+// The first density pass of a substep lists, per snow particle, its snow candidates within h plus
+// a skin of NL_SKIN h (those beyond h marked NL_FAR; link formation skips them).  While the snow
+// keeps its sort (DevState::skin_ok) the iterations' density passes take the snow's own sums from
+// these lists, each pair put to the exact test, in place of some 300 candidates in 27 cells, and
+// list no own neighbours again (NL_OWN_SKIN): the PBF, contact and friction passes read the same
+// lists.  The sums are those of the traversal, term by term: the lists are in traversal order, and
+// a kept sort keeps every cell's members.  A pair that comes within h has one end that moved more
+// than half the skin: the rank pass marks the 27 cells around such a particle, and in marked cells
+// the traversal is taken, as it is for a list that a stale cell range went into (NL_STALE: those
+// members' own cells may lie elsewhere).
+// Density + lambda pass at rest: 832 -> 577 us at 1.18M particles (the frame 22.9 -> 19.6 ms), 144
+// -> 112 us at 153.8k (4.08 -> 3.78 ms).  A resting block's particles move 2e-4 m a substep by
+// gravity and 99% of them less than 6e-4 m in all, at h = 0.04; skins of 0.02, 0.03 and 0.045 h
+// gave 3.78, 3.77, 3.80 and 19.6, 19.8, 20.0 ms.  Where the snow is sorted at every point (the
+// melt, batches in which some scene always is) the lists' extra candidates cost about 0.5%.
+constexpr float NL_SKIN = 0.02f;
+constexpr uint32_t NL_FAR = 1u << 30;        // in an entry
+constexpr uint32_t NL_STALE = 1u << 30;      // in a count of the lists with a skin
+constexpr uint32_t NL_OWN_SKIN = 1u << 30;   // in a count of the iteration's lists
 struct NList {
     uint32_t* e;       // entry k of slot s at e[k * stride + s]: j | cell << 25 | set << 30
     uint32_t* cnt;     // per slot: own | other << 10 | boundary << 20 (| NL_OVF)
     uint32_t stride;   // 2 * capacity: water slots [0, cap), snow slots [cap, 2 cap)
     uint32_t cap;
+    const uint32_t *skin_e, *skin_cnt;   // the substep's snow lists with a skin (null: not used)
+    const uint32_t* skin_far;            // per cell: the last substep that marked it
 };
 struct NLWriter {
     uint32_t* e;
@@ -184,7 +205,9 @@ __device__ __forceinline__ float3 seg_pbf_own(const DevParams& P, float3 acc, co
         const uint32_t en = S.at(k), j = en & NL_J_MASK, cell = (en >> 25) & 31u;
         if (cell != cur) { if (cur != 0xFFu) acc = add3(acc, cs); cs = f3(0.f, 0.f, 0.f); cur = cell; }
         float3 dv = sub3(p, v.pos(j));
-        float d = sqrtf(dot3(dv, dv));   // a recorded candidate: d < h
+        const float d2 = dot3(dv, dv);
+        if (!(d2 < P.h2_lt)) continue;   // lists with a skin hold more
+        float d = sqrtf(d2);
         float3 gr = G_spiky_in(P, dv, d);
         float lj = v.attr(lam_s, lam_o, j), cj = v.attr(con_s, con_o, j);
         cs = add3(cs, sc3(cj * lam_scorr(P, li + lj, d, dt), gr));
@@ -287,6 +310,7 @@ __device__ __forceinline__ bool segments(const NList& L, uint32_t slot, Seg& own
     if (c & NL_OVF) return false;
     const uint32_t a = c & 1023u, b = (c >> 10) & 1023u, d = (c >> 20) & 1023u;
     own = Seg{L.e, L.stride, slot, 0u, a};
+    if (c & NL_OWN_SKIN) own = Seg{L.skin_e, L.stride, slot, 0u, L.skin_cnt[slot] & 1023u};
     oth = Seg{L.e, L.stride, slot, a, a + b};
     bnd = Seg{L.e, L.stride, slot, a + b, a + b + d};
     return true;
@@ -299,7 +323,7 @@ __device__ __forceinline__ bool segments(const NList& L, uint32_t slot, Seg& own
 // own C and neighbour positions only, so both come out of one traversal.  Each quantity
 // keeps its own per-cell accumulation in the reference's loop order.
 // one candidate of acc_WG
-template <bool LAMBDA>
+template <bool LAMBDA, bool SKIN = false>
 __device__ __forceinline__ void wg_term(const DevParams& P, float& cs, float& cg, float4 q, float3 p, uint32_t j,
                                         bool vol, int mode, float m_self, float m_j, NLWriter* wr, int cell, int set)
 {
@@ -320,20 +344,24 @@ __device__ __forceinline__ void wg_term(const DevParams& P, float& cs, float& cg
             float3 gc = sc3(sc, G_spiky_in(P, dv, d));
             cg += dot3(gc, gc);
         }
+    } else if (SKIN && d2 < P.s2) {
+        wr->push(j, cell, 1);   // NL_FAR
     }
 }
-template <bool LAMBDA>
+template <bool LAMBDA, bool SKIN = false>
 __device__ __forceinline__ void acc_WG(const DevParams& P, float& rho, float& gs, const SetView& v, float3 p,
                                        const Nbhd& nb, uint32_t skip, bool vol, int mode, float m_self,
                                        const float* mass_s, const float* mass_o, NLWriter* wr = nullptr, int set = 0,
-                                       float* dpart = nullptr, uint32_t* dmask = nullptr)
+                                       float* dpart = nullptr, uint32_t* dmask = nullptr, bool* stale = nullptr)
 {
     const P2 pp = bcast2(p);
+    const float cull = SKIN ? P.s2_cull : P.h2_cull;
     FOR27 {
         float cs = 0.f, cg = 0.f;
         uint32_t s, e;
         if (v.range_nb(nb, ox, oy, oz, s, e)) {
             const int cell = CELL27;
+            if (SKIN) *stale |= !(s < v.n && __ldg(v.gh + s) == nb.hash(ox, oy, oz));
             if (e <= v.n) {
                 // current entries only: the compact sorted copies.  Candidates are screened
                 // two at a time with packed arithmetic; ptxas may contract its multiply-adds,
@@ -343,24 +371,24 @@ __device__ __forceinline__ void acc_WG(const DevParams& P, float& rho, float& gs
                 for (; j + 1 < e; j += 2) {
                     const float4 q0 = __ldg(v.p4 + j), q1 = __ldg(v.p4 + j + 1);
                     const float2 dd = d2_pair(pp, q0, q1);
-                    if (dd.x < P.h2_cull && j != skip) {
+                    if (dd.x < cull && j != skip) {
                         const float mj = (LAMBDA && mode == 2) ? __ldg(mass_s + j) : 0.f;
-                        wg_term<LAMBDA>(P, cs, cg, q0, p, j, vol, mode, m_self, mj, wr, cell, set);
+                        wg_term<LAMBDA, SKIN>(P, cs, cg, q0, p, j, vol, mode, m_self, mj, wr, cell, set);
                     }
-                    if (dd.y < P.h2_cull && j + 1 != skip) {
+                    if (dd.y < cull && j + 1 != skip) {
                         const float mj = (LAMBDA && mode == 2) ? __ldg(mass_s + j + 1) : 0.f;
-                        wg_term<LAMBDA>(P, cs, cg, q1, p, j + 1, vol, mode, m_self, mj, wr, cell, set);
+                        wg_term<LAMBDA, SKIN>(P, cs, cg, q1, p, j + 1, vol, mode, m_self, mj, wr, cell, set);
                     }
                 }
                 if (j < e && j != skip) {
                     const float mj = (LAMBDA && mode == 2) ? __ldg(mass_s + j) : 0.f;
-                    wg_term<LAMBDA>(P, cs, cg, __ldg(v.p4 + j), p, j, vol, mode, m_self, mj, wr, cell, set);
+                    wg_term<LAMBDA, SKIN>(P, cs, cg, __ldg(v.p4 + j), p, j, vol, mode, m_self, mj, wr, cell, set);
                 }
             } else {
                 for (uint32_t j = s; j < e; ++j) {
                     if (j == skip) continue;
                     const float mj = (LAMBDA && mode == 2) ? v.attr(mass_s, mass_o, j) : 0.f;
-                    wg_term<LAMBDA>(P, cs, cg, v.pw(j), p, j, vol, mode, m_self, mj, wr, cell, set);
+                    wg_term<LAMBDA, SKIN>(P, cs, cg, v.pw(j), p, j, vol, mode, m_self, mj, wr, cell, set);
                 }
             }
         }
@@ -373,6 +401,36 @@ __device__ __forceinline__ void acc_WG(const DevParams& P, float& rho, float& gs
         }
         if (LAMBDA) gs += cg;
     }
+}
+// the same sums for a snow particle and its own set from its list with a skin, entries taken four
+// at a time
+__device__ __forceinline__ void acc_skin(const DevParams& P, float& rho, float& gs, const NList& L, uint32_t slot,
+                                         uint32_t n, const SetView& v, float3 p)
+{
+    const Seg S{L.skin_e, L.stride, slot, 0u, n};
+    float cs = 0.f, cg = 0.f;
+    uint32_t cur = 0u;
+    for (uint32_t k = 0u; k < n; k += 4u) {
+        uint32_t en[4];
+        float4 q[4];
+#pragma unroll
+        for (uint32_t u = 0u; u < 4u; ++u) en[u] = S.at(umin32(k + u, n - 1u));
+#pragma unroll
+        for (uint32_t u = 0u; u < 4u; ++u) q[u] = v.pw(en[u] & NL_J_MASK);
+#pragma unroll
+        for (uint32_t u = 0u; u < 4u; ++u) {
+            if (k + u >= n) break;
+            const uint32_t cell = (en[u] >> 25) & 31u;
+            if (cell != cur) {
+                rho += cs; gs += cg;
+                cs = cg = 0.f;
+                cur = cell;
+            }
+            wg_term<true>(P, cs, cg, q[u], p, en[u] & NL_J_MASK, false, 0, 0.f, 0.f, nullptr, 0, 0);
+        }
+    }
+    rho += cs;
+    gs += cg;
 }
 // Sums over the boundary set of every boundary particle (own term included): the opening
 // terms of its density and lambda sums, the same in every pass of a call since the boundary
@@ -439,14 +497,22 @@ template <bool LAMBDA>
 // and snow sums take the boundary's terms either way, through its compact sorted copies.
 __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restrict__ S, SetView vs, SetView vd,
                                                  SetView vb, Sets X, Sorted ss, Sorted sd, Sorted sb, NList L,
-                                                 int with_bnd, BndBase base)
+                                                 int with_bnd, BndBase base, float4* __restrict__ skin_p4)
 {
     wait_prior();
     const uint32_t ns = S->n_sph, nd = S->n_dem, nb = S->n_b, nbt = with_bnd ? nb : 0u;
     vs.n = ns; vd.n = nd; vb.n = nb;
     const bool ready = S->base_ready != 0u;
     const float3 z = f3(0.f, 0.f, 0.f);
-    if (LAMBDA && blockIdx.x == 0 && threadIdx.x == 0) S->far_move = 0u;   // the lists are new
+    const bool skin = LAMBDA && S->skin_ok != 0u;
+    const uint32_t epoch = S->epoch;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (LAMBDA) {
+            S->far_move = 0u;   // the lists are new
+        } else {
+            S->skin_ok = 1u;
+        }
+    }
     GRID_LOOP(t, ns + nd + nbt) {
         float rho, gs = dot3(z, z);
         const snowb_particle_data* D;
@@ -461,13 +527,24 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
             lam_s = w ? ss.lambda : sd.lambda;
             o = own.gi[i];
             float3 p = xyz(own.p4[i]); GCell g = grid_pos(P, p, own.scene(i));
-            const Nbhd nb = make_nbhd(P, g, p, P.h2_cull);
+            const Nbhd nb = make_nbhd(P, g, p, LAMBDA || w ? P.h2_cull : P.s2_cull);
             rho = D->mass[o] * P.W0;
             NLWriter wr{L.e, L.stride, (w ? 0u : L.cap) + i, 0u};
             // the density+lambda pass lists all three sets for the PBF and contact passes; the
             // substep's first density pass lists the snow-snow candidates for link formation
             NLWriter* pw = (LAMBDA || !w) ? &wr : nullptr;
-            acc_WG<LAMBDA>(P, rho, gs, own, p, nb, i, false, 0, 0.f, nullptr, nullptr, pw, 0);
+            const uint32_t listed = skin && !w && L.skin_far[nb.hash(0, 0, 0)] != epoch ? L.skin_cnt[wr.slot] : NL_OVF;
+            const bool use_skin = !(listed & (NL_OVF | NL_STALE));
+            bool stale = false;
+            if (use_skin) {
+                acc_skin(P, rho, gs, L, wr.slot, listed & 1023u, own, p);
+            } else if (LAMBDA || w) {
+                acc_WG<LAMBDA>(P, rho, gs, own, p, nb, i, false, 0, 0.f, nullptr, nullptr, pw, 0);
+            } else {
+                acc_WG<LAMBDA, true>(P, rho, gs, own, p, nb, i, false, 0, 0.f, nullptr, nullptr, pw, 0, nullptr, nullptr,
+                                     &stale);
+                skin_p4[i] = own.p4[i];
+            }
             const uint32_t n_own = wr.n;
             if (!LAMBDA) pw = nullptr;
             acc_WG<LAMBDA>(P, rho, gs, oth, p, nb, SNOWB_UMAX, false, 0, 0.f, nullptr, nullptr, pw, 1);
@@ -475,10 +552,10 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
             acc_WG<LAMBDA>(P, rho, gs, vb, p, nb, SNOWB_UMAX, true, 1, D->mass[o], nullptr, nullptr, pw, 2);
             if (LAMBDA) {
                 const uint32_t n_bnd = wr.n - n_own - n_oth;
-                L.cnt[wr.slot] = wr.n > NLIST_K ? NL_OVF : (n_own | (n_oth << 10) | (n_bnd << 20));
+                L.cnt[wr.slot] = wr.n > NLIST_K ? NL_OVF : (n_own | (n_oth << 10) | (n_bnd << 20) | (use_skin ? NL_OWN_SKIN : 0u));
                 if (wr.n > NLIST_K) atomicAdd(&S->n_nl_ovf, 1u);
             } else if (!w) {
-                L.cnt[wr.slot] = n_own > NLIST_K ? NL_OVF : n_own;
+                L.cnt[wr.slot] = n_own > NLIST_K ? NL_OVF : (n_own | (stale ? NL_STALE : 0u));
             }
         } else {
             // boundary: density sums the sets in the order (b, snow, water), lambda (b, water,

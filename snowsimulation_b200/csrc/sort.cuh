@@ -96,6 +96,8 @@ struct SortPair {
     int begin;
     uint32_t ncells;
     int clear_all;
+    const float4* skin_p4;                // see NL_SKIN
+    uint32_t* skin_far;
     __device__ __forceinline__ bool sorts(int k) const { return on[k] && (!S || S->resort[k] != 0u); }
     __device__ __forceinline__ uint32_t size(int k) const { return on[k] ? *a[k].n : 0u; }
 };
@@ -110,6 +112,7 @@ __device__ __forceinline__ void begin_substep(DevState* S)
 {
     S->n0_sph = S->n_sph; S->n0_dem = S->n_dem;
     S->n_freeze = 0; S->n_melt = 0; S->changed = 0; S->n_active = 0; S->n_links = 0; S->n_nl_ovf = 0;
+    S->skin_ok = 0; ++S->epoch;
     for (int c = 0; c < 8; ++c) S->sc_count[c] = 0u;
 }
 __global__ void k_sort_hash(DevParams P, const __grid_constant__ SortPair Q)
@@ -128,6 +131,7 @@ __global__ void k_sort_hash(DevParams P, const __grid_constant__ SortPair Q)
                 else ++Q.S->sorts_kept[k];
             }
     }
+    if (Q.S && m[1] && blockIdx.x == 0 && threadIdx.x == 0) Q.S->skin_ok = 0u;   // the lists hold sorted indices
     const uint32_t n0 = m[0] ? Q.size(0) : 0u, n = n0 + (m[1] ? Q.size(1) : 0u);
     const uint32_t lane = threadIdx.x & 31u;
     // whole warps iterate together so the chunk counts can be aggregated with warp votes
@@ -316,11 +320,12 @@ __device__ __forceinline__ uint32_t stable_rank(const uint32_t* __restrict__ tmp
 // sort (no particle left its cell, same set size): grid_hash, grid_index and the cell table are
 // already what this sort would write, so only the gathered outputs are refreshed, sorted slot
 // by sorted slot.
-__global__ void k_sort_rank(const __grid_constant__ SortPair Q)
+__global__ void k_sort_rank(DevParams P, const __grid_constant__ SortPair Q)
 {
     wait_prior();
     const bool s0 = Q.sorts(0), s1 = Q.sorts(1);
     const uint32_t n0 = Q.size(0), n = n0 + Q.size(1);
+    const bool skin = Q.S && Q.on[1] && !s1 && Q.S->skin_ok != 0u;
     GRID_LOOP(t, n) {
         const int k = t < n0 ? 0 : 1;
         const SortSide& A = Q.a[k];
@@ -337,6 +342,14 @@ __global__ void k_sort_rank(const __grid_constant__ SortPair Q)
             o = A.cd.grid_index[p];
         }
         const float3 q = ldv3(A.pos, o);
+        if (k && skin) {
+            const float3 d = sub3(q, xyz(Q.skin_p4[p]));
+            if (!(dot3(d, d) <= P.skin_move2)) {   // the lists of the cells around are not to be used
+                const Nbhd nb = make_nbhd(P, grid_pos(P, q, A.sid_o ? A.sid_o[o] : 0u), q, 0.f);
+                const uint32_t now = Q.S->epoch;
+                FOR27 Q.skin_far[nb.hash(ox, oy, oz)] = now;
+            }
+        }
         st3(A.cd.sorted_pos, p, q);
         A.p4[p] = make_float4(q.x, q.y, q.z, A.w[o]);
         A.invm_s[p] = A.invm[o];
