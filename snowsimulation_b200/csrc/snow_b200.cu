@@ -177,7 +177,7 @@ struct Ctx {
     DevState* S = nullptr;
     DevState* S_host = nullptr;
     uint32_t* err_dev = nullptr;
-    cudaStream_t side = nullptr;          // second stream for the water sort (see sort_pair)
+    cudaStream_t side = nullptr;          // second stream: the interlink terms (see links_beside)
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaStream_t side2 = nullptr;         // third stream (the water PBF pass beside the snow passes)
     cudaEvent_t fork2 = nullptr, join2 = nullptr;
