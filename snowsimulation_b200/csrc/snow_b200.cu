@@ -554,14 +554,17 @@ struct StepArgs {
         dynamic, cd_on;
     float dTe;
     int stop_after;
-    const uint32_t *sid_sph, *sid_dem, *sid_bnd;   // batched runs: scene id per slot (else null)
-    uint32_t* sid_buf;
     int xsph_thread[2];   // XSPH of the water / snow set in the one-thread form (sizes at the call)
     uint32_t particles;   // water + snow at the call (phase changes keep the sum)
     // passes in their one-warp forms (set sizes at the call): density and link filter, heat,
     // snow contacts, friction (1: unless the neighbour lists hold, 2: always)
     int small, small_heat, small_contact, small_friction;
+    const uint32_t *sid_sph, *sid_dem, *sid_bnd;   // batched runs: scene id per slot (else null)
+    uint32_t* sid_buf;
 };
+// The struct's bytes are the key of the captured graph: a padding byte, which nothing sets, would
+// make equal calls differ (the first call of a program was captured a second time by the next).
+static_assert(sizeof(StepArgs) == 8 * sizeof(void*) + 3 * sizeof(snowb_cell_data) + 24 * sizeof(int), "no padding");
 
 
 // ------------------------------------------------------------------ adjoint tape
@@ -1455,13 +1458,13 @@ static int run_steps(snowb_particle_data* sph, uint32_t* sph_size, snowb_particl
     const uint32_t xs_d = opt.quirks == SNOWB_QUIRKS_REFERENCE ? umin32(coverage(*sph_size), *dem_size) : *dem_size;
     StepArgs a{sph, dem, bnd, buf, nb, full, scd, dcd, bcd, dt, iterations,
                fl[0], fl[1], fl[2], fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10], dTe, opt.stop_after,
-               batch ? batch->scene_sph : nullptr, batch ? batch->scene_dem : nullptr,
-               batch ? batch->scene_boundary : nullptr, batch ? batch->scene_buffer : nullptr,
                {xs_s > XSPH_WARP_MAX ? 1 : 0, xs_d > XSPH_WARP_MAX ? 1 : 0}, *sph_size + *dem_size,
                *sph_size + *dem_size <= DENSITY_WARP_MAX ? 1 : 0,
                *sph_size + *dem_size <= (opt.quirks == SNOWB_QUIRKS_REFERENCE ? HEAT_WARP_MAX_REF : HEAT_WARP_MAX) ? 1 : 0,
                *dem_size <= CONTACT_WARP_MAX ? 1 : 0,
-               *dem_size <= FRICTION_WARP_MAX ? 2 : (*dem_size <= FRICTION_BOTH_MAX ? 1 : 0)};
+               *dem_size <= FRICTION_WARP_MAX ? 2 : (*dem_size <= FRICTION_BOTH_MAX ? 1 : 0),
+               batch ? batch->scene_sph : nullptr, batch ? batch->scene_dem : nullptr,
+               batch ? batch->scene_boundary : nullptr, batch ? batch->scene_buffer : nullptr};
     LAUNCH1(k_set_state, c.S, *sph_size, *dem_size, nb);
     if (batch)
         LAUNCH(k_check_scenes, full > nb ? full : nb, 256, P, c.S, a.sid_sph, a.sid_dem, a.sid_bnd);
