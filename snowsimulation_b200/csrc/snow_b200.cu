@@ -555,10 +555,11 @@ struct StepArgs {
     float dTe;
     int stop_after;
     int xsph_thread[2];   // XSPH of the water / snow set in the one-thread form (sizes at the call)
-    uint32_t particles;   // water + snow at the call (phase changes keep the sum)
-    // passes in their one-warp forms (set sizes at the call): density and link filter, heat,
-    // snow contacts, friction (1: unless the neighbour lists hold, 2: always)
-    int small, small_heat, small_contact, small_friction;
+    // passes in their one-warp forms, by the set sizes at the call: density, link filter, heat, snow
+    // contacts, friction (1: unless the neighbour lists hold, 2: always).  The sizes themselves stay
+    // out: these bytes are part of the key of the captured graph, and a host that adds or removes
+    // particles between calls keeps its graph.  `full` sizes the launches; every pass loops.
+    int small_density, small_links, small_heat, small_contact, small_friction;
     const uint32_t *sid_sph, *sid_dem, *sid_bnd;   // batched runs: scene id per slot (else null)
     uint32_t* sid_buf;
 };
@@ -769,9 +770,9 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // iterations leaves the boundary out here.
     const int bnd_first = !(beside && a.iterations > 0);
     // warps of the one-warp density form: a particle each, 32 boundary particles each
-    const uint64_t dwork = 32ull * (a.particles + (a.nb + 31u) / 32u);
-    if (a.small)
-        TLAUNCH_AS("k_density<false>", k_density_warp<false>, 256, bnd_first ? dwork : 32ull * a.particles, 128, P, S, vs,
+    const uint64_t dwork = 32ull * (full + (a.nb + 31u) / 32u);
+    if (a.small_density)
+        TLAUNCH_AS("k_density<false>", k_density_warp<false>, 256, bnd_first ? dwork : 32ull * full, 128, P, S, vs,
                    vd, vb, X, ss, sd, sb, NL2, bnd_first, c.b.base);
     else
         TLAUNCH(k_density<false>, 256, bnd_first ? work3 : 2 * full, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL2,
@@ -780,7 +781,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // in a whole substep the phase flags pass commits the new temperatures itself
     const int commit_in_flags = beside && a.temperature && a.change_phase;
     if (a.temperature) {
-        if (a.small_heat) TLAUNCH_AS("k_heat", k_heat_warp, SMALL_TPB, 32ull * a.particles, SMALL_TPB, P, S, vs, vd, X, a.dt);
+        if (a.small_heat) TLAUNCH_AS("k_heat", k_heat_warp, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd, X, a.dt);
         else if (P.quirks == SNOWB_QUIRKS_REFERENCE) {
             TLAUNCH_AS("k_heat", k_heat<true>, 256, 2 * full, 128, P, S, vs, vd, X, a.dt, nullptr, nullptr);
         } else {
@@ -819,7 +820,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         // link formation over a view of the snow set: the set's own, or its copy
         auto form = [&](const SetView& v) -> int {
             const SCList scl = sc_lists(P);
-            if (a.small && P.maxc <= SNOWB_MAXC_FAST)
+            if (a.small_links)
                 TLAUNCH_AS("k_link_filter", k_link_filter_warp, 128, 32ull * full, 128, P, S, v, *a.dem, a.dynamic,
                            c.active, NL2, scl);
             else
@@ -884,7 +885,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         const bool links_beside = beside && a.interlink;
         if (links_beside) TRY(on_side(c.side, c.fork, link_terms));
         // density + lambda in one pass (stage boundaries base+1 and base+2 coincide)
-        if (a.small)
+        if (a.small_density)
             TLAUNCH_AS("k_density<true>", k_density_warp<true>, 256, dwork, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1,
                        c.b.base);
         else
@@ -1458,8 +1459,9 @@ static int run_steps(snowb_particle_data* sph, uint32_t* sph_size, snowb_particl
     const uint32_t xs_d = opt.quirks == SNOWB_QUIRKS_REFERENCE ? umin32(coverage(*sph_size), *dem_size) : *dem_size;
     StepArgs a{sph, dem, bnd, buf, nb, full, scd, dcd, bcd, dt, iterations,
                fl[0], fl[1], fl[2], fl[3], fl[4], fl[5], fl[6], fl[7], fl[8], fl[9], fl[10], dTe, opt.stop_after,
-               {xs_s > XSPH_WARP_MAX ? 1 : 0, xs_d > XSPH_WARP_MAX ? 1 : 0}, *sph_size + *dem_size,
+               {xs_s > XSPH_WARP_MAX ? 1 : 0, xs_d > XSPH_WARP_MAX ? 1 : 0},
                *sph_size + *dem_size <= DENSITY_WARP_MAX ? 1 : 0,
+               *sph_size + *dem_size <= DENSITY_WARP_MAX && P.maxc <= SNOWB_MAXC_FAST ? 1 : 0,
                *sph_size + *dem_size <= (opt.quirks == SNOWB_QUIRKS_REFERENCE ? HEAT_WARP_MAX_REF : HEAT_WARP_MAX) ? 1 : 0,
                *dem_size <= CONTACT_WARP_MAX ? 1 : 0,
                *dem_size <= FRICTION_WARP_MAX ? 2 : (*dem_size <= FRICTION_BOTH_MAX ? 1 : 0),
