@@ -1567,6 +1567,9 @@ static int connect_links(const DevParams& P, snowb_particle_data* dem, uint32_t 
     if (!dem) return fail(SNOWB_ERR_INVALID, "null pointer");
     if (n == 0) return SNOWB_OK;
     if (P.gsx < 4 || P.gsy < 4 || P.gsz < 4) return fail(SNOWB_ERR_INVALID, "grid must be at least 4 cells per axis");
+    // indices share a word with their cell (NL_J_MASK); the neighbour lists of so many particles
+    // (206 GB) would not fit the GPU either
+    if (n > NL_J_MASK) return fail(SNOWB_ERR_INVALID, "more than 2^25 particles per set");
     TRY(ensure_ctx(g_ctx.cap > n ? g_ctx.cap : n, g_ctx.bcap ? g_ctx.bcap : 1, P.ncells));
     Ctx& c = g_ctx;
     LAUNCH1(k_set_state, c.S, 0u, n, 0u);
