@@ -131,8 +131,10 @@ static int dalloc(T** p, size_t count)
 {
     *p = nullptr;
     if (count == 0) count = 1;
-    CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T)));
-    return SNOWB_OK;
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
+    if (e == cudaSuccess) return SNOWB_OK;
+    cudaGetLastError();   // no later launch's error
+    return fail(SNOWB_ERR_CUDA, "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes: " + cudaGetErrorString(e));
 }
 
 struct SetBufs {
@@ -244,17 +246,8 @@ static int alloc_sort(SetBufs& s, uint32_t cap, uint32_t ncells, bool attrs)
     }
     return SNOWB_OK;
 }
-// (Re)create the context for the current device with room for `full` particles per set,
-// `nb` boundary particles and `ncells` cells.
-static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
+static int make_ctx(Ctx& c, int dev, uint32_t full, uint32_t nb, uint32_t ncells, uint32_t maxc)
 {
-    int dev = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    Ctx& c = g_ctx;
-    const uint32_t maxc = g_sim.maximum_connection > 0 ? g_sim.maximum_connection : 1;
-    if (c.device == dev && c.cap >= full && c.bcap >= nb && c.ncells == ncells && c.maxc >= maxc) return SNOWB_OK;
-    free_ctx(c);
-    ++g_ctx_gen;
     c.device = dev;
     c.cap = full > 0 ? full : 1;
     c.bcap = nb > 0 ? nb : 1;
@@ -326,6 +319,22 @@ static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
     g_sms = sms;
     return SNOWB_OK;
 }
+// (Re)create the context for the current device with room for `full` particles per set,
+// `nb` boundary particles and `ncells` cells.  One that cannot be made whole is not kept: its sizes
+// would let the next call run on buffers that are not there.
+static int ensure_ctx(uint32_t full, uint32_t nb, uint32_t ncells)
+{
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    Ctx& c = g_ctx;
+    const uint32_t maxc = g_sim.maximum_connection > 0 ? g_sim.maximum_connection : 1;
+    if (c.device == dev && c.cap >= full && c.bcap >= nb && c.ncells == ncells && c.maxc >= maxc) return SNOWB_OK;
+    free_ctx(c);
+    ++g_ctx_gen;
+    const int rc = make_ctx(c, dev, full, nb, ncells, maxc);
+    if (rc != SNOWB_OK) free_ctx(c);
+    return rc;
+}
 // the link passes' super-cell lists (warp form only: maximum_connection <= SNOWB_MAXC_FAST)
 static SCList sc_lists(const DevParams& P)
 {
@@ -340,7 +349,9 @@ static int ensure_gen(uint32_t n, uint32_t ncells)
     if (c.gen.key && c.gen_cap >= n && c.ncells == ncells) return SNOWB_OK;
     free_set(c.gen);
     c.gen_cap = n > 0 ? n : 1;
-    return alloc_sort(c.gen, c.gen_cap, ncells, false);
+    const int rc = alloc_sort(c.gen, c.gen_cap, ncells, false);
+    if (rc != SNOWB_OK) free_set(c.gen);
+    return rc;
 }
 
 // ------------------------------------------------------------------ launch helpers
@@ -639,7 +650,12 @@ static int tape_hook(const StepArgs& a, int kind, int it)
     Tape& tp = g_tape;
     if (kind == 0 && tp.used == tp.steps.size()) {
         tp.steps.emplace_back();
-        TRY(tape_alloc_step(tp.steps.back()));
+        const int rc = tape_alloc_step(tp.steps.back());
+        if (rc != SNOWB_OK) {
+            for (void* p : tp.steps.back().bufs) cudaFree(p);
+            tp.steps.pop_back();
+            return rc;
+        }
     }
     TapeStep& T = tp.steps[tp.used];
     const size_t b3[2] = {(size_t)tp.n[0] * 12, (size_t)tp.n[1] * 12};
@@ -1064,13 +1080,8 @@ static void adj_free()
     for (void* p : g_adj.bufs) cudaFree(p);
     g_adj = AdjBufs();
 }
-static int adj_ensure(uint32_t cap, uint32_t bcap, uint32_t ncells)
+static int adj_make(AdjBufs& B, int dev, uint32_t cap, uint32_t bcap, uint32_t ncells)
 {
-    int dev = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    AdjBufs& B = g_adj;
-    if (B.device == dev && B.cap >= cap && B.bcap >= bcap && B.ncells == ncells) return SNOWB_OK;
-    adj_free();
     B.device = dev; B.cap = cap; B.bcap = bcap; B.ncells = ncells;
     auto A = [&](auto** p, size_t n) -> int { TRY(dalloc(p, n)); B.bufs.push_back(*p); return SNOWB_OK; };
     for (int s = 0; s < 2; ++s) {
@@ -1089,6 +1100,17 @@ static int adj_ensure(uint32_t cap, uint32_t bcap, uint32_t ncells)
     for (float*& q : B.part) TRY(A(&q, 2 * (size_t)cap));
     TRY(A(&B.nbuf, 4)); TRY(A(&B.gp, 4));
     return SNOWB_OK;
+}
+static int adj_ensure(uint32_t cap, uint32_t bcap, uint32_t ncells)
+{
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    AdjBufs& B = g_adj;
+    if (B.device == dev && B.cap >= cap && B.bcap >= bcap && B.ncells == ncells) return SNOWB_OK;
+    adj_free();
+    const int rc = adj_make(B, dev, cap, bcap, ncells);
+    if (rc != SNOWB_OK) adj_free();
+    return rc;
 }
 static inline snowb_float3* F3(float* p) { return reinterpret_cast<snowb_float3*>(p); }
 static inline const snowb_float3* F3(const float* p) { return reinterpret_cast<const snowb_float3*>(p); }
