@@ -230,6 +230,14 @@ static void free_ctx(Ctx& c)
     if (c.ev_links) cudaEventDestroy(c.ev_links);
     c = Ctx();
 }
+// Memsets of new buffers run in the legacy stream and return before they are done, and a stream of
+// the caller's that does not block on it would read the buffers before (behind work of the caller's
+// in the legacy stream, long before).  Whoever makes buffers waits once.
+static int wait_memsets()
+{
+    CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+    return SNOWB_OK;
+}
 static int alloc_sort(SetBufs& s, uint32_t cap, uint32_t ncells, bool attrs)
 {
     TRY(dalloc(&s.key, cap)); TRY(dalloc(&s.slot, cap)); TRY(dalloc(&s.tmp, cap)); TRY(dalloc(&s.val, cap));
@@ -244,7 +252,7 @@ static int alloc_sort(SetBufs& s, uint32_t cap, uint32_t ncells, bool attrs)
         TRY(dalloc(&s.p4, cap)); TRY(dalloc(&s.invm, cap)); TRY(dalloc(&s.contrib, cap)); TRY(dalloc(&s.lambda, cap));
         TRY(dalloc(&s.sid, cap));
     }
-    return SNOWB_OK;
+    return wait_memsets();
 }
 static int make_ctx(Ctx& c, int dev, uint32_t full, uint32_t nb, uint32_t ncells, uint32_t maxc)
 {
@@ -317,7 +325,7 @@ static int make_ctx(Ctx& c, int dev, uint32_t full, uint32_t nb, uint32_t ncells
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     g_max_blocks = sms * 16;
     g_sms = sms;
-    return SNOWB_OK;
+    return wait_memsets();
 }
 // (Re)create the context for the current device with room for `full` particles per set,
 // `nb` boundary particles and `ncells` cells.  One that cannot be made whole is not kept: its sizes
@@ -1049,6 +1057,7 @@ static int tape_start_call(const DevParams& P, snowb_particle_data* sph, uint32_
     if (!tp.viol) {
         TRY(dalloc(&tp.viol, 1));
         CUDA_TRY(cudaMemset(tp.viol, 0, sizeof(uint32_t)));
+        TRY(wait_memsets());
     }
     tp.sph = *sph; tp.dem = *dem; tp.bnd = *bnd; tp.bcd = bcd; tp.P = P; tp.dt = dt;
     tp.correct_dem = fl[0]; tp.friction = fl[2]; tp.temperature = fl[3]; tp.dem_visc = fl[7];
