@@ -350,7 +350,8 @@ int snowb_write_bgeo_host(const float* positions, uint32_t n, const char* path, 
  * Times the tunable kernels of the substep (neighbour passes, link colouring, apply) under
  * nine launch shapes (64/128/256 threads per block x grid caps of 8/16/64 blocks per SM),
  * each over `substeps` graph-replayed substeps timed from CUDA-event nodes, and keeps the
- * fastest shape per kernel and work-size bucket (floor(log2(threads of work))).  The
+ * fastest shape per kernel and work-size bucket (floor(log2(threads of work)); 32 more for
+ * the form of a pass that runs one warp per particle, a kernel of its own).  The
  * arguments are those of snowb_snow_simulation_ex (batch: NULL for one scene, else the
  * batch of snowb_batch_snow_simulation); the state advances by 9 x (substeps + 1) substeps,
  * so callers snapshot it first if they need it.  Launch shapes never change results. */

@@ -463,31 +463,45 @@ static cudaError_t launch_prior(void (*kernel)(E...), unsigned grid, int tpb, A&
 // snowb_autotune, which times every candidate shape from CUDA-event nodes inside the
 // substep's graph.  Launch shapes never change results: every thread's work and every
 // reduction order are independent of the block and grid shape.
+// A pass with several forms is profiled under the pass's name, whichever form runs.  Its forms are
+// different kernels, which count their work differently (32 threads a particle against one), so
+// the one-warp form's shapes stand under the pass's name in buckets of their own, TUNE_WARP and
+// up (fewer than 2^31 threads: at most 62), and while candidates are timed each form is timed
+// under its kernel's name.  The lower buckets keep their meaning, so tables saved before there
+// were one-warp forms still hold.
+constexpr int TUNE_WARP = 32;
 struct TuneEntry {
     std::string name;
     int bucket, tpb, capm;
 };
+struct TuneSeen {
+    std::string name, timed_as;
+    int bucket;
+};
 static std::vector<TuneEntry> g_tune;
 static uint64_t g_tune_gen = 0;        // bumped when the table or the forced shape changes (graph key)
 static int g_tune_force_tpb = 0, g_tune_force_capm = 0;
-static std::vector<std::pair<std::string, int>> g_tune_seen;   // (kernel, bucket) launched while forcing
+static std::vector<TuneSeen> g_tune_seen;   // launched while forcing
 static inline int ilog2_u64(uint64_t x)
 {
     int b = 0;
     while (x > 1) { x >>= 1; ++b; }
     return b;
 }
-static void tune_pick(const char* name, uint64_t work, int tpb0, int max_tpb, int& tpb, unsigned& grid)
+// kernel: the form that runs; first: its first bucket.  Returns the name to profile it under.
+static const char* tune_pick(const char* name, const char* kernel, int first, uint64_t work, int tpb0, int max_tpb,
+                             int& tpb, unsigned& grid)
 {
-    const int bucket = ilog2_u64(work ? work : 1);
+    const int bucket = first + ilog2_u64(work ? work : 1);
     tpb = tpb0;
     int capm = 0;
     if (g_tune_force_tpb) {
         tpb = g_tune_force_tpb < max_tpb ? g_tune_force_tpb : max_tpb;
         capm = g_tune_force_capm;
         bool seen = false;
-        for (auto& e : g_tune_seen) seen |= e.first == name && e.second == bucket;
-        if (!seen) g_tune_seen.emplace_back(name, bucket);
+        for (auto& e : g_tune_seen) seen |= e.timed_as == kernel && e.bucket == bucket;
+        if (!seen) g_tune_seen.push_back(TuneSeen{name, kernel, bucket});
+        name = kernel;
     } else {
         for (const auto& e : g_tune)
             if (e.bucket == bucket && e.name == name) { tpb = e.tpb; capm = e.capm; break; }
@@ -498,22 +512,20 @@ static void tune_pick(const char* name, uint64_t work, int tpb0, int max_tpb, in
     const uint64_t cap = capm ? (uint64_t)capm * g_sms : (uint64_t)g_max_blocks;
     if (b > cap) b = cap;
     grid = (unsigned)b;
+    return name;
 }
-#define TLAUNCH(kernel, max_tpb, work, tpb0, ...)                                            \
+#define TLAUNCH_FORM(name, first, kernel, max_tpb, work, tpb0, ...)                          \
     do {                                                                                     \
         int _tpb;                                                                            \
         unsigned _grid;                                                                      \
-        tune_pick(#kernel, (work), (tpb0), (max_tpb), _tpb, _grid);                          \
-        KL(kernel, _grid, _tpb, __VA_ARGS__);                                                \
+        const char* _name = tune_pick(name, #kernel, first, (work), (tpb0), (max_tpb), _tpb, _grid); \
+        KL_AS(_name, kernel, _grid, _tpb, __VA_ARGS__);                                      \
     } while (0)
-// a pass with several forms is profiled and tuned under the pass's name, whichever form runs
-#define TLAUNCH_AS(name, kernel, max_tpb, work, tpb0, ...)                                   \
-    do {                                                                                     \
-        int _tpb;                                                                            \
-        unsigned _grid;                                                                      \
-        tune_pick(name, (work), (tpb0), (max_tpb), _tpb, _grid);                             \
-        KL_AS(name, kernel, _grid, _tpb, __VA_ARGS__);                                       \
-    } while (0)
+#define TLAUNCH(kernel, max_tpb, work, tpb0, ...) TLAUNCH_FORM(#kernel, 0, kernel, max_tpb, work, tpb0, __VA_ARGS__)
+// the one-thread form of a pass of another name, and a pass's one-warp form
+#define TLAUNCH_AS(name, kernel, max_tpb, work, tpb0, ...) TLAUNCH_FORM(name, 0, kernel, max_tpb, work, tpb0, __VA_ARGS__)
+#define TLAUNCH_WARP(name, kernel, max_tpb, work, tpb0, ...) \
+    TLAUNCH_FORM(name, TUNE_WARP, kernel, max_tpb, work, tpb0, __VA_ARGS__)
 // tunable only when `tunable` holds (else the built-in shape)
 #define TLAUNCH_IF(tunable, kernel, max_tpb, work, tpb0, ...)                                \
     do {                                                                                     \
@@ -796,7 +808,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // warps of the one-warp density form: a particle each, 32 boundary particles each
     const uint64_t dwork = 32ull * (full + (a.nb + 31u) / 32u);
     if (a.small_density)
-        TLAUNCH_AS("k_density<false>", k_density_warp<false>, 256, bnd_first ? dwork : 32ull * full, 128, P, S, vs,
+        TLAUNCH_WARP("k_density<false>", k_density_warp<false>, 256, bnd_first ? dwork : 32ull * full, 128, P, S, vs,
                    vd, vb, X, ss, sd, sb, NL2, bnd_first, c.b.base);
     else
         TLAUNCH(k_density<false>, 256, bnd_first ? work3 : 2 * full, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL2,
@@ -805,7 +817,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
     // in a whole substep the phase flags pass commits the new temperatures itself
     const int commit_in_flags = beside && a.temperature && a.change_phase;
     if (a.temperature) {
-        if (a.small_heat) TLAUNCH_AS("k_heat", k_heat_warp, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd, X, a.dt);
+        if (a.small_heat) TLAUNCH_WARP("k_heat", k_heat_warp, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd, X, a.dt);
         else if (P.quirks == SNOWB_QUIRKS_REFERENCE) {
             TLAUNCH_AS("k_heat", k_heat<true>, 256, 2 * full, 128, P, S, vs, vd, X, a.dt, nullptr, nullptr);
         } else {
@@ -845,7 +857,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         auto form = [&](const SetView& v) -> int {
             const SCList scl = sc_lists(P);
             if (a.small_links)
-                TLAUNCH_AS("k_link_filter", k_link_filter_warp, 128, 32ull * full, 128, P, S, v, *a.dem, a.dynamic,
+                TLAUNCH_WARP("k_link_filter", k_link_filter_warp, 128, 32ull * full, 128, P, S, v, *a.dem, a.dynamic,
                            c.active, NL2, scl);
             else
                 TLAUNCH(k_link_filter, 256, full, 128, P, S, v, *a.dem, a.dynamic, c.active, NL2, scl);
@@ -910,7 +922,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         if (links_beside) TRY(on_side(c.side, c.fork, link_terms));
         // density + lambda in one pass (stage boundaries base+1 and base+2 coincide)
         if (a.small_density)
-            TLAUNCH_AS("k_density<true>", k_density_warp<true>, 256, dwork, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1,
+            TLAUNCH_WARP("k_density<true>", k_density_warp<true>, 256, dwork, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1,
                        c.b.base);
         else
             TLAUNCH(k_density<true>, 256, work3, 128, P, S, vs, vd, vb, X, ss, sd, sb, NL, 1, c.b.base, nullptr);
@@ -929,7 +941,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         if (links_beside)
             TRY(on_side(c.side3, c.fork3, [&]() -> int {
                 if (a.small_contact)
-                    TLAUNCH_AS("k_dem_corr<true>", k_dem_corr_warp<true>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd,
+                    TLAUNCH_WARP("k_dem_corr<true>", k_dem_corr_warp<true>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd,
                                vb, X, ss, sd, sb, F, c.contact);
                 else
                     TLAUNCH(k_dem_corr<true>, 256, full, 128, P, S, vs, vd, vb, X, ss, sd, sb, F, NL, c.contact);
@@ -941,7 +953,7 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
         STOP(base + 3);
         if (!links_beside) {
             if (a.small_contact)
-                TLAUNCH_AS("k_dem_corr<false>", k_dem_corr_warp<false>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd,
+                TLAUNCH_WARP("k_dem_corr<false>", k_dem_corr_warp<false>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vs, vd,
                            vb, X, ss, sd, sb, F, nullptr);
             else
                 TLAUNCH(k_dem_corr<false>, 256, full, 128, P, S, vs, vd, vb, X, ss, sd, sb, F, NL, nullptr);
@@ -978,13 +990,13 @@ static int substep(const DevParams& P, const StepArgs& a, bool step_sph, bool st
             const int unless = a.small_friction == 1 ? 1 : 0;
             if (beside) {
                 if (a.small_friction)
-                    TLAUNCH_AS("k_friction<true>", k_friction_warp<true>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vd,
+                    TLAUNCH_WARP("k_friction<true>", k_friction_warp<true>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vd,
                                vb, X, sd, sb, fr_lists ? 1 : 0, unless, track_d);
                 if (a.small_friction != 2)
                     TLAUNCH(k_friction<true>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, unless, track_d);
             } else {
                 if (a.small_friction)
-                    TLAUNCH_AS("k_friction<false>", k_friction_warp<false>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vd,
+                    TLAUNCH_WARP("k_friction<false>", k_friction_warp<false>, SMALL_TPB, 32ull * full, SMALL_TPB, P, S, vd,
                                vb, X, sd, sb, fr_lists ? 1 : 0, unless, track_d);
                 if (a.small_friction != 2)
                     TLAUNCH(k_friction<false>, 256, full, 128, P, S, vd, vb, X, sd, sb, NL, fr_lists ? 1 : 0, unless, track_d);
@@ -1972,7 +1984,7 @@ int snowb_autotune(snowb_particle_data* sph, uint32_t* sph_size, snowb_particle_
     if (rc != SNOWB_OK) return rc;
     for (const auto& sb : g_tune_seen) {
         size_t idx = 0;
-        while (idx < names.size() && names[idx] != sb.first) ++idx;
+        while (idx < names.size() && names[idx] != sb.timed_as) ++idx;
         if (idx == names.size()) continue;
         int best = -1;
         for (int c = 0; c < 9; ++c)
@@ -1980,10 +1992,10 @@ int snowb_autotune(snowb_particle_data* sph, uint32_t* sph_size, snowb_particle_
         if (best < 0) continue;
         bool found = false;
         for (auto& e : g_tune)
-            if (e.name == sb.first && e.bucket == sb.second) {
+            if (e.name == sb.name && e.bucket == sb.bucket) {
                 e.tpb = tpbs[best / 3]; e.capm = caps[best % 3]; found = true;
             }
-        if (!found) g_tune.push_back(TuneEntry{sb.first, sb.second, tpbs[best / 3], caps[best % 3]});
+        if (!found) g_tune.push_back(TuneEntry{sb.name, sb.bucket, tpbs[best / 3], caps[best % 3]});
     }
     ++g_tune_gen;
     return SNOWB_OK;
