@@ -416,8 +416,11 @@ int snowb_read_sizes(uint32_t* sph_size, uint32_t* dem_size);
  * neighbour lists that overflowed in the substep's density+lambda passes, (index 15 unused),
  * then for the water and the snow set: the pending full-sort flags (2), the last sort
  * decisions (2), and since the call started the sort points that sorted in full (2) and
- * those that kept the previous sort because no particle had left its cell (2).
- * Copies min(n, 24) values into out (blocks). */
+ * those that kept the previous sort because no particle had left its cell (2); and since the
+ * call started, for the snow's neighbour lists with a skin: density+lambda passes that read
+ * them, particles that walked the cells in such a pass all the same, and particles found
+ * beyond half the skin at a sort point.
+ * Copies min(n, 27) values into out (blocks). */
 int snowb_device_counters(uint32_t* out, int n);
 
 /* Default quirk mode of snowb_snow_simulation (SNOWB_QUIRKS_REFERENCE initially). */

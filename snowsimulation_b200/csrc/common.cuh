@@ -67,6 +67,10 @@ struct DevState {
     // started.
     uint32_t moved[2], resort[2];
     uint32_t sorts_full[2], sorts_kept[2];
+    // Snow lists with a skin (NL_SKIN), since the call started: density+lambda passes that read
+    // them, particles that walked the cells in such a pass all the same (marked, or their list
+    // overflowed or met a stale range), particles found beyond half the skin at a sort point.
+    uint32_t skin_passes, skin_walks, skin_marks;
     // a snow particle moved more than FR_LIST_MOVE since the iteration's neighbour lists
     // were built (set by k_apply, cleared by the density+lambda pass)
     uint32_t far_move;

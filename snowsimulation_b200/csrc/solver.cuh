@@ -509,6 +509,7 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (LAMBDA) {
             S->far_move = 0u;   // the lists are new
+            if (skin) ++S->skin_passes;
         } else {
             S->skin_ok = 1u;
         }
@@ -539,6 +540,7 @@ __global__ void __launch_bounds__(256) k_density(DevParams P, DevState* __restri
             if (use_skin) {
                 acc_skin(P, rho, gs, L, wr.slot, listed & 1023u, own, p);
             } else if (LAMBDA || w) {
+                if (skin && !w) atomicAdd(&S->skin_walks, 1u);
                 acc_WG<LAMBDA>(P, rho, gs, own, p, nb, i, false, 0, 0.f, nullptr, nullptr, pw, 0);
             } else {
                 acc_WG<LAMBDA, true>(P, rho, gs, own, p, nb, i, false, 0, 0.f, nullptr, nullptr, pw, 0, nullptr, nullptr,
@@ -2039,6 +2041,7 @@ __global__ void k_set_state(DevState* S, uint32_t ns, uint32_t nd, uint32_t nb)
         S->tail_dirty = 1u;
         // ... and the particles: the first sort point of a call sorts both sets in full
         for (int k = 0; k < 2; ++k) { S->moved[k] = 1u; S->table_any[k] = 1u; S->sorts_full[k] = 0u; S->sorts_kept[k] = 0u; }
+        S->skin_passes = S->skin_walks = S->skin_marks = 0u;
         for (int c = 0; c < 8; ++c) S->sc_count[c] = 0u;
         S->clean_hi[0] = SNOWB_UMAX; S->clean_hi[1] = SNOWB_UMAX;
         S->base_ready = 0u;   // ... and the boundary

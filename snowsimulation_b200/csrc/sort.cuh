@@ -348,6 +348,7 @@ __global__ void k_sort_rank(DevParams P, const __grid_constant__ SortPair Q)
                 const Nbhd nb = make_nbhd(P, grid_pos(P, q, A.sid_o ? A.sid_o[o] : 0u), q, 0.f);
                 const uint32_t now = Q.S->epoch;
                 FOR27 Q.skin_far[nb.hash(ox, oy, oz)] = now;
+                atomicAdd(&Q.S->skin_marks, 1u);
             }
         }
         st3(A.cd.sorted_pos, p, q);
