@@ -15,7 +15,7 @@
 // particles in ascending sorted index.  A particle only edits its own slots and those of
 // neighbours within h, i.e. in adjacent cells; same-coloured super-cells are at least
 // three cells apart, so they never touch the same particle and run in parallel, one
-// thread per super-cell.  A prefilter marks the particles that can change anything:
+// block per super-cell (one thread above SNOWB_MAXC_FAST slots).  A prefilter marks the particles that can change anything:
 // links are never removed during the pass and counts only grow, so a particle whose
 // count already reaches its cap, or whose candidates are all linked already, is a no-op.
 #pragma once
@@ -460,79 +460,7 @@ __global__ void __launch_bounds__(256) k_link_filter(DevParams P, DevState* S, S
         }
     }
 }
-// connect_and_record_cell (:4127-4252) + connect_and_record_d (:4255-4284) for one particle.
-// Only this thread edits particle o and its neighbours during the colour phase, so o's
-// slots, count and tolerance are kept in registers (M <= SNOWB_MAXC_FAST); every record
-// write goes through to memory, where the partner search reads it.  Candidates are
-// screened with the exact squared-distance test (dist < h <=> d2 < h2_lt).
-__device__ void link_particle_fast(const DevParams& P, const SetView& vd, const snowb_particle_data& d, uint32_t i,
-                                   int dynamic, DevState* S)
-{
-    const uint32_t M = P.maxc;
-    const float3 p = vd.pos(i);
-    const uint32_t o = vd.gi[i];
-    const GCell g = grid_pos(P, p, vd.scene(i));
-    const uint32_t tol = link_tolerance(P, d.T[o], dynamic);
-    const uint32_t base = o * M;
-    uint32_t count = d.iter_end[o] - base;
-    uint32_t r[SNOWB_MAXC_FAST];
-#pragma unroll
-    for (int k = 0; k < SNOWB_MAXC_FAST; ++k) r[k] = (uint32_t)k < M ? d.connect_record[base + k] : 0u;
-    FOR27 {
-        uint32_t s, e;
-        if (!vd.range(P, g, ox, oy, oz, s, e)) continue;
-        for (uint32_t j = s; j < e; ++j) {
-            if (j == i) continue;
-            const float3 dv = sub3(p, vd.pos(j));
-            const float d2 = dot3(dv, dv);
-            if (!(d2 < P.h2_lt) || !(count < tol)) continue;
-            const uint32_t o1 = vd.gi[j];
-            const float dist = sqrtf(d2);
-            bool dup = false;
-            int free_k = -1;
-#pragma unroll
-            for (int k = 0; k < SNOWB_MAXC_FAST; ++k) {
-                if ((uint32_t)k < M) {
-                    dup |= r[k] == o1;
-                    if (free_k < 0 && r[k] == SNOWB_UMAX) free_k = k;
-                }
-            }
-            if (dup) break;               // the reference returns from the cell helper
-            if (free_k < 0) continue;     // no free slot: the claim loop finds nothing
-            d.connect_record[base + free_k] = o1;           // claim
-            bool valid = false;
-            const uint32_t b1 = o1 * M;
-            if (d.iter_end[o1] < b1 + M)
-                for (uint32_t q = b1; q < b1 + M; ++q)
-                    if (d.connect_record[q] == SNOWB_UMAX) {
-                        d.connect_record[q] = o;
-                        d.connect_length[q] = dist;
-                        d.iter_end[o1]++;
-                        if (o1 >= vd.n) atomicOr(&S->tail_dirty, 1u);
-                        if (o1 == o) {                       // self link (stale cell range)
-                            ++count;
-#pragma unroll
-                            for (int k = 0; k < SNOWB_MAXC_FAST; ++k)
-                                if ((uint32_t)k == q - base) r[k] = o;
-                        }
-                        valid = true;
-                        break;
-                    }
-            if (valid) {
-                d.connect_length[base + free_k] = dist;
-                ++count;
-                d.iter_end[o] = base + count;
-#pragma unroll
-                for (int k = 0; k < SNOWB_MAXC_FAST; ++k)
-                    if (k == free_k) r[k] = o1;
-                atomicAdd(&S->n_links, 1u);
-            } else {
-                d.connect_record[base + free_k] = SNOWB_UMAX;
-            }
-        }
-    }
-}
-// A particle's links by one warp.  The sequential rule of link_particle_fast, for up to 32
+// A particle's links by one warp.  The sequential rule of link_particle, for up to 32
 // candidates in traversal order (lane k holds candidate k), resolved at once:
 //  - a candidate that o is already linked to ends its cell, so it and the later candidates
 //    of its cell drop out;
@@ -972,7 +900,8 @@ __global__ void __launch_bounds__(LINK_TPB, 3) k_link_colour_warp(DevParams P, D
         __syncthreads();
     }
 }
-// general maximum_connection: the plain restatement with every access in memory
+// connect_and_record_cell (:4127-4252) + connect_and_record_d (:4255-4284) for one particle, the
+// sequential rule as it stands with every access in memory (maximum_connection > SNOWB_MAXC_FAST)
 __device__ void link_particle(const DevParams& P, const SetView& vd, const snowb_particle_data& d, uint32_t i,
                               int dynamic, DevState* S)
 {
@@ -1040,7 +969,7 @@ __global__ void k_copy_link_view(SetView v, uint32_t full, uint32_t ncells, floa
         if (k < ncells) { cs[k] = v.cs[k]; ce[k] = v.ce[k]; }
     }
 }
-// one colour: one thread per super-cell of that colour
+// one colour: one thread per super-cell of that colour (maximum_connection > SNOWB_MAXC_FAST)
 __global__ void k_link_colour(DevParams P, DevState* S, SetView vd, snowb_particle_data dem,
                               const uint8_t* __restrict__ active, uint32_t colour, int dynamic)
 {
@@ -1059,10 +988,7 @@ __global__ void k_link_colour(DevParams P, DevState* S, SetView vd, snowb_partic
                     uint32_t b = 0;
                     const uint32_t n = current_range(vd, h, b);
                     for (uint32_t i = b; i < b + n; ++i)
-                        if (active[i]) {
-                            if (P.maxc <= SNOWB_MAXC_FAST) link_particle_fast(P, vd, dem, i, dynamic, S);
-                            else link_particle(P, vd, dem, i, dynamic, S);
-                        }
+                        if (active[i]) link_particle(P, vd, dem, i, dynamic, S);
                 }
     }
 }

@@ -1570,7 +1570,7 @@ static int sort_pairs(uint32_t nc, snowb_cell_data cd, uint32_t n)
     CUDA_TRY(cudaMemsetAsync(g_ctx.err_dev, 0, sizeof(uint32_t), g_stream));
     LAUNCH(k_key_count, n, 256, cd.grid_hash, cd.grid_index, n, nc, B.key, B.val, B.slot, B.cnt, g_ctx.err_dev);
     const unsigned nb = (nc + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    KL(k_block_sums, nb, SCAN_TPB, B.cnt, nc, B.bsum, nullptr);
+    KL(k_block_sums, nb, SCAN_TPB, B.cnt, nc, B.bsum);
     KL(k_cell_scan, nb, SCAN_TPB, B.cnt, B.bsum, nc, B.off);
     LAUNCH(k_scatter, n, 256, B.key, B.slot, B.off, B.tmp, n);
     LAUNCH(k_rank_pairs, n, 256, B.key, B.val, B.off, B.tmp, cd.grid_hash, cd.grid_index, n);
@@ -1770,7 +1770,7 @@ int snowb_sort_particles_static(snowb_cell_data cd, uint32_t n)
     CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(uint32_t), g_stream));
     const unsigned nb = (nc + SCAN_CHUNK - 1) / SCAN_CHUNK;
     KL_PLAIN(k_key_count, blocks_for(n, 256), 256, cd.grid_hash, cd.grid_index, n, nc, key, val, slot, cnt, err);
-    KL_PLAIN(k_block_sums, nb, SCAN_TPB, cnt, nc, bsum, nullptr);
+    KL_PLAIN(k_block_sums, nb, SCAN_TPB, cnt, nc, bsum);
     KL_PLAIN(k_cell_scan, nb, SCAN_TPB, cnt, bsum, nc, off);
     KL_PLAIN(k_scatter, blocks_for(n, 256), 256, key, slot, off, tmp, n);
     KL_PLAIN(k_rank_pairs, blocks_for(n, 256), 256, key, val, off, tmp, cd.grid_hash, cd.grid_index, n);

@@ -69,9 +69,9 @@ __device__ __forceinline__ uint32_t prefix_of_blocks(const uint32_t* bsum, uint3
 
 // One or two sets sorted by the same four launches (the water and the snow set of a sort
 // point): the particle passes run over both sets' particles end to end, the scan over both
-// cell tables.  Two chains of launches on two streams, forked and joined at each sort point,
-// were 56 launches and 32 event calls a substep; these are 28 launches (issuing a substep: 330 ->
-// 230 us of host time; one substep of 208 particles 512 -> 480 us).
+// cell tables.  Two chains of launches on two streams, forked and joined at each sort point, were
+// 56 launches and 32 event calls a substep; these are 32 launches at its eight sort points
+// (issuing a substep: 330 -> 230 us of host time; one substep of 208 particles 512 -> 480 us).
 struct SortSide {
     const snowb_float3* pos;
     const float *w, *invm, *contrib;      // mass, massInv, contrib by original index
@@ -172,11 +172,9 @@ __global__ void k_key_count(const uint32_t* __restrict__ keys, const uint32_t* _
 }
 
 // ------------------------------------------------------------------ 2. scan of counts
-__global__ void k_block_sums(const uint32_t* __restrict__ cnt, uint32_t ncells, uint32_t* __restrict__ bsum,
-                             const uint32_t* cond)
+__global__ void k_block_sums(const uint32_t* __restrict__ cnt, uint32_t ncells, uint32_t* __restrict__ bsum)
 {
     wait_prior();
-    if (cond && *cond == 0) return;
     __shared__ uint32_t sm[SCAN_TPB / 32];
     const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
     uint32_t s = 0;
