@@ -139,7 +139,7 @@ static int dalloc(T** p, size_t count)
 
 struct SetBufs {
     uint32_t *key = nullptr, *slot = nullptr, *tmp = nullptr, *cnt = nullptr, *off = nullptr, *bsum = nullptr;
-    uint32_t *sup = nullptr, *dirty = nullptr;
+    uint32_t* dirty = nullptr;
     uint32_t* val = nullptr;
     float4* p4 = nullptr;
     float *invm = nullptr, *contrib = nullptr, *lambda = nullptr, *mass = nullptr;
@@ -194,7 +194,7 @@ static uint64_t g_ctx_gen = 0;   // bumped whenever the scratch buffers are (re)
 static void free_set(SetBufs& s)
 {
     void* ptrs[] = {s.key, s.slot, s.tmp, s.cnt, s.off, s.bsum, s.val, s.p4, s.invm, s.contrib, s.lambda, s.mass,
-                    s.sid, s.sup, s.dirty, s.base.rho, s.base.gs};
+                    s.sid, s.dirty, s.base.rho, s.base.gs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     s = SetBufs();
@@ -245,8 +245,7 @@ static int alloc_sort(SetBufs& s, uint32_t cap, uint32_t ncells, bool attrs)
     TRY(dalloc(&s.bsum, ncells / SCAN_CHUNK + 2));
     CUDA_TRY(cudaMemset(s.cnt, 0, sizeof(uint32_t) * ncells));
     CUDA_TRY(cudaMemset(s.bsum, 0, sizeof(uint32_t) * (ncells / SCAN_CHUNK + 2)));
-    TRY(dalloc(&s.sup, ncells / SCAN_CHUNK / SUP_CHUNKS + 2)); TRY(dalloc(&s.dirty, ncells / SCAN_CHUNK + 2));
-    CUDA_TRY(cudaMemset(s.sup, 0, sizeof(uint32_t) * (ncells / SCAN_CHUNK / SUP_CHUNKS + 2)));
+    TRY(dalloc(&s.dirty, ncells / SCAN_CHUNK + 2));
     CUDA_TRY(cudaMemset(s.dirty, 0xff, sizeof(uint32_t) * (ncells / SCAN_CHUNK + 2)));
     if (attrs) {
         TRY(dalloc(&s.p4, cap)); TRY(dalloc(&s.invm, cap)); TRY(dalloc(&s.contrib, cap)); TRY(dalloc(&s.lambda, cap));
@@ -551,7 +550,7 @@ static SortSide sort_side(SetBufs& B, const snowb_particle_data& D, const snowb_
                           const uint32_t* sid_o = nullptr)
 {
     return SortSide{D.predict_positions, D.mass, D.massInv, D.contrib, n, B.key, B.slot, B.tmp, B.cnt, B.off, B.bsum,
-                    B.sup, B.dirty, sid_o, sid_o ? B.sid : nullptr, cd, B.p4, B.invm, B.contrib};
+                    B.dirty, sid_o, sid_o ? B.sid : nullptr, cd, B.p4, B.invm, B.contrib};
 }
 // work: particles of the sorted sets together
 static int sort_sets(const DevParams& P, const SortPair& Q, uint64_t work)

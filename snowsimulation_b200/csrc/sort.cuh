@@ -77,7 +77,7 @@ struct SortSide {
     const float *w, *invm, *contrib;      // mass, massInv, contrib by original index
     const uint32_t* n;                    // set size (device)
     uint32_t *key, *slot, *tmp, *cnt, *off;
-    uint32_t *bsum, *sup;                 // particles per scan chunk, and per SUP_CHUNKS chunks; zero between sorts
+    uint32_t* bsum;                       // particles per scan chunk; zero between sorts
     uint32_t* dirty;                      // per scan chunk: its part of cell_start may hold entries
     const uint32_t* sid_o;                // scene ids by original index (batched runs) or null
     uint32_t* sid_s;
@@ -101,8 +101,6 @@ struct SortPair {
     __device__ __forceinline__ bool sorts(int k) const { return on[k] && (!S || S->resort[k] != 0u); }
     __device__ __forceinline__ uint32_t size(int k) const { return on[k] ? *a[k].n : 0u; }
 };
-constexpr uint32_t SUP_CHUNKS = 64;       // scan chunks per entry of `sup`, used past SUP_MIN chunks
-constexpr uint32_t SUP_MIN = 1024;
 
 // ------------------------------------------------------------------ 1. hash + count
 // Hash of pos[o] (calcHashD :194-212) and its cell's and scan chunk's counts (one chunk atomic
@@ -150,10 +148,7 @@ __global__ void k_sort_hash(DevParams P, const __grid_constant__ SortPair Q)
             chunk = h / (uint32_t)SCAN_CHUNK;
         }
         const uint32_t peers = __match_any_sync(0xffffffffu, chunk | (uint32_t)k << 30);
-        if (live && lane == (uint32_t)(__ffs(peers) - 1)) {
-            atomicAdd(A.bsum + chunk, (uint32_t)__popc(peers));
-            if (Q.ncells > SUP_MIN * SCAN_CHUNK) atomicAdd(A.sup + chunk / SUP_CHUNKS, (uint32_t)__popc(peers));
-        }
+        if (live && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(A.bsum + chunk, (uint32_t)__popc(peers));
     }
 }
 // sort_particles path: keys and values already in (grid_hash, grid_index).
@@ -243,7 +238,6 @@ __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ 
 {
     wait_prior();
     __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
-    __shared__ uint32_t s_prefix;
     const int k = blockIdx.x < chunks ? 0 : 1;
     const uint32_t chunk = blockIdx.x - (k ? chunks : 0u);
     const SortSide& A = Q.a[k];
@@ -259,21 +253,11 @@ __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ 
         if (threadIdx.x == 0) A.dirty[chunk] = dirty && end > clear ? 1u : 0u;
         return;
     }
-    if (threadIdx.x < 32) {
-        uint32_t p = 0;
-        if (Q.ncells > SUP_MIN * SCAN_CHUNK) {
-            const uint32_t s0 = chunk / SUP_CHUNKS;
-            p = prefix_of_blocks(A.sup, s0) + prefix_of_blocks(A.bsum + s0 * SUP_CHUNKS, chunk - s0 * SUP_CHUNKS);
-        } else {
-            p = prefix_of_blocks(A.bsum, chunk);
-        }
-        if (threadIdx.x == 0) {
-            s_prefix = p;
-            A.dirty[chunk] = 1u;
-        }
-    }
-    __syncthreads();
-    scan_chunk(A.cnt, Q.ncells, A.off, A.cd.cell_start, clear, chunk, s_prefix, sm);
+    uint32_t before = 0, prefix;
+    for (uint32_t c = threadIdx.x; c < chunk; c += SCAN_TPB) before += A.bsum[c];
+    block_excl_scan(before, sm, prefix);
+    if (threadIdx.x == 0) A.dirty[chunk] = 1u;
+    scan_chunk(A.cnt, Q.ncells, A.off, A.cd.cell_start, clear, chunk, prefix, sm);
 }
 
 // ------------------------------------------------------------------ 3. scatter
@@ -299,8 +283,8 @@ __global__ void k_sort_scatter(const __grid_constant__ SortPair Q, uint32_t chun
         A.tmp[A.off[A.key[o]] + A.slot[o]] = o;
     }
     GRID_LOOP(c, chunks) {
-        if (s0) { Q.a[0].bsum[c] = 0u; Q.a[0].sup[c / SUP_CHUNKS] = 0u; }
-        if (s1) { Q.a[1].bsum[c] = 0u; Q.a[1].sup[c / SUP_CHUNKS] = 0u; }
+        if (s0) Q.a[0].bsum[c] = 0u;
+        if (s1) Q.a[1].bsum[c] = 0u;
     }
 }
 
