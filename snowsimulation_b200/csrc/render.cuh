@@ -101,35 +101,41 @@ __device__ __forceinline__ bool sprite_fragment(const SpriteVtx& v, int px, int 
              fminf(fmaxf(diff * v.col.z, 0.f), 1.f));
     return true;
 }
-// Splats: SPLAT lanes take a particle and walk its covered pixels row by row, so one access of
+// Splats: LANES lanes take a particle and walk its covered pixels row by row, so one access of
 // a warp falls into fewer sectors of the image than 32 sprites' addresses would, and a lane has
 // a few pixels in turn instead of a whole sprite.  Draws of 148k and 6k sprites of 6 x 6 pixels
 // on 1280 x 720, mean: 24.3 us with one thread per particle, 16.9 with 4 lanes (2: 19.7; 8: 19.6).
+// A sprite of up to about two and a half pixels a side is not worth sharing: its vertex, formed
+// in every lane, is the work (1.18M sprites, point view seen from 3 m, point size 2: 49 us with
+// one lane, 71 with four; 6: 57 and 76; 8, a side of 2.7: 80 and 83; 12: 129 and 103).  The side
+// follows from the point size over the distance, of which the host knows the first;
+// SPLAT_ONE_SIZE is where the forms meet at 3 m (at 5 m: 52 us against 73 there, and they meet
+// at 14).
+constexpr float SPLAT_ONE_SIZE = 8.f;
 // READ: the depth that stands at a pixel is read first and a fragment that cannot win is dropped
 // before its arithmetic and its atomic (depths only fall during a launch, so an old value drops
 // nothing that belongs in the image).  It takes the wait for a read per pixel and saves atomics
 // on one address: the fluid view's default camera, whose far snow block puts about 200 sprites
 // on a pixel, 36.7 -> 27.1 us; the point view at about 25 a pixel, 16.9 -> 21.0 us, so it stays
 // out there.
-constexpr uint32_t SPLAT = 4;
-template <class F>
+template <uint32_t LANES, class F>
 __device__ __forceinline__ void splat_pixels(int x0, int x1, int y0, int y1, F&& f)
 {
     const int w = x1 - x0;
     if (w <= 0) return;
-    int px = x0 + (int)(threadIdx.x & (SPLAT - 1u)), py = y0;
+    int px = x0 + (int)(threadIdx.x & (LANES - 1u)), py = y0;
     while (true) {
         while (px >= x1) { px -= w; ++py; }
         if (py >= y1) return;
         f(px, py);
-        px += (int)SPLAT;
+        px += (int)LANES;
     }
 }
 #define SPLAT_LOOP(i, n, block, blocks)                                                    \
-    for (uint32_t i = ((block) * blockDim.x + threadIdx.x) / SPLAT; i < (n);               \
-         i += (blocks) * blockDim.x / SPLAT)
+    for (uint32_t i = ((block) * blockDim.x + threadIdx.x) / LANES; i < (n);               \
+         i += (blocks) * blockDim.x / LANES)
 
-template <bool READ>
+template <uint32_t LANES, bool READ>
 __device__ __forceinline__ void splat_points(const RenderCam& c, const RenderColour& rc,
                                              const snowb_float3* __restrict__ pos, uint32_t n, uint32_t draw,
                                              unsigned long long* zbuf, uint32_t block, uint32_t blocks)
@@ -143,18 +149,19 @@ __device__ __forceinline__ void splat_points(const RenderCam& c, const RenderCol
         uint32_t db;
         memcpy(&db, &v.depth, 4);
         const unsigned long long key = ((unsigned long long)db << 32) | ((unsigned long long)draw << 27) | i;
-        splat_pixels(x0, x1, y0, y1, [&](int px, int py) {
+        splat_pixels<LANES>(x0, x1, y0, y1, [&](int px, int py) {
             unsigned long long* const z = zbuf + (size_t)py * c.W + px;
             float3 rgb;
             if ((!READ || key < *z) && sprite_fragment(v, px, py, rgb)) atomicMin(z, key);
         });
     }
 }
+template <uint32_t LANES>
 __global__ void __launch_bounds__(128) kr_depth(RenderCam c, RenderColour rc, const snowb_float3* __restrict__ pos,
                                                 uint32_t n, uint32_t draw, unsigned long long* zbuf)
 {
     wait_prior();
-    splat_points<false>(c, rc, pos, n, draw, zbuf, blockIdx.x, gridDim.x);
+    splat_points<LANES, false>(c, rc, pos, n, draw, zbuf, blockIdx.x, gridDim.x);
 }
 // one pixel of the image, in one 16-byte store where the image is aligned for it (v4)
 __device__ __forceinline__ void put_pixel(float* __restrict__ rgba, uint32_t k, float4 o, int v4)

@@ -2081,13 +2081,22 @@ int snowb_render_clear_colour(const snowb_camera* cam, const float* clear_rgba, 
     return SNOWB_OK;
 }
 
-// one block per SPLAT * n threads, not fewer that loop: sprites differ in size and finished
+// one block per lanes * n threads, not fewer that loop: sprites differ in size and finished
 // blocks make room for the next
-static unsigned splat_blocks(uint32_t n, int tpb)
+static unsigned splat_blocks(uint32_t n, uint32_t lanes, int tpb)
 {
-    const uint64_t b = ((uint64_t)SPLAT * n + tpb - 1) / tpb;
+    const uint64_t b = ((uint64_t)lanes * n + tpb - 1) / tpb;
     return b < 1 ? 1u : (b > 0xffffffull ? 0xffffffu : (unsigned)b);
 }
+
+// a splat kernel with the lanes that suit the point size (SPLAT_ONE_SIZE); `lanes` in the arguments
+// is that number
+#define SPLAT_LAUNCH(kernel, point_size, grid, tpb, ...)                                   \
+    do {                                                                                   \
+        const uint32_t lanes = (point_size) <= SPLAT_ONE_SIZE ? 1u : 4u;                   \
+        if (lanes == 1u) KL_AS(#kernel, kernel<1u>, (grid), tpb, __VA_ARGS__);             \
+        else KL_AS(#kernel, kernel<4u>, (grid), tpb, __VA_ARGS__);                         \
+    } while (0)
 
 static RenderColour render_colour(const snowb_point_colour* colour)
 {
@@ -2112,7 +2121,7 @@ int snowb_render_points(const snowb_particle_data* set, uint32_t n, const snowb_
     if (n == 0) return SNOWB_OK;
     const RenderColour rc = render_colour(colour);
     const float* T = rc.temp ? set->T : nullptr;
-    KL(kr_depth, splat_blocks(n, 128), 128, c, rc, set->positions, n, draw, zbuf);
+    SPLAT_LAUNCH(kr_depth, c.point_size, splat_blocks(n, lanes, 128), 128, c, rc, set->positions, n, draw, zbuf);
     LAUNCH(kr_shade, (uint64_t)c.W * c.H, 256, c, rc, set->positions, T, draw, zbuf, rgba, aligned16(rgba));
     return SNOWB_OK;
 }
@@ -2211,7 +2220,8 @@ int snowb_ssfr_sphere_depth(const snowb_particle_data* set, uint32_t n, const sn
     TRY(ssfr_cam(cam, ssfr, c));
     if (!set || !ssfr || !depth) return fail(SNOWB_ERR_INVALID, "null pointer");
     if (n == 0) return SNOWB_OK;
-    KL(ks_sphere_depth, splat_blocks(n, 128), 128, c, set->positions, n, reinterpret_cast<uint32_t*>(depth));
+    SPLAT_LAUNCH(ks_sphere_depth, c.point_size, splat_blocks(n, lanes, 128), 128, c, set->positions, n,
+                 reinterpret_cast<uint32_t*>(depth));
     return SNOWB_OK;
 }
 
@@ -2221,7 +2231,7 @@ int snowb_ssfr_thickness(const snowb_particle_data* set, uint32_t n, const snowb
     TRY(ssfr_cam(cam, nullptr, c));
     if (!set || !thick) return fail(SNOWB_ERR_INVALID, "null pointer");
     if (n == 0) return SNOWB_OK;
-    KL(ks_thickness, splat_blocks(n, 128), 128, c, set->positions, n, thick);
+    SPLAT_LAUNCH(ks_thickness, c.point_size, splat_blocks(n, lanes, 128), 128, c, set->positions, n, thick);
     return SNOWB_OK;
 }
 
@@ -2285,12 +2295,12 @@ int snowb_render_fluid(const snowb_particle_data* sph, uint32_t n_sph, const sno
     const RenderColour col = render_colour(snow_colour);
     uint32_t* const sdepth = reinterpret_cast<uint32_t*>(scene_depth);
     LAUNCH(ks_view_clear, np, 256, (uint32_t)np, zbuf, thick, sdepth, reinterpret_cast<uint32_t*>(fdepth));
-    const uint32_t b_snow = splat_blocks(n_dem, 128), b_water = splat_blocks(n_sph, 128);
-    KL(ks_view_splat, b_snow + b_water, 128, rc, col, c, dem->positions, n_dem, sph->positions, n_sph, zbuf,
-       reinterpret_cast<uint32_t*>(fdepth), thick, b_snow);
-    const uint32_t b_px = blocks_for(np, 256), b_depth = splat_blocks(n_dem, 256);
-    KL(ks_view_filter, b_px + b_depth, 256, rc, col, c, s, dem->positions, col.temp ? dem->T : nullptr, n_dem, zbuf,
-       scene, fdepth, tmp, sdepth, b_px);
+    SPLAT_LAUNCH(ks_view_splat, c.point_size, splat_blocks(n_dem, lanes, 128) + splat_blocks(n_sph, lanes, 128), 128, rc, col,
+                 c, dem->positions, n_dem, sph->positions, n_sph, zbuf, reinterpret_cast<uint32_t*>(fdepth), thick,
+                 splat_blocks(n_dem, lanes, 128));
+    const uint32_t b_px = blocks_for(np, 256);
+    SPLAT_LAUNCH(ks_view_filter, c.point_size, b_px + splat_blocks(n_dem, lanes, 256), 256, rc, col, c, s,
+                 dem->positions, col.temp ? dem->T : nullptr, n_dem, zbuf, scene, fdepth, tmp, sdepth, b_px);
     LAUNCH(ks_bilateral, np, 256, c, s, tmp, smooth, 1);
     LAUNCH(ks_compose, np, 256, c, s, smooth, thick, scene, scene_depth, rgba, 1, aligned16(rgba));
     return SNOWB_OK;

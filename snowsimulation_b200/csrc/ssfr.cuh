@@ -89,10 +89,10 @@ __device__ __forceinline__ bool sphere_coord(const DepthVtx& v, int px, int py, 
     return true;
 }
 
-// One set's spheres, SPLAT lanes a particle (see splat_pixels).  DEPTH: into depth (float bits,
+// One set's spheres, LANES lanes a particle (see splat_pixels).  DEPTH: into depth (float bits,
 // cleared to 1.0), the minimum over fragments.  THICK: thickness, 32.32 fixed point per pixel.
 // MASK: only where mask (another set's depth) lies inside 0..1.
-template <bool DEPTH, bool THICK, bool MASK>
+template <uint32_t LANES, bool DEPTH, bool THICK, bool MASK>
 __device__ __forceinline__ void splat_spheres(const SsfrCam& c, const snowb_float3* __restrict__ pos, uint32_t n,
                                               uint32_t* depth, unsigned long long* thick,
                                               const float* __restrict__ mask, uint32_t block, uint32_t blocks)
@@ -103,7 +103,7 @@ __device__ __forceinline__ void splat_spheres(const SsfrCam& c, const snowb_floa
         int x0, x1, y0, y1;
         sprite_span(v.xw, v.side, c.W, x0, x1);
         sprite_span(v.yw, v.side, c.H, y0, y1);
-        splat_pixels(x0, x1, y0, y1, [&](int px, int py) {
+        splat_pixels<LANES>(x0, x1, y0, y1, [&](int px, int py) {
             const size_t k = (size_t)py * c.W + px;
             if (MASK) {
                 const float m = mask[k];
@@ -127,17 +127,19 @@ __device__ __forceinline__ void splat_spheres(const SsfrCam& c, const snowb_floa
         });
     }
 }
+template <uint32_t LANES>
 __global__ void __launch_bounds__(128) ks_sphere_depth(SsfrCam c, const snowb_float3* __restrict__ pos, uint32_t n,
                                                        uint32_t* depth)
 {
     wait_prior();
-    splat_spheres<true, false, false>(c, pos, n, depth, nullptr, nullptr, blockIdx.x, gridDim.x);
+    splat_spheres<LANES, true, false, false>(c, pos, n, depth, nullptr, nullptr, blockIdx.x, gridDim.x);
 }
+template <uint32_t LANES>
 __global__ void __launch_bounds__(128) ks_thickness(SsfrCam c, const snowb_float3* __restrict__ pos, uint32_t n,
                                                     unsigned long long* thick)
 {
     wait_prior();
-    splat_spheres<false, true, false>(c, pos, n, nullptr, thick, nullptr, blockIdx.x, gridDim.x);
+    splat_spheres<LANES, false, true, false>(c, pos, n, nullptr, thick, nullptr, blockIdx.x, gridDim.x);
 }
 __device__ __forceinline__ float thickness_value(unsigned long long q, float clear_r)
 {
@@ -307,6 +309,7 @@ __global__ void ks_view_clear(uint32_t npix, unsigned long long* __restrict__ zb
         scene_depth[k] = fluid_depth[k] = 0x3f800000u;
     }
 }
+template <uint32_t LANES>
 __global__ void __launch_bounds__(128) ks_view_splat(RenderCam rc, RenderColour col, SsfrCam c,
                                                      const snowb_float3* __restrict__ snow, uint32_t n_snow,
                                                      const snowb_float3* __restrict__ water, uint32_t n_water,
@@ -314,11 +317,12 @@ __global__ void __launch_bounds__(128) ks_view_splat(RenderCam rc, RenderColour 
                                                      unsigned long long* thick, uint32_t split)
 {
     wait_prior();
-    if (blockIdx.x < split) splat_points<true>(rc, col, snow, n_snow, 0u, zbuf, blockIdx.x, split);
+    if (blockIdx.x < split) splat_points<LANES, true>(rc, col, snow, n_snow, 0u, zbuf, blockIdx.x, split);
     else
-        splat_spheres<true, true, false>(c, water, n_water, fluid_depth, thick, nullptr, blockIdx.x - split,
+        splat_spheres<LANES, true, true, false>(c, water, n_water, fluid_depth, thick, nullptr, blockIdx.x - split,
                                          gridDim.x - split);
 }
+template <uint32_t LANES>
 __global__ void __launch_bounds__(256) ks_view_filter(RenderCam rc, RenderColour col, SsfrCam c, SsfrShade s,
                                                       const snowb_float3* __restrict__ snow,
                                                       const float* __restrict__ T, uint32_t n_snow,
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(256) ks_view_filter(RenderCam rc, RenderColour
     wait_prior();
     __shared__ BilateralTaps B;
     if (blockIdx.x >= split) {
-        splat_spheres<true, false, true>(c, snow, n_snow, scene_depth, nullptr, fluid_depth, blockIdx.x - split,
+        splat_spheres<LANES, true, false, true>(c, snow, n_snow, scene_depth, nullptr, fluid_depth, blockIdx.x - split,
                                          gridDim.x - split);
         return;
     }
