@@ -14,11 +14,10 @@
 // term in which it takes part, from its own constraint and from its neighbours', so no
 // atomics are needed except for the scalar parameter gradients.
 //
-// The neighbour passes run one warp per particle (warp_neighbors): with the few thousand
-// particles that are differentiated, one thread each left most of the GPU idle while it
-// walked up to 81 cells one candidate after another (9,216 particles, us a launch: fields
-// 90 -> 43, lambda adjoint 99 -> 19, positions 130 -> 43, friction 81 -> 25, XSPH 79 -> 20,
-// heat 94 -> 31).
+// The neighbour passes run one warp per particle (warp_neighbors) where one thread each leaves most
+// of the GPU idle while it walks up to 81 cells one candidate after another (9,216 particles, us a
+// launch: fields 90 -> 43, lambda adjoint 99 -> 19, positions 130 -> 43, friction 81 -> 25, XSPH
+// 79 -> 20, heat 94 -> 31), and one thread per particle above ADJ_WARP_MAX.
 //
 // Notation: r = x_i - x_j, d = |r|.  For a radial vector function F(r) = f(d) r its
 // Jacobian is J = f I + (f'(d)/d) r r^T (symmetric, even in r).
@@ -155,9 +154,69 @@ __device__ __forceinline__ void warp_neighbors(const SetView& v, float3 p, uint3
         }
     }
 }
-// sum a of the ordered sums, for every lane
-__device__ __forceinline__ float sum_of(float acc, int a) { return __shfl_sync(0xffffffffu, acc, a); }
-__device__ __forceinline__ float3 sum3_of(float acc, int a) { return f3(sum_of(acc, a), sum_of(acc, a + 1), sum_of(acc, a + 2)); }
+// The passes below are written once for both forms: WARP, a particle to a warp, lane a < NA holding
+// sum a; else a particle to a thread, which holds all sums and walks the cells itself.  Either way
+// a sum's addends are added neighbour by neighbour in traversal order.
+template <bool WARP, int NA>
+struct AdjSums {
+    float v[WARP ? 1 : NA];
+    __device__ __forceinline__ AdjSums()
+    {
+#pragma unroll
+        for (int a = 0; a < (WARP ? 1 : NA); ++a) v[a] = 0.f;
+    }
+    __device__ __forceinline__ void start(int a, float x)
+    {
+        if (!WARP) v[WARP ? 0 : a] = x;
+        else if ((threadIdx.x & 31u) == (uint32_t)a) v[0] = x;
+    }
+    // sum a, for every lane
+    __device__ __forceinline__ float of(int a) const { return WARP ? __shfl_sync(0xffffffffu, v[0], a) : v[WARP ? 0 : a]; }
+    __device__ __forceinline__ float3 of3(int a) const { return f3(of(a), of(a + 1), of(a + 2)); }
+};
+// where a particle looks for neighbours: its cell, and a lane's own one of the 27 around it
+template <bool WARP>
+struct AdjCell {
+    GCell g;
+    uint32_t h;
+    __device__ __forceinline__ AdjCell(const DevParams& P, float3 p) : g(grid_pos(P, p)), h(WARP ? lane_cell(P, g) : 0u) {}
+};
+template <int M, bool WARP, int NA, class F>
+__device__ __forceinline__ void adj_neighbors(const DevParams& P, const SetView& v, float3 p, const AdjCell<WARP>& c,
+                                              uint32_t skip, float cut, AdjBuf& W, AdjSums<WARP, NA>& sums, F&& terms)
+{
+    if constexpr (WARP) {
+        warp_neighbors<NA, M>(v, p, c.h, skip, cut, W, sums.v[0], terms);
+    } else {
+        FOR27 {
+            uint32_t s, e;
+            if (!v.range(P, c.g, ox, oy, oz, s, e)) continue;
+            for (uint32_t j = s; j < e; ++j) {
+                const float3 r = sub3(p, xyz(__ldg(v.p4 + j)));
+                if (j == skip || !(dot3(r, r) < cut)) continue;
+                float out[NA * M];
+                terms(j, out);
+#pragma unroll
+                for (int a = 0; a < NA; ++a)
+#pragma unroll
+                    for (int q = 0; q < M; ++q) sums.v[a] += out[a * M + q];
+            }
+        }
+    }
+}
+// particles t < n of such a pass; the thread that writes a particle's results
+#define ADJ_LOOP(WARP, t, n)                                                                      \
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> ((WARP) ? 5 : 0); t < (n);        \
+         t += (gridDim.x * blockDim.x) >> ((WARP) ? 5 : 0))
+#define ADJ_LEAD(WARP) (!(WARP) || (threadIdx.x & 31u) == 0u)
+// Up to so many particles (water + snow) the passes run one warp each, above it one thread each.
+// One warp | one thread, us a launch, at 9.2k, 47.9k, 83.5k and 153.8k particles: fields 43 | 102,
+// 91 | 138, 148 | 148, 244 | 156; positions 43 | 122, 134 | 181, 220 | 201, 390 | 283; friction
+// 25 | 84, 90 | 104, 150 | 116, 274 | 199; XSPH 20 | 83, 60 | 127, 94 | 124, 165 | 139; heat 30 | 95,
+// 118 | 130, 200 | 136, 363 | 192 (the lambda adjoint, fewer neighbours, stays with one warp).  A
+// gradient of three substeps meets at 75k: 17.1 | 17.8 ms at 70.2k, 18.4 | 17.8 at 83.5k, and
+// 26.2 | 22.2 at 153.8k.
+constexpr uint32_t ADJ_WARP_MAX = 75000;
 // addend q of the three sums from a on (M addends each)
 template <int M>
 __device__ __forceinline__ void put3(float* out, int a, int q, float3 x)
@@ -194,11 +253,11 @@ __device__ __forceinline__ void field_store(const DevParams& P, const AdjField& 
 }
 // a particle's density (sum 0) and gradient-square (sum 1) terms from the entries of set v (vol:
 // the boundary, whose lambda denominator scales with the volume over m_of(j))
-template <class F>
-__device__ __forceinline__ void field_terms(const DevParams& P, const SetView& v, float3 p, uint32_t h, uint32_t skip,
-                                            bool vol, AdjBuf& W, float& acc, F&& m_of)
+template <bool WARP, class F>
+__device__ __forceinline__ void field_terms(const DevParams& P, const SetView& v, float3 p, const AdjCell<WARP>& c,
+                                            uint32_t skip, bool vol, AdjBuf& W, AdjSums<WARP, 2>& acc, F&& m_of)
 {
-    warp_neighbors<2, 1>(v, p, h, skip, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+    adj_neighbors<1>(P, v, p, c, skip, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
         const float4 q = __ldg(v.p4 + j);
         const float3 r = sub3(p, xyz(q));
         const float d = sqrtf(dot3(r, r));
@@ -220,40 +279,44 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_boundary_base(DevParams P, uint32_
     vb.n = nb;
     WARP_LOOP(i, nb) {
         const float3 p = xyz(vb.p4[i]);
-        float acc = lane == 0u ? (P.rho0 * X.bnd.volume[vb.gi[i]]) * P.W0 : 0.f;
-        field_terms(P, vb, p, lane_cell(P, grid_pos(P, p)), i, true, W, acc,
-                    [&](uint32_t j) { return X.bnd.mass[vb.gi[j]]; });
-        if (lane == 0u) rho0[i] = acc;
-        if (lane == 1u) S0[i] = acc;
+        AdjSums<true, 2> acc;
+        acc.start(0, (P.rho0 * X.bnd.volume[vb.gi[i]]) * P.W0);
+        field_terms(P, vb, p, AdjCell<true>(P, p), i, true, W, acc, [&](uint32_t j) { return X.bnd.mass[vb.gi[j]]; });
+        if (lane == 0u) rho0[i] = acc.v[0];
+        if (lane == 1u) S0[i] = acc.v[0];
     }
 }
+// first: the particles (water, snow, boundary in that order) before it are not taken; the one-thread
+// form takes the water and snow, and the boundary comes from the other form
+template <bool WARP>
 __global__ void __launch_bounds__(ADJ_TPB) ka_fields(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
                                                      SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
                                                      AdjField fb, const float* __restrict__ rho0,
-                                                     const float* __restrict__ S0)
+                                                     const float* __restrict__ S0, uint32_t first)
 {
     wait_prior();
-    __shared__ AdjBuf bufs[ADJ_TPB / 32];
-    AdjBuf& W = bufs[threadIdx.x >> 5];
+    __shared__ AdjBuf bufs[WARP ? ADJ_TPB / 32 : 1];
+    AdjBuf& W = bufs[WARP ? threadIdx.x >> 5 : 0];
     vw.n = nw; vs.n = ns; vb.n = nb;
-    const uint32_t lane = threadIdx.x & 31u;
-    WARP_LOOP(t, nw + ns + (nb + 31u) / 32u) {
+    ADJ_LOOP(WARP, t0, nw + ns + (WARP ? (nb + 31u) / 32u : 0u) - first) {
+        const uint32_t t = t0 + first;
         if (t < nw + ns) {
             const bool w = t < nw;
             const uint32_t i = w ? t : t - nw;
             const SetView& own = w ? vw : vs;
             const uint32_t o = own.gi[i];
             const float3 p = xyz(own.p4[i]);
-            const uint32_t h = lane_cell(P, grid_pos(P, p));
+            const AdjCell<WARP> c(P, p);
             const float mi = (w ? X.sph.mass : X.dem.mass)[o];
             auto m_of = [&](uint32_t) { return mi; };
-            float acc = lane == 0u ? mi * P.W0 : 0.f;
-            field_terms(P, vw, p, h, w ? i : SNOWB_UMAX, false, W, acc, m_of);
-            field_terms(P, vs, p, h, w ? SNOWB_UMAX : i, false, W, acc, m_of);
-            field_terms(P, vb, p, h, SNOWB_UMAX, true, W, acc, m_of);
-            const float S = sum_of(acc, 1);
-            if (lane == 0u) field_store(P, w ? fw : fs, o, acc, S);
-        } else {
+            AdjSums<WARP, 2> acc;
+            acc.start(0, mi * P.W0);
+            field_terms(P, vw, p, c, w ? i : SNOWB_UMAX, false, W, acc, m_of);
+            field_terms(P, vs, p, c, w ? SNOWB_UMAX : i, false, W, acc, m_of);
+            field_terms(P, vb, p, c, SNOWB_UMAX, true, W, acc, m_of);
+            const float rho = acc.of(0), S = acc.of(1);
+            if (ADJ_LEAD(WARP)) field_store(P, w ? fw : fs, o, rho, S);
+        } else if constexpr (WARP) {
             boundary_patch(
                 t - nw - ns, nb,
                 [&](uint32_t i) {
@@ -263,14 +326,16 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_fields(DevParams P, uint32_t nw, u
                 },
                 [&](uint32_t i) {
                     const float3 p = xyz(vb.p4[i]);
-                    const uint32_t o = vb.gi[i], h = lane_cell(P, grid_pos(P, p));
+                    const uint32_t o = vb.gi[i];
+                    const AdjCell<true> c(P, p);
                     auto m_of = [&](uint32_t j) { return X.bnd.mass[vb.gi[j]]; };
-                    float acc = lane == 0u ? (P.rho0 * X.bnd.volume[o]) * P.W0 : 0.f;
-                    field_terms(P, vw, p, h, SNOWB_UMAX, false, W, acc, m_of);
-                    field_terms(P, vs, p, h, SNOWB_UMAX, false, W, acc, m_of);
-                    field_terms(P, vb, p, h, i, true, W, acc, m_of);
-                    const float S = sum_of(acc, 1);
-                    if (lane == 0u) field_store(P, fb, o, acc, S);
+                    AdjSums<true, 2> acc;
+                    acc.start(0, (P.rho0 * X.bnd.volume[o]) * P.W0);
+                    field_terms(P, vw, p, c, SNOWB_UMAX, false, W, acc, m_of);
+                    field_terms(P, vs, p, c, SNOWB_UMAX, false, W, acc, m_of);
+                    field_terms(P, vb, p, c, i, true, W, acc, m_of);
+                    const float rho = acc.of(0), S = acc.of(1);
+                    if (ADJ_LEAD(true)) field_store(P, fb, o, rho, S);
                 });
         }
     }
@@ -359,22 +424,22 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_pbf_lambar(DevParams P, uint32_t n
 // terms of rho-bar (which also carries the XSPH and heat contributions at these
 // positions when they were accumulated before).  pbf != 0 adds the constraint terms;
 // pbf == 0 runs the density part alone (heat, substep start).
+template <bool WARP>
 __global__ void __launch_bounds__(ADJ_TPB) ka_pos_rev(DevParams P, uint32_t nw, uint32_t ns, uint32_t nb, SetView vw,
                                                   SetView vs, SetView vb, Sets X, AdjField fw, AdjField fs,
                                                   AdjField fb, AdjSet aw, AdjSet as, float* __restrict__ kst, int pbf, int contact)
 {
     wait_prior();
-    __shared__ AdjBuf bufs[ADJ_TPB / 32];
-    AdjBuf& W = bufs[threadIdx.x >> 5];
+    __shared__ AdjBuf bufs[WARP ? ADJ_TPB / 32 : 1];
+    AdjBuf& W = bufs[WARP ? threadIdx.x >> 5 : 0];
     vw.n = nw; vs.n = ns; vb.n = nb;
-    const uint32_t lane = threadIdx.x & 31u;
-    WARP_LOOP(t, nw + ns) {
+    ADJ_LOOP(WARP, t, nw + ns) {
         const int set = t < nw ? 0 : 1;
         const uint32_t i = set == 0 ? t : t - nw;
         const SetView& own = set == 0 ? vw : vs;
         const uint32_t o = own.gi[i];
         const float3 p = xyz(own.p4[i]);
-        const uint32_t h = lane_cell(P, grid_pos(P, p));
+        const AdjCell<WARP> c(P, p);
         const AdjField& Fi = set == 0 ? fw : fs;
         const AdjSet& Ai = set == 0 ? aw : as;
         const snowb_particle_data& Di = set == 0 ? X.sph : X.dem;
@@ -383,12 +448,12 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_pos_rev(DevParams P, uint32_t nw, 
         const float lam_i = pbf ? Fi.lam[o] : 0.f;
         const float3 ui = pbf ? ldv3(Ai.u, o) : f3(0.f, 0.f, 0.f);
         // sums 0..2: position adjoint (up to four addends a neighbour); 3..5: k_stretch direction
-        float acc = 0.f;
+        AdjSums<WARP, 6> acc;
         for (int k = 0; k < 3; ++k) {
             const SetView& v = k == 0 ? vw : (k == 1 ? vs : vb);
             const AdjField& Fj = k == 0 ? fw : (k == 1 ? fs : fb);
             const bool self = k == set;
-            warp_neighbors<6, 4>(v, p, h, self ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+            adj_neighbors<4>(P, v, p, c, self ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
 #pragma unroll
                 for (int q = 0; q < 24; ++q) out[q] = 0.f;
                 const float4 q = __ldg(v.p4 + j);
@@ -463,8 +528,8 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_pos_rev(DevParams P, uint32_t nw, 
                 }
             });
         }
-        const float3 xb = sum3_of(acc, 0), kst_dir = sum3_of(acc, 3);
-        if (lane == 0u) {
+        const float3 xb = acc.of3(0), kst_dir = acc.of3(3);
+        if (ADJ_LEAD(WARP)) {
             st3(Ai.xb, o, add3(ldv3(Ai.xb, o), xb));
             if (pbf) kst[t] = set == 1 ? dot3(ui, kst_dir) : 0.f;
         }
@@ -615,22 +680,23 @@ __device__ __forceinline__ void friction_vjp(const DevParams& P, float3 dx, floa
 }
 // snow particles at the friction pass's positions (sorted view vs) and the start
 // positions after integration x0p; u = sor * adjoint of the positions after friction.
+template <bool WARP>
 __global__ void __launch_bounds__(ADJ_TPB) ka_friction_rev(DevParams P, uint32_t ns, uint32_t nb, SetView vs, SetView vb,
                                                            Sets X, AdjSet as)
 {
     wait_prior();
-    __shared__ AdjBuf bufs[ADJ_TPB / 32];
-    AdjBuf& W = bufs[threadIdx.x >> 5];
+    __shared__ AdjBuf bufs[WARP ? ADJ_TPB / 32 : 1];
+    AdjBuf& W = bufs[WARP ? threadIdx.x >> 5 : 0];
     vs.n = ns; vb.n = nb;
-    WARP_LOOP(i, ns) {
+    ADJ_LOOP(WARP, i, ns) {
         const uint32_t o = vs.gi[i];
         const float3 p = xyz(vs.p4[i]);
-        const uint32_t h = lane_cell(P, grid_pos(P, p));
+        const AdjCell<WARP> c(P, p);
         const float3 op0 = ldv3(as.x0p, o);
         const float w0 = X.dem.massInv[o];
         const float3 ui = ldv3(as.u, o);
-        float acc = 0.f;   // sums 0..2: positions, 3..5: start positions; two addends a neighbour
-        warp_neighbors<6, 2>(vs, p, h, i, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+        AdjSums<WARP, 6> acc;   // sums 0..2: positions, 3..5: start positions; two addends a neighbour
+        adj_neighbors<2>(P, vs, p, c, i, P.r2_le, W, acc, [&](uint32_t j, float* out) {
             const float3 pp1 = xyz(__ldg(vs.p4 + j));
             const float3 r = sub3(p, pp1);
             const float d = sqrtf(dot3(r, r));
@@ -646,15 +712,15 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_friction_rev(DevParams P, uint32_t
             put3<2>(out, 0, 1, sub3(dxb, rb));
             put3<2>(out, 3, 1, sc3(-1.f, dxb));
         });
-        warp_neighbors<6, 1>(vb, p, h, SNOWB_UMAX, P.r2_le, W, acc, [&](uint32_t j, float* out) {
+        adj_neighbors<1>(P, vb, p, c, SNOWB_UMAX, P.r2_le, W, acc, [&](uint32_t j, float* out) {
             const float3 r = sub3(p, xyz(__ldg(vb.p4 + j)));
             float3 dxb, rb;
             friction_vjp(P, sub3(p, op0), w0, X.bnd.massInv[vb.gi[j]], sqrtf(dot3(r, r)), r, ui, dxb, rb);
             put3<1>(out, 0, 0, add3(dxb, rb));
             put3<1>(out, 3, 0, sc3(-1.f, dxb));
         });
-        const float3 pb = sum3_of(acc, 0), x0b = sum3_of(acc, 3);
-        if ((threadIdx.x & 31u) == 0u) {
+        const float3 pb = acc.of3(0), x0b = acc.of3(3);
+        if (ADJ_LEAD(WARP)) {
             st3(as.xb, o, add3(ldv3(as.xb, o), pb));
             st3(as.x0b, o, add3(ldv3(as.x0b, o), x0b));
         }
@@ -667,6 +733,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_friction_rev(DevParams P, uint32_t
 // (own sum: velocity, position and density adjoints), warps [nA, nA + nB) particles of
 // B (as neighbours of A).  Outputs are added to vbA/vbB (velocity adjoints), xbA/xbB and
 // rhobA/rhobB.  A's own velocity adjoint keeps its identity term.
+template <bool WARP>
 __global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA, uint32_t nB, SetView vA, SetView vB,
                                                    const snowb_float3* __restrict__ velA,
                                                    const snowb_float3* __restrict__ velB,
@@ -677,22 +744,21 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA,
                                                    snowb_float3* xbB, float* rhobA, float* rhobB)
 {
     wait_prior();
-    __shared__ AdjBuf bufs[ADJ_TPB / 32];
-    AdjBuf& W = bufs[threadIdx.x >> 5];
+    __shared__ AdjBuf bufs[WARP ? ADJ_TPB / 32 : 1];
+    AdjBuf& W = bufs[WARP ? threadIdx.x >> 5 : 0];
     vA.n = nA; vB.n = nB;
-    const uint32_t lane = threadIdx.x & 31u;
-    WARP_LOOP(t, nA + nB) {
+    ADJ_LOOP(WARP, t, nA + nB) {
         const bool inA = t < nA;
         const uint32_t i = inA ? t : t - nA;
         const SetView& own = inA ? vA : vB;
         const uint32_t o = own.gi[i];
         const float3 p = xyz(own.p4[i]);
-        const uint32_t h = lane_cell(P, grid_pos(P, p));
+        const AdjCell<WARP> cell(P, p);
         const float3 vi = ldv3(inA ? velA : velB, o);
         const float mi = (inA ? massA : massB)[o], rhoi = (inA ? rhoA : rhoB)[o];
         const float ai = mi / rhoi;
         // sums 0..2: positions (two addends a neighbour), 3..5: velocities, 6: density, 7: weights
-        float acc = 0.f;
+        AdjSums<WARP, 8> acc;
         // i as a neighbour of A-particle j: c a_i (v_i - v_j) W, adjoint g_j
         auto as_neighbor = [&](float* out, int q, uint32_t oj, float3 vj, float3 r, float d, float Wd) {
             const float3 gj = ldv3(gb, oj);
@@ -706,7 +772,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA,
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const SetView& v = k == 0 ? vA : vB;
-                warp_neighbors<8, 2>(v, p, h, k == 0 ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+                adj_neighbors<2>(P, v, p, cell, k == 0 ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
                     for (int q = 0; q < 16; ++q) out[q] = 0.f;
                     const float3 r = sub3(p, xyz(__ldg(v.p4 + j)));
                     const float d = sqrtf(dot3(r, r));
@@ -720,20 +786,20 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA,
                     if (k == 0) as_neighbor(out, 1, oj, vj, r, d, Wd);
                 });
             }
-            vb = add3(sum3_of(acc, 3), sc3(1.f - c * sum_of(acc, 7), gi));
+            vb = add3(acc.of3(3), sc3(1.f - c * acc.of(7), gi));
         } else {
-            warp_neighbors<8, 2>(vA, p, h, SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+            adj_neighbors<2>(P, vA, p, cell, SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
                 for (int q = 0; q < 16; ++q) out[q] = 0.f;
                 const float3 r = sub3(p, xyz(__ldg(vA.p4 + j)));
                 const float d = sqrtf(dot3(r, r));
                 const uint32_t oj = vA.gi[j];
                 as_neighbor(out, 0, oj, ldv3(velA, oj), r, d, W_poly6(P, d));
             });
-            vb = sum3_of(acc, 3);
+            vb = acc.of3(3);
         }
-        const float3 xb = sum3_of(acc, 0);
-        const float rb = sum_of(acc, 6);
-        if (lane == 0u) {
+        const float3 xb = acc.of3(0);
+        const float rb = acc.of(6);
+        if (ADJ_LEAD(WARP)) {
             snowb_float3 *const vo = inA ? vbA : vbB, *const xo = inA ? xbA : xbB;
             st3(vo, o, add3(ldv3(vo, o), vb));
             st3(xo, o, add3(ldv3(xo, o), xb));
@@ -747,6 +813,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_xsph_rev(DevParams P, uint32_t nA,
 // both sets (fixed quirks).  Tb = adjoint of T1 in, T0b = adjoint of T out; rho-bar and
 // position adjoints added; conductivity gradients accumulated.
 __device__ __forceinline__ float kh(float ki, float kj) { return ((4.f * ki) * kj) / (ki + kj); }
+template <bool WARP>
 __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw, uint32_t ns, SetView vw, SetView vs,
                                                    Sets X, const float* __restrict__ Tw, const float* __restrict__ Ts,
                                                    const float* __restrict__ Tbw, const float* __restrict__ Tbs,
@@ -755,17 +822,16 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw,
                                                        float dt)
 {
     wait_prior();
-    __shared__ AdjBuf bufs[ADJ_TPB / 32];
-    AdjBuf& W = bufs[threadIdx.x >> 5];
+    __shared__ AdjBuf bufs[WARP ? ADJ_TPB / 32 : 1];
+    AdjBuf& W = bufs[WARP ? threadIdx.x >> 5 : 0];
     vw.n = nw; vs.n = ns;
-    const uint32_t lane = threadIdx.x & 31u;
-    WARP_LOOP(t, nw + ns) {
+    ADJ_LOOP(WARP, t, nw + ns) {
         const int set = t < nw ? 0 : 1;
         const uint32_t i = set == 0 ? t : t - nw;
         const SetView& own = set == 0 ? vw : vs;
         const uint32_t o = own.gi[i];
         const float3 p = xyz(own.p4[i]);
-        const uint32_t h = lane_cell(P, grid_pos(P, p));
+        const AdjCell<WARP> c(P, p);
         const float Ti = (set == 0 ? Tw : Ts)[o];
         const float Tbi = (set == 0 ? Tbw : Tbs)[o];
         const float ki = set == 0 ? P.k_water : P.k_snow;
@@ -774,7 +840,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw,
         const float rhoi = (set == 0 ? fw.rho : fs.rho)[o];
         const float bi = dt / (Ci * rhoi);
         // sums 0: T, 1: weights, 2: dT, 3: density, 4, 5: conductivities, 6..8: positions
-        float acc = 0.f;
+        AdjSums<WARP, 9> acc;
         for (int k = 0; k < 2; ++k) {
             const SetView& v = k == 0 ? vw : vs;
             const float kj = k == 0 ? P.k_water : P.k_snow;
@@ -788,7 +854,7 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw,
                 dkw = 4.f * P.k_snow * P.k_snow / s2;
                 dks = 4.f * P.k_water * P.k_water / s2;
             }
-            warp_neighbors<9, 1>(v, p, h, k == set ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
+            adj_neighbors<1>(P, v, p, c, k == set ? i : SNOWB_UMAX, P.h2_lt, W, acc, [&](uint32_t j, float* out) {
                 const float3 r = sub3(p, xyz(__ldg(v.p4 + j)));
                 const float d = sqrtf(dot3(r, r));
                 const uint32_t oj = v.gi[j];
@@ -814,11 +880,11 @@ __global__ void __launch_bounds__(ADJ_TPB) ka_heat_rev(DevParams P, uint32_t nw,
                 out[5] = q * dks;
             });
         }
-        const float T0b = sum_of(acc, 0) + Tbi * (1.f - bi * sum_of(acc, 1));
-        const float rb = sum_of(acc, 3) + -Tbi * (bi / rhoi) * sum_of(acc, 2);
-        const float gkw = sum_of(acc, 4), gks = sum_of(acc, 5);
-        const float3 xb = sum3_of(acc, 6);
-        if (lane == 0u) {
+        const float T0b = acc.of(0) + Tbi * (1.f - bi * acc.of(1));
+        const float rb = acc.of(3) + -Tbi * (bi / rhoi) * acc.of(2);
+        const float gkw = acc.of(4), gks = acc.of(5);
+        const float3 xb = acc.of3(6);
+        if (ADJ_LEAD(WARP)) {
             (set == 0 ? T0bw : T0bs)[o] = T0b;
             (set == 0 ? fw.rhob : fs.rhob)[o] += rb;
             const AdjSet& A = set == 0 ? aw : as;

@@ -1145,6 +1145,12 @@ static int dcopy(void* dst, const void* src, size_t bytes)
     return SNOWB_OK;
 }
 
+// a reverse pass over `n` particles in the form that suits the sets' size (ADJ_WARP_MAX)
+#define ADJ_LAUNCH(kernel, n, ...)                                                                       \
+    do {                                                                                                 \
+        if (warp) KL_AS(#kernel, kernel<true>, blocks_for(32ull * (n), ADJ_TPB), ADJ_TPB, __VA_ARGS__);   \
+        else KL_AS(#kernel, kernel<false>, blocks_for((n), ADJ_TPB), ADJ_TPB, __VA_ARGS__);               \
+    } while (0)
 // reverse of one recorded substep; gx/gv/gT (per set) hold the adjoint of the state after
 // it on entry and the adjoint of the state before it on return
 static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2], float* const gT[2], float* gL)
@@ -1176,10 +1182,16 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         for (int s = 0; s < 3; ++s) TRY(zero(F[s].rhob, fb[s]));
         return SNOWB_OK;
     };
+    const bool warp = (uint64_t)nw + ns <= ADJ_WARP_MAX;
     // a warp per water and snow particle, one per 32 boundary particles
     const uint64_t bwork = 32ull * ((uint64_t)nw + ns + (nb + 31u) / 32u);
     auto fields = [&]() -> int {
-        LAUNCH(ka_fields, bwork, ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], B.brho0, B.bS0);
+        if (!warp)
+            KL_AS("ka_fields", ka_fields<false>, blocks_for((uint64_t)nw + ns, ADJ_TPB), ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X,
+                  F[0], F[1], F[2], B.brho0, B.bS0, 0u);
+        const uint32_t first = warp ? 0u : nw + ns;   // the one-thread form leaves the boundary
+        KL_AS("ka_fields", ka_fields<true>, blocks_for(bwork - 32ull * first, ADJ_TPB), ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X,
+              F[0], F[1], F[2], B.brho0, B.bS0, first);
         return SNOWB_OK;
     };
     // 1. fields at the last iteration's input positions (densities read by the XSPH)
@@ -1193,12 +1205,12 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
     for (int s = 0; s < 2; ++s) { TRY(zero(B.VB[s], b3[s])); TRY(zero(B.XBX[s], b3[s])); }
     TRY(dcopy(B.GVW, gv[0], b3[0]));
     if (tp.dem_visc)
-        LAUNCH(ka_xsph_rev, 32ull * (ns + nw), ADJ_TPB, P, ns, nw, vs, vw, F3(T.vf[1]), F3(T.vw1), tp.dem.mass, tp.sph.mass,
+        ADJ_LAUNCH(ka_xsph_rev, ns + nw, P, ns, nw, vs, vw, F3(T.vf[1]), F3(T.vw1), tp.dem.mass, tp.sph.mass,
                F[1].rho, F[0].rho, P.dem_visc, F3(gv[1]), F3(B.VB[1]), F3(B.GVW), F3(B.XBX[1]), F3(B.XBX[0]),
                F[1].rhob, F[0].rhob);
     else
         TRY(dcopy(B.VB[1], gv[1], b3[1]));
-    LAUNCH(ka_xsph_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, vw, vs, F3(T.vf[0]), F3(T.vf[1]), tp.sph.mass, tp.dem.mass, F[0].rho,
+    ADJ_LAUNCH(ka_xsph_rev, nw + ns, P, nw, ns, vw, vs, F3(T.vf[0]), F3(T.vf[1]), tp.sph.mass, tp.dem.mass, F[0].rho,
            F[1].rho, P.sph_visc, F3(B.GVW), F3(B.VB[0]), F3(B.VB[1]), F3(B.XBX[0]), F3(B.XBX[1]), F[0].rhob,
            F[1].rhob);
     // 3. finalize: x = x_new, v = (x_new - x0p)/dt
@@ -1214,7 +1226,7 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         if (tp.friction) {
             if (it != last) TRY(sort2(T.xmid[0][it], T.xmid[1][it]));
             LAUNCH(ka_scale3, ns, 256, ns, F3(B.U[1]), P.sor, F3(B.XB[1]));
-            LAUNCH(ka_friction_rev, 32ull * ns, ADJ_TPB, P, ns, nb, vs, vb, X, AS);
+            ADJ_LAUNCH(ka_friction_rev, ns, P, ns, nb, vs, vb, X, AS);
         }
         if (it == last && tp.friction)
             for (int s = 0; s < 2; ++s) LAUNCH(ka_axpy3, n[s], 256, n[s], F3(B.XB[s]), F3(B.XB[s]), 1.f, F3(B.XBX[s]));
@@ -1222,7 +1234,7 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         TRY(fields());
         for (int s = 0; s < 2; ++s) LAUNCH(ka_scale3, n[s], 256, n[s], F3(B.U[s]), P.sor, F3(B.XB[s]));
         LAUNCH(ka_pbf_lambar, bwork, ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW);
-        LAUNCH(ka_pos_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW, AS, B.part[0],
+        ADJ_LAUNCH(ka_pos_rev, nw + ns, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], AW, AS, B.part[0],
                1, tp.correct_dem);
         LAUNCH(ka_param_sum, nw + ns, 128, nw + ns, B.part[0], nullptr, G.g + 1, nullptr);
         if (tp.interlink)
@@ -1241,10 +1253,10 @@ static int adj_substep(const TapeStep& T, float* const gx[2], float* const gv[2]
         TRY(fields());
         AdjSet HW{F3(B.XH[0]), F3(B.U[0]), F3(B.X0B[0]), F3(T.x0p[0])};
         AdjSet HS{F3(B.XH[1]), F3(B.U[1]), F3(B.X0B[1]), F3(T.x0p[1])};
-        LAUNCH(ka_heat_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, vw, vs, X, T.T0[0], T.T0[1], gT[0], gT[1], B.T0B[0], B.T0B[1],
+        ADJ_LAUNCH(ka_heat_rev, nw + ns, P, nw, ns, vw, vs, X, T.T0[0], T.T0[1], gT[0], gT[1], B.T0B[0], B.T0B[1],
                F[0], F[1], HW, HS, B.part[0], B.part[1], tp.dt);
         LAUNCH(ka_param_sum, nw + ns, 128, nw + ns, B.part[0], B.part[1], G.g + 2, G.g + 3);
-        LAUNCH(ka_pos_rev, 32ull * (nw + ns), ADJ_TPB, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], HW, HS, B.part[0], 0,
+        ADJ_LAUNCH(ka_pos_rev, nw + ns, P, nw, ns, nb, vw, vs, vb, X, F[0], F[1], F[2], HW, HS, B.part[0], 0,
                0);
         TRY(zero_rhob());
         for (int s = 0; s < 2; ++s) TRY(dcopy(gT[s], B.T0B[s], fb[s]));
