@@ -186,22 +186,31 @@ __global__ void k_block_sums(const uint32_t* __restrict__ cnt, uint32_t ncells, 
     }
 }
 
-// off[c] = exclusive prefix of cnt (c <= ncells), cnt re-zeroed, for the scan chunk `chunk` whose
-// particles come after `prefix` others; cells from `clear` on keep their cell_start (null: none
-// is cleared)
+// off[c] = exclusive prefix of cnt (c <= ncells), cnt re-zeroed, for the scan chunk `chunk`; bsum:
+// the counts of the chunks, of which the block's threads sum those before it side by side, in the
+// same steps as the scan; cells from `clear` on keep their cell_start (null: none is cleared)
+struct ScanShared {
+    uint32_t scan[SCAN_TPB / 32 + 1], before[SCAN_TPB / 32];
+};
 __device__ __forceinline__ void scan_chunk(uint32_t* __restrict__ cnt, uint32_t ncells, uint32_t* __restrict__ off,
                                            uint32_t* __restrict__ cell_start, uint32_t clear, uint32_t chunk,
-                                           uint32_t prefix, uint32_t* sm)
+                                           const uint32_t* bsum, ScanShared& sm)
 {
     const uint32_t base = chunk * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
+    uint32_t before = 0;
+    for (uint32_t c = threadIdx.x; c < chunk; c += SCAN_TPB) before += bsum[c];
     uint32_t v[SCAN_ITEMS], t = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         v[k] = base + k < ncells ? cnt[base + k] : 0u;
         t += v[k];
     }
+    before = warp_sum(before);
+    if ((threadIdx.x & 31) == 0) sm.before[threadIdx.x >> 5] = before;
     uint32_t total;
-    uint32_t ex = block_excl_scan(t, sm, total) + prefix;
+    uint32_t ex = block_excl_scan(t, sm.scan, total);   // its barriers cover sm.before too
+#pragma unroll
+    for (int w = 0; w < SCAN_TPB / 32; ++w) ex += sm.before[w];
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         const uint32_t c = base + k;
@@ -220,14 +229,8 @@ __global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restri
                             uint32_t* __restrict__ off)
 {
     wait_prior();
-    __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
-    __shared__ uint32_t s_prefix;
-    if (threadIdx.x < 32) {
-        const uint32_t p = prefix_of_blocks(bsum, blockIdx.x);
-        if (threadIdx.x == 0) s_prefix = p;
-    }
-    __syncthreads();
-    scan_chunk(cnt, ncells, off, nullptr, 0u, blockIdx.x, s_prefix, sm);
+    __shared__ ScanShared sm;
+    scan_chunk(cnt, ncells, off, nullptr, 0u, blockIdx.x, bsum, sm);
 }
 // A block takes a scan chunk of a set.  A chunk without particles only has its part of
 // cell_start cleared, if entries may be left there (dirty); its offsets are not written, and no
@@ -237,7 +240,7 @@ __global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restri
 __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ SortPair Q, uint32_t chunks)
 {
     wait_prior();
-    __shared__ uint32_t sm[SCAN_TPB / 32 + 1];
+    __shared__ ScanShared sm;
     const int k = blockIdx.x < chunks ? 0 : 1;
     const uint32_t chunk = blockIdx.x - (k ? chunks : 0u);
     const SortSide& A = Q.a[k];
@@ -253,11 +256,8 @@ __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ 
         if (threadIdx.x == 0) A.dirty[chunk] = dirty && end > clear ? 1u : 0u;
         return;
     }
-    uint32_t before = 0, prefix;
-    for (uint32_t c = threadIdx.x; c < chunk; c += SCAN_TPB) before += A.bsum[c];
-    block_excl_scan(before, sm, prefix);
     if (threadIdx.x == 0) A.dirty[chunk] = 1u;
-    scan_chunk(A.cnt, Q.ncells, A.off, A.cd.cell_start, clear, chunk, prefix, sm);
+    scan_chunk(A.cnt, Q.ncells, A.off, A.cd.cell_start, clear, chunk, A.bsum, sm);
 }
 
 // ------------------------------------------------------------------ 3. scatter
