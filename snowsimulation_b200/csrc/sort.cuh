@@ -235,7 +235,7 @@ __global__ void k_cell_scan(uint32_t* __restrict__ cnt, const uint32_t* __restri
 // A block takes a scan chunk of a set.  A chunk without particles only has its part of
 // cell_start cleared, if entries may be left there (dirty); its offsets are not written, and no
 // pass reads them: most chunks of a batch's wide grid, or above a scene, are empty (32 scenes,
-// 8,192 chunks, where every block also summed all earlier chunks: 79 us a set, 26 us both).
+// 8,192 chunks, where every block also summed all earlier chunks: 79 us a set, 27 us both).
 // cell_start is cleared for c < clear (min(n, ncells) reproduces the reference's partial memset, Q1).
 __global__ void __launch_bounds__(SCAN_TPB) k_sort_scan(const __grid_constant__ SortPair Q, uint32_t chunks)
 {

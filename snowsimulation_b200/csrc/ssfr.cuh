@@ -297,7 +297,8 @@ __global__ void ks_fill(uint32_t npix, uint32_t* __restrict__ depth_bits, uint32
 //     filter pass | the snow's sphere depth, only where the water has a depth inside 0..1:
 //     the composite compares it nowhere else (a filtered depth is 0 or 1 wherever the
 //     unfiltered one is).
-// The README-scale view at 1600 x 900 (148k snow, 6k water): 172 -> 88 us for the call.
+// The README-scale view at 1600 x 900 (148k snow, 6k water): 172 -> 88 us for the call, 75 since
+// launches overlap the end of the one before (launch_prior).
 __global__ void ks_view_clear(uint32_t npix, unsigned long long* __restrict__ zbuf,
                               unsigned long long* __restrict__ thick, uint32_t* __restrict__ scene_depth,
                               uint32_t* __restrict__ fluid_depth)
